@@ -137,9 +137,13 @@ def _states(g, channels, B: int, S: int, layout: str = 'bhsd') -> torch.Tensor:
     return x.mul_(sigma[:, None]).add_(offset[:, None]).to(torch.bfloat16)
 
 
+def _exponent_counts(x: torch.Tensor) -> torch.Tensor:
+    return torch.bincount(((x.reshape(-1).view(torch.int16).int() >> 7) & 0xFF), minlength=256).cpu()
+
+
 def _calibrated(g, channels, nbits: int = 0):
     """(right, nbits) for these channels from a draw of their own; ``nbits`` 0: the adjuster's choice."""
-    hist = codec.exponent_hist(_states(g, channels, 1, 256)).cpu()
+    hist = _exponent_counts(_states(g, channels, 1, 256))
     if nbits == 0:
         return codec.analysis_best_bits(hist)
     cover = torch.nn.functional.avg_pool1d(hist.double()[None], 2 ** nbits - 1, stride=1)[0]
@@ -167,7 +171,7 @@ def prepare(case: dict, seed: int) -> dict:
     if kind in ('unflat', 'flat'):
         w = torch.randn(case['rows'], case['cols'], generator=g, device='cuda')
         w = w.mul_(0.02 * torch.exp(0.3 * torch.randn(case['rows'], 1, generator=g, device='cuda'))).to(torch.bfloat16)
-        hist = codec.exponent_hist(w.view(1, 1, -1, 8)).cpu().double()
+        hist = _exponent_counts(w).double()
         n = case['nbits']
         right = int(torch.nn.functional.avg_pool1d(hist[None], 2 ** n - 1, stride=1)[0].argmax()) + 2 ** n - 2
         w = _to_share(g, w, (right, n), 'w')
@@ -180,16 +184,11 @@ def prepare(case: dict, seed: int) -> dict:
         return st
     if kind == 'session':
         return _prepare_session(st, g)
-    B, H, S, D = case['B'], case['H'], case['S'], case['D']
-    spread = 0.5 if kind == 'attend' else 1.0
-    ck, cv = _channels(g, H, D, True, s=spread), _channels(g, H, D, False, s=spread)
-    layout = case.get('layout', 'bhsd')
-    k, v = _states(g, ck, B, S, layout), _states(g, cv, B, S, layout)
+    S = case['S']
+    k, v, pk, pv = _keys_values(case, g)
     if kind == 'adjust':
         st.update(k=k, v=v)
         return st
-    pk, pv = _calibrated(g, ck, case['nbits']), _calibrated(g, cv, case['nbits'])
-    k, v = _to_share(g, k, pk, 'k'), _to_share(g, v, pv, 'v')
     if kind == 'pack':
         st.update(k=k, v=v, pk=pk, pv=pv)
     elif kind == 'layer':
@@ -203,8 +202,25 @@ def prepare(case: dict, seed: int) -> dict:
         st['ks'], st['vs'] = kc.segments(), vc.segments()
         st['kt'], st['vt'] = k[:, :, full:].contiguous(), v[:, :, full:].contiguous()
         st['ktab'], st['vtab'] = codec.build_segment_table(st['ks']), codec.build_segment_table(st['vs'])
-        st['q'] = (0.5 * torch.randn(B, H * case['G'], D, generator=g, device='cuda')).to(torch.bfloat16)
+        st['q'] = _query(case, g)
     return st
+
+
+def _keys_values(case: dict, g):
+    """Keys, values and their windows (none for the adjuster, which is to find them)."""
+    kind, B, H, S, D = (case[x] for x in ('kind', 'B', 'H', 'S', 'D'))
+    spread = 0.5 if kind == 'attend' else 1.0
+    ck, cv = _channels(g, H, D, True, s=spread), _channels(g, H, D, False, s=spread)
+    layout = case.get('layout', 'bhsd')
+    k, v = _states(g, ck, B, S, layout), _states(g, cv, B, S, layout)
+    if kind == 'adjust':
+        return k, v, None, None
+    pk, pv = _calibrated(g, ck, case['nbits']), _calibrated(g, cv, case['nbits'])
+    return _to_share(g, k, pk, 'k'), _to_share(g, v, pv, 'v'), pk, pv
+
+
+def _query(case: dict, g) -> torch.Tensor:
+    return (0.5 * torch.randn(case['B'], case['H'] * case['G'], case['D'], generator=g, device='cuda')).to(torch.bfloat16)
 
 
 def _prepare_session(st: dict, g) -> dict:
@@ -307,6 +323,31 @@ def work(case: dict) -> dict:
     if kind == 'attend':
         return {'bytes': 2 * _packed_bytes(n, case['nbits']) + 4 * B * H * case['G'] * D, 'flops': 4 * n * case['G']}
     return {'bytes': 2 * (2 * n + _packed_bytes(n, case['nbits'])), 'flops': 0}
+
+
+def _attention64(q, k, v) -> torch.Tensor:
+    """softmax(q K^T / sqrt(D)) V of one query token per sequence in 64 bits, one sequence and key head at a time."""
+    B, H, S, D = k.shape
+    q = q.reshape(B, H, -1, D)
+    out = torch.empty(q.shape, dtype=torch.float64, device=q.device)
+    for b in range(B):
+        for h in range(H):
+            p = torch.softmax(q[b, h].double() @ k[b, h].double().T / math.sqrt(D), dim=-1)
+            out[b, h] = p @ v[b, h].double()
+    return out
+
+
+def exact(case: dict, seed: int):
+    """What ``run`` returns where that is computed numbers, i.e. attention; everything else is bytes and whole numbers."""
+    g = torch.Generator('cuda').manual_seed(int(seed))
+    if case['kind'] == 'attend':
+        k, v, *_ = _keys_values(case, g)
+        q = _query(case, g)
+        return _attention64(q, k, v).view(q.shape)
+    if case['kind'] == 'session' and case['route'] == 'fused':
+        st = _prepare_session({'case': case}, g)
+        return [[_attention64(st['q'], k, v).view(st['q'].shape) for k, v in zip(st['k'], st['v'])], None, None, None, None]
+    return None
 
 
 def tolerance(case: dict):

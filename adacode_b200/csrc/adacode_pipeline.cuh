@@ -33,7 +33,7 @@ struct PipeGeom {
     static constexpr int kThreads = kConsumers + 32;        // + the producer warp
     static constexpr int kUnit = kConsumers * kPCPT * 16;   // elements per unit
     static constexpr int kCtasPerSm = CTAS;
-    static constexpr int kEscStage = kUnit / 2;             // bytes of a tile's escape stream staged with a unit
+    static constexpr int kEscStage = 8192;                  // bytes of a tile's escape stream staged with a unit
 };
 using WideGeom = PipeGeom<16, 2>;
 using NarrowGeom = PipeGeom<8, 4>;
@@ -193,15 +193,14 @@ template <class G>
 struct alignas(128) UnpackStageT {
     alignas(128) uint8_t sm[G::kUnit];
     alignas(128) uint8_t codes[G::kUnit / 2];
-    alignas(128) uint8_t esc[G::kEscStage + 16];
+    // (a granule of slack in front, one behind, and the words that place_escapes reads ahead)
+    alignas(128) uint8_t esc[G::kEscStage + 48];
     alignas(16) UnitMeta meta;
 };
 
 template <class G>
 struct alignas(128) UnpackSmemT {
     UnpackStageT<G> stage[kStages];
-    alignas(128) uint16_t out[G::kUnit];
-    alignas(16) uint32_t lut[1024];   // decode table of the current (left, nbits)
     // Unit descriptions live in a ring of their own, twice as deep as the stages: a consumer reads
     // the destination of unit i after it has released stage i % kStages, and the producer writes
     // the description of unit i + 2 * kStages only after every consumer has released unit
@@ -210,7 +209,9 @@ struct alignas(128) UnpackSmemT {
     alignas(16) UnitMeta meta_ring[2 * kStages];
     alignas(8) uint64_t full[kStages];
     alignas(8) uint64_t empty[kStages];
-    int warp_tot[G::kWarps];
+    // escapes per consumer warp of a unit, by the unit's parity: a warp writes those of unit i + 2 only
+    // behind the barrier of unit i + 1, which no warp reaches before it has read those of unit i
+    int warp_tot[2][G::kWarps];
 };
 using UnpackStage = UnpackStageT<WideGeom>;
 static_assert(sizeof(UnpackStageT<WideGeom>) % 128 == 0 && sizeof(UnpackStageT<NarrowGeom>) % 128 == 0,
@@ -411,108 +412,117 @@ __device__ __forceinline__ void decode_chunks(const Stage &st, const uint32_t *l
     }
 }
 
+// A 16-element chunk of a destination row.  32 bytes leave in one instruction where they are aligned
+// (a warp then writes 1 KB of whole sectors at once), in two otherwise.
+__device__ __forceinline__ void store_chunk(uint16_t *dst, const uint32_t (&w)[8], bool wide) {
+    if (wide) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(w[0]), "r"(w[1]),
+                     "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                     : "memory");
+    } else {
+        reinterpret_cast<uint4 *>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        reinterpret_cast<uint4 *>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+}
+
+// Escapes of one group whose bytes are not (all) staged in shared memory: byte by byte, from global
+// memory beyond the window; a stream that is too short is flagged and gives exponent 0.  Returns the
+// bytes in their places (elements 0..3, 4..7).
+__device__ __forceinline__ uint2 gather_escapes(uint32_t z, int r, const uint8_t *esc_smem, int staged, const UnitMeta &m,
+                                                int32_t *status) {
+    const uint8_t *g_esc = m.esc;
+    const long long g_len = m.esc_len, g_start = m.esc_tile_start;
+    uint2 e = make_uint2(0u, 0u);
+#pragma unroll 1
+    for (; z != 0; z &= z - 1, ++r) {
+        const int k = (__ffs((int)z) - 1) >> 2;
+        uint32_t v = 0;
+        if (r < staged) v = esc_smem[r];
+        else if (g_start + r < g_len) v = g_esc[g_start + r];
+        else atomicOr(status, ADACODE_STATUS_ESCAPE_UNDERRUN);
+        const uint32_t at = v << (8 * (k & 3));
+        if (k < 4) e.x |= at;
+        else e.y |= at;
+    }
+    return e;
+}
+
+// One unit: staged planes -> registers -> global memory.  The codes are expanded, the escapes placed
+// and the bf16 words put together in registers (about 6 instructions per element, see spread8), and
+// whole sectors are stored straight from there.  The only CTA-wide barrier is the one between the
+// escape counts of the warps and their sum.  Bound by DRAM: the time hardly depends on the code length
+// or the share of escapes any more.  Keys and values of [16, 8, 8192, 128] (537 M elements moved):
+// n = 3, 5 % escapes 189 -> 183 us, n = 2, 34 % escapes 341 -> 179 us, n = 4 169 -> 183 us (76-81 % of
+// 6.65 TB/s).  The finished unit through shared memory and a bulk store instead: 229 us; three
+// stages 191 us, five CTAs per SM 223 us.
 template <int N, class G>
 __device__ __forceinline__ void unpack_unit(UnpackSmemT<G> &s, const UnpackStageT<G> &st, const UnitMeta &meta,
-                                            uint64_t *empty_bar, int &consumed, int D, int32_t *status, bool broken) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // only what the common path needs is read from the unit's description up front; the fields of
-    // the rare global-memory escape path and the destination are read where they are used
-    const int esc_staged = meta.esc_staged, esc_shift = meta.esc_shift;
+                                            uint64_t *empty_bar, int *warp_tot, int &consumed, const ExpTable &tab,
+                                            const int (&row)[kPCPT], const int (&col)[kPCPT], int32_t *status,
+                                            bool broken) {
+    constexpr int CB = 2 * N;   // code bytes per 16-element chunk
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (meta.first_unit_of_tile) consumed = 0;
     const int chunks = meta.elems >> 4;
-
-    uint4 o[kPCPT][2];
-    uint32_t zm[kPCPT][2];
-    int zc[kPCPT];
-    decode_chunks<N>(st, s.lut, chunks, o, zm, zc);
-    int incl[kPCPT];
-    const int wtot = warp_scan_counts(zc, incl);
-    if (lane == 0) s.warp_tot[warp] = wtot;
-    bulk_wait_read();          // the previous unit's store has finished reading s.out
-    consumer_sync<G::kConsumers>();
-    int wprefix, unit_tot;
-    cross_warp_prefix<G::kWarps>(s.warp_tot, wprefix, unit_tot);
-    static_assert(kPCPT == 2, "the escape loop below walks the two chunks of a thread together");
     const int c0 = warp * (kPCPT * 32) + lane;
+
+    uint32_t nib[kPCPT][2], z[kPCPT][2];
+    int zc[kPCPT];
 #pragma unroll
     for (int k = 0; k < kPCPT; ++k) {
         const int c = c0 + k * 32;
-        if (c < chunks) {
-            uint16_t *ow = s.out + c * 16;
-            reinterpret_cast<uint4 *>(ow)[0] = o[k][0];
-            reinterpret_cast<uint4 *>(ow)[1] = o[k][1];
+        uint32_t x[2] = {0u, 0u};
+        const bool valid = c < chunks;
+        if (valid) load_codes16<N>(st.codes + c * CB, x);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            nib[k][q] = spread8<N>(x[q]);
+            z[k][q] = valid ? escape_mask<N>(nib[k][q]) : 0u;
         }
+        zc[k] = escapes_of(z[k][0]) + escapes_of(z[k][1]);
     }
-    if (zc[0] + zc[1] != 0) {
-        // ranks inside the tile of the first escape of either chunk
-        const int r0 = consumed + wprefix + incl[0] - zc[0], r1 = consumed + wprefix + incl[1] - zc[1];
-        const bool staged = (zc[0] == 0 || r0 + zc[0] <= esc_staged) && (zc[1] == 0 || r1 + zc[1] <= esc_staged);
-        if (staged) {
-            // One loop over the escapes of both chunks (four groups): a warp iterates as often as its
-            // busiest lane has escapes, and per-lane totals over 32 elements vary much less than
-            // per-group counts over 8, so this takes about half the iterations of four separate loops.
-            // mask: chunk 0 elements 0..15, then chunk 1 elements 0..15, from the most significant bit.
-            uint32_t todo = (compress_slots<N>(zm[0][0]) << 24) | (compress_slots<N>(zm[0][1]) << 16) |
-                            (compress_slots<N>(zm[1][0]) << 8) | compress_slots<N>(zm[1][1]);
-            // The exponent field in s.out is zero at escaped positions (code 0 decodes to 0), so the
-            // escape byte is OR-ed in with a shared-memory reduction: no read-modify-write round trip.
-            const uint8_t *ep = st.esc + esc_shift + r0;
-            const int skip = r1 - r0 - zc[0];             // from chunk 0's escapes to chunk 1's
-            uint32_t *ow32 = reinterpret_cast<uint32_t *>(s.out + c0 * 16);
-            int n = 0;
-            while (todo) {
-                const int i = __clz(todo);
-                todo &= ~(0x80000000u >> i);
-                const uint32_t e = ep[n + (i >> 4) * skip];
-                ++n;
-                // chunk 1 lies 32 chunks = 256 words further on; (i >> 1) & 7 is the word inside the chunk
-                atomicOr(ow32 + (((i >> 4) << 8) | ((i >> 1) & 7)), e << (7 + 16 * (i & 1)));
-            }
+    int incl[kPCPT];
+    const int wtot = warp_scan_counts(zc, incl);
+    if (lane == 0) warp_tot[warp] = wtot;
+    consumer_sync<G::kConsumers>();
+    int wprefix, unit_tot;
+    cross_warp_prefix<G::kWarps>(warp_tot, wprefix, unit_tot);
+    const int staged = meta.esc_staged, shift = meta.esc_shift;
+    uint16_t *const dst = meta.dst;
+    const long long ds = meta.ds;
+    const bool wide = ((((uintptr_t)dst) | ((uintptr_t)ds * 2)) & 31) == 0;
+    const uint32_t *words = reinterpret_cast<const uint32_t *>(st.esc);
+    const auto word = [words](uint32_t i) { return words[i]; };
+#pragma unroll
+    for (int k = 0; k < kPCPT; ++k) {
+        const int r0 = consumed + wprefix + incl[k] - zc[k];     // rank inside the tile of the chunk's first escape
+        const int r1 = r0 + escapes_of(z[k][0]);
+        uint32_t e0[2], e1[2];
+        lookup8<N>(nib[k][0], tab, e0);
+        lookup8<N>(nib[k][1], tab, e1);
+        if (r0 + zc[k] <= staged || zc[k] == 0) {
+            // (a chunk without escapes may rank beyond the window: it reads the window's first words)
+            place_escapes(z[k][0], (uint32_t)(shift + (zc[k] ? r0 : 0)), word, e0);
+            place_escapes(z[k][1], (uint32_t)(shift + (zc[k] ? r1 : 0)), word, e1);
         } else {
-            // beyond the staged window (or beyond the stream): fetch from global memory
-            const uint8_t *g_esc = meta.esc;
-            const long long g_len = meta.esc_len, g_start = meta.esc_tile_start;
-#pragma unroll 1
-            for (int k = 0; k < kPCPT; ++k) {
-                uint16_t *ow = s.out + (c0 + k * 32) * 16;
-                int r = k == 0 ? r0 : r1;
-#pragma unroll 1
-                for (int q = 0; q < 2; ++q) {
-                    // (selects, not zm[k][q]: a run-time index would move the array to local memory)
-                    uint32_t z = k == 0 ? (q == 0 ? zm[0][0] : zm[0][1]) : (q == 0 ? zm[1][0] : zm[1][1]);
-                    while (z) {
-                        const int pos = 31 - __clz(z);
-                        z ^= 1u << pos;
-                        uint32_t e = 0;
-                        if (r < esc_staged) e = st.esc[esc_shift + r];
-                        else if (g_start + r < g_len) e = g_esc[g_start + r];
-                        else atomicOr(status, ADACODE_STATUS_ESCAPE_UNDERRUN);
-                        ++r;
-                        uint16_t *pw = ow + (q * 8 + 7 - pos / N);
-                        *pw = (uint16_t)((*pw & 0x807Fu) | (e << 7));
-                    }
-                }
-            }
+            const uint2 g0 = gather_escapes(z[k][0], r0, st.esc + shift, staged, meta, status);
+            e0[0] |= g0.x, e0[1] |= g0.y;
+            const uint2 g1 = gather_escapes(z[k][1], r1, st.esc + shift, staged, meta, status);
+            e1[0] |= g1.x, e1[1] |= g1.y;
         }
+        uint4 sv = make_uint4(0, 0, 0, 0);
+        const bool valid = c0 + k * 32 < chunks;
+        if (valid) sv = *reinterpret_cast<const uint4 *>(st.sm + (c0 + k * 32) * 16);
+        uint32_t w[8];
+        assemble4(sv.x, e0[0], w[0], w[1]);
+        assemble4(sv.y, e0[1], w[2], w[3]);
+        assemble4(sv.z, e1[0], w[4], w[5]);
+        assemble4(sv.w, e1[1], w[6], w[7]);
+        if (valid && !broken) store_chunk(dst + (long long)row[k] * ds + col[k], w, wide);
     }
     consumed += unit_tot;
-    mbar_arrive(empty_bar);    // this thread no longer reads the stage
-    fence_async_smem();
-    consumer_sync<G::kConsumers>();
-    const long long ds = meta.ds;
-    if (broken) {
-        // (nothing is stored)
-    } else if (ds == D) {
-        if (tid == 0 && meta.elems > 0) {
-            bulk_store(meta.dst, s.out, (uint32_t)meta.elems * 2u);
-            bulk_commit();
-        }
-    } else {
-        const int rows = meta.elems / D;
-        uint16_t *const dst = meta.dst;
-        for (int r = tid; r < rows; r += G::kConsumers) bulk_store(dst + (long long)r * ds, s.out + r * D, (uint32_t)D * 2u);
-        bulk_commit();
-    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty_bar);    // this warp no longer reads the stage
 }
 
 // Consumer warp: wait (bounded) until unit `it` is loaded; false if the wait gave up.
@@ -525,14 +535,17 @@ __device__ __forceinline__ bool wait_loaded(UnpackSmemT<G> &s, uint32_t it, int3
     return loaded;
 }
 
-// Units it, it + 1, ... as long as they carry code length N and window `left` (the decode table
-// in s.lut); returns the first unit that does not, already waited for, or n_units.
+// Units it, it + 1, ... as long as they carry code length N and window `left`; returns the first unit
+// that does not, already waited for, or n_units.
 template <int N, class G>
 __device__ __forceinline__ uint32_t unpack_run(UnpackSmemT<G> &s, uint32_t it, uint32_t n_units, int left, int &consumed,
-                                               bool &broken, int D, int32_t *status, uint32_t poll_limit) {
+                                               const int (&row)[kPCPT], const int (&col)[kPCPT], bool &broken,
+                                               int32_t *status, uint32_t poll_limit) {
+    const ExpTable tab = exp_table<N>(left);
     for (;;) {
         const int stg = it % kStages;
-        unpack_unit<N>(s, s.stage[stg], s.meta_ring[it % (2 * kStages)], &s.empty[stg], consumed, D, status, broken);
+        unpack_unit<N>(s, s.stage[stg], s.meta_ring[it % (2 * kStages)], &s.empty[stg], s.warp_tot[it & 1], consumed, tab,
+                       row, col, status, broken);
         if (++it >= n_units) return it;
         broken |= !wait_loaded(s, it, status, poll_limit);
         const UnitMeta &next = s.meta_ring[it % (2 * kStages)];
@@ -562,7 +575,7 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_unpack_pipe(cons
 #pragma unroll
         for (int i = 0; i < kStages; ++i) {
             mbar_init(&s.full[i], 1);
-            mbar_init(&s.empty[i], G::kConsumers);
+            mbar_init(&s.empty[i], G::kWarps);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -623,7 +636,14 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_unpack_pipe(cons
     // ---------------- consumer warps ----------------
     int consumed = 0;
     bool broken = false;                  // a wait of this warp ran out: compute on, store nothing
-    int lut_left = 0, lut_nbits = 0;      // what s.lut currently encodes (nbits 0: nothing yet)
+    // row and column of this thread's chunks inside a unit (a chunk never crosses a row: D % 16 == 0)
+    int row[kPCPT], col[kPCPT];
+#pragma unroll
+    for (int k = 0; k < kPCPT; ++k) {
+        const int e0 = ((tid >> 5) * (kPCPT * 32) + k * 32 + (tid & 31)) * 16;
+        row[k] = e0 / a0.D;
+        col[k] = e0 - row[k] * a0.D;
+    }
     // (the consumers only count units: which tile a unit belongs to is in its description)
     const uint32_t my_units =
         n_tiles > (long long)blockIdx.x
@@ -631,27 +651,19 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_unpack_pipe(cons
             : 0u;
     // Units of one code length and window are handled by a loop of their own (unpack_run<N>), so
     // that the compiler schedules each code length's loop body by itself; this outer loop only
-    // takes over when the table has to change.
+    // takes over when the code length or the window changes.
     uint32_t it = 0;
     while (it < my_units) {
         broken |= !wait_loaded(s, it, a0.status, ja.poll_limit);      // returns at once if unpack_run waited already
         const UnitMeta &meta = s.meta_ring[it % (2 * kStages)];
-        const int nb = meta.nbits, lf = meta.left;
-        if (nb != lut_nbits || lf != lut_left) {
-            // uniform over the CTA: every consumer read the same description.  The previous unit
-            // ended with a consumer barrier, so nobody still reads the old table.
-            build_decode_lut(s.lut, nb, lf, G::kConsumers);
-            lut_nbits = nb, lut_left = lf;
-            consumer_sync<G::kConsumers>();
-        }
-        switch (nb) {
-            case 1: it = unpack_run<1>(s, it, my_units, lf, consumed, broken, a0.D, a0.status, ja.poll_limit); break;
-            case 2: it = unpack_run<2>(s, it, my_units, lf, consumed, broken, a0.D, a0.status, ja.poll_limit); break;
-            case 3: it = unpack_run<3>(s, it, my_units, lf, consumed, broken, a0.D, a0.status, ja.poll_limit); break;
-            default: it = unpack_run<4>(s, it, my_units, lf, consumed, broken, a0.D, a0.status, ja.poll_limit); break;
+        const int lf = meta.left;
+        switch (meta.nbits) {
+            case 1: it = unpack_run<1>(s, it, my_units, lf, consumed, row, col, broken, a0.status, ja.poll_limit); break;
+            case 2: it = unpack_run<2>(s, it, my_units, lf, consumed, row, col, broken, a0.status, ja.poll_limit); break;
+            case 3: it = unpack_run<3>(s, it, my_units, lf, consumed, row, col, broken, a0.status, ja.poll_limit); break;
+            default: it = unpack_run<4>(s, it, my_units, lf, consumed, row, col, broken, a0.status, ja.poll_limit); break;
         }
     }
-    bulk_wait_all();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 

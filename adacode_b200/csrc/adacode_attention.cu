@@ -5,7 +5,8 @@
 // the G query heads that share a KV head, online softmax in fp32, weighted sum of the decoded V
 // tile.  The cache is split along the sequence (flash-decoding): grid = (splits, B * Hkv), each
 // CTA owns a run of 128-token tiles of one (batch, kv head) and leaves (max, sum, numerator)
-// partials that a second kernel combines.
+// partials that a second kernel combines.  The plain kernel comes first; the pipelined tensor-core
+// one, which every call takes unless ADACODE_ATTN_SIMPLE=1 is set, follows below.
 //
 // The reference has no such kernel (its attention path materialises dense K/V first; the module
 // its validation script imports, ops/kv_attention.py, is absent from its tree), so numerics are
@@ -16,6 +17,8 @@
 #include "adacode.h"
 
 #include <stdlib.h>
+
+#include <atomic>
 
 namespace {
 
@@ -318,59 +321,59 @@ __global__ void k_decode_attn_combine(const float *__restrict__ part_o, const fl
 }
 
 // =======================================================================================
-// Pipelined variant for head_dim 128: the unpack pipeline (producer warp, bulk copies into a
-// two-stage ring, 16 consumer warps decoding out of shared memory) feeding tensor-core products.
-// A decoded tile lives in shared memory as 128 rows (tokens) of 256 bytes whose 16-byte pieces are
-// XOR-swizzled with the row index, so that ldmatrix reads it with few bank conflicts both as
-// K (token-major, for scores) and, transposed, as V (for the weighted sum).
-//   scores  S[t][g]   = sum_d K[t][d] q[g][d]   : mma.m16n8k16, A = K rows, B = q (8 query heads)
-//   output  O^T[d][g] = sum_t V[t][d] P[t][g]   : mma.m16n8k16, A = V^T (ldmatrix.trans), B = P
-// Warps 0..7 own 16 tokens (scores) resp. 16 output columns (weighted sum) each.
+// Pipelined tensor-core variant: bulk copies into a ring of units (one unit = one tile, as in the
+// unpack pipeline) feeding mma.sync straight from registers.  A tile of 128 tokens is split over the
+// eight warps, sixteen tokens each, and what a thread decodes is what the
+// tensor core wants from that thread, so a decoded tile never goes through shared memory:
+//   scores  S^T[g][t] = sum_d q[g][d] K[t][d]  : A = q, B = K^T.  Thread (i, j) = (lane / 4, lane % 4)
+//           owns D / 4 consecutive elements of token i; the order of the contraction over d is free,
+//           so k-step s takes elements 4 s .. 4 s + 3 of the four threads of a token.
+//   output  O^T[d][g] = sum_t V[t][d] P[t][g]  : A = V^T, B = P^T.  The scores' accumulators are the B
+//           operand as they are.  Thread (i, j) owns columns i D / 8 .. of tokens 4 j .. 4 j + 3 and
+//           pairs up tokens with byte permutes.
+// The online softmax is each warp's own (running maximum, sum and numerator over its sixteen-token
+// slabs); the warps meet once per unit, for the escape counts before each one's first element, and
+// once at the end, to merge.  Behind a unit's barrier the unit before it has been read by everyone, so
+// its stage is refilled after that, by one warp in turn: no producer warp (whose registers the others can
+// use) and no barrier for free stages.
+// Keys and values of [16, 8, 8192, 128], 3 bits, 5 % escapes: 4 query heads per KV head 301 -> 215 us, 16
+// 588 -> 251 us; [16, 4, 8192, 64] (the plain kernel before) 221 -> 78 and 423 -> 90 us.  The floor is the packed
+// bytes, 58 us; what bounds it is the integer pipe (47 % busy) and, with sixteen warps per SM, instruction
+// latency and fetches.  The version before put every decoded tile into shared memory, let half of its warps
+// multiply and met four times per tile.
 // =======================================================================================
 
-constexpr int kAD = 128;                 // head_dim of this variant
-constexpr int kQPad = kAD + 8;           // padded rows of the small operand matrices (272 bytes)
+constexpr int kAWarps = 8;
+constexpr int kAThreads = kAWarps * 32;
+constexpr int kAStages = 3;
 constexpr float kLog2e = 1.4426950408889634f;
 
-struct AttnPipeSmem {
-    UnpackStage stage[kStages];
-    alignas(128) uint8_t tile[kTileTokens * kAD * 2];
-    alignas(16) uint32_t lut[2][1024];            // [0] keys, [1] values
-    alignas(16) uint16_t q[kMaxGroup][kQPad];     // queries, bf16
-    alignas(16) uint16_t p[kMaxGroup][kQPad];     // probabilities of the current tile, bf16, [head][token]
-    float red_max[8][kMaxGroup];                  // per-warp partial maxima
-    float red_sum[8][kMaxGroup];                  // per-warp partial sums
-    float m[2][kMaxGroup];                        // running max (log2 domain), double-buffered by tile parity
-    float l[kMaxGroup];
-    float alpha[kMaxGroup];
-    alignas(8) uint64_t full[kStages];
-    alignas(8) uint64_t empty[kStages];
-    int warp_tot[kPWarps];
+template <int D>
+struct alignas(128) AttnStage {
+    static constexpr int kEscStage = kTileTokens * D / 2;
+    alignas(128) uint8_t sm[kTileTokens * D];
+    alignas(128) uint8_t codes[kTileTokens * D / 2];
+    alignas(128) uint8_t esc[kEscStage + kEscSlack];
 };
 
-// Byte offset of 16-byte piece `piece` of row `row` in the swizzled tile.  Only the two low bits of
-// the row enter the XOR: ldmatrix then sees two-way conflicts (eight rows, four patterns), which
-// hardly matters at sixteen ldmatrix per warp and tile, and in return rows r and r + 4 share one
-// pattern, so the second chunk of a thread (32 chunks = 4 rows further on) lies exactly 1024 bytes
-// after the first and the second piece of a chunk at its first piece's offset XOR 16.
-__device__ __forceinline__ uint32_t swz(int row, int piece) {
-    return (uint32_t)(row * 256 + ((piece ^ (row & 3)) << 4));
-}
-__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-}
-__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+template <int D>
+struct AttnPipeSmem {
+    AttnStage<D> stage[kAStages];
+    alignas(16) UnitMeta meta[kAStages];
+    alignas(16) uint16_t q[16 * (D + 8)];         // queries (sixteen heads per CTA only)
+    alignas(16) TileSrc src[32];                  // where the units of the current run of 32 lie
+    float m[kAWarps][16];                         // running max per warp and head (log2 domain)
+    float l[kAWarps][16];
+    alignas(8) uint64_t full[kAStages];
+    alignas(16) int warp_tot[2][kAWarps];         // escapes per warp of a unit, by the unit's parity
+};
+
+__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1) {
     asm volatile(
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ uint32_t f32_to_bf16_bits(float x) {
     uint32_t u = __float_as_uint(x);
@@ -378,96 +381,313 @@ __device__ __forceinline__ uint32_t f32_to_bf16_bits(float x) {
     return u >> 16;
 }
 
-// Decode one staged unit (a whole 128 x 128 tile) into the swizzled tile.  Same steps as the
-// unpack kernel's consumer: zero-slot masks, warp scan, cross-warp prefix (one barrier), table
-// decode, escapes OR-ed in.  Ends with a consumer barrier: the tile is complete on return.
-template <int N>
-__device__ __forceinline__ void decode_unit_swz(AttnPipeSmem &s, const UnpackStage &st, uint64_t *empty_bar,
-                                                const uint32_t *lut, int32_t *status) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const UnitMeta m = st.meta;
-    const int chunks = m.elems >> 4;
+// Elements from one query row to the next in shared memory (padded: the rows start in different banks).
+template <int D>
+constexpr int kQRow = D + 8;
 
-    uint4 o[kPCPT][2];
-    uint32_t zm[kPCPT][2];
-    int zc[kPCPT];
-    decode_chunks<N>(st, lut, chunks, o, zm, zc);
-    int incl[kPCPT];
-    const int wtot = warp_scan_counts(zc, incl);
-    if (lane == 0) s.warp_tot[warp] = wtot;
-    consumer_sync();           // also: every warp is done reading the previous tile
-    int wprefix, unit_tot;
-    cross_warp_prefix(s.warp_tot, wprefix, unit_tot);
-    static_assert(kPCPT == 2, "the escape loop below walks the two chunks of a thread together");
-    const int c0 = warp * (kPCPT * 32) + lane;
-    const uint32_t off0 = swz(c0 >> 3, (c0 & 7) * 2);          // chunk 0, first piece
-    uint32_t *tile32 = reinterpret_cast<uint32_t *>(s.tile);
-#pragma unroll
-    for (int k = 0; k < kPCPT; ++k) {
-        if (c0 + k * 32 < chunks) {
-            *reinterpret_cast<uint4 *>(s.tile + off0 + 1024 * k) = o[k][0];
-            *reinterpret_cast<uint4 *>(s.tile + (off0 ^ 16u) + 1024 * k) = o[k][1];
-        }
+// What a warp carries along.  HG: groups of eight query heads (1 or 2).
+template <int D, int HG>
+struct AttnState {
+    // O^T: [HG][d pair][c0: (d, head 2 j), c1: (d, head 2 j + 1), c2, c3: d + 1], d = i D / 8 + 2 pair
+    float o[HG][D / 16][4];
+    float m[HG], l[HG];                           // head i (+ 8): running max, this thread's part of the sum
+    uint32_t q[HG == 1 ? D / 8 : 1];              // one group: q[head i][j D / 4 ..], bf16 pairs
+    const uint16_t *q_smem;                       // two (too many registers): the same in shared memory, head i
+    uint32_t p[HG][2];                            // probabilities of the current slab, tokens 4 j .. 4 j + 3
+    uint32_t p2[HG][2], p3[HG][2];                // what rounding p to bf16 (once, twice) left over
+};
+
+// Bf16 terms of a probability that go through the tensor core, which has time to spare: two at head_dim
+// 128 (17 bits or more), three, all of the 24 bits, at head_dim 64 (whose kernel worked in fp32 before).
+// The denominators sum p as it is.
+template <int D>
+constexpr int kTermsP = D == 64 ? 3 : 2;
+
+// Scores += k-step `step` of the token this thread owns: its elements 4 step .. 4 step + 3.
+template <int D, int HG>
+__device__ __forceinline__ void score_words(const AttnState<D, HG> &st, int step, uint32_t w0, uint32_t w1, float (&c)[4]) {
+    if constexpr (HG == 1) {
+        mma_bf16(c, st.q[2 * step], 0u, st.q[2 * step + 1], 0u, w0, w1);
+    } else {
+        const uint2 lo = *reinterpret_cast<const uint2 *>(st.q_smem + 4 * step);
+        const uint2 hi = *reinterpret_cast<const uint2 *>(st.q_smem + 8 * kQRow<D> + 4 * step);
+        mma_bf16(c, lo.x, hi.x, lo.y, hi.y, w0, w1);
     }
-    if (zc[0] + zc[1] != 0) {
-        const int r0 = wprefix + incl[0] - zc[0], r1 = wprefix + incl[1] - zc[1];     // ranks inside the tile
-        const bool staged = (zc[0] == 0 || r0 + zc[0] <= m.esc_staged) && (zc[1] == 0 || r1 + zc[1] <= m.esc_staged);
-        const uint32_t base_w = off0 >> 2;
-        if (staged) {
-            // one loop over the escapes of both chunks, as in the unpack kernel: chunk 0 elements
-            // 0..15, then chunk 1 elements 0..15, from the most significant bit of the mask
-            uint32_t todo = (compress_slots<N>(zm[0][0]) << 24) | (compress_slots<N>(zm[0][1]) << 16) |
-                            (compress_slots<N>(zm[1][0]) << 8) | compress_slots<N>(zm[1][1]);
-            const uint8_t *ep = st.esc + m.esc_shift + r0;
-            const int skip = r1 - r0 - zc[0];
-            int n = 0;
-            while (todo) {
-                const int i = __clz(todo);
-                todo &= ~(0x80000000u >> i);
-                const uint32_t e = ep[n + (i >> 4) * skip];
-                ++n;
-                const uint32_t t = (uint32_t)i >> 1;         // bit 2: second piece; bits 0..1: word in the piece
-                atomicOr(tile32 + ((base_w ^ (t & 4u)) + (((uint32_t)i >> 4) << 8) + (t & 3u)), e << (7 + 16 * (i & 1)));
-            }
-        } else {
-            // beyond the staged window (or beyond the stream): fetch from global memory
-#pragma unroll 1
-            for (int k = 0; k < kPCPT; ++k) {
-                int r = k == 0 ? r0 : r1;
-#pragma unroll 1
-                for (int q = 0; q < 2; ++q) {
-                    uint32_t z = k == 0 ? (q == 0 ? zm[0][0] : zm[0][1]) : (q == 0 ? zm[1][0] : zm[1][1]);
-                    uint32_t *w32 = tile32 + ((base_w ^ ((uint32_t)q << 2)) + ((uint32_t)k << 8));
-                    while (z) {
-                        const int pos = 31 - __clz(z);
-                        z ^= 1u << pos;
-                        const int el = 7 - pos / N;
-                        uint32_t e = 0;
-                        if (r < m.esc_staged) e = st.esc[m.esc_shift + r];
-                        else if (m.esc_tile_start + r < m.esc_len) e = m.esc[m.esc_tile_start + r];
-                        else atomicOr(status, ADACODE_STATUS_ESCAPE_UNDERRUN);
-                        ++r;
-                        atomicOr(w32 + (el >> 1), e << (7 + 16 * (el & 1)));
-                    }
-                }
-            }
-        }
-    }
-    mbar_arrive(empty_bar);
-    consumer_sync();
 }
 
-// Dense rows [t0, t0 + 128) of `base` into the swizzled tile, zero beyond `len`.  Barrier before
-// (the previous tile is no longer read) and after (the tile is complete).
-__device__ __forceinline__ void load_dense_tile_swz(AttnPipeSmem &s, const uint16_t *base, long long ss, int t0, int len) {
-    consumer_sync();
-    for (int i = threadIdx.x; i < kTileTokens * (kAD / 2); i += kConsumerThreads) {
-        const int row = i >> 6, w = i & 63;
-        uint32_t v = 0;
-        if (t0 + row < len) v = *reinterpret_cast<const uint32_t *>(base + (long long)(t0 + row) * ss + 2 * w);
-        *reinterpret_cast<uint32_t *>(s.tile + swz(row, w >> 2) + (w & 3) * 4) = v;
+// Online softmax of one slab: c[a] holds S^T of n-tile a (heads i and i + 8, tokens 4 j + 2 a, + 1);
+// `valid`: tokens of the slab that exist (16 for a packed one).
+template <int D, int HG>
+__device__ __forceinline__ void softmax_slab(AttnState<D, HG> &st, const float (&c)[2][4], float sc2, int valid) {
+    const int j = threadIdx.x & 3;
+#pragma unroll
+    for (int h = 0; h < HG; ++h) {
+        float s[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const float v = c[t >> 1][2 * h + (t & 1)] * sc2;
+            s[t] = 4 * j + t < valid ? v : -INFINITY;
+        }
+        float mx = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
+        mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, 2));
+        const float mn = fmaxf(st.m[h], mx);
+        const float ref = mn == -INFINITY ? 0.f : mn;         // (all scores so far minus infinity: weights 0, not NaN)
+        const float alpha = exp2f(st.m[h] - ref);
+        st.m[h] = mn;
+        float sum = 0.f;
+        uint32_t b[4], b2[4], b3[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const float p = exp2f(s[t] - ref);
+            sum += p;
+            b[t] = f32_to_bf16_bits(p);
+            const float r = p - __uint_as_float(b[t] << 16);
+            b2[t] = f32_to_bf16_bits(r);
+            b3[t] = f32_to_bf16_bits(r - __uint_as_float(b2[t] << 16));
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            st.p[h][u] = b[2 * u] | (b[2 * u + 1] << 16);
+            st.p2[h][u] = b2[2 * u] | (b2[2 * u + 1] << 16);
+            if (kTermsP<D> == 3) st.p3[h][u] = b3[2 * u] | (b3[2 * u + 1] << 16);
+        }
+        st.l[h] = st.l[h] * alpha + sum;
+        // the accumulators hold heads 2 j and 2 j + 1: fetch those heads' factors
+        const float a0 = __shfl_sync(kFull, alpha, 8 * j), a1 = __shfl_sync(kFull, alpha, 8 * j + 4);
+        if (__any_sync(kFull, alpha != 1.f)) {
+#pragma unroll
+            for (int e = 0; e < D / 16; ++e) {
+                st.o[h][e][0] *= a0, st.o[h][e][1] *= a1;
+                st.o[h][e][2] *= a0, st.o[h][e][3] *= a1;
+            }
+        }
     }
-    consumer_sync();
+}
+
+// One pair of columns of the slab's V: w[m] = columns (2 e, 2 e + 1) of token 4 j + m.
+template <int D, int HG>
+__device__ __forceinline__ void accumulate_words(AttnState<D, HG> &st, int e, const uint32_t (&w)[4]) {
+    const uint32_t a0 = __byte_perm(w[0], w[1], 0x5410), a1 = __byte_perm(w[0], w[1], 0x7632);
+    const uint32_t a2 = __byte_perm(w[2], w[3], 0x5410), a3 = __byte_perm(w[2], w[3], 0x7632);
+#pragma unroll
+    for (int h = 0; h < HG; ++h) {
+        if (kTermsP<D> == 3) mma_bf16(st.o[h][e], a0, a1, a2, a3, st.p3[h][0], st.p3[h][1]);
+        mma_bf16(st.o[h][e], a0, a1, a2, a3, st.p2[h][0], st.p2[h][1]);
+        mma_bf16(st.o[h][e], a0, a1, a2, a3, st.p[h][0], st.p[h][1]);
+    }
+}
+
+// Escapes of the tile before this warp's first one: the warps' counts, through shared memory.
+__device__ __forceinline__ int escapes_before_warp(int *warp_tot, int mine) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) warp_tot[warp] = mine;
+    __syncthreads();
+    return (int)__reduce_add_sync(kFull, (unsigned)(lane < warp ? warp_tot[lane & (kAWarps - 1)] : 0));
+}
+
+// Escape bytes of one group into its exponent bytes, from the staged window or, beyond it, from global memory.
+__device__ __forceinline__ void fill_escapes(uint32_t z, int rank, bool staged, const uint8_t *esc, const UnitMeta &meta,
+                                             int32_t *status, uint32_t (&e)[2]) {
+    const int shift = meta.esc_shift;
+    if (staged) {
+        const uint32_t *words = reinterpret_cast<const uint32_t *>(esc);
+        place_escapes(z, shift + rank, [words](int i) { return words[i]; }, e);
+    } else {
+        const uint2 g = gather_escapes(z, rank, esc + shift, meta.esc_staged, meta, status);
+        e[0] |= g.x, e[1] |= g.y;
+    }
+}
+
+// Scores of a staged K tile: this warp's sixteen tokens.
+template <int N, int D, int HG>
+__device__ __forceinline__ void score_unit(AttnState<D, HG> &st, const AttnStage<D> &stage, const UnitMeta &meta, int *warp_tot,
+                                           float sc2, int32_t *status) {
+    constexpr int NG = D / 32;                    // groups of eight elements in a thread's quarter of a token
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const ExpTable tab = exp_table<N>(meta.left);
+    // n-tile a, column i is token 4 (i / 2) + 2 a + i % 2: a thread's probabilities are then those of tokens 4 j ..
+    const int tok0 = warp * 16 + 4 * (lane >> 3) + ((lane >> 2) & 1);
+    const int base = tok0 * D + (lane & 3) * (D / 4);
+    uint32_t nib[2][NG];
+    int cnt[2];
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+        const int off = base + 2 * a * D;
+        uint32_t x[NG];
+        if constexpr (NG == 4) load_codes32<N>(stage.codes + off * N / 8, x);
+        else load_codes16<N>(stage.codes + off * N / 8, x);
+        cnt[a] = 0;
+#pragma unroll
+        for (int q = 0; q < NG; ++q) {
+            nib[a][q] = spread8<N>(x[q]);
+            cnt[a] += escapes_of(escape_mask<N>(nib[a][q]));
+        }
+    }
+    // ranks: four tokens at a time, eight lanes each; tile a = 0 comes before a = 1 in every four
+    uint32_t x = (uint32_t)cnt[0] | ((uint32_t)cnt[1] << 16);
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) {
+        const uint32_t u = __shfl_up_sync(kFull, x, d, 8);
+        if ((lane & 7) >= d) x += u;
+    }
+    const uint32_t tot = __shfl_sync(kFull, x, 7, 8);
+    const int t0 = (int)(tot & 0xFFFFu), four = t0 + (int)(tot >> 16);
+    int pre = four;
+#pragma unroll
+    for (int d = 8; d < 32; d <<= 1) {
+        const int u = __shfl_up_sync(kFull, pre, d);
+        if (lane >= d) pre += u;
+    }
+    const int mine = __shfl_sync(kFull, pre, 31);
+    pre += escapes_before_warp(warp_tot, mine) - four;
+    const int rank[2] = {pre + (int)(x & 0xFFFFu) - cnt[0], pre + t0 + (int)(x >> 16) - cnt[1]};
+    // (a warp none of whose escapes lies beyond the window, i.e. nearly every one)
+    const bool staged = __all_sync(kFull, rank[1] + cnt[1] <= meta.esc_staged);
+    float c[2][4];
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+        c[a][0] = c[a][1] = c[a][2] = c[a][3] = 0.f;
+        const int off = base + 2 * a * D;
+        int r = rank[a];
+#pragma unroll
+        for (int q = 0; q < NG; q += 2) {
+            const uint4 sv = *reinterpret_cast<const uint4 *>(stage.sm + off + 8 * q);
+            const uint32_t sw[4] = {sv.x, sv.y, sv.z, sv.w};
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const uint32_t z = escape_mask<N>(nib[a][q + u]);
+                uint32_t e[2];
+                lookup8<N>(nib[a][q + u], tab, e);
+                fill_escapes(z, r, staged, stage.esc + kEscFront, meta, status, e);
+                r += escapes_of(z);
+                uint32_t w[4];
+                assemble4(sw[2 * u], e[0], w[0], w[1]);
+                assemble4(sw[2 * u + 1], e[1], w[2], w[3]);
+                score_words(st, 2 * (q + u), w[0], w[1], c[a]);
+                score_words(st, 2 * (q + u) + 1, w[2], w[3], c[a]);
+            }
+        }
+    }
+    softmax_slab(st, c, sc2, 16);
+}
+
+// Weighted sum over a staged V tile: this warp's sixteen tokens.
+template <int N, int D, int HG>
+__device__ __forceinline__ void accumulate_unit(AttnState<D, HG> &st, const AttnStage<D> &stage, const UnitMeta &meta,
+                                                int *warp_tot, int32_t *status) {
+    constexpr int NG = D / 64;                    // groups of eight elements in a thread's columns of a token
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = lane >> 2, j = lane & 3;
+    const ExpTable tab = exp_table<N>(meta.left);
+    const int base = (warp * 16 + 4 * j) * D + i * (D / 8);
+    uint32_t nib[4][NG];
+    uint32_t x = 0;                               // escapes of this thread's four pieces, a byte each (at most 16)
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        const int off = base + m * D;
+        uint32_t raw[NG];
+        if constexpr (NG == 2) load_codes16<N>(stage.codes + off * N / 8, raw);
+        else raw[0] = load_codes8<N>(stage.codes + off * N / 8);
+        uint32_t cnt = 0;
+#pragma unroll
+        for (int q = 0; q < NG; ++q) {
+            nib[m][q] = spread8<N>(raw[q]);
+            cnt += (uint32_t)escapes_of(escape_mask<N>(nib[m][q]));
+        }
+        x |= cnt << (8 * m);
+    }
+    const uint32_t own = x;
+    // ranks: token by token, the eight threads of a token one after the other (sums of at most 128)
+#pragma unroll
+    for (int d = 4; d < 32; d <<= 1) {
+        const uint32_t u = __shfl_up_sync(kFull, x, d);
+        if (lane >= d) x += u;
+    }
+    const uint32_t rows = __shfl_sync(kFull, x, 28 + j);
+    const int rt[4] = {(int)(rows & 0xFFu), (int)((rows >> 8) & 0xFFu), (int)((rows >> 16) & 0xFFu), (int)(rows >> 24)};
+    const int four = rt[0] + rt[1] + rt[2] + rt[3];
+    int pre = four;
+#pragma unroll
+    for (int d = 1; d < 4; d <<= 1) {
+        const int u = __shfl_up_sync(kFull, pre, d, 4);
+        if (j >= d) pre += u;
+    }
+    const int mine = __shfl_sync(kFull, pre, 3);
+    pre += escapes_before_warp(warp_tot, mine) - four;
+    const bool staged = __all_sync(kFull, pre + four <= meta.esc_staged);
+    int rank[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        rank[m] = pre + (int)((x >> (8 * m)) & 0xFFu) - (int)((own >> (8 * m)) & 0xFFu);
+        pre += rt[m];
+    }
+#pragma unroll
+    for (int q = 0; q < NG; ++q) {
+        uint32_t w[4][4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const uint2 sv = *reinterpret_cast<const uint2 *>(stage.sm + base + m * D + 8 * q);
+            const uint32_t z = escape_mask<N>(nib[m][q]);
+            uint32_t e[2];
+            lookup8<N>(nib[m][q], tab, e);
+            fill_escapes(z, rank[m], staged, stage.esc + kEscFront, meta, status, e);
+            rank[m] += escapes_of(z);
+            assemble4(sv.x, e[0], w[0][m], w[1][m]);
+            assemble4(sv.y, e[1], w[2][m], w[3][m]);
+        }
+#pragma unroll
+        for (int p = 0; p < 4; ++p) accumulate_words(st, 4 * q + p, w[p]);
+    }
+}
+
+// WORDS 32-bit words from a row that starts on a 16-byte boundary (wide) or only on a 4-byte one.
+template <int WORDS>
+__device__ __forceinline__ void load_row(const uint16_t *p, bool wide, uint32_t (&w)[WORDS]) {
+    if (wide) {
+#pragma unroll
+        for (int i = 0; i < WORDS / 4; ++i) {
+            const uint4 v = reinterpret_cast<const uint4 *>(p)[i];
+            w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < WORDS; ++i) w[i] = reinterpret_cast<const uint32_t *>(p)[i];
+    }
+}
+
+// One slab of sixteen tokens of the dense residual, straight from global memory; `valid` of them exist.
+template <int D, int HG>
+__device__ __forceinline__ void dense_slab(AttnState<D, HG> &st, const uint16_t *k, const uint16_t *v, long long ss, int valid,
+                                           bool wide, float sc2) {
+    const int lane = threadIdx.x & 31, i = lane >> 2, j = lane & 3;
+    float c[2][4];
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+        const int t = 4 * (i >> 1) + 2 * a + (i & 1);
+        uint32_t w[D / 8];
+#pragma unroll
+        for (int u = 0; u < D / 8; ++u) w[u] = 0u;
+        if (t < valid) load_row(k + t * ss + j * (D / 4), wide, w);
+        c[a][0] = c[a][1] = c[a][2] = c[a][3] = 0.f;
+#pragma unroll
+        for (int s = 0; s < D / 16; ++s) score_words(st, s, w[2 * s], w[2 * s + 1], c[a]);
+    }
+    softmax_slab(st, c, sc2, valid);
+#pragma unroll
+    for (int part = 0; part < D / 64; ++part) {
+        uint32_t w[4][4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) w[m][u] = 0u;
+            if (4 * j + m < valid) load_row(v + (4 * j + m) * ss + i * (D / 8) + 8 * part, wide, w[m]);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const uint32_t col[4] = {w[0][e], w[1][e], w[2][e], w[3][e]};
+            accumulate_words(st, 4 * part + e, col);
+        }
+    }
 }
 
 struct AttnPipeArgs {
@@ -475,142 +695,33 @@ struct AttnPipeArgs {
     UnpackPipeArgs k, v;      // table form, used through resolve_tile
 };
 
-// Scores of the K tile in shared memory against the group's queries, online-softmax bookkeeping
-// and the tile's probabilities (bf16, s.p).  Called by all consumer warps; warps 0..7 work (and meet
-// at a barrier of their own), the others go straight on to the next unit's register phase.
-__device__ __forceinline__ void score_tile(AttnPipeSmem &s, int valid, float sc2, int parity) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g0 = 2 * (lane & 3), r0 = lane >> 2;
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
-    if (warp < 8) {
-        const uint32_t tile_base = smem_u32(s.tile);
-        const int t0 = warp * 16;
-        const int lrow = t0 + (lane & 7) + ((lane >> 3) & 1) * 8;
-        const int lp = lane >> 4;
-#pragma unroll
-        for (int ks = 0; ks < kAD / 16; ++ks) {
-            uint32_t af[4];
-            ldsm_x4(tile_base + swz(lrow, 2 * ks + lp), af);
-            const uint32_t b0 = *reinterpret_cast<const uint32_t *>(&s.q[r0][16 * ks + g0]);
-            const uint32_t b1 = *reinterpret_cast<const uint32_t *>(&s.q[r0][16 * ks + 8 + g0]);
-            mma_bf16(c, af, b0, b1);
-        }
-        const int ta = t0 + r0, tb = ta + 8;
-        c[0] = ta < valid ? c[0] * sc2 : -INFINITY;
-        c[1] = ta < valid ? c[1] * sc2 : -INFINITY;
-        c[2] = tb < valid ? c[2] * sc2 : -INFINITY;
-        c[3] = tb < valid ? c[3] * sc2 : -INFINITY;
-        float v0 = fmaxf(c[0], c[2]), v1 = fmaxf(c[1], c[3]);
-#pragma unroll
-        for (int d = 4; d < 32; d <<= 1) {
-            v0 = fmaxf(v0, __shfl_xor_sync(kFull, v0, d));
-            v1 = fmaxf(v1, __shfl_xor_sync(kFull, v1, d));
-        }
-        if (lane < 4) {
-            s.red_max[warp][g0] = v0;
-            s.red_max[warp][g0 + 1] = v1;
-        }
-        asm volatile("bar.sync 2, 256;" ::: "memory");      // the eight math warps only; the others run ahead
-        float mn[2], al[2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            float tm = s.red_max[0][g0 + j];
-#pragma unroll
-            for (int w = 1; w < 8; ++w) tm = fmaxf(tm, s.red_max[w][g0 + j]);
-            const float mo = s.m[parity][g0 + j];
-            mn[j] = fmaxf(mo, tm);
-            al[j] = mo == -INFINITY ? 0.f : exp2f(mo - mn[j]);
-        }
-        // probabilities, rounded to bf16 (what the tensor cores multiply with; the sums use the same)
-        const uint32_t b00 = f32_to_bf16_bits(c[0] == -INFINITY ? 0.f : exp2f(c[0] - mn[0]));
-        const uint32_t b01 = f32_to_bf16_bits(c[1] == -INFINITY ? 0.f : exp2f(c[1] - mn[1]));
-        const uint32_t b10 = f32_to_bf16_bits(c[2] == -INFINITY ? 0.f : exp2f(c[2] - mn[0]));
-        const uint32_t b11 = f32_to_bf16_bits(c[3] == -INFINITY ? 0.f : exp2f(c[3] - mn[1]));
-        s.p[g0][ta] = (uint16_t)b00;
-        s.p[g0 + 1][ta] = (uint16_t)b01;
-        s.p[g0][ta + 8] = (uint16_t)b10;
-        s.p[g0 + 1][ta + 8] = (uint16_t)b11;
-        float s0 = __uint_as_float(b00 << 16) + __uint_as_float(b10 << 16);
-        float s1 = __uint_as_float(b01 << 16) + __uint_as_float(b11 << 16);
-#pragma unroll
-        for (int d = 4; d < 32; d <<= 1) {
-            s0 += __shfl_xor_sync(kFull, s0, d);
-            s1 += __shfl_xor_sync(kFull, s1, d);
-        }
-        if (lane < 4) {
-            s.red_sum[warp][g0] = s0;
-            s.red_sum[warp][g0 + 1] = s1;
-            if (warp == 0) {
-                s.m[parity ^ 1][g0] = mn[0];
-                s.m[parity ^ 1][g0 + 1] = mn[1];
-                s.alpha[g0] = al[0];
-                s.alpha[g0 + 1] = al[1];
-            }
-        }
-    }
-}
-
-// oacc = oacc * alpha + V^T P for the V tile in shared memory; warp 0 also folds the tile's
-// probability sums into the running denominators.  The caller has passed a barrier since score_tile.
-__device__ __forceinline__ void accumulate_tile(AttnPipeSmem &s, float (&oacc)[4]) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g0 = 2 * (lane & 3), r0 = lane >> 2;
-    if (warp >= 8) return;
-    const float a0 = s.alpha[g0], a1 = s.alpha[g0 + 1];
-    oacc[0] *= a0, oacc[1] *= a1, oacc[2] *= a0, oacc[3] *= a1;
-    const uint32_t tile_base = smem_u32(s.tile);
-    const int m_piece = warp * 2 + ((lane >> 3) & 1);            // output columns 16 warp .. 16 warp + 15
-    const int lt = (lane & 7) + (lane >> 4) * 8;
-#pragma unroll
-    for (int ks = 0; ks < kTileTokens / 16; ++ks) {
-        uint32_t af[4];
-        ldsm_x4_trans(tile_base + swz(16 * ks + lt, m_piece), af);
-        const uint32_t b0 = *reinterpret_cast<const uint32_t *>(&s.p[r0][16 * ks + g0]);
-        const uint32_t b1 = *reinterpret_cast<const uint32_t *>(&s.p[r0][16 * ks + 8 + g0]);
-        mma_bf16(oacc, af, b0, b1);
-    }
-    if (warp == 0 && lane < kMaxGroup) {
-        float t = 0.f;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) t += s.red_sum[w][lane];
-        s.l[lane] = s.l[lane] * s.alpha[lane] + t;
-    }
-}
-
-__global__ void __launch_bounds__(kPipeThreads, 2) k_decode_attn_pipe(const AttnPipeArgs pa) {
+template <int D, int HG>
+__global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_constant__ AttnPipeArgs pa) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    AttnPipeSmem &s = *reinterpret_cast<AttnPipeSmem *>(smem_raw);
+    AttnPipeSmem<D> &s = *reinterpret_cast<AttnPipeSmem<D> *>(smem_raw);
     const AttnArgs &a = pa.a;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int bh = blockIdx.x, split = blockIdx.y;      // (batch, KV head) on x: no 65 535 limit
     const int b = bh / a.Hkv, hkv = bh - b * a.Hkv;
-    const int Gt = a.G, gz = blockIdx.z * kMaxGroup;     // eight query heads of the group per CTA
-    const int G = Gt - gz < kMaxGroup ? Gt - gz : kMaxGroup;
+    const int Gt = a.G, gz = blockIdx.z * 8 * HG;        // 8 or 16 query heads of the group per CTA
+    const int G = Gt - gz < 8 * HG ? Gt - gz : 8 * HG;
 
     if (tid == 0) {
 #pragma unroll
-        for (int i = 0; i < kStages; ++i) {
+        for (int i = 0; i < kAStages; ++i) {
             mbar_init(&s.full[i], 1);
-            mbar_init(&s.empty[i], kConsumerThreads);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // launched as a programmatic dependent of its predecessor in the stream: no global memory is touched above
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    // queries (zero rows beyond G), running statistics
-    for (int i = tid; i < kMaxGroup * kQPad; i += kPipeThreads) {
-        const int g = i / kQPad, d = i - g * kQPad;
-        uint16_t v = 0;
-        if (g < G && d < kAD) v = a.q[(long long)b * a.q_sb + (long long)(hkv * Gt + gz + g) * a.q_sh + d];
-        s.q[g][d] = v;
-        s.p[g][d] = 0;
-    }
-    if (tid < kMaxGroup) {
-        s.m[0][tid] = s.m[1][tid] = -INFINITY;
-        s.l[tid] = 0.f;
-        s.alpha[tid] = 0.f;
+    if (tid < kAStages) {
+        // an empty unit: what a consumer sees if it gives up waiting before the first description is written
+        UnitMeta &m = s.meta[tid];
+        m.dst = nullptr, m.esc = nullptr, m.esc_len = 0, m.esc_tile_start = 0, m.esc_staged = 0, m.esc_shift = 0;
+        m.elems = 0, m.left = 0, m.nbits = 1, m.first_unit_of_tile = 1, m.ds = 0;
     }
     __syncthreads();
+    // launched as a programmatic dependent of its predecessor in the stream: no global memory is touched above
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 
     const int tail_tiles = (a.tail_len + kTileTokens - 1) / kTileTokens;
     const int items = a.n_seg + tail_tiles;
@@ -620,103 +731,160 @@ __global__ void __launch_bounds__(kPipeThreads, 2) k_decode_attn_pipe(const Attn
     const int pk_last = last < a.n_seg ? last : a.n_seg;
     const int n_units = 2 * (pk_last - pk_first);          // K tile, V tile, K tile, ...
 
-    if (tid >= kConsumerThreads) {
-        // ---------------- producer warp ----------------
-        uint32_t it = 0;
-        for (int base = 0; base < n_units; base += 32) {
-            TileSrc mine = {};
-            const int u = base + lane;
-            if (u < n_units) {
-                const long long tile = (long long)(pk_first + (u >> 1)) * pa.k.BH + bh;
-                mine = (u & 1) ? resolve_tile(pa.v, tile) : resolve_tile(pa.k, tile);
+    // Start the copies of unit u (a whole warp; units in ascending order).  The sources of 32 units are looked
+    // up at a time, one per lane: two dependent round trips to global memory for all of them.
+    const auto issue = [&](int u) {
+        if (u >= n_units) return;
+        if ((u & 31) == 0) {
+            const int mine = u + lane;
+            if (mine < n_units) {
+                const long long tile = (long long)(pk_first + (mine >> 1)) * pa.k.BH + bh;
+                s.src[lane] = (mine & 1) ? resolve_tile(pa.v, tile) : resolve_tile(pa.k, tile);
             }
-            const int n_here = n_units - base < 32 ? n_units - base : 32;
-            for (int j = 0; j < n_here; ++j, ++it) {
-                const TileSrc t = shfl_tile(mine, j);
-                const EscWindow w = esc_window(t);
-                const int stg = it % kStages;
-                mbar_wait(&s.empty[stg], ((it / kStages) & 1) ^ 1, a.status);
-                issue_unit(s.stage[stg], s.stage[stg].meta, &s.full[stg], t, w, 0, kTileTokens, kAD, nullptr, true, a.status);
-            }
+            __syncwarp();
         }
-        return;
+        const TileSrc &t = s.src[u & 31];
+        const EscWindow w = esc_window(t, AttnStage<D>::kEscStage);
+        const int stg = u % kAStages;
+        AttnStage<D> &st = s.stage[stg];
+        issue_unit(st.sm, st.codes, st.esc + kEscFront, s.meta[stg], &s.full[stg], t, w, 0, kTileTokens, D, nullptr, true, a.status);
+    };
+    if (warp == 0) {
+        for (int u = 0; u < kAStages - 1; ++u) issue(u);
     }
 
-    // ---------------- consumer warps ----------------
+    const int i = lane >> 2, j = lane & 3;
     const float sc2 = a.scale * kLog2e;                      // scores are kept in the log2 domain
-    float oacc[4] = {0.f, 0.f, 0.f, 0.f};                    // O^T[d = 16 warp + lane/4 (+8)][2 (lane%4), +1]
-    int parity = 0;                                          // tiles seen & 1: which m[] holds the running max
-    int lut_left[2] = {0, 0}, lut_nbits[2] = {0, 0};
-    for (int u = 0; u < n_units; ++u) {
-        const int stg = u % kStages, which = u & 1;
-        if (lane == 0) mbar_wait(&s.full[stg], (u / kStages) & 1, a.status);
-        __syncwarp();
-        const UnpackStage &st = s.stage[stg];
-        const int nb = st.meta.nbits, lf = st.meta.left;
-        if (nb != lut_nbits[which] || lf != lut_left[which]) {
-            // uniform over the CTA; the previous user of this table finished before the last barrier
-            build_decode_lut(s.lut[which], nb, lf, kConsumerThreads);
-            lut_nbits[which] = nb, lut_left[which] = lf;
-            consumer_sync();
-        }
-        switch (nb) {
-            case 1: decode_unit_swz<1>(s, st, &s.empty[stg], s.lut[which], a.status); break;
-            case 2: decode_unit_swz<2>(s, st, &s.empty[stg], s.lut[which], a.status); break;
-            case 3: decode_unit_swz<3>(s, st, &s.empty[stg], s.lut[which], a.status); break;
-            default: decode_unit_swz<4>(s, st, &s.empty[stg], s.lut[which], a.status); break;
-        }
-        if (which == 0) {
-            score_tile(s, kTileTokens, sc2, parity);
-        } else {
-            accumulate_tile(s, oacc);
-            parity ^= 1;
-        }
+    AttnState<D, HG> st;
+#pragma unroll
+    for (int h = 0; h < HG; ++h) {
+        st.m[h] = -INFINITY, st.l[h] = 0.f;
+#pragma unroll
+        for (int e = 0; e < D / 16; ++e) st.o[h][e][0] = st.o[h][e][1] = st.o[h][e][2] = st.o[h][e][3] = 0.f;
     }
-    // dense residual tiles that fall into this split
+    const uint16_t *qb = a.q + (long long)b * a.q_sb + (long long)(hkv * Gt + gz) * a.q_sh;
+    if constexpr (HG == 1) {                                 // (query rows are only known to be 2-byte aligned)
+        const uint16_t *row = qb + (long long)i * a.q_sh + j * (D / 4);
+#pragma unroll
+        for (int u = 0; u < D / 8; ++u) st.q[u] = i < G ? (uint32_t)row[2 * u] | ((uint32_t)row[2 * u + 1] << 16) : 0u;
+    } else {
+        for (int x = tid; x < 16 * D; x += kAThreads) {
+            const int g = x / D, d = x - g * D;
+            s.q[g * kQRow<D> + d] = g < G ? qb[(long long)g * a.q_sh + d] : (uint16_t)0;
+        }
+        st.q_smem = s.q + i * kQRow<D> + j * (D / 4);
+        __syncthreads();
+    }
+    for (int u = 0; u < n_units; ++u) {
+        const int stg = u % kAStages;
+        mbar_wait(&s.full[stg], (u / kAStages) & 1, a.status);      // (every lane: the ready case is three instructions)
+        __syncwarp();
+        const AttnStage<D> &stage = s.stage[stg];
+        const UnitMeta &meta = s.meta[stg];
+        int *wt = s.warp_tot[u & 1];
+        if ((u & 1) == 0) {
+            switch (meta.nbits) {
+                case 1: score_unit<1, D, HG>(st, stage, meta, wt, sc2, a.status); break;
+                case 2: score_unit<2, D, HG>(st, stage, meta, wt, sc2, a.status); break;
+                case 3: score_unit<3, D, HG>(st, stage, meta, wt, sc2, a.status); break;
+                default: score_unit<4, D, HG>(st, stage, meta, wt, sc2, a.status); break;
+            }
+        } else {
+            switch (meta.nbits) {
+                case 1: accumulate_unit<1, D, HG>(st, stage, meta, wt, a.status); break;
+                case 2: accumulate_unit<2, D, HG>(st, stage, meta, wt, a.status); break;
+                case 3: accumulate_unit<3, D, HG>(st, stage, meta, wt, a.status); break;
+                default: accumulate_unit<4, D, HG>(st, stage, meta, wt, a.status); break;
+            }
+        }
+        // every warp has passed this unit's barrier, so the stage of the unit before it is free
+        if (warp == (u & (kAWarps - 1))) issue(u + kAStages - 1);
+    }
+    // dense residual tiles that fall into this split, a slab per warp
     const int tl_first = first > a.n_seg ? first - a.n_seg : 0;
     const int tl_last = last > a.n_seg ? last - a.n_seg : 0;
-    for (int j = tl_first; j < tl_last; ++j) {
-        const int t0 = j * kTileTokens;
-        const int valid = a.tail_len - t0 < kTileTokens ? a.tail_len - t0 : kTileTokens;
-        const long long off = (long long)b * a.t_sb + (long long)hkv * a.t_sh;
-        load_dense_tile_swz(s, a.k_tail + off, a.t_ss, t0, a.tail_len);
-        score_tile(s, valid, sc2, parity);
-        load_dense_tile_swz(s, a.v_tail + off, a.t_ss, t0, a.tail_len);
-        accumulate_tile(s, oacc);
-        parity ^= 1;
+    const long long toff = (long long)b * a.t_sb + (long long)hkv * a.t_sh;
+    const bool wide = ((((uintptr_t)a.k_tail | (uintptr_t)a.v_tail) & 15) | (uintptr_t)((a.t_sb | a.t_sh | a.t_ss) & 7)) == 0;
+    for (int t = tl_first; t < tl_last; ++t) {
+        const int t0 = t * kTileTokens + warp * 16;
+        const int valid = a.tail_len - t0 < 16 ? a.tail_len - t0 : 16;
+        if (valid > 0)
+            dense_slab(st, a.k_tail + toff + t0 * a.t_ss, a.v_tail + toff + t0 * a.t_ss, a.t_ss, valid, wide, sc2);
     }
-    consumer_sync();
+
+    // ---------------- merge the warps ----------------
+#pragma unroll
+    for (int h = 0; h < HG; ++h) {
+        st.l[h] += __shfl_xor_sync(kFull, st.l[h], 1);
+        st.l[h] += __shfl_xor_sync(kFull, st.l[h], 2);
+        if (j == 0) {
+            s.m[warp][8 * h + i] = st.m[h];
+            s.l[warp][8 * h + i] = st.l[h];
+        }
+    }
+    __syncthreads();                       // also: every unit has been read, the stages are free
+    // numerators of all warps, one group of eight heads at a time: [warp][head][d], rows padded by four words
+    constexpr int kRow = D + 4;
+    float *acc = reinterpret_cast<float *>(s.stage);
+    static_assert(sizeof(s.stage) >= sizeof(float) * kAWarps * 8 * kRow, "the stages hold the numerators of the merge");
     const long long slot = (long long)bh * a.n_splits + split;
-    if (warp < 8) {
-        const int g0 = 2 * (lane & 3), d0 = warp * 16 + (lane >> 2);
-        if (g0 < G) {
-            a.part_o[(slot * Gt + gz + g0) * kAD + d0] = oacc[0];
-            a.part_o[(slot * Gt + gz + g0) * kAD + d0 + 8] = oacc[2];
+#pragma unroll
+    for (int h = 0; h < HG; ++h) {
+        float f[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int g = 8 * h + 2 * j + u;
+            float mx = s.m[0][g];
+#pragma unroll
+            for (int w = 1; w < kAWarps; ++w) mx = fmaxf(mx, s.m[w][g]);
+            f[u] = s.m[warp][g] == -INFINITY ? 0.f : exp2f(s.m[warp][g] - mx);
         }
-        if (g0 + 1 < G) {
-            a.part_o[(slot * Gt + gz + g0 + 1) * kAD + d0] = oacc[1];
-            a.part_o[(slot * Gt + gz + g0 + 1) * kAD + d0 + 8] = oacc[3];
+#pragma unroll
+        for (int e = 0; e < D / 16; ++e) {
+            float *r0 = acc + (warp * 8 + 2 * j) * kRow + i * (D / 8) + 2 * e, *r1 = r0 + kRow;
+            *reinterpret_cast<float2 *>(r0) = make_float2(st.o[h][e][0] * f[0], st.o[h][e][2] * f[0]);
+            *reinterpret_cast<float2 *>(r1) = make_float2(st.o[h][e][1] * f[1], st.o[h][e][3] * f[1]);
         }
+        __syncthreads();
+        for (int x = tid; x < 8 * D; x += kAThreads) {
+            const int g = x / D, d = x - g * D;
+            if (8 * h + g < G) {
+                float v = 0.f;
+#pragma unroll
+                for (int w = 0; w < kAWarps; ++w) v += acc[(w * 8 + g) * kRow + d];
+                a.part_o[(slot * Gt + gz + 8 * h + g) * D + d] = v;
+            }
+        }
+        if (h + 1 < HG) __syncthreads();
     }
     if (tid < G) {
-        const float m2 = s.m[parity][tid];
-        a.part_ml[(slot * Gt + gz + tid) * 2 + 0] = m2 == -INFINITY ? -INFINITY : m2 / kLog2e;   // natural-log domain
-        a.part_ml[(slot * Gt + gz + tid) * 2 + 1] = s.l[tid];
+        float mx = s.m[0][tid];
+#pragma unroll
+        for (int w = 1; w < kAWarps; ++w) mx = fmaxf(mx, s.m[w][tid]);
+        float l = 0.f;
+#pragma unroll
+        for (int w = 0; w < kAWarps; ++w) l += s.m[w][tid] == -INFINITY ? 0.f : s.l[w][tid] * exp2f(s.m[w][tid] - mx);
+        a.part_ml[(slot * Gt + gz + tid) * 2 + 0] = mx == -INFINITY ? -INFINITY : mx / kLog2e;   // natural-log domain
+        a.part_ml[(slot * Gt + gz + tid) * 2 + 1] = l;
     }
+    // do not leave while a copy into this CTA's shared memory may still be in flight (see k_unpack_pipe)
+    if (warp == 0 && launch_timed_out(a.status))
+        for (int u = n_units > kAStages ? n_units - kAStages : 0; u < n_units; ++u)
+            mbar_wait(&s.full[u % kAStages], (u / kAStages) & 1, a.status);
 }
 
-static_assert(sizeof(AttnPipeSmem) <= 113 * 1024, "two CTAs of the pipelined kernel must fit one SM");
+static_assert(sizeof(AttnPipeSmem<128>) <= 113 * 1024, "two CTAs of the pipelined kernel must fit one SM");
 
 constexpr int kMaxSplits = 128;
 
 // Splits per (batch, KV head): the grid should fill a whole number of waves of resident CTAs
-// (two per SM for the pipelined kernel, three for the plain one).  One, two and three waves are
+// (two per SM).  One, two and three waves are
 // tried and the fullest wins; fewer waves on ties (more tiles per CTA, less per-CTA overhead).
-int pick_splits(int B, int Hkv, int items, int D) {
+int pick_splits(int B, int Hkv, int items) {
     int sms = 148;
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long slots = (long long)sms * (D == kAD ? 2 : 3);
+    const long long slots = (long long)sms * 2;
     const long long bh = (long long)B * Hkv;
     int best = 1;
     double best_fill = 0.0;
@@ -748,6 +916,23 @@ cudaError_t launch_as_dependent(void (*kernel)(KArgs...), dim3 grid, int threads
     cfg.attrs = attr, cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
+
+template <int D, int HG>
+int launch_attn_pipe(const AttnPipeArgs &pa, dim3 grid, cudaStream_t st) {
+    // the kernel's limit of dynamic shared memory is raised once per device
+    static std::atomic<bool> done[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return ADACODE_ERR_CUDA;
+    if (dev < 0 || dev >= 64 || !done[dev].load(std::memory_order_acquire)) {
+        if (cudaFuncSetAttribute(k_decode_attn_pipe<D, HG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(AttnPipeSmem<D>)) != cudaSuccess)
+            return ADACODE_ERR_CUDA;
+        if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
+    }
+    return launch_as_dependent(k_decode_attn_pipe<D, HG>, grid, kAThreads, sizeof(AttnPipeSmem<D>), st, pa) == cudaSuccess
+               ? ADACODE_OK
+               : ADACODE_ERR_CUDA;
+}
 }  // namespace
 
 extern "C" {
@@ -767,7 +952,16 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
     if (B <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0 || n_segments < 0 || tail_len < 0) return ADACODE_ERR_INVALID_ARG;
     const int G = Hq / Hkv;
     if (seq_tile != kTileTokens || (D != 64 && D != 128)) return ADACODE_ERR_INVALID_ARG;
-    const int head_groups = (G + kMaxGroup - 1) / kMaxGroup;      // CTAs along z, eight query heads each
+    // ADACODE_ATTN_SIMPLE=1 forces the plain kernel
+    static const bool force_simple = [] {
+        const char *v = getenv("ADACODE_ATTN_SIMPLE");
+        return v && v[0] == '1';
+    }();
+    // CTAs along z: up to eight query heads share a CTA, or up to sixteen: what costs is the decode of the
+    // cache, which they share.  The plain kernel takes eight.
+    const bool two_groups = G > 8 && !force_simple;
+    const int heads_per_cta = two_groups ? 16 : kMaxGroup;
+    const int head_groups = (G + heads_per_cta - 1) / heads_per_cta;
     if (head_groups > 65535) return ADACODE_ERR_INVALID_ARG;
     if (!q_bf16 || !out_bf16 || !workspace || !status) return ADACODE_ERR_INVALID_ARG;
     if (n_segments > 0 && (!k_segments_dev || !v_segments_dev)) return ADACODE_ERR_INVALID_ARG;
@@ -776,7 +970,7 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
         return ADACODE_ERR_INVALID_ARG;
     const int items = n_segments + (tail_len + kTileTokens - 1) / kTileTokens;
     if (items == 0) return ADACODE_ERR_INVALID_ARG;
-    if (n_splits <= 0) n_splits = pick_splits(B, Hkv * head_groups, items, D);
+    if (n_splits <= 0) n_splits = pick_splits(B, Hkv * head_groups, items);
     if (n_splits > kMaxSplits) n_splits = kMaxSplits;
     if (workspace_bytes < adacode_decode_attn_workspace_bytes(B, Hq, D, n_splits)) return ADACODE_ERR_WORKSPACE;
     AttnArgs a;
@@ -789,23 +983,7 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
     a.part_ml = a.part_o + (size_t)B * Hq * n_splits * D;
     a.status = status;
     cudaStream_t st = (cudaStream_t)stream;
-    static bool attr_set[64] = {false};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return ADACODE_ERR_CUDA;
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        if (cudaFuncSetAttribute(k_decode_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AttnSmem)) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(k_decode_attn_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sizeof(AttnPipeSmem)) != cudaSuccess)
-            return ADACODE_ERR_CUDA;
-        attr_set[dev] = true;
-    }
-    // head_dim 128: the pipelined tensor-core kernel; ADACODE_ATTN_SIMPLE=1 forces the plain one
-    static const bool force_simple = [] {
-        const char *v = getenv("ADACODE_ATTN_SIMPLE");
-        return v && v[0] == '1';
-    }();
-    if (D == kAD && !force_simple) {
+    if (!force_simple) {
         AttnPipeArgs pa;
         pa.a = a;
         UnpackPipeArgs u;
@@ -817,10 +995,14 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
         u.dst = nullptr, u.db = 0, u.dh = 0, u.ds = 0, u.status = status;
         pa.k = u, pa.v = u;
         pa.k.seg = k_segments_dev, pa.v.seg = v_segments_dev;
-        if (launch_as_dependent(k_decode_attn_pipe, dim3(B * Hkv, n_splits, head_groups), kPipeThreads,
-                                sizeof(AttnPipeSmem), st, pa) != cudaSuccess)
-            return ADACODE_ERR_CUDA;
+        const dim3 grid(B * Hkv, n_splits, head_groups);
+        const int rc = D == 128 ? (two_groups ? launch_attn_pipe<128, 2>(pa, grid, st) : launch_attn_pipe<128, 1>(pa, grid, st))
+                                : (two_groups ? launch_attn_pipe<64, 2>(pa, grid, st) : launch_attn_pipe<64, 1>(pa, grid, st));
+        if (rc != ADACODE_OK) return rc;
     } else {
+        if (cudaFuncSetAttribute(k_decode_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AttnSmem)) !=
+            cudaSuccess)
+            return ADACODE_ERR_CUDA;
         k_decode_attn<<<dim3(B * Hkv, n_splits, head_groups), kAttnThreads, sizeof(AttnSmem), st>>>(a);
     }
     if (cudaGetLastError() != cudaSuccess) return ADACODE_ERR_CUDA;

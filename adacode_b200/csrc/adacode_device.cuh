@@ -274,30 +274,40 @@ __device__ __forceinline__ void decode_group(const uint32_t *lut, uint32_t g, ui
 // ---- decode in registers ---------------------------------------------------------------------
 // Eight codes at a time, without shared-memory lookups and without a loop over the escapes.  The
 // exponent fields are put together as bytes, four elements to a 32-bit word:
-//   1. the codes are spread to one nibble per element, element 0 lowest (for N <= 3 each code's
-//      bits come out reversed: the bytes are filled from the most significant bit, so one bit
-//      reversal brings the elements into ascending order);
+//   1. the codes are spread to one nibble per element.  The first element's code has the most
+//      significant bits of a group, so element k lies in nibble 7 - k, and in the words below the
+//      last of four elements has the lowest byte;
 //   2. a byte permute looks four exponents up at once in a table of at most eight bytes that lives
 //      in two registers (N = 4 has sixteen values and adds the window's left edge bytewise);
 //   3. z has one bit per element that escaped (code 0).  A product with 0x11111111 gives every
-//      nibble its inclusive count of escapes, and from it the selector with which a byte permute
-//      drops the next escape bytes of the stream into their places (zero bytes elsewhere);
+//      nibble the number of escapes from its element to the last one, and from it the selector with
+//      which a byte permute drops the escape bytes that end here into their places (zero bytes
+//      elsewhere);
 //   4. sign, mantissa and exponent bytes are merged and interleaved into bf16 pairs.
-// About 6 instructions per element, none of them divergent; the table lookups and the
-// per-escape loop that this replaces took 15.8 on keys and values with 6 % escapes.
+// About 6 instructions per element, none of them divergent and all on the full-rate integer and
+// multiply pipes (bringing the elements into ascending order with one bit reversal per group made
+// that unit, a quarter as fast, the bottleneck at 85 % busy); the table lookups and the per-escape
+// loop that this replaces took 15.8 on keys and values with 6 % escapes.
 
 struct ExpTable { uint32_t a, b; };
+
+// bits of a where the mask has ones, of b elsewhere: one instruction
+__device__ __forceinline__ uint32_t bit_select(uint32_t mask, uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xE4;" : "=r"(r) : "r"(a), "r"(b), "r"(mask));
+    return r;
+}
 
 template <int N>
 __device__ __forceinline__ ExpTable exp_table(int left) {
     ExpTable t = {0u, 0u};
-    const auto v = [left](int c) { return (uint32_t)(c + left) & 0xFFu; };
-    if constexpr (N == 1) t.a = v(1) << 8;
-    else if constexpr (N == 2) t.a = (v(2) << 8) | (v(1) << 16) | (v(3) << 24);
-    else if constexpr (N == 3) {
-        t.a = (v(4) << 8) | (v(2) << 16) | (v(6) << 24);
-        t.b = v(1) | (v(5) << 8) | (v(3) << 16) | (v(7) << 24);
-    } else t.a = (uint32_t)left;
+    if constexpr (N == 4) {
+        t.a = (uint32_t)left;
+    } else {
+        const auto v = [left](int c) { return (uint32_t)(c + left) & 0xFFu; };
+        t.a = (v(1) << 8) | (v(2) << 16) | (v(3) << 24);
+        t.b = v(4) | (v(5) << 8) | (v(6) << 16) | (v(7) << 24);
+    }
     return t;
 }
 
@@ -305,30 +315,77 @@ __device__ __forceinline__ ExpTable exp_table(int left) {
 template <int N>
 __device__ __forceinline__ void load_codes16(const uint8_t *s, uint32_t (&x)[2]) {
     if constexpr (N == 1) {
-        const uint32_t v = __brev((uint32_t) * reinterpret_cast<const uint16_t *>(s));
-        x[0] = v >> 24, x[1] = (v >> 16) & 0xFFu;
+        const uint32_t v = *reinterpret_cast<const uint16_t *>(s);
+        x[0] = v & 0xFFu, x[1] = v >> 8;
     } else if constexpr (N == 2) {
-        const uint32_t v = __brev(__byte_perm(*reinterpret_cast<const uint32_t *>(s), 0u, 0x0123));
-        x[0] = __byte_perm(v, 0u, 0x4140), x[1] = __byte_perm(v, 0u, 0x4342);
+        const uint32_t v = *reinterpret_cast<const uint32_t *>(s);
+        x[0] = __byte_perm(v, 0u, 0x4041), x[1] = __byte_perm(v, 0u, 0x4243);
     } else if constexpr (N == 3) {
         const uint16_t *p = reinterpret_cast<const uint16_t *>(s);
         const uint32_t lo = (uint32_t)p[0] | ((uint32_t)p[1] << 16), hi = p[2];
-        x[0] = __brev(__byte_perm(lo, 0u, 0x0124));
-        x[1] = __brev(__byte_perm(lo, hi, 0x3456));
+        x[0] = __byte_perm(lo, 0u, 0x4012);
+        x[1] = __byte_perm(lo, hi, 0x6345);
     } else {
         const uint2 v = *reinterpret_cast<const uint2 *>(s);
-        x[0] = v.x, x[1] = v.y;
+        x[0] = __byte_perm(v.x, 0u, 0x0123), x[1] = __byte_perm(v.y, 0u, 0x0123);
     }
 }
 
-// One nibble per element (N = 4: as stored, the even elements in the high halves of the bytes).
+// The same for the eight elements of one group, whose N code bytes lie on an N-byte boundary
+// (N = 3: anywhere).
+template <int N>
+__device__ __forceinline__ uint32_t load_codes8(const uint8_t *s) {
+    if constexpr (N == 1) return s[0];
+    else if constexpr (N == 2) return __byte_perm((uint32_t) * reinterpret_cast<const uint16_t *>(s), 0u, 0x4041);
+    else if constexpr (N == 3) return ((uint32_t)s[0] << 16) | ((uint32_t)s[1] << 8) | s[2];
+    else return __byte_perm(*reinterpret_cast<const uint32_t *>(s), 0u, 0x0123);
+}
+
+// The same for 32 elements (four groups) whose 4 N code bytes lie on a 4 N-byte boundary (N = 3: 4 bytes).
+template <int N>
+__device__ __forceinline__ void split_codes32(const uint32_t (&w)[N], uint32_t (&x)[4]) {
+    if constexpr (N == 1) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) x[q] = (w[0] >> (8 * q)) & 0xFFu;
+    } else if constexpr (N == 2) {
+        x[0] = __byte_perm(w[0], 0u, 0x4041), x[1] = __byte_perm(w[0], 0u, 0x4243);
+        x[2] = __byte_perm(w[1], 0u, 0x4041), x[3] = __byte_perm(w[1], 0u, 0x4243);
+    } else if constexpr (N == 3) {
+        // (the highest byte is arbitrary: spread8 ignores it)
+        x[0] = __byte_perm(w[0], 0u, 0x4012);
+        x[1] = __byte_perm(w[0], w[1], 0x5345);
+        x[2] = __byte_perm(w[1], w[2], 0x4234);
+        x[3] = __byte_perm(w[2], 0u, 0x4123);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) x[q] = __byte_perm(w[q], 0u, 0x0123);
+    }
+}
+template <int N>
+__device__ __forceinline__ void load_codes32(const uint8_t *s, uint32_t (&x)[4]) {
+    uint32_t w[N];
+    if constexpr (N == 2) {
+        const uint2 v = *reinterpret_cast<const uint2 *>(s);
+        w[0] = v.x, w[1] = v.y;
+    } else if constexpr (N == 4) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(s);
+        w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) w[i] = reinterpret_cast<const uint32_t *>(s)[i];
+    }
+    split_codes32<N>(w, x);
+}
+
+// One nibble per element.
 template <int N>
 __device__ __forceinline__ uint32_t spread8(uint32_t x) {
     uint32_t nib = x;
     if constexpr (N == 3) {
-        nib = (x & 0x00000FFFu) | ((x << 4) & 0x0FFF0000u);
-        nib = (nib & 0x003F003Fu) | ((nib << 2) & 0x3F003F00u);
-        nib = (nib & 0x07070707u) | ((nib << 1) & 0x70707070u);
+        // (what a step leaves between the fields it moves is cleared by the last mask)
+        nib = bit_select(0xFFFF0000u, x << 4, x);
+        nib = bit_select(0xFF00FF00u, nib << 2, nib);
+        nib = bit_select(0xF0F0F0F0u, nib << 1, nib) & 0x77777777u;
     } else if constexpr (N == 2) {                     // x: eight bits in each half
         nib = (x | (x << 4)) & 0x0F0F0F0Fu;
         nib = (nib | (nib << 2)) & 0x33333333u;
@@ -340,13 +397,12 @@ __device__ __forceinline__ uint32_t spread8(uint32_t x) {
     return nib;
 }
 
-// z: bit 4 k set where element k escaped
+// z: bit 4 (7 - k) set where element k escaped
 template <int N>
 __device__ __forceinline__ uint32_t escape_mask(uint32_t nib) {
     if constexpr (N == 4) {
-        uint32_t t = nib | (nib >> 1);
-        t = ~(t | (t >> 2));
-        return ((t >> 4) & 0x01010101u) | ((t << 4) & 0x10101010u);
+        const uint32_t t = nib | (nib >> 1);
+        return ~(t | (t >> 2)) & 0x11111111u;
     } else if constexpr (N == 3) {
         return (~(nib + 0x77777777u) & 0x88888888u) >> 3;
     } else if constexpr (N == 2) {
@@ -356,7 +412,7 @@ __device__ __forceinline__ uint32_t escape_mask(uint32_t nib) {
     }
 }
 
-// e[0], e[1]: exponent bytes of elements 0..3 and 4..7, zero where the element escaped
+// e[0], e[1]: exponent bytes of elements 0..3 and 4..7 (the last one lowest), zero where the element escaped
 template <int N>
 __device__ __forceinline__ void lookup8(uint32_t nib, const ExpTable &t, uint32_t (&e)[2]) {
     if constexpr (N == 4) {
@@ -365,36 +421,40 @@ __device__ __forceinline__ void lookup8(uint32_t nib, const ExpTable &t, uint32_
         const uint32_t no = ((odd + 0x0F0F0F0Fu) >> 4) & 0x01010101u;
         // (no carry between bytes: a code that was written stands for an exponent of 0..255)
         const uint32_t ee = ne * t.a + even, eo = no * t.a + odd;
-        e[0] = __byte_perm(ee, eo, 0x5140);
-        e[1] = __byte_perm(ee, eo, 0x7362);
+        e[0] = __byte_perm(ee, eo, 0x3726);
+        e[1] = __byte_perm(ee, eo, 0x1504);
     } else {
-        e[0] = __byte_perm(t.a, t.b, nib);
-        e[1] = __byte_perm(t.a, t.b, nib >> 16);
+        e[0] = __byte_perm(t.a, t.b, nib >> 16);
+        e[1] = __byte_perm(t.a, t.b, nib);
     }
 }
 
 // escapes among the eight elements of z
 __device__ __forceinline__ int escapes_of(uint32_t z) { return (int)((z * 0x11111111u) >> 28); }
 
-// Put the next escape bytes of a stream into e (as lookup8 left it).  `word(i)` is the stream's aligned
-// 32-bit word i and `r` the byte at which these eight elements' escapes begin.  Three words are read
-// whether they are needed or not.
+// Put the escape bytes of these eight elements, which begin at byte `r` of a stream, into e (as lookup8
+// left it).  `word(i)` is the stream's aligned 32-bit word i; of the words from the one before r's to
+// two behind it three are read, whether they are needed or not.
 template <typename Words>
-__device__ __forceinline__ void place_escapes(uint32_t z, uint32_t r, const Words &word, uint32_t (&e)[2]) {
-    const uint32_t i = r >> 2, sh = r << 3;                // (the funnel shifts take sh modulo 32)
+__device__ __forceinline__ void place_escapes(uint32_t z, int r, const Words &word, uint32_t (&e)[2]) {
+    const uint32_t suffix = z * 0x11111111u;               // nibble 7 - k: escapes among elements k..7 (at most 8)
+    const uint32_t last8 = (suffix >> 9) & 0x78u;          // 8 x escapes among elements 4..7
+    const int mid8 = 8 * r + (int)(suffix >> 28) * 8 - (int)last8;       // 8 x where those begin
+    const int i = (mid8 >> 5) - 1;
     const uint32_t w0 = word(i), w1 = word(i + 1), w2 = word(i + 2);
-    const uint32_t a = __funnelshift_r(w0, w1, sh), b = __funnelshift_r(w1, w2, sh);
-    const uint32_t incl = z * 0x11111111u;                 // nibble k: escapes among elements 0..k (at most 8)
-    const uint32_t c = __funnelshift_rc(a, b, (incl >> 9) & 0x78u);      // behind the escapes of elements 0..3
-    // nibble k of a selector: the rank of an escape inside its four elements, 4..7 (a zero byte) otherwise
-    e[0] |= __byte_perm(a, 0u, z * (0x1111u - 5u) + 0x4444u);
-    e[1] |= __byte_perm(c, 0u, (z >> 16) * (0x1111u - 5u) + 0x4444u);
+    const uint32_t a = __funnelshift_r(w0, w1, (uint32_t)mid8);          // the four bytes before that place
+    const uint32_t b = __funnelshift_r(w1, w2, (uint32_t)mid8);
+    const uint32_t c = __funnelshift_rc(a, b, last8);                    // the four bytes before the end
+    // a nibble of a selector: the s-th escape from the end of four elements takes byte 4 - s of the word
+    // (bytes 4..7 of the pair), any other element a zero byte (0..3)
+    e[0] |= __byte_perm(0u, a, 0x3333u - (z >> 16) * (0x1111u - 5u));
+    e[1] |= __byte_perm(0u, c, 0x3333u - z * (0x1111u - 5u));
 }
 
-// Two bf16 pairs from four sign/mantissa bytes and four exponent bytes.
+// Two bf16 pairs from four sign/mantissa bytes and their exponent bytes (the last one lowest).
 __device__ __forceinline__ void assemble4(uint32_t sm, uint32_t e, uint32_t &w0, uint32_t &w1) {
-    const uint32_t lo = ((e << 7) & 0x80808080u) | (sm & 0x7F7F7F7Fu);
-    const uint32_t hi = ((e >> 1) & 0x7F7F7F7Fu) | (sm & 0x80808080u);
-    w0 = __byte_perm(lo, hi, 0x5140);
-    w1 = __byte_perm(lo, hi, 0x7362);
+    // exponents to bits 7..14 of each half (the product runs on the multiply pipe), the rest from the byte
+    // of sign and mantissa doubled
+    w0 = bit_select(0x7F807F80u, __byte_perm(e, 0u, 0x4243) * 128u, __byte_perm(sm, 0u, 0x1100));
+    w1 = bit_select(0x7F807F80u, __byte_perm(e, 0u, 0x4041) * 128u, __byte_perm(sm, 0u, 0x3322));
 }

@@ -5,9 +5,9 @@
 //
 // One CTA = W consumer warps + 1 producer warp, persistent over tiles.  A "unit" is a run of
 // whole token rows of one tile, at most W x 1024 elements.  Two geometries are built: the wide one
-// (16 warps, units of a whole 128 x 128 tile, 2 CTAs per SM) for the pack kernel and the fused
-// attention kernel, the narrow one (8 warps, units of 8192 elements, 4 CTAs per SM) for the unpack
-// kernel, which measured 5-8 % faster with four smaller pipelines per SM than with two large ones.
+// (16 warps, units of a whole 128 x 128 tile, 2 CTAs per SM) for the pack kernel, the narrow one
+// (8 warps, units of 8192 elements, 4 CTAs per SM) for the unpack kernel, which measured 5-8 % faster
+// with four smaller pipelines per SM than with two large ones.
 // The pack kernel measured 7 % slower that way (twice the escape slots and unit counts to
 // compact) and takes the narrow geometry only for tiles of at most 8192 elements, which would
 // leave half the threads of a wide unit idle.
@@ -38,7 +38,7 @@ struct PipeGeom {
 using WideGeom = PipeGeom<16, 2>;
 using NarrowGeom = PipeGeom<8, 4>;
 
-// the wide geometry under the names the pack kernel and the attention kernel use
+// the wide geometry under the names that the helpers default to
 constexpr int kPWarps = WideGeom::kWarps;
 constexpr int kConsumerThreads = WideGeom::kConsumers;
 constexpr int kPipeThreads = WideGeom::kThreads;
@@ -172,7 +172,11 @@ __host__ __device__ inline int unit_rows_for(int seq_tile, int D) {
 // unpack
 // ---------------------------------------------------------------------------------------
 
-constexpr int kEscStage = WideGeom::kEscStage;
+// Bytes of an escape buffer that are not for escapes: kEscFront in front of the first granule, because
+// place_escapes reads the word before an escape, and behind the last one a granule and the words it
+// reads ahead.
+constexpr int kEscFront = 16;
+constexpr int kEscSlack = kEscFront + 32;
 
 struct UnitMeta {
     uint16_t *dst;            // first element of the unit in the destination
@@ -193,9 +197,7 @@ template <class G>
 struct alignas(128) UnpackStageT {
     alignas(128) uint8_t sm[G::kUnit];
     alignas(128) uint8_t codes[G::kUnit / 2];
-    // (a granule of slack in front, one behind, and the words that place_escapes reads ahead)
-    alignas(128) uint8_t esc[G::kEscStage + 48];
-    alignas(16) UnitMeta meta;
+    alignas(128) uint8_t esc[G::kEscStage + kEscSlack];
 };
 
 template <class G>
@@ -213,7 +215,6 @@ struct alignas(128) UnpackSmemT {
     // behind the barrier of unit i + 1, which no warp reaches before it has read those of unit i
     int warp_tot[2][G::kWarps];
 };
-using UnpackStage = UnpackStageT<WideGeom>;
 static_assert(sizeof(UnpackStageT<WideGeom>) % 128 == 0 && sizeof(UnpackStageT<NarrowGeom>) % 128 == 0,
               "stage buffers must stay 128-byte aligned");
 
@@ -310,13 +311,12 @@ struct EscWindow {
     int win, tail, staged, shift;
 };
 
-template <int ESC_STAGE = kEscStage>
-__device__ __forceinline__ EscWindow esc_window(const TileSrc &t) {
+__device__ __forceinline__ EscWindow esc_window(const TileSrc &t, int most) {
     EscWindow w;
     // stage no more than the stream really holds, so that a short stream is reported as such
     long long avail = t.esc_len - t.esc_start;
     if (avail > t.esc_cnt) avail = t.esc_cnt;
-    if (avail > ESC_STAGE) avail = ESC_STAGE;
+    if (avail > most) avail = most;
     w.staged = avail > 0 ? (int)avail : 0;
     const uint8_t *ea = t.esc + t.esc_start;
     w.shift = (int)((uintptr_t)ea & 15);
@@ -332,15 +332,14 @@ __device__ __forceinline__ EscWindow esc_window(const TileSrc &t) {
     return w;
 }
 
-// Producer warp, stage known to be free: describe the unit (rows [row0, row0 + rows) of tile t) in
-// `m` and start its bulk copies against `full_bar`.
-template <class Stage>
-__device__ __forceinline__ void issue_unit(Stage &st, UnitMeta &m, uint64_t *full_bar, const TileSrc &t,
-                                           const EscWindow &w, int row0, int rows, int D, uint16_t *dst,
+// One warp, stage known to be free: describe the unit (rows [row0, row0 + rows) of tile t) in `m` and
+// start its bulk copies against `full_bar`.
+__device__ __forceinline__ void issue_unit(uint8_t *s_sm, uint8_t *s_codes, uint8_t *s_esc, UnitMeta &m, uint64_t *full_bar,
+                                           const TileSrc &t, const EscWindow &w, int row0, int rows, int D, uint16_t *dst,
                                            bool first_unit, int32_t *status, bool withhold = false) {
     const int lane = threadIdx.x & 31;
     if (w.tail > 0) {
-        if (lane < w.tail) st.esc[w.win + lane] = w.a0[w.win + lane];
+        if (lane < w.tail) s_esc[w.win + lane] = w.a0[w.win + lane];
         __syncwarp();
     }
     if (lane == 0) {
@@ -368,46 +367,9 @@ __device__ __forceinline__ void issue_unit(Stage &st, UnitMeta &m, uint64_t *ful
             mbar_arrive_expect_tx(full_bar, 0);
         } else {
             mbar_arrive_expect_tx(full_bar, (uint32_t)elems + cbytes + (uint32_t)w.win);
-            bulk_load(st.sm, src_sm, (uint32_t)elems, full_bar);
-            bulk_load(st.codes, src_cd, cbytes, full_bar);
-            if (w.win > 0) bulk_load(st.esc, w.a0, (uint32_t)w.win, full_bar);
-        }
-    }
-}
-
-// Register phase of a unit, shared by the unpack kernel and the fused attention kernel: every
-// consumer thread decodes its kPCPT chunks of the staged planes into registers (exponent fields
-// from the table, 0 where the code is 0; sign and mantissa merged in) and notes where the
-// escapes are (zm: one bit per code-0 slot of each group word; zc: their number per chunk).
-template <int N, class Stage>
-__device__ __forceinline__ void decode_chunks(const Stage &st, const uint32_t *lut, int chunks,
-                                              uint4 (&o)[kPCPT][2], uint32_t (&zm)[kPCPT][2], int (&zc)[kPCPT]) {
-    constexpr int CB = 2 * N;   // code bytes per 16-element chunk
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < kPCPT; ++k) {
-        const int c = warp * (kPCPT * 32) + k * 32 + lane;
-        uint32_t g[2] = {0u, 0u};
-        uint4 sv = make_uint4(0, 0, 0, 0);
-        const bool valid = c < chunks;
-        if (valid) {
-            sv = *reinterpret_cast<const uint4 *>(st.sm + c * 16);
-            load_chunk_codes<N, 16>(st.codes + c * CB, g);
-        }
-        const uint32_t sw[4] = {sv.x, sv.y, sv.z, sv.w};
-        zc[k] = 0;
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            zm[k][q] = valid ? zero_slots<N>(g[q]) : 0u;
-            zc[k] += __popc(zm[k][q]);
-            uint32_t ew[4];
-            decode_group<N>(lut, g[q], ew);
-            const uint32_t s0 = sw[2 * q], s1 = sw[2 * q + 1];
-            // sign and mantissa: each byte doubled into its 16-bit lane, then masked into place
-            o[k][q].x = ew[0] | (__byte_perm(s0, 0u, 0x1100) & 0x807F807Fu);
-            o[k][q].y = ew[1] | (__byte_perm(s0, 0u, 0x3322) & 0x807F807Fu);
-            o[k][q].z = ew[2] | (__byte_perm(s1, 0u, 0x1100) & 0x807F807Fu);
-            o[k][q].w = ew[3] | (__byte_perm(s1, 0u, 0x3322) & 0x807F807Fu);
+            bulk_load(s_sm, src_sm, (uint32_t)elems, full_bar);
+            bulk_load(s_codes, src_cd, cbytes, full_bar);
+            if (w.win > 0) bulk_load(s_esc, w.a0, (uint32_t)w.win, full_bar);
         }
     }
 }
@@ -427,22 +389,23 @@ __device__ __forceinline__ void store_chunk(uint16_t *dst, const uint32_t (&w)[8
 
 // Escapes of one group whose bytes are not (all) staged in shared memory: byte by byte, from global
 // memory beyond the window; a stream that is too short is flagged and gives exponent 0.  Returns the
-// bytes in their places (elements 0..3, 4..7).
-__device__ __forceinline__ uint2 gather_escapes(uint32_t z, int r, const uint8_t *esc_smem, int staged, const UnitMeta &m,
+// bytes in their places (elements 0..3, 4..7, the last one lowest).
+__device__ __noinline__ uint2 gather_escapes(uint32_t z, int r, const uint8_t *esc_smem, int staged, const UnitMeta &m,
                                                 int32_t *status) {
     const uint8_t *g_esc = m.esc;
     const long long g_len = m.esc_len, g_start = m.esc_tile_start;
     uint2 e = make_uint2(0u, 0u);
 #pragma unroll 1
-    for (; z != 0; z &= z - 1, ++r) {
-        const int k = (__ffs((int)z) - 1) >> 2;
+    for (; z != 0; ++r) {
+        const int at = 31 - __clz((int)z);                 // the first element has the highest nibble
+        z ^= 1u << at;
         uint32_t v = 0;
         if (r < staged) v = esc_smem[r];
         else if (g_start + r < g_len) v = g_esc[g_start + r];
         else atomicOr(status, ADACODE_STATUS_ESCAPE_UNDERRUN);
-        const uint32_t at = v << (8 * (k & 3));
-        if (k < 4) e.x |= at;
-        else e.y |= at;
+        const uint32_t b = v << (2 * (at & 15));
+        if (at >= 16) e.x |= b;
+        else e.y |= b;
     }
     return e;
 }
@@ -450,16 +413,18 @@ __device__ __forceinline__ uint2 gather_escapes(uint32_t z, int r, const uint8_t
 // One unit: staged planes -> registers -> global memory.  The codes are expanded, the escapes placed
 // and the bf16 words put together in registers (about 6 instructions per element, see spread8), and
 // whole sectors are stored straight from there.  The only CTA-wide barrier is the one between the
-// escape counts of the warps and their sum.  Bound by DRAM: the time hardly depends on the code length
-// or the share of escapes any more.  Keys and values of [16, 8, 8192, 128] (537 M elements moved):
-// n = 3, 5 % escapes 189 -> 183 us, n = 2, 34 % escapes 341 -> 179 us, n = 4 169 -> 183 us (76-81 % of
-// 6.65 TB/s).  The finished unit through shared memory and a bulk store instead: 229 us; three
-// stages 191 us, five CTAs per SM 223 us.
+// escape counts of the warps and their sum.
+// Keys and values of [16, 8, 8192, 128] in one launch (537 M elements), with the lookups, the escape loop and the
+// bulk store that were here before and now: n = 3, 5 % escapes 188.6 -> 177.7 us (5.2 TB/s, 81 % of what a plain
+// copy reaches), n = 2, 34 % escapes 340 -> 177 us, n = 4, 0.1 % escapes 169.7 -> 170.8 us; [1, 8, 20480, 128]
+// 38.8 -> 35.0 us.  The integer pipe is 64 % busy, issue slots 60 %; the rest is waiting at the barrier and for
+// loads.  Tried and slower: no producer warp (one warp in turn refills; the others wait for it at the next
+// barrier) 201 us; one tile per warp without shared memory or barriers 217-219 us; the finished unit through
+// shared memory and a bulk store, which leaves room for three CTAs per SM, 229 us; five CTAs per SM (spills) 223 us.
 template <int N, class G>
-__device__ __forceinline__ void unpack_unit(UnpackSmemT<G> &s, const UnpackStageT<G> &st, const UnitMeta &meta,
-                                            uint64_t *empty_bar, int *warp_tot, int &consumed, const ExpTable &tab,
-                                            const int (&row)[kPCPT], const int (&col)[kPCPT], int32_t *status,
-                                            bool broken) {
+__device__ __forceinline__ void unpack_unit(const UnpackStageT<G> &st, const UnitMeta &meta, int *warp_tot, int &consumed,
+                                            const ExpTable &tab, const int (&row)[kPCPT], const int (&col)[kPCPT],
+                                            uint64_t *empty_bar, int32_t *status, bool broken) {
     constexpr int CB = 2 * N;   // code bytes per 16-element chunk
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (meta.first_unit_of_tile) consumed = 0;
@@ -471,13 +436,12 @@ __device__ __forceinline__ void unpack_unit(UnpackSmemT<G> &s, const UnpackStage
 #pragma unroll
     for (int k = 0; k < kPCPT; ++k) {
         const int c = c0 + k * 32;
-        uint32_t x[2] = {0u, 0u};
-        const bool valid = c < chunks;
-        if (valid) load_codes16<N>(st.codes + c * CB, x);
+        uint32_t x[2];
+        load_codes16<N>(st.codes + c * CB, x);             // (beyond the unit's end: what lies there, not used)
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             nib[k][q] = spread8<N>(x[q]);
-            z[k][q] = valid ? escape_mask<N>(nib[k][q]) : 0u;
+            z[k][q] = c < chunks ? escape_mask<N>(nib[k][q]) : 0u;
         }
         zc[k] = escapes_of(z[k][0]) + escapes_of(z[k][1]);
     }
@@ -485,42 +449,42 @@ __device__ __forceinline__ void unpack_unit(UnpackSmemT<G> &s, const UnpackStage
     const int wtot = warp_scan_counts(zc, incl);
     if (lane == 0) warp_tot[warp] = wtot;
     consumer_sync<G::kConsumers>();
-    int wprefix, unit_tot;
-    cross_warp_prefix<G::kWarps>(warp_tot, wprefix, unit_tot);
+    const int others = warp_tot[lane & (G::kWarps - 1)];
+    const int before = consumed + (int)__reduce_add_sync(kFull, (unsigned)(lane < warp ? others : 0));
+    consumed += (int)__reduce_add_sync(kFull, (unsigned)(lane < G::kWarps ? others : 0));
+    const uint8_t *const esc = st.esc + kEscFront;
     const int staged = meta.esc_staged, shift = meta.esc_shift;
     uint16_t *const dst = meta.dst;
     const long long ds = meta.ds;
     const bool wide = ((((uintptr_t)dst) | ((uintptr_t)ds * 2)) & 31) == 0;
-    const uint32_t *words = reinterpret_cast<const uint32_t *>(st.esc);
-    const auto word = [words](uint32_t i) { return words[i]; };
+    const uint32_t *words = reinterpret_cast<const uint32_t *>(esc);
+    const auto word = [words](int i) { return words[i]; };
+    // (a warp none of whose escapes lies beyond the window, i.e. nearly every one)
+    const bool in_window = __all_sync(kFull, before + incl[kPCPT - 1] <= staged);
 #pragma unroll
     for (int k = 0; k < kPCPT; ++k) {
-        const int r0 = consumed + wprefix + incl[k] - zc[k];     // rank inside the tile of the chunk's first escape
+        const int r0 = before + incl[k] - zc[k];               // rank inside the tile of the chunk's first escape
         const int r1 = r0 + escapes_of(z[k][0]);
         uint32_t e0[2], e1[2];
         lookup8<N>(nib[k][0], tab, e0);
         lookup8<N>(nib[k][1], tab, e1);
-        if (r0 + zc[k] <= staged || zc[k] == 0) {
-            // (a chunk without escapes may rank beyond the window: it reads the window's first words)
-            place_escapes(z[k][0], (uint32_t)(shift + (zc[k] ? r0 : 0)), word, e0);
-            place_escapes(z[k][1], (uint32_t)(shift + (zc[k] ? r1 : 0)), word, e1);
+        if (in_window) {
+            place_escapes(z[k][0], shift + r0, word, e0);
+            place_escapes(z[k][1], shift + r1, word, e1);
         } else {
-            const uint2 g0 = gather_escapes(z[k][0], r0, st.esc + shift, staged, meta, status);
+            const uint2 g0 = gather_escapes(z[k][0], r0, esc + shift, staged, meta, status);
             e0[0] |= g0.x, e0[1] |= g0.y;
-            const uint2 g1 = gather_escapes(z[k][1], r1, st.esc + shift, staged, meta, status);
+            const uint2 g1 = gather_escapes(z[k][1], r1, esc + shift, staged, meta, status);
             e1[0] |= g1.x, e1[1] |= g1.y;
         }
-        uint4 sv = make_uint4(0, 0, 0, 0);
-        const bool valid = c0 + k * 32 < chunks;
-        if (valid) sv = *reinterpret_cast<const uint4 *>(st.sm + (c0 + k * 32) * 16);
+        const uint4 sv = *reinterpret_cast<const uint4 *>(st.sm + (c0 + k * 32) * 16);
         uint32_t w[8];
         assemble4(sv.x, e0[0], w[0], w[1]);
         assemble4(sv.y, e0[1], w[2], w[3]);
         assemble4(sv.z, e1[0], w[4], w[5]);
         assemble4(sv.w, e1[1], w[6], w[7]);
-        if (valid && !broken) store_chunk(dst + (long long)row[k] * ds + col[k], w, wide);
+        if (c0 + k * 32 < chunks && !broken) store_chunk(dst + (long long)row[k] * ds + col[k], w, wide);
     }
-    consumed += unit_tot;
     __syncwarp();
     if (lane == 0) mbar_arrive(empty_bar);    // this warp no longer reads the stage
 }
@@ -528,11 +492,8 @@ __device__ __forceinline__ void unpack_unit(UnpackSmemT<G> &s, const UnpackStage
 // Consumer warp: wait (bounded) until unit `it` is loaded; false if the wait gave up.
 template <class G>
 __device__ __forceinline__ bool wait_loaded(UnpackSmemT<G> &s, uint32_t it, int32_t *status, uint32_t poll_limit) {
-    bool loaded = true;
-    if ((threadIdx.x & 31) == 0) loaded = mbar_wait(&s.full[it % kStages], (it / kStages) & 1, status, poll_limit);
-    loaded = __shfl_sync(kFull, loaded, 0);
-    __syncwarp();          // orders the other lanes' reads of the stage after lane 0's wait
-    return loaded;
+    // (every lane waits: the ready case is three instructions)
+    return __all_sync(kFull, mbar_wait(&s.full[it % kStages], (it / kStages) & 1, status, poll_limit));
 }
 
 // Units it, it + 1, ... as long as they carry code length N and window `left`; returns the first unit
@@ -544,8 +505,8 @@ __device__ __forceinline__ uint32_t unpack_run(UnpackSmemT<G> &s, uint32_t it, u
     const ExpTable tab = exp_table<N>(left);
     for (;;) {
         const int stg = it % kStages;
-        unpack_unit<N>(s, s.stage[stg], s.meta_ring[it % (2 * kStages)], &s.empty[stg], s.warp_tot[it & 1], consumed, tab,
-                       row, col, status, broken);
+        unpack_unit<N>(s.stage[stg], s.meta_ring[it % (2 * kStages)], s.warp_tot[it & 1], consumed, tab, row, col,
+                       &s.empty[stg], status, broken);
         if (++it >= n_units) return it;
         broken |= !wait_loaded(s, it, status, poll_limit);
         const UnitMeta &next = s.meta_ring[it % (2 * kStages)];
@@ -612,13 +573,14 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_unpack_pipe(cons
             const int n_here = (int)(my_tiles - base < 32 ? my_tiles - base : 32);
             for (int j = 0; j < n_here; ++j) {
                 const TileSrc t = shfl_tile(mine, j);
-                const EscWindow w = esc_window<G::kEscStage>(t);
+                const EscWindow w = esc_window(t, G::kEscStage);
                 for (int u = 0; u < units_per_tile; ++u, ++it) {
                     const int stg = it % kStages;
                     mbar_wait(&s.empty[stg], ((it / kStages) & 1) ^ 1, a0.status, ja.poll_limit);
                     const int row0 = u * unit_rows;
                     const int rows = min(unit_rows, a0.seq_tile - row0);
-                    issue_unit(s.stage[stg], s.meta_ring[it % (2 * kStages)], &s.full[stg], t, w, row0, rows, a0.D,
+                    UnpackStageT<G> &st = s.stage[stg];
+                    issue_unit(st.sm, st.codes, st.esc + kEscFront, s.meta_ring[it % (2 * kStages)], &s.full[stg], t, w, row0, rows, a0.D,
                                t.dst + (long long)row0 * t.ds,
                                u == 0, a0.status, blockIdx.x == 0 && (int)it == ja.withhold_unit);
                 }

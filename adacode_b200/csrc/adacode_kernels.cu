@@ -483,34 +483,119 @@ __global__ void __launch_bounds__(kThreads) k_unpack_segments(const UnpackCommon
 // histogram and adjuster
 // ---------------------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(kThreads) k_hist(const uint16_t *__restrict__ src, int64_t sb, int64_t sh,
-                                                   int64_t ss, int H, int S, int D, int64_t n_rows,
-                                                   int32_t *__restrict__ hist) {
-    __shared__ int s_hist[kWarps][256];
-    const int tid = threadIdx.x, warp = tid >> 5;
-    for (int i = tid; i < kWarps * 256; i += kThreads) (&s_hist[0][0])[i] = 0;
-    __syncthreads();
-    const int vec_per_row = D / 8;
-    const int64_t n_vec = n_rows * vec_per_row;
-    for (int64_t i = (int64_t)blockIdx.x * kThreads + tid; i < n_vec; i += (int64_t)gridDim.x * kThreads) {
-        const int64_t row = i / vec_per_row;
-        const int col = (int)(i - row * vec_per_row) * 8;
-        const int64_t bh = row / S;
-        const int s = (int)(row - bh * S);
-        const int b = (int)(bh / H), h = (int)(bh - (int64_t)b * H);
-        const uint4 v = *reinterpret_cast<const uint4 *>(src + b * sb + h * sh + s * ss + col);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+// Exponent histogram.  One shared-memory atomic per element on a histogram that a warp shares costs the
+// conflicts of 32 lanes on the few exponents that nearly all elements have.  Here every lane counts in
+// bytes of its own: 64 words per lane, word (e & 63) of lane l in bank l, byte e >> 6 of it, so that
+// 32 lanes never meet in a bank whatever the exponents are.  A lane's bytes are added up over the warp
+// before they can overflow (kHistUnits units of 32 elements a lane).
+//
+// The source is `runs` contiguous pieces of `run_vec` 16-byte vectors (the host merges dimensions, see
+// flatten_runs); a warp takes units of kHistVec x 32 vectors of one run, and loads the next unit
+// while it counts the current one.  SHORT: runs too short for that are walked vector by vector.
+constexpr int kHistVec = 4;
+constexpr int kHistUnits = 7;                                  // 7 * 32 = 224 <= 255
+
+struct HistRuns {
+    const uint16_t *src;
+    int64_t runs, run_vec;
+    int64_t n1, n0;              // run r -> (r / (n1 n0), r / n0 % n1, r % n0)
+    int64_t s2, s1, s0;          // element strides of those indices
+    int32_t *hist;
+};
+
+__device__ __forceinline__ const uint4 *hist_run(const HistRuns &a, uint32_t r) {
+    const uint32_t q = r / (uint32_t)a.n0, i0 = r - q * (uint32_t)a.n0;
+    const uint32_t i2 = q / (uint32_t)a.n1, i1 = q - i2 * (uint32_t)a.n1;
+    return reinterpret_cast<const uint4 *>(a.src + i2 * a.s2 + i1 * a.s1 + i0 * a.s0);
+}
+
+__device__ __forceinline__ void hist_count(uint32_t *mine, uint32_t w) {
+    // exponent of the low bf16: bits 7..14 (the word's row) and 13..14 (its byte)
+    const uint32_t v = w >> 16;
+    atomicAdd(mine + ((w & 0x1F80u) >> 2), 1u << ((w >> 10) & 0x18u));
+    atomicAdd(mine + ((v & 0x1F80u) >> 2), 1u << ((v >> 10) & 0x18u));
+}
+
+// Add the byte counters of a warp (64 rows of 32 words) to the CTA's histogram and clear them.
+__device__ __forceinline__ void hist_flush(uint32_t *rows, int *s_hist) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+        const int r = half * 32 + lane;
+        uint32_t lo = 0, hi = 0;                               // bytes 0 and 2, bytes 1 and 3: 16-bit sums (32 * 224 fit)
+#pragma unroll 8
+        for (int k = 0; k < 32; ++k) {
+            const uint32_t v = rows[r * 32 + ((lane + k) & 31)];
+            lo += v & 0x00FF00FFu;
+            hi += (v >> 8) & 0x00FF00FFu;
+        }
+        const uint32_t c[4] = {lo & 0xFFFFu, hi & 0xFFFFu, lo >> 16, hi >> 16};
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            atomicAdd(&s_hist[warp][(w[q] >> 7) & 0xFFu], 1);
-            atomicAdd(&s_hist[warp][(w[q] >> 23) & 0xFFu], 1);
+        for (int b = 0; b < 4; ++b)
+            if (c[b] != 0) atomicAdd(&s_hist[b * 64 + r], (int)c[b]);
+    }
+    __syncwarp();
+    for (int i = lane; i < 512; i += 32) reinterpret_cast<uint4 *>(rows)[i] = make_uint4(0, 0, 0, 0);
+    __syncwarp();
+}
+
+template <bool SHORT>
+__global__ void __launch_bounds__(kThreads) k_hist(const __grid_constant__ HistRuns a) {
+    extern __shared__ __align__(16) uint32_t s_rows[];         // [warp][64][32]
+    __shared__ int s_hist[256];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < kWarps * 512; i += kThreads) reinterpret_cast<uint4 *>(s_rows)[i] = make_uint4(0, 0, 0, 0);
+    s_hist[tid] = 0;
+    __syncthreads();
+    uint32_t *rows = s_rows + warp * 2048, *mine = rows + lane;
+    int pending = 0;
+    if constexpr (SHORT) {
+        const int64_t n_vec = a.runs * a.run_vec;
+        for (int64_t base = ((int64_t)blockIdx.x * kWarps + warp) * 32; base < n_vec; base += (int64_t)gridDim.x * kThreads) {
+            const int64_t i = base + lane;
+            if (i < n_vec) {
+                const int64_t r = i / a.run_vec, q = r / a.n0, i2 = q / a.n1;
+                const uint16_t *run = a.src + i2 * a.s2 + (q - i2 * a.n1) * a.s1 + (r - q * a.n0) * a.s0;
+                const uint4 v = reinterpret_cast<const uint4 *>(run)[i - r * a.run_vec];
+                hist_count(mine, v.x), hist_count(mine, v.y), hist_count(mine, v.z), hist_count(mine, v.w);
+            }
+            if (++pending == kHistUnits * kHistVec) hist_flush(rows, s_hist), pending = 0;
+        }
+    } else {
+        const uint32_t run_vec = (uint32_t)a.run_vec, per_run = (run_vec + 32 * kHistVec - 1) / (32 * kHistVec);
+        const uint32_t units = (uint32_t)a.runs * per_run, step = gridDim.x * kWarps;
+        uint4 cur[kHistVec], nxt[kHistVec];
+        // (a lane beyond the end of its run loads nothing and counts nothing: `have` says how many it has)
+        const auto load = [&](uint32_t u, uint4 (&v)[kHistVec]) {
+            int have = 0;
+            if (u < units) {
+                const uint32_t r = u / per_run, at = (u - r * per_run) * (32 * kHistVec) + lane;
+                const uint4 *p = hist_run(a, r) + at;
+#pragma unroll
+                for (int k = 0; k < kHistVec; ++k)
+                    if (at + 32 * k < run_vec) v[k] = __ldg(p + 32 * k), ++have;
+            }
+            return have;
+        };
+        uint32_t u = blockIdx.x * kWarps + warp;
+        int have = load(u, cur);
+        while (u < units) {
+            u += step;
+            const int have_next = load(u, nxt);
+#pragma unroll
+            for (int k = 0; k < kHistVec; ++k)
+                if (k < have) hist_count(mine, cur[k].x), hist_count(mine, cur[k].y), hist_count(mine, cur[k].z), hist_count(mine, cur[k].w);
+#pragma unroll
+            for (int k = 0; k < kHistVec; ++k) cur[k] = nxt[k];
+            have = have_next;
+            if (++pending == kHistUnits) hist_flush(rows, s_hist), pending = 0;
         }
     }
+    if (pending > 0) hist_flush(rows, s_hist);
     __syncthreads();
-    int total = 0;
-#pragma unroll
-    for (int i = 0; i < kWarps; ++i) total += s_hist[i][tid];
-    if (total != 0) atomicAdd(hist + tid, total);
+    const int total = s_hist[tid];
+    if (total != 0) atomicAdd(a.hist + tid, total);
 }
 
 // One warp per histogram: fifteen rounds of "largest remaining count, lowest bin on ties"
@@ -697,6 +782,34 @@ int launch_dependent(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStr
     cfg.attrs = attr, cfg.numAttrs = 1;
     ADACODE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args));
     return ADACODE_OK;
+}
+
+// A [B, H, S, D] view (unit stride along D) as runs of contiguous vectors in any order: dimensions of one
+// entry drop out, the others are sorted by stride and each that continues the one inside it is merged.
+HistRuns flatten_runs(int64_t sb, int64_t sh, int64_t ss, int64_t B, int64_t H, int64_t S, int64_t D) {
+    int64_t size[3] = {B, H, S}, stride[3] = {sb, sh, ss};
+    for (int i = 0; i < 2; ++i)
+        for (int j = 0; j < 2 - i; ++j)
+            if (stride[j] < stride[j + 1]) {
+                const int64_t t = stride[j], u = size[j];
+                stride[j] = stride[j + 1], size[j] = size[j + 1];
+                stride[j + 1] = t, size[j + 1] = u;
+            }
+    int64_t run = D, n[3] = {1, 1, 1}, st[3] = {0, 0, 0};    // outer dimensions, innermost first
+    int k = 0;
+    for (int i = 2; i >= 0; --i) {
+        if (size[i] == 1) continue;
+        if (k == 0 && stride[i] == run) run *= size[i];
+        else if (k > 0 && stride[i] == st[k - 1] * n[k - 1]) n[k - 1] *= size[i];
+        else n[k] = size[i], st[k] = stride[i], ++k;
+    }
+    HistRuns a;
+    a.src = nullptr, a.hist = nullptr;
+    a.run_vec = run / 8;
+    a.runs = n[0] * n[1] * n[2];
+    a.n0 = n[0], a.n1 = n[1];
+    a.s0 = st[0], a.s1 = st[1], a.s2 = st[2];
+    return a;
 }
 
 template <class G>
@@ -1185,13 +1298,23 @@ int adacode_hist_bf16(const void *src_bf16, int64_t stride_b, int64_t stride_h, 
     if (n_rows == 0) return ADACODE_OK;
     if (!src_bf16 || ((uintptr_t)src_bf16 & 15) != 0 || ((stride_b | stride_h | stride_s) & 7))
         return ADACODE_ERR_INVALID_ARG;
-    const int64_t n_vec = n_rows * (D / 8);
-    int64_t blocks = (n_vec + kThreads * 4 - 1) / (kThreads * 4);
-    const int64_t cap = (int64_t)sm_count() * 8;
-    if (blocks > cap) blocks = cap;
-    if (blocks < 1) blocks = 1;
-    k_hist<<<(int)blocks, kThreads, 0, (cudaStream_t)stream>>>((const uint16_t *)src_bf16, stride_b, stride_h,
-                                                              stride_s, H, S, D, n_rows, hist256);
+    HistRuns a = flatten_runs(stride_b, stride_h, stride_s, B, H, S, D);
+    a.src = (const uint16_t *)src_bf16, a.hist = hist256;
+    // Runs shorter than half a warp's unit leave most of its lanes idle, and 32-bit indices must do.
+    const bool by_vector = a.run_vec < 16 * kHistVec || a.runs * a.run_vec >= (1ll << 31);
+    const size_t smem = (size_t)kWarps * 64 * 32 * 4;
+    const int64_t units = by_vector ? (a.runs * a.run_vec + 31) / 32
+                                    : a.runs * ((a.run_vec + 32 * kHistVec - 1) / (32 * kHistVec));
+    const int64_t want = (units + kWarps - 1) / kWarps, cap = (int64_t)sm_count() * 3;
+    const int blocks = (int)(want < cap ? want : cap);
+    int rc;
+    if (by_vector) {
+        if ((rc = ensure_dynamic_smem(k_hist<true>, smem)) != ADACODE_OK) return rc;
+        k_hist<true><<<blocks, kThreads, smem, (cudaStream_t)stream>>>(a);
+    } else {
+        if ((rc = ensure_dynamic_smem(k_hist<false>, smem)) != ADACODE_OK) return rc;
+        k_hist<false><<<blocks, kThreads, smem, (cudaStream_t)stream>>>(a);
+    }
     ADACODE_CUDA_TRY(cudaGetLastError());
     return ADACODE_OK;
 }

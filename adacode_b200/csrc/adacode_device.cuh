@@ -458,3 +458,24 @@ __device__ __forceinline__ void assemble4(uint32_t sm, uint32_t e, uint32_t &w0,
     w0 = bit_select(0x7F807F80u, __byte_perm(e, 0u, 0x4243) * 128u, __byte_perm(sm, 0u, 0x1100));
     w1 = bit_select(0x7F807F80u, __byte_perm(e, 0u, 0x4041) * 128u, __byte_perm(sm, 0u, 0x3322));
 }
+
+// ---- encode in registers ---------------------------------------------------------------------
+// The exponents of a word's two bf16 as codes in its 16-bit halves, 0 outside the window: one packed
+// add-and-minimum takes exponent - left, where everything below the window wraps to a large value and
+// everything beyond it is cut to 2**N, whose low N bits are 0 again.  `neg_left` is -left in both halves.
+// (A table in shared memory, one byte lookup per element, took a load and two bank conflicts each: pack of keys and
+// values [16, 8, 8192, 128] at 3 bits 222.6 us with it, 209.8 us without; with the histogram 241 and 219 us.)
+template <int N>
+__device__ __forceinline__ uint32_t encode_pair(uint32_t w, uint32_t neg_left) {
+    constexpr uint32_t kTop = (1u << N) * 0x10001u;
+    return __viaddmin_u16x2((w >> 7) & 0x00FF00FFu, neg_left, kTop) & (kTop - 0x10001u);
+}
+
+// Eight codes (four words of encode_pair) as one group word, element 0 in the most significant bits.
+template <int N>
+__device__ __forceinline__ uint32_t join_codes(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t p3) {
+    constexpr uint32_t kStep = 1u << (2 * N);
+    const uint32_t u = p0 * kStep + p1, v = p2 * kStep + p3;       // low half: elements 0, 2 (4, 6), high half: 1, 3 (5, 7)
+    constexpr uint32_t kWeights = (1u << N) | (1u << 8);           // low half x 2**N + high half
+    return __dp2a_lo(v, kWeights, __dp2a_lo(u, kWeights, 0u) * (kStep * kStep));
+}

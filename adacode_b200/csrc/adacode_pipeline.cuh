@@ -141,24 +141,6 @@ __device__ __forceinline__ int warp_scan_counts(const int (&cnt)[kPCPT], int (&i
     return total;
 }
 
-// Exclusive prefix of this warp and the total over all consumer warps, from the per-warp totals
-// in shared memory: lane i reads warp i's total, one warp scan, two shuffles.
-template <int W = kPWarps>
-__device__ __forceinline__ void cross_warp_prefix(const int *warp_tot, int &prefix, int &total) {
-    static_assert(W <= 32, "one lane per consumer warp");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int x = lane < W ? warp_tot[lane] : 0;
-#pragma unroll
-    for (int d = 1; d < W; d <<= 1) {
-        const int u = __shfl_up_sync(kFull, x, d);
-        if (lane >= d) x += u;
-    }
-    total = __shfl_sync(kFull, x, W - 1);
-    const int incl = __shfl_sync(kFull, x, warp);
-    const int own = __shfl_sync(kFull, lane < W ? warp_tot[lane] : 0, warp);
-    prefix = incl - own;
-}
-
 // Rows of one tile handled per unit: whole rows, a multiple of 8 (so that code bytes per unit are a
 // multiple of 16), at most UNIT elements (D <= UNIT / 8).
 template <int UNIT = kUnitElems>
@@ -716,10 +698,8 @@ struct alignas(128) PackStageT {
 template <class G>
 struct alignas(128) PackSmemT {
     PackStageT<G> stage[kStages];
-    alignas(128) uint8_t sm[G::kUnit];
     alignas(128) uint8_t codes[G::kUnit / 2];
     alignas(128) uint8_t esc[G::kUnit];      // worst case: every element of a unit escapes
-    alignas(16) uint8_t lut[256];      // exponent -> code (0 = outside the window)
     alignas(16) PackUnitMeta meta_ring[2 * kStages];   // unit descriptions (see UnpackSmemT::meta_ring)
     alignas(8) uint64_t full[kStages];
     alignas(8) uint64_t empty[kStages];
@@ -926,14 +906,13 @@ __device__ __forceinline__ void flush_code_counts(uint32_t (&cnt2)[HistRegs<N>::
 template <int N, bool HIST, class G, bool FULL>
 __device__ __forceinline__ void pack_unit(PackSmemT<G> &s, const PackStageT<G> &st, const PackUnitMeta &m,
                                           uint64_t *empty_bar, int &running, uint32_t (&cnt2)[HistRegs<N>::v],
-                                          bool broken) {
+                                          uint32_t neg_left, bool broken) {
     constexpr int CB = 2 * N;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // (m lives in the description ring: its destination fields are read where the unit is stored)
     if (m.first_unit_of_tile) running = 0;
     const int chunks = FULL ? G::kUnit / 16 : m.elems >> 4;
 
-    uint4 smv[kPCPT];
     uint32_t g[kPCPT * 2], zm[kPCPT][2];
     int zc[kPCPT];
 #pragma unroll
@@ -947,28 +926,20 @@ __device__ __forceinline__ void pack_unit(PackSmemT<G> &s, const PackStageT<G> &
             w1 = p[1];
         }
         const uint32_t w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-        uint32_t smw[4];
-        uint32_t gg[2] = {0u, 0u};
+        uint32_t smw[4], pair[8];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            // four elements: their low bytes [e0 m6..m0] and high bytes [s e7..e1]
-            const uint32_t lo4 = __byte_perm(w[2 * q], w[2 * q + 1], 0x6420);
-            const uint32_t hi4 = __byte_perm(w[2 * q], w[2 * q + 1], 0x7531);
-            smw[q] = (hi4 & 0x80808080u) | (lo4 & 0x7F7F7F7Fu);
-            const uint32_t e4 = ((hi4 & 0x7F7F7F7Fu) << 1) | ((lo4 >> 7) & 0x01010101u);
+        for (int q = 0; q < 4; ++q)       // four elements: their low bytes [e0 m6..m0] and high bytes [s e7..e1]
+            smw[q] = bit_select(0x80808080u, __byte_perm(w[2 * q], w[2 * q + 1], 0x7531), __byte_perm(w[2 * q], w[2 * q + 1], 0x6420));
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t code = s.lut[__byte_perm(e4, 0u, 0x4440 | j)];     // byte j of e4; 0 when out of the window
-                const int el = 4 * q + j;
-                gg[el >> 3] = code * (1u << ((7 - (el & 7)) * N)) + gg[el >> 3];
-            }
-        }
+        for (int i = 0; i < 8; ++i) pair[i] = encode_pair<N>(w[i], neg_left);
+        const uint32_t gg[2] = {join_codes<N>(pair[0], pair[1], pair[2], pair[3]),
+                                join_codes<N>(pair[4], pair[5], pair[6], pair[7])};
         g[2 * k] = valid ? gg[0] : 0u;
         g[2 * k + 1] = valid ? gg[1] : 0u;
         zm[k][0] = valid ? zero_slots<N>(gg[0]) : 0u;
         zm[k][1] = valid ? zero_slots<N>(gg[1]) : 0u;
         zc[k] = __popc(zm[k][0]) + __popc(zm[k][1]);
-        smv[k] = make_uint4(smw[0], smw[1], smw[2], smw[3]);
+        if (valid && !broken) *reinterpret_cast<uint4 *>(m.sm_dst + c * 16) = make_uint4(smw[0], smw[1], smw[2], smw[3]);
     }
     if (HIST) {
         count_codes_overlaid<N, kPCPT * 2>(g, cnt2);
@@ -983,15 +954,15 @@ __device__ __forceinline__ void pack_unit(PackSmemT<G> &s, const PackStageT<G> &
     if (lane == 0) s.warp_tot[warp] = wtot;
     bulk_wait_read();      // the previous unit's stores have finished reading the out buffers
     consumer_sync<G::kConsumers>();
-    int wprefix, unit_tot;
-    cross_warp_prefix<G::kWarps>(s.warp_tot, wprefix, unit_tot);
+    const int others = s.warp_tot[lane & (G::kWarps - 1)];
+    const int wprefix = (int)__reduce_add_sync(kFull, (unsigned)(lane < warp ? others : 0));
+    const int unit_tot = (int)__reduce_add_sync(kFull, (unsigned)(lane < G::kWarps ? others : 0));
     static_assert(kPCPT == 2, "the escape loop below walks the two chunks of a thread together");
     const int c0 = warp * (kPCPT * 32) + lane;
 #pragma unroll
     for (int k = 0; k < kPCPT; ++k) {
         const int c = c0 + k * 32;
         if (FULL || c < chunks) {
-            *reinterpret_cast<uint4 *>(s.sm + c * 16) = smv[k];
             const uint32_t gg[2] = {g[2 * k], g[2 * k + 1]};
             store_chunk_codes<N, 16>(s.codes + c * CB, gg);
         }
@@ -1020,7 +991,6 @@ __device__ __forceinline__ void pack_unit(PackSmemT<G> &s, const PackStageT<G> &
     running += unit_tot;
     if (tid == 0 && !broken) {
         if (m.elems > 0) {
-            bulk_store(m.sm_dst, s.sm, (uint32_t)m.elems);
             bulk_store(m.code_dst, s.codes, (uint32_t)m.elems * N / 8);
             if (unit_tot > 0) bulk_store(m.esc_dst, s.esc, (uint32_t)((unit_tot + 15) & ~15));
             bulk_commit();
@@ -1136,8 +1106,7 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const 
         const int job = s.meta_ring[it % (2 * kStages)].job;
         if (job != cur_job) {
             // Uniform over the CTA (every consumer reads the same sequence of units): hand the finished
-            // job's histogram over and build the new job's code table.  The previous unit ended with
-            // a consumer barrier, so nobody still encodes with the old table.
+            // job's histogram over.
             if (HIST && cur_job >= 0) flush_code_counts<N>(cnt2, cur_left, s.hist);
             consumer_sync<G::kConsumers>();
             if (HIST && cur_job >= 0 && tid < 256) {
@@ -1147,17 +1116,14 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const 
             }
             cur_job = job;
             cur_left = pa.job[job].left;
-            if (tid < 256) {
-                const uint32_t code = (uint32_t)tid - (uint32_t)cur_left;
-                s.lut[tid] = (uint8_t)(code > ((1u << N) - 1u) ? 0u : code);
-            }
             consumer_sync<G::kConsumers>();
         }
+        const uint32_t neg_left = ((uint32_t)(-cur_left) & 0xFFFFu) * 0x10001u;
         for (;;) {
             const int stg = it % kStages;
             const PackUnitMeta &meta = s.meta_ring[it % (2 * kStages)];
-            if (meta.elems == G::kUnit) pack_unit<N, HIST, G, true>(s, s.stage[stg], meta, &s.empty[stg], running, cnt2, broken);
-            else pack_unit<N, HIST, G, false>(s, s.stage[stg], meta, &s.empty[stg], running, cnt2, broken);
+            if (meta.elems == G::kUnit) pack_unit<N, HIST, G, true>(s, s.stage[stg], meta, &s.empty[stg], running, cnt2, neg_left, broken);
+            else pack_unit<N, HIST, G, false>(s, s.stage[stg], meta, &s.empty[stg], running, cnt2, neg_left, broken);
             // the per-thread counters are 16-bit fields and grow by at most 32 per unit
             if (HIST && (it & 1023u) == 1023u) flush_code_counts<N>(cnt2, cur_left, s.hist);
             if (++it >= my_units) break;

@@ -885,6 +885,14 @@ int launch_pack_pipe(PackPipeArgs &pa, int nbits, cudaStream_t st) {
         hist = hist || pa.job[j].hist != nullptr;
         max_blocks = pa.job[j].n_blocks > max_blocks ? pa.job[j].n_blocks : max_blocks;
     }
+    // one warp per tile; few enough CTAs that the final per-bin atomics of the histogram stay cheap
+    const int64_t job_tiles = (int64_t)max_blocks * pa.BH;
+    const int64_t want = (job_tiles + kWarps - 1) / kWarps;
+    const int64_t cap = ((int64_t)sm_count() * 4 + pa.n_jobs - 1) / pa.n_jobs;
+    const dim3 cgrid((unsigned)(want < cap ? want : cap), (unsigned)pa.n_jobs);
+    // The compaction's CTAs find their tiles' offsets themselves as long as each can add up all counts
+    // before its tiles and has a thread for each of them; beyond that the pack kernel's last CTA scans.
+    pa.scan_in_pack = pa.n_tiles > kSumTiles || job_tiles > (int64_t)cgrid.x * kThreads;
     int rc;
     switch (nbits + (narrow ? 4 : 0)) {
         case 1: rc = launch_pack_pipe_n<1, WideGeom>(pa, hist, st); break;
@@ -897,11 +905,6 @@ int launch_pack_pipe(PackPipeArgs &pa, int nbits, cudaStream_t st) {
         default: rc = launch_pack_pipe_n<4, NarrowGeom>(pa, hist, st); break;
     }
     if (rc != ADACODE_OK) return rc;
-    // one warp per tile; few enough CTAs that the final per-bin atomics of the histogram stay cheap
-    const int64_t job_tiles = (int64_t)max_blocks * pa.BH;
-    const int64_t want = (job_tiles + kWarps - 1) / kWarps;
-    const int64_t cap = ((int64_t)sm_count() * 4 + pa.n_jobs - 1) / pa.n_jobs;
-    const dim3 cgrid((unsigned)(want < cap ? want : cap), (unsigned)pa.n_jobs);
     // (a programmatic dependent of the pack kernel: it is set up, and clears its histogram copies, while
     // the pack kernel's last CTAs still run)
     return hist ? launch_dependent(k_compact_units<true>, cgrid, kThreads, 0, st, pa)

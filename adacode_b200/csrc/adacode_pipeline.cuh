@@ -738,6 +738,7 @@ struct PackPipeArgs {
     int64_t *blk_off;         // over all blocks of the launch: escapes before global block i (n_blocks_total + 1)
     unsigned int *done;       // zero on entry, zero on exit
     int unit_rows, units_per_tile;
+    int scan_in_pack;         // offsets by the pack kernel's last CTA (else by the compaction's CTAs)
     int32_t *status;
     uint32_t poll_limit;      // bound of every on-chip wait (kMaxPolls unless a test lowered it)
 };
@@ -1142,6 +1143,7 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const 
     bulk_wait_all();
     // the compaction pass may be set up from here on (it waits for this launch to complete before it reads)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!pa.scan_in_pack) return;
     __threadfence();
     consumer_sync<G::kConsumers>();
     if (tid == 0) {
@@ -1214,8 +1216,65 @@ __device__ __forceinline__ void compact_tile_units(const PackPipeArgs &pa, const
     }
 }
 
+// Offsets of the escapes of tiles [lt0, lt0 + n) of a job (n <= kThreads), by the whole CTA: their inclusive
+// counts inside the segment and the segments' offsets go to the caller's arrays, s_off[i] is tile lt0 + i's
+// first byte in the job's stream and s_cnt[i] its count.  Every CTA adds up all the counts before its own
+// tiles: with at most kSumTiles of them that is a microsecond of reads from L2, while one CTA that
+// scans them alone keeps the others waiting.  Keys and values in one launch, 3 bits: [16, 8, 8192, 128] (16 384 tiles)
+// 209.8 -> 193.3 us, [1, 8, 20480, 128] (2560 tiles) 43.4 -> 39.1 us, one block of [1, 8, 128, 128] 14.2 -> 10.4 us.
+constexpr int64_t kSumTiles = 65536;
+
+__device__ __forceinline__ void tile_offsets(const PackPipeArgs &pa, const PackJob &jb, int lt0, int n, int *s_off, int *s_cnt,
+                                             int *s_red) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int seg0 = lt0 / pa.BH, seg0_tile = seg0 * pa.BH;
+    const int first = (int)jb.tile0, mid = first + seg0_tile, last = first + lt0;
+    // counts before segment seg0 and from there to lt0, four at a time (the array starts on a 256-byte boundary)
+    int before_seg = 0, in_seg = 0;
+#pragma unroll 4
+    for (int v = (first >> 2) + tid; v < (last + 3) >> 2; v += kThreads) {
+        const int4 q = __ldcg(reinterpret_cast<const int4 *>(pa.tile_counts) + v);
+        const int c[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = 4 * v + i;
+            before_seg += t >= first && t < mid ? c[i] : 0;
+            in_seg += t >= mid && t < last ? c[i] : 0;
+        }
+    }
+    const int c = tid < n ? __ldcg(pa.tile_counts + last + tid) : 0;
+    int incl = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int u = __shfl_up_sync(kFull, incl, d);
+        if (lane >= d) incl += u;
+    }
+    before_seg = (int)__reduce_add_sync(kFull, (unsigned)before_seg);
+    in_seg = (int)__reduce_add_sync(kFull, (unsigned)in_seg);
+    if (lane == 31) s_red[warp] = before_seg, s_red[kWarps + warp] = in_seg, s_red[2 * kWarps + warp] = incl;
+    __syncthreads();
+    int seg_start = 0, start = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+        seg_start += s_red[w];
+        start += s_red[w] + s_red[kWarps + w];
+        if (w < warp) incl += s_red[2 * kWarps + w];
+    }
+    const int off = start + incl - c;                     // escapes of the job before tile lt0 + tid
+    s_off[tid] = off;
+    s_cnt[tid] = c;
+    __syncthreads();
+    if (tid < n) {
+        const int lt = lt0 + tid, seg = lt / pa.BH;
+        const int at = seg == seg0 ? seg_start : s_off[seg * pa.BH - lt0];
+        jb.tile_base[lt] = off + c - at;
+        if (lt - seg * pa.BH == pa.BH - 1) jb.seg_off[seg + 1] = (int64_t)(off + c);
+        if (lt == 0) jb.seg_off[0] = 0;
+    }
+}
+
 // Gather every unit's escape bytes from its scratch slot into the compact per-segment stream.
-// Tile t of global block i starts at blk_off[i] - blk_off[first block of the job] + tile_base[t] -
+// With scan_in_pack tile t of global block i starts at blk_off[i] - blk_off[first block of the job] + tile_base[t] -
 // count[t] in its job's stream.  blockIdx.y is the job; one warp per tile; all of a tile's metadata
 // is fetched with independent loads (one memory round trip).
 // With HIST the escaped exponents are counted here (whole warps of escape bytes) rather than one
@@ -1236,18 +1295,30 @@ __global__ void __launch_bounds__(kThreads) k_compact_units(const __grid_constan
     // launched as a programmatic dependent of the pack kernel: nothing that kernel wrote is read above
     asm volatile("griddepcontrol.wait;" ::: "memory");
     int *my_hist = &s_hist[HIST ? warp : 0][HIST ? (lane & 3) : 0][0];
-    const int64_t warp_global = (int64_t)blockIdx.x * kWarps + warp;
-    const int64_t n_warps = (int64_t)gridDim.x * kWarps;
     const int64_t job_tiles = (int64_t)jb.n_blocks * pa.BH;
-    const int64_t job_off = __ldg(pa.blk_off + jb.blk0);
-    for (int64_t lt = warp_global; lt < job_tiles; lt += n_warps) {
-        const int64_t t = jb.tile0 + lt;
-        // independent loads: one round trip
-        const int c = __ldg(pa.tile_counts + t);
-        const int tb = __ldg(jb.tile_base + lt);
-        const int64_t so = __ldg(pa.blk_off + t / pa.BH) - job_off;
-        if (c == 0) continue;
-        compact_tile_units(pa, jb, t, so + tb - c, c, my_hist, do_hist);
+    if (!pa.scan_in_pack) {
+        __shared__ int s_off[kThreads], s_cnt[kThreads], s_red[3 * kWarps];
+        const int per = (int)((job_tiles + gridDim.x - 1) / gridDim.x);
+        const int64_t lt0 = (int64_t)blockIdx.x * per;
+        const int n = (int)(job_tiles - lt0 < per ? job_tiles - lt0 : per);
+        if (n > 0) {                                       // (uniform over the CTA)
+            tile_offsets(pa, jb, (int)lt0, n, s_off, s_cnt, s_red);
+            for (int i = warp; i < n; i += kWarps)
+                if (s_cnt[i] != 0) compact_tile_units(pa, jb, jb.tile0 + lt0 + i, s_off[i], s_cnt[i], my_hist, do_hist);
+        }
+    } else {
+        const int64_t warp_global = (int64_t)blockIdx.x * kWarps + warp;
+        const int64_t n_warps = (int64_t)gridDim.x * kWarps;
+        const int64_t job_off = __ldg(pa.blk_off + jb.blk0);
+        for (int64_t lt = warp_global; lt < job_tiles; lt += n_warps) {
+            const int64_t t = jb.tile0 + lt;
+            // independent loads: one round trip
+            const int c = __ldg(pa.tile_counts + t);
+            const int tb = __ldg(jb.tile_base + lt);
+            const int64_t so = __ldg(pa.blk_off + t / pa.BH) - job_off;
+            if (c == 0) continue;
+            compact_tile_units(pa, jb, t, so + tb - c, c, my_hist, do_hist);
+        }
     }
     if (do_hist) {
         __syncthreads();

@@ -84,3 +84,22 @@ def test_histogram_of_any_view(cuda_device, shape):
         got = codec.exponent_hist(t).cpu().numpy()
         e = (t.contiguous().view(torch.int16).cpu().numpy().astype(np.int64) >> 7) & 0xFF
         assert np.array_equal(got, np.bincount(e.ravel(), minlength=256))
+
+
+@pytest.mark.parametrize('B,H,blocks,D', [(1, 1, 1, 128), (1, 3, 1, 64), (3, 1, 333, 16), (1, 5, 2400, 16), (2, 4, 8193, 16)])
+def test_offsets_of_many_tiles(cuda_device, B, H, blocks, D):
+    """Escape offsets of two tensors of one launch, from one tile up to 131 088 (two tensors of 65 544 tiles: beyond what
+    the compaction's CTAs add up themselves), against sums of the tiles' own counts; then the round trip."""
+    from adacode_b200 import codec
+    g = torch.Generator(device=cuda_device).manual_seed(blocks)
+    k, v = (torch.randn(B, H, blocks * 128, D, generator=g, device=cuda_device).to(torch.bfloat16) for _ in range(2))
+    chunks = codec.pack_pair(k, v, (127, 3), (126, 3), 128)[:2]
+    for x, c, right in zip((k, v), chunks, (127, 126)):
+        e = (x.view(torch.int16).to(torch.int32) >> 7) & 0xFF
+        out = ((e <= right - 7) | (e > right)).view(B, H, blocks, 128 * D).sum(-1).permute(2, 0, 1).reshape(blocks, B * H)
+        assert torch.equal(c.tile_base.long(), out.cumsum(1))
+        assert torch.equal(c.seg_offsets_dev, torch.cat([torch.zeros_like(out[:1, 0]), out.sum(1).cumsum(0)]))
+        back = torch.empty_like(x)
+        codec.unpack_chunk(c, back)
+        assert torch.equal(_bits(back), _bits(x))
+    codec.check_device_status(cuda_device)

@@ -29,7 +29,7 @@ EXPORTED_SYMBOLS = (
     'adacode_pack_tiles', 'adacode_unpack_tiles', 'adacode_unpack_segments', 'adacode_hist_bf16',
     'adacode_choose_params', 'adacode_choose_params_host', 'adacode_calibrate_host', 'adacode_pack_tiles_static',
     'adacode_decode_attn_workspace_bytes', 'adacode_decode_attn', 'adacode_copy_to_host',
-    'adacode_pack_jobs', 'adacode_unpack_jobs', 'adacode_max_jobs', 'adacode_debug_set_wait_limit',
+    'adacode_pack_jobs', 'adacode_unpack_jobs', 'adacode_unpack_jobs_with_rows', 'adacode_copy_rows', 'adacode_max_jobs', 'adacode_debug_set_wait_limit',
     'adacode_flat_block_elems', 'adacode_unpack_flat',
 )
 
@@ -60,6 +60,16 @@ class UnpackJob(ctypes.Structure):
         ('segments_dev', ctypes.c_void_p), ('n_segments', ctypes.c_int32), ('reserved', ctypes.c_int32),
         ('dst_bf16', ctypes.c_void_p), ('dstride_b', ctypes.c_int64), ('dstride_h', ctypes.c_int64),
         ('dstride_s', ctypes.c_int64),
+    ]
+
+
+class RowCopy(ctypes.Structure):
+    """``struct adacode_row_copy``."""
+    _fields_ = [
+        ('src_bf16', ctypes.c_void_p), ('dst_bf16', ctypes.c_void_p),
+        ('src_b', ctypes.c_int64), ('src_h', ctypes.c_int64), ('src_s', ctypes.c_int64),
+        ('dst_b', ctypes.c_int64), ('dst_h', ctypes.c_int64), ('dst_s', ctypes.c_int64),
+        ('B', ctypes.c_int32), ('H', ctypes.c_int32), ('rows', ctypes.c_int32), ('D', ctypes.c_int32),
     ]
 
 
@@ -124,6 +134,10 @@ def lib() -> ctypes.CDLL:
     L.adacode_pack_jobs.argtypes = [vp, i32, i32, i32, i32, i32, i32, vp, sz, vp, vp]
     L.adacode_unpack_jobs.restype = i32
     L.adacode_unpack_jobs.argtypes = [vp, i32, i32, i32, i32, i32, vp, vp]
+    L.adacode_unpack_jobs_with_rows.restype = i32
+    L.adacode_unpack_jobs_with_rows.argtypes = [vp, i32, i32, i32, i32, i32, vp, i32, vp, vp]
+    L.adacode_copy_rows.restype = i32
+    L.adacode_copy_rows.argtypes = [vp, i32, vp]
     _lib = L
     return L
 

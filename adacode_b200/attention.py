@@ -20,7 +20,8 @@ from typing import Optional, Sequence
 import torch
 
 from . import _lib
-from .codec import _scratch_for, _stream_ptr, build_segment_table
+from .codec import _scratch_for, build_segment_table
+from .rows import on_device, stream_ptr
 
 _SEQ_TILE = 128
 _MAX_SPLITS = 128
@@ -100,12 +101,12 @@ def decode_attention(query: torch.Tensor, key_segments: Sequence, value_segments
     elif out.dtype != torch.bfloat16 or tuple(out.shape) != (B, Hq, D) or not out.is_contiguous():
         raise ValueError('out must be a contiguous bf16 [B, Hq, D] tensor')
     tb, th, ts = (key_tail.stride()[:3] if tail_len else (0, 0, 0))
-    with torch.cuda.device(dev):
+    with on_device(dev):
         rc = L.adacode_decode_attn(
             q.data_ptr(), q.stride(0), q.stride(1),
             key_table.data_ptr() if n_seg else None, value_table.data_ptr() if n_seg else None, n_seg,
             key_tail.data_ptr() if tail_len else None, value_tail.data_ptr() if tail_len else None, tail_len,
             tb, th, ts, B, Hq, Hkv, _SEQ_TILE, D, float(scale), out.data_ptr(), ws.data_ptr(), ws.numel(),
-            int(n_splits), sc.status.data_ptr(), _stream_ptr(dev))
+            int(n_splits), sc.status.data_ptr(), stream_ptr(dev))
     _lib.check(rc, 'adacode_decode_attn')
     return out.unsqueeze(2) if squeeze else out

@@ -17,6 +17,7 @@ from typing import Any, Optional, Sequence
 import torch
 
 from . import _lib
+from .rows import on_device, stream_ptr
 
 _SUPPORTED_TILE_NBITS = (1, 2, 3, 4)
 _DEFAULT_TILE_NBITS = 3
@@ -59,10 +60,6 @@ def _scratch_for(device: torch.device) -> _DeviceScratch:
     return s
 
 
-def _stream_ptr(device: torch.device) -> int:
-    return int(torch.cuda.current_stream(device).cuda_stream)
-
-
 def read_back(t: torch.Tensor):
     """Host copy (numpy array of ``t``'s shape and dtype) of a small device tensor.
 
@@ -80,7 +77,7 @@ def read_back(t: torch.Tensor):
     if sc.mailbox is None or sc.mailbox.numel() < nbytes:
         sc.mailbox = torch.empty(max(1 << 16, nbytes), dtype=torch.uint8).pin_memory()
     stream = torch.cuda.current_stream(dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         rc = _lib.lib().adacode_copy_to_host(t.data_ptr(), sc.mailbox.data_ptr(), nbytes, int(stream.cuda_stream))
     if rc == _lib.ERR_INVALID_ARG:
         return t.cpu().numpy()           # pinned memory this device cannot address: plain copy
@@ -372,12 +369,12 @@ def _pack_launch(p: _PendingPack, capacity: int, hist_t) -> torch.Tensor:
     ws = sc.workspace_for(n_tiles, p.seq_tile * p.D)
     esc = torch.empty(capacity, dtype=torch.uint8, device=p.dev)
     sb, sh, ss, _ = p.x.stride()
-    with torch.cuda.device(p.dev):
+    with on_device(p.dev):
         rc = _lib.lib().adacode_pack_tiles(
             p.x.data_ptr(), sb, sh, ss, p.B, p.H, p.n_blocks, p.seq_tile, p.D, p.right, p.nbits,
             p.sign_mant.data_ptr(), p.codes.data_ptr(), esc.data_ptr(), capacity, p.tile_base.data_ptr(),
             p.meta.data_ptr(), 0 if hist_t is None else hist_t.data_ptr(), ws.data_ptr(), ws.numel(),
-            p.meta.data_ptr() + 8 * (p.n_blocks + 1), _stream_ptr(p.dev))
+            p.meta.data_ptr() + 8 * (p.n_blocks + 1), stream_ptr(p.dev))
     _lib.check(rc, 'adacode_pack_tiles')
     return esc
 
@@ -400,10 +397,10 @@ def _pack_launch_jobs(ps: Sequence[_PendingPack]) -> None:
         jb.escapes_capacity = p.cap
         jb.tile_base, jb.seg_escape_offsets = p.tile_base.data_ptr(), p.meta.data_ptr()
         jb.hist256 = 0 if p.hist is None else p.hist.data_ptr()
-    with torch.cuda.device(dev):
+    with on_device(dev):
         rc = _lib.lib().adacode_pack_jobs(
             ctypes.addressof(jobs), len(ps), first.B, first.H, first.seq_tile, first.D, first.nbits,
-            ws.data_ptr(), ws.numel(), first.meta.data_ptr() + 8 * (first.n_blocks + 1), _stream_ptr(dev))
+            ws.data_ptr(), ws.numel(), first.meta.data_ptr() + 8 * (first.n_blocks + 1), stream_ptr(dev))
     _lib.check(rc, 'adacode_pack_jobs')
 
 
@@ -411,7 +408,7 @@ def pack_blocks_finish(p: _PendingPack, host_meta):
     """Finish a launch given the host copy of its ``meta`` (int64[n_blocks + 2]): re-run with the
     exact capacity if the escape buffer was too small, trim it, build the ``PackedChunk``."""
     n_blocks = p.n_blocks
-    offsets = [int(v) for v in host_meta[: n_blocks + 1]]
+    offsets = host_meta[: n_blocks + 1].tolist()
     total = offsets[-1]
     status = int(host_meta[n_blocks + 1]) & 0xFFFFFFFF
     escapes = p.escapes
@@ -495,11 +492,11 @@ def unpack_chunk(chunk: PackedChunk, dst: torch.Tensor, seq_offset: int = 0) -> 
     view = dst[:, :, seq_offset:]
     db, dh, ds, _ = dst.stride()
     seg_off = chunk.seg_offsets_dev
-    with torch.cuda.device(dev):
+    with on_device(dev):
         rc = _lib.lib().adacode_unpack_tiles(
             chunk.sign_mant.data_ptr(), chunk.codes.data_ptr(), chunk.escapes.data_ptr(), chunk.escapes.numel(),
             chunk.tile_base.data_ptr(), seg_off.data_ptr(), B, H, chunk.n_blocks, T, D,
-            chunk.left, chunk.nbits, view.data_ptr(), db, dh, ds, sc.status.data_ptr(), _stream_ptr(dev))
+            chunk.left, chunk.nbits, view.data_ptr(), db, dh, ds, sc.status.data_ptr(), stream_ptr(dev))
     _lib.check(rc, 'adacode_unpack_tiles')
 
 
@@ -619,19 +616,29 @@ def unpack_segments(segments: Sequence[TiledCompressedTensor], dst: torch.Tensor
         return
     first = segments[0]
     B, H, T, D = first.original_shape
-    for seg in segments:
-        if tuple(seg.original_shape) != (B, H, T, D):
-            raise ValueError('all segments of one call must share [batch, kv_heads, seq_tile, head_dim]')
+    _check_one_shape(segments, (B, H, T, D))
     _check_dst(dst, B, H, D, 0)
     dev = dst.device
     sc = _scratch_for(dev)
     if table is None:
         table = build_segment_table(segments, seq_offsets, dev)
     db, dh, ds, _ = dst.stride()
-    with torch.cuda.device(dev):
+    with on_device(dev):
         rc = _lib.lib().adacode_unpack_segments(table.data_ptr(), len(segments), B, H, T, D, dst.data_ptr(),
-                                                db, dh, ds, sc.status.data_ptr(), _stream_ptr(dev))
+                                                db, dh, ds, sc.status.data_ptr(), stream_ptr(dev))
     _lib.check(rc, 'adacode_unpack_segments')
+
+
+def _check_one_shape(segs: Sequence, shape0: tuple) -> None:
+    """Refuse segments of another [batch, kv_heads, seq_tile, head_dim]; segments of one chunk have one shape."""
+    chunk = None
+    for seg in segs:
+        if type(seg) is SegmentRef:
+            if seg.chunk is chunk:
+                continue
+            chunk = seg.chunk
+        if tuple(seg.original_shape) != shape0:
+            raise ValueError('all segments of one call must share [batch, kv_heads, seq_tile, head_dim]')
 
 
 def unpack_segments_multi(jobs: Sequence[tuple]) -> None:
@@ -648,26 +655,54 @@ def unpack_segments_multi(jobs: Sequence[tuple]) -> None:
         for segs, dst, table in jobs:
             unpack_segments(segs, dst, table=table)
         return
-    B, H, T, D = shape0
+    _unpack_with_rows([(segs, dst, table, None) for segs, dst, table in jobs], shape0)
+
+
+def _unpack_with_rows(jobs: Sequence[tuple], shape: tuple) -> None:
+    B, H, T, D = shape
     dev = jobs[0][1].device
-    sc = _scratch_for(dev)
-    arr = (_lib.UnpackJob * len(jobs))()
-    keep = []
-    for rec, (segs, dst, table) in zip(arr, jobs):
-        for seg in segs:
-            if tuple(seg.original_shape) != shape0:
-                raise ValueError('all segments of one call must share [batch, kv_heads, seq_tile, head_dim]')
+    records, rows, keep = [], [], []
+    for segs, dst, table, row in jobs:
+        _check_one_shape(segs, shape)
         _check_dst(dst, B, H, D, 0)
         if table is None:
             table = build_segment_table(segs, None, dev)
         keep.append(table)
         db, dh, ds, _ = dst.stride()
-        rec.segments_dev, rec.n_segments = table.data_ptr(), len(segs)
-        rec.dst_bf16, rec.dstride_b, rec.dstride_h, rec.dstride_s = dst.data_ptr(), db, dh, ds
-    with torch.cuda.device(dev):
-        rc = _lib.lib().adacode_unpack_jobs(ctypes.addressof(arr), len(jobs), B, H, T, D, sc.status.data_ptr(),
-                                            _stream_ptr(dev))
-    _lib.check(rc, 'adacode_unpack_jobs')
+        records.append((table.data_ptr(), len(segs), 0, dst.data_ptr(), db, dh, ds))
+        if row is not None:
+            rows.append(row)
+    arr = (_lib.UnpackJob * len(records))(*records)
+    row_arr = (_lib.RowCopy * len(rows))(*rows) if rows else None
+    with on_device(dev):
+        rc = _lib.lib().adacode_unpack_jobs_with_rows(
+            ctypes.addressof(arr), len(records), B, H, T, D, None if row_arr is None else ctypes.addressof(row_arr),
+            len(rows), _scratch_for(dev).status.data_ptr(), stream_ptr(dev))
+    _lib.check(rc, 'adacode_unpack_jobs_with_rows')
+
+
+def unpack_with_tails(parts: Sequence[tuple], prefix: int, rows: int) -> None:
+    """Dense keys and values of one layer: for every ``(segments, table, dense, tail)`` the segments are unpacked into
+    the front of the contiguous ``dense`` [B, H, prefix + rows, D] and the first ``rows`` tokens of ``tail``
+    [B, H, capacity, D] copied behind them, in one launch for parts of one shape."""
+    jobs = []
+    for segs, table, dense, tail in parts:
+        row = None
+        if rows:
+            B, H, _, D = dense.shape
+            if tail.shape[0] != B or tail.shape[1] != H or tail.shape[3] != D or tail.shape[2] < rows:
+                raise ValueError(f'tail {tuple(tail.shape)} does not fit {tuple(dense.shape)}')
+            if tail.device != dense.device or tail.dtype != torch.bfloat16 or tail.stride(3) != 1:
+                raise ValueError('tail must be a bf16 tensor with unit stride along head_dim on the device of the dense one')
+            db, dh, ds, _ = dense.stride()
+            row = (tail.data_ptr(), dense.data_ptr() + 2 * prefix * ds, *tail.stride()[:3], db, dh, ds, B, H, rows, D)
+        jobs.append((segs, dense, table, row))
+    shapes = [tuple(p[0][0].original_shape) for p in parts]
+    if all(s == shapes[0] for s in shapes):
+        _unpack_with_rows(jobs, shapes[0])
+    else:
+        for job, shape in zip(jobs, shapes):
+            _unpack_with_rows([job], shape)
 
 
 def exponent_hist(x: torch.Tensor, hist_out: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -679,8 +714,8 @@ def exponent_hist(x: torch.Tensor, hist_out: Optional[torch.Tensor] = None) -> t
     hist = hist_out if hist_out is not None else torch.zeros(256, dtype=torch.int32, device=dev)
     B, H, S, D = x.shape
     sb, sh, ss, _ = x.stride()
-    with torch.cuda.device(dev):
-        rc = _lib.lib().adacode_hist_bf16(x.data_ptr(), sb, sh, ss, B, H, S, D, hist.data_ptr(), _stream_ptr(dev))
+    with on_device(dev):
+        rc = _lib.lib().adacode_hist_bf16(x.data_ptr(), sb, sh, ss, B, H, S, D, hist.data_ptr(), stream_ptr(dev))
     _lib.check(rc, 'adacode_hist_bf16')
     return hist
 
@@ -694,8 +729,8 @@ def choose_params_device(hists: torch.Tensor) -> torch.Tensor:
     dev = h.device
     _scratch_for(dev)
     out = torch.empty((h.shape[0], 2), dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
-        rc = _lib.lib().adacode_choose_params(h.data_ptr(), h.shape[0], out.data_ptr(), _stream_ptr(dev))
+    with on_device(dev):
+        rc = _lib.lib().adacode_choose_params(h.data_ptr(), h.shape[0], out.data_ptr(), stream_ptr(dev))
     _lib.check(rc, 'adacode_choose_params')
     return out
 

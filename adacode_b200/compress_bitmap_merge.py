@@ -14,6 +14,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib, codec
+from .rows import on_device, stream_ptr
 
 _BLOCK_GAPS = (8, 4, 8, 2)
 _MAX_ELEMS_PER_CALL = 1 << 30
@@ -187,9 +188,9 @@ class CompressorBitMap:
         dev = self.device
         sc = codec._scratch_for(dev)
         esc = self.invalid_exp
-        stream = codec._stream_ptr(dev)
+        stream = stream_ptr(dev)
         L = _lib.lib()
-        with torch.cuda.device(dev):
+        with on_device(dev):
             if n_whole:
                 rc = L.adacode_unpack_flat(self.sign_mass_data.data_ptr(), self.exp_data.data_ptr(),
                                            esc.data_ptr() if esc.numel() else 0, esc.numel(),

@@ -843,6 +843,7 @@ int launch_unpack_pipe(const UnpackPipeArgs &a, cudaStream_t st) {
     ja.job[0] = a;
     ja.tile0[0] = 0, ja.tile0[1] = a.n_tiles;
     ja.n_jobs = 1;
+    ja.rows.n = 0;
     return launch_unpack_pipe(ja, st);
 }
 
@@ -915,6 +916,39 @@ template <int N, int CH>
 void launch_pack(const PackArgs &a, int grid, cudaStream_t st) {
     if (a.hist) k_pack<N, CH, true><<<grid, kThreads, 0, st>>>(a);
     else k_pack<N, CH, false><<<grid, kThreads, 0, st>>>(a);
+}
+
+// Rows alone: a few kilobytes as a rule (a token's keys and values), bound by the launch.
+__global__ void __launch_bounds__(kThreads) k_copy_rows(const __grid_constant__ RowCopies rc) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    copy_rows(rc.copy[blockIdx.y], blockIdx.x * kThreads + threadIdx.x, gridDim.x * kThreads);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Copies that have anything to move, checked.
+int take_rows(const adacode_row_copy *copies, int n_copies, RowCopies &rc, int64_t &most) {
+    if (n_copies < 0 || n_copies > kMaxJobs || (n_copies > 0 && !copies)) return ADACODE_ERR_INVALID_ARG;
+    rc.n = 0;
+    most = 0;
+    for (int i = 0; i < n_copies; ++i) {
+        const adacode_row_copy &c = copies[i];
+        if (c.B < 0 || c.H < 0 || c.rows < 0 || c.D < 0 || c.D % 8 != 0) return ADACODE_ERR_INVALID_ARG;
+        if ((int64_t)c.B * c.H == 0 || c.rows == 0 || c.D == 0) continue;
+        if (!c.src_bf16 || !c.dst_bf16 || (((uintptr_t)c.src_bf16 | (uintptr_t)c.dst_bf16) & 15) != 0 ||
+            ((c.src_b | c.src_h | c.src_s | c.dst_b | c.dst_h | c.dst_s) & 7) != 0)
+            return ADACODE_ERR_INVALID_ARG;
+        const int64_t bh = (int64_t)c.B * c.H, row_vec = (int64_t)c.rows * (c.D / 8);
+        if (bh >= (1ll << 31) || row_vec >= (1ll << 31) || bh * row_vec >= (1ll << 31)) return ADACODE_ERR_TOO_LARGE;
+        most = bh * row_vec > most ? bh * row_vec : most;
+        rc.copy[rc.n++] = c;
+    }
+    return ADACODE_OK;
+}
+
+int launch_copy_rows(const RowCopies &rc, int64_t most, cudaStream_t st) {
+    if (rc.n == 0) return ADACODE_OK;
+    const int64_t want = (most + kThreads - 1) / kThreads, cap = (int64_t)sm_count() * 8;
+    return launch_dependent(k_copy_rows, dim3((unsigned)(want < cap ? want : cap), (unsigned)rc.n), kThreads, 0, st, rc);
 }
 
 // Word-wise copy of a small device buffer into host memory that the device can address (pinned
@@ -1256,8 +1290,20 @@ int adacode_unpack_flat(const uint8_t *sign_mant, const uint8_t *codes, const ui
     return ADACODE_OK;
 }
 
+int adacode_copy_rows(const adacode_row_copy *copies, int n_copies, void *stream) {
+    RowCopies rc;
+    int64_t most;
+    const int ok = take_rows(copies, n_copies, rc, most);
+    return ok != ADACODE_OK ? ok : launch_copy_rows(rc, most, (cudaStream_t)stream);
+}
+
 int adacode_unpack_jobs(const adacode_unpack_job *jobs, int n_jobs, int B, int H, int seq_tile, int D,
                         int32_t *status, void *stream) {
+    return adacode_unpack_jobs_with_rows(jobs, n_jobs, B, H, seq_tile, D, nullptr, 0, status, stream);
+}
+
+int adacode_unpack_jobs_with_rows(const adacode_unpack_job *jobs, int n_jobs, int B, int H, int seq_tile, int D,
+                                  const adacode_row_copy *copies, int n_copies, int32_t *status, void *stream) {
     if (n_jobs < 0 || n_jobs > kMaxJobs || (n_jobs > 0 && !jobs)) return ADACODE_ERR_INVALID_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     const bool pipe = pipeline_enabled() && pipeline_shape_ok(seq_tile, D);
@@ -1265,6 +1311,9 @@ int adacode_unpack_jobs(const adacode_unpack_job *jobs, int n_jobs, int B, int H
     memset(&ja, 0, sizeof(ja));
     int n = 0;
     long long tile0 = 0;
+    int64_t most;
+    const int rows_ok = take_rows(copies, n_copies, ja.rows, most);
+    if (rows_ok != ADACODE_OK) return rows_ok;
     for (int j = 0; j < n_jobs; ++j) {
         const adacode_unpack_job &jb = jobs[j];
         if (jb.n_segments < 0) return ADACODE_ERR_INVALID_ARG;
@@ -1288,7 +1337,7 @@ int adacode_unpack_jobs(const adacode_unpack_job *jobs, int n_jobs, int B, int H
         tile0 += n_tiles;
         ++n;
     }
-    if (!pipe || n == 0) return ADACODE_OK;
+    if (!pipe || n == 0) return launch_copy_rows(ja.rows, most, st);
     ja.tile0[n] = tile0;
     ja.n_jobs = n;
     return launch_unpack_pipe(ja, st);

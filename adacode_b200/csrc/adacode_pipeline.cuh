@@ -498,9 +498,29 @@ __device__ __forceinline__ uint32_t unpack_run(UnpackSmemT<G> &s, uint32_t it, u
 
 constexpr int kMaxJobs = 8;
 
+// A dense copy of bf16 rows (adacode_row_copy), by `n_workers` threads of which this is `worker`.
+__device__ __forceinline__ void copy_rows(const adacode_row_copy &c, uint32_t worker, uint32_t n_workers) {
+    const uint32_t vec = (uint32_t)c.D / 8, rows = (uint32_t)c.rows;
+    const uint32_t total = (uint32_t)c.B * (uint32_t)c.H * rows * vec;      // (checked by the host: below 2**31)
+#pragma unroll 2
+    for (uint32_t i = worker; i < total; i += n_workers) {
+        const uint32_t r = i / vec, v = i - r * vec, bh = r / rows, t = r - bh * rows;
+        const uint32_t b = bh / (uint32_t)c.H, h = bh - b * (uint32_t)c.H;
+        const uint16_t *src = (const uint16_t *)c.src_bf16 + b * c.src_b + h * c.src_h + t * c.src_s;
+        uint16_t *dst = (uint16_t *)c.dst_bf16 + b * c.dst_b + h * c.dst_h + t * c.dst_s;
+        reinterpret_cast<uint4 *>(dst)[v] = reinterpret_cast<const uint4 *>(src)[v];
+    }
+}
+
+struct RowCopies {
+    adacode_row_copy copy[kMaxJobs];
+    int n;
+};
+
 // Up to kMaxJobs destinations in one launch; job j owns the tiles [tile0[j], tile0[j + 1]).
 struct UnpackJobsArgs {
     UnpackPipeArgs job[kMaxJobs];
+    RowCopies rows;           // dense rows that go along
     long long tile0[kMaxJobs + 1];
     int n_jobs;
     uint32_t poll_limit;      // bound of every on-chip wait (kMaxPolls unless a test lowered it)
@@ -578,6 +598,9 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_unpack_pipe(cons
     }
 
     // ---------------- consumer warps ----------------
+    // the dense rows first, while the first units are on their way
+    for (int j = 0; j < ja.rows.n; ++j)
+        copy_rows(ja.rows.copy[j], blockIdx.x * (uint32_t)G::kConsumers + tid, gridDim.x * (uint32_t)G::kConsumers);
     int consumed = 0;
     bool broken = false;                  // a wait of this warp ran out: compute on, store nothing
     // row and column of this thread's chunks inside a unit (a chunk never crosses a row: D % 16 == 0)

@@ -34,6 +34,7 @@ from transformers import Cache
 from transformers.cache_utils import DynamicLayer
 
 from . import codec
+from .rows import copy_rows
 from .codec import SegmentRef, TiledCompressedTensor
 
 _SUPPORTED_LAYOUTS = ('segmented_tiled', 'legacy', 'tiled')
@@ -117,9 +118,14 @@ class _Residual:
         q = int(states.shape[-2])
         if q == 0:
             return
-        self._reserve(states, self.length + q, block)
-        self.buf[:, :, self.length: self.length + q].copy_(states)
+        copy_rows([(states, self.room(states, block))])
         self.length += q
+
+    def room(self, states: torch.Tensor, block: int) -> torch.Tensor:
+        """Where ``states`` goes, behind the tail; they belong to it once they are copied and counted."""
+        q = int(states.shape[-2])
+        self._reserve(states, self.length + q, block)
+        return self.buf[:, :, self.length: self.length + q]
 
     def drop_front(self, count: int) -> None:
         """Forget the first ``count`` tokens, moving what follows to the front."""
@@ -342,8 +348,11 @@ class float11Layer(DynamicLayer):
         return self._res_k.tensor(), self._res_v.tensor()
 
     def _append_residual(self, key_states: torch.Tensor, value_states: torch.Tensor) -> None:
-        self._res_k.append(key_states, self.block_size)
-        self._res_v.append(value_states, self.block_size)
+        new = [(states, res) for states, res in ((key_states, self._res_k), (value_states, self._res_v))
+               if int(states.shape[-2]) > 0]
+        copy_rows([(states, res.room(states, self.block_size)) for states, res in new])
+        for states, res in new:
+            res.length += int(states.shape[-2])
 
     @staticmethod
     def _extract_exponent_histogram(states: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -615,37 +624,44 @@ class float11Layer(DynamicLayer):
         return outs[0], outs[1]
 
     def _materialize_into_workspace(self):
-        res_k, res_v = self._active_residual_tensors()
-        res_len = 0 if res_k is None else int(res_k.shape[-2])
+        res_len = self._res_k.length if self._res_k.buf is not None else 0
         prefix = self._compressed_prefix_seq_len
         total = prefix + res_len
-        outs = []
+        outs, tails = [], []
+        pairs = (('k', self._key_segments, self._res_k), ('v', self._value_segments, self._res_v))
         if self.dense_workspace == 'shared':
-            # keys and values are decoded by one launch when they have one shape
-            todo = []
-            for which, segs in (('k', self._key_segments), ('v', self._value_segments)):
+            # keys, values and the tails behind them are written by one launch when keys and values have one shape
+            parts = []
+            for which, segs, res in pairs:
                 B, H, _, D = segs[0].original_shape
                 dense = self._workspace.view(self.cache_device, which, (B, H, total, D))
-                todo.append((segs, dense, self._segment_table(which, segs)))
-            codec.unpack_segments_multi(todo)
-        for i, (which, segs, res) in enumerate((('k', self._key_segments, res_k), ('v', self._value_segments, res_v))):
-            B, H, _, D = segs[0].original_shape
-            if self.dense_workspace == 'shared':
-                dense = todo[i][1]
+                parts.append((segs, self._segment_table(which, segs), dense, res.buf))
+                outs.append(dense)
+            if all(dense.is_cuda and (not res_len or (tail.device == dense.device and not tail.requires_grad))
+                   for _, _, dense, tail in parts):
+                codec.unpack_with_tails(parts, prefix, res_len)
             else:
-                # per-layer mirror: lossless packing never changes a token's bits, so whatever was
-                # written once stays valid; only blocks not yet present are decoded
-                mirror = self._layer_mirror(which, (B, H, D), total)
-                done = self._mirror_valid[which]
-                if done < prefix:
-                    first = done // self.seq_tile_size
-                    offs = [i * self.seq_tile_size for i in range(first, len(segs))]
-                    codec.unpack_segments(segs[first:], mirror, seq_offsets=offs)
-                dense = mirror[:, :, :total]
-                self._mirror_valid[which] = total
+                codec.unpack_segments_multi([(segs, dense, table) for segs, table, dense, _ in parts])
+                if res_len:
+                    for _, _, dense, tail in parts:
+                        dense[:, :, prefix:total].copy_(tail[:, :, :res_len])
+            return outs[0], outs[1]
+        for which, segs, res in pairs:
+            B, H, _, D = segs[0].original_shape
+            # per-layer mirror: lossless packing never changes a token's bits, so whatever was
+            # written once stays valid; only blocks not yet present are decoded
+            mirror = self._layer_mirror(which, (B, H, D), total)
+            done = self._mirror_valid[which]
+            if done < prefix:
+                first = done // self.seq_tile_size
+                offs = [i * self.seq_tile_size for i in range(first, len(segs))]
+                codec.unpack_segments(segs[first:], mirror, seq_offsets=offs)
+            dense = mirror[:, :, :total]
+            self._mirror_valid[which] = total
             if res_len:
-                dense[:, :, prefix:total].copy_(res)
+                tails.append((res.tensor(), dense[:, :, prefix:total]))
             outs.append(dense)
+        copy_rows(tails)
         return outs[0], outs[1]
 
     def _layer_mirror(self, which: str, bhd: tuple, total: int) -> torch.Tensor:

@@ -233,6 +233,24 @@ typedef struct adacode_unpack_job {
 int adacode_unpack_jobs(const adacode_unpack_job *jobs, int n_jobs, int B, int H, int seq_tile, int D,
                         int32_t *status, void *stream);
 
+/* A dense copy of bf16 rows: dst[b][h][t][:] = src[b][h][t][:] for b < B, h < H, t < rows, D elements each (D % 8 == 0).
+ * Pointers on 16-byte boundaries, strides multiples of 8 elements; source and destination do not overlap. */
+typedef struct adacode_row_copy {
+    const void *src_bf16;
+    void *dst_bf16;
+    int64_t src_b, src_h, src_s;
+    int64_t dst_b, dst_h, dst_s;
+    int32_t B, H, rows, D;
+} adacode_row_copy;
+
+/* Up to adacode_max_jobs() row copies in one launch (a token's keys and values appended to the
+ * residual: Tensor.copy_ twice, float_cache_utils.py:860-881).  `copies` is host memory. */
+int adacode_copy_rows(const adacode_row_copy *copies, int n_copies, void *stream);
+
+/* adacode_unpack_jobs and adacode_copy_rows (the not yet packed tails behind the segments) in ONE launch. */
+int adacode_unpack_jobs_with_rows(const adacode_unpack_job *jobs, int n_jobs, int B, int H, int seq_tile, int D,
+                                  const adacode_row_copy *copies, int n_copies, int32_t *status, void *stream);
+
 /* Elements per escape-base block of the flat layout for a code length: 128 * {8, 4, 8, 2}[nbits - 1]
  * (compress_bitmap_merge.py:653-657, invalid_block_size); 0 for an invalid nbits. */
 int adacode_flat_block_elems(int nbits);

@@ -483,121 +483,6 @@ __global__ void __launch_bounds__(kThreads) k_unpack_segments(const UnpackCommon
 // histogram and adjuster
 // ---------------------------------------------------------------------------------------
 
-// Exponent histogram.  One shared-memory atomic per element on a histogram that a warp shares costs the
-// conflicts of 32 lanes on the few exponents that nearly all elements have.  Here every lane counts in
-// bytes of its own: 64 words per lane, word (e & 63) of lane l in bank l, byte e >> 6 of it, so that
-// 32 lanes never meet in a bank whatever the exponents are.  A lane's bytes are added up over the warp
-// before they can overflow (kHistUnits units of 32 elements a lane).
-//
-// The source is `runs` contiguous pieces of `run_vec` 16-byte vectors (the host merges dimensions, see
-// flatten_runs); a warp takes units of kHistVec x 32 vectors of one run, and loads the next unit
-// while it counts the current one.  SHORT: runs too short for that are walked vector by vector.
-constexpr int kHistVec = 4;
-constexpr int kHistUnits = 7;                                  // 7 * 32 = 224 <= 255
-
-struct HistRuns {
-    const uint16_t *src;
-    int64_t runs, run_vec;
-    int64_t n1, n0;              // run r -> (r / (n1 n0), r / n0 % n1, r % n0)
-    int64_t s2, s1, s0;          // element strides of those indices
-    int32_t *hist;
-};
-
-__device__ __forceinline__ const uint4 *hist_run(const HistRuns &a, uint32_t r) {
-    const uint32_t q = r / (uint32_t)a.n0, i0 = r - q * (uint32_t)a.n0;
-    const uint32_t i2 = q / (uint32_t)a.n1, i1 = q - i2 * (uint32_t)a.n1;
-    return reinterpret_cast<const uint4 *>(a.src + i2 * a.s2 + i1 * a.s1 + i0 * a.s0);
-}
-
-__device__ __forceinline__ void hist_count(uint32_t *mine, uint32_t w) {
-    // exponent of the low bf16: bits 7..14 (the word's row) and 13..14 (its byte)
-    const uint32_t v = w >> 16;
-    atomicAdd(mine + ((w & 0x1F80u) >> 2), 1u << ((w >> 10) & 0x18u));
-    atomicAdd(mine + ((v & 0x1F80u) >> 2), 1u << ((v >> 10) & 0x18u));
-}
-
-// Add the byte counters of a warp (64 rows of 32 words) to the CTA's histogram and clear them.
-__device__ __forceinline__ void hist_flush(uint32_t *rows, int *s_hist) {
-    const int lane = threadIdx.x & 31;
-    __syncwarp();
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-        const int r = half * 32 + lane;
-        uint32_t lo = 0, hi = 0;                               // bytes 0 and 2, bytes 1 and 3: 16-bit sums (32 * 224 fit)
-#pragma unroll 8
-        for (int k = 0; k < 32; ++k) {
-            const uint32_t v = rows[r * 32 + ((lane + k) & 31)];
-            lo += v & 0x00FF00FFu;
-            hi += (v >> 8) & 0x00FF00FFu;
-        }
-        const uint32_t c[4] = {lo & 0xFFFFu, hi & 0xFFFFu, lo >> 16, hi >> 16};
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-            if (c[b] != 0) atomicAdd(&s_hist[b * 64 + r], (int)c[b]);
-    }
-    __syncwarp();
-    for (int i = lane; i < 512; i += 32) reinterpret_cast<uint4 *>(rows)[i] = make_uint4(0, 0, 0, 0);
-    __syncwarp();
-}
-
-template <bool SHORT>
-__global__ void __launch_bounds__(kThreads) k_hist(const __grid_constant__ HistRuns a) {
-    extern __shared__ __align__(16) uint32_t s_rows[];         // [warp][64][32]
-    __shared__ int s_hist[256];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < kWarps * 512; i += kThreads) reinterpret_cast<uint4 *>(s_rows)[i] = make_uint4(0, 0, 0, 0);
-    s_hist[tid] = 0;
-    __syncthreads();
-    uint32_t *rows = s_rows + warp * 2048, *mine = rows + lane;
-    int pending = 0;
-    if constexpr (SHORT) {
-        const int64_t n_vec = a.runs * a.run_vec;
-        for (int64_t base = ((int64_t)blockIdx.x * kWarps + warp) * 32; base < n_vec; base += (int64_t)gridDim.x * kThreads) {
-            const int64_t i = base + lane;
-            if (i < n_vec) {
-                const int64_t r = i / a.run_vec, q = r / a.n0, i2 = q / a.n1;
-                const uint16_t *run = a.src + i2 * a.s2 + (q - i2 * a.n1) * a.s1 + (r - q * a.n0) * a.s0;
-                const uint4 v = reinterpret_cast<const uint4 *>(run)[i - r * a.run_vec];
-                hist_count(mine, v.x), hist_count(mine, v.y), hist_count(mine, v.z), hist_count(mine, v.w);
-            }
-            if (++pending == kHistUnits * kHistVec) hist_flush(rows, s_hist), pending = 0;
-        }
-    } else {
-        const uint32_t run_vec = (uint32_t)a.run_vec, per_run = (run_vec + 32 * kHistVec - 1) / (32 * kHistVec);
-        const uint32_t units = (uint32_t)a.runs * per_run, step = gridDim.x * kWarps;
-        uint4 cur[kHistVec], nxt[kHistVec];
-        // (a lane beyond the end of its run loads nothing and counts nothing: `have` says how many it has)
-        const auto load = [&](uint32_t u, uint4 (&v)[kHistVec]) {
-            int have = 0;
-            if (u < units) {
-                const uint32_t r = u / per_run, at = (u - r * per_run) * (32 * kHistVec) + lane;
-                const uint4 *p = hist_run(a, r) + at;
-#pragma unroll
-                for (int k = 0; k < kHistVec; ++k)
-                    if (at + 32 * k < run_vec) v[k] = __ldg(p + 32 * k), ++have;
-            }
-            return have;
-        };
-        uint32_t u = blockIdx.x * kWarps + warp;
-        int have = load(u, cur);
-        while (u < units) {
-            u += step;
-            const int have_next = load(u, nxt);
-#pragma unroll
-            for (int k = 0; k < kHistVec; ++k)
-                if (k < have) hist_count(mine, cur[k].x), hist_count(mine, cur[k].y), hist_count(mine, cur[k].z), hist_count(mine, cur[k].w);
-#pragma unroll
-            for (int k = 0; k < kHistVec; ++k) cur[k] = nxt[k];
-            have = have_next;
-            if (++pending == kHistUnits) hist_flush(rows, s_hist), pending = 0;
-        }
-    }
-    if (pending > 0) hist_flush(rows, s_hist);
-    __syncthreads();
-    const int total = s_hist[tid];
-    if (total != 0) atomicAdd(a.hist + tid, total);
-}
-
 // One warp per histogram: fifteen rounds of "largest remaining count, lowest bin on ties"
 // reproduce a stable descending sort's first fifteen entries.
 __global__ void k_choose_params(const int32_t *__restrict__ hists, int n_hists, int32_t *__restrict__ out) {
@@ -657,6 +542,156 @@ __global__ void k_choose_params(const int32_t *__restrict__ hists, int n_hists, 
 }
 
 #include "adacode_pipeline.cuh"
+
+// Exponent histogram.  Nearly all exponents of a tensor lie in a window of fifteen, so they are counted as the
+// pack kernel counts its codes: four-bit codes against a window that each warp takes from the first values
+// it sees, one population count per subset of the code bits over 32 elements (count_codes_overlaid), and one
+// shared-memory atomic for each of the few elements outside.  The window only decides the speed.
+// [16, 8, 8192, 128] (268 MB): one atomic per element on bins shared by a warp 113 us, byte counters of each lane's own
+// 97 us (an atomic of 32 lanes in 32 banks still takes several cycles), this 81 us (3.3 TB/s, bound by the integer
+// pipe); three CTAs per SM 87 us.  One block of [1, 8, 128, 128]: 6.3 -> 4.3 us.
+//
+// The source is `runs` contiguous pieces of `run_vec` 16-byte vectors (the host merges dimensions, see
+// flatten_runs); a warp takes units of kHistVec x 32 vectors of one run, and loads the next unit
+// while it counts the current one.  SHORT: runs too short for that are walked vector by vector.
+constexpr int kHistVec = 4;
+constexpr int kHistBits = 4;
+constexpr int kHistFlush = 1024;                               // units between flushes of the 16-bit counters
+constexpr int kHistCtas = 4;                                   // per SM
+constexpr int kHistCopies = 4;                                 // of the bins that the atomics go to, by lane
+
+struct HistRuns {
+    const uint16_t *src;
+    int64_t runs, run_vec;
+    int64_t n1, n0;              // run r -> (r / (n1 n0), r / n0 % n1, r % n0)
+    int64_t s2, s1, s0;          // element strides of those indices
+    int32_t *hist;
+};
+
+__device__ __forceinline__ const uint4 *hist_run(const HistRuns &a, uint32_t r) {
+    const uint32_t q = r / (uint32_t)a.n0, i0 = r - q * (uint32_t)a.n0;
+    const uint32_t i2 = q / (uint32_t)a.n1, i1 = q - i2 * (uint32_t)a.n1;
+    return reinterpret_cast<const uint4 *>(a.src + i2 * a.s2 + i1 * a.s1 + i0 * a.s0);
+}
+
+struct HistState {
+    uint32_t cnt[HistRegs<kHistBits>::v];
+    uint32_t neg_left;
+    int left, units;             // units: since the last flush; -1: no window yet
+};
+
+// Count the first `have` of V vectors of this lane (V * 8 elements at most); `scratch`: V vectors per lane.
+template <int V>
+__device__ __forceinline__ void hist_count(HistState &st, const uint4 (&v)[V], int have, uint4 *scratch, int *s_hist) {
+    const int lane = threadIdx.x & 31;
+    if (st.units < 0) {
+        // the window ends at the largest finite exponent among this unit's first vectors
+        uint32_t m = 0;
+        if (have > 0) {
+            const uint32_t w[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t e0 = (w[i] >> 7) & 0xFFu, e1 = (w[i] >> 23) & 0xFFu;
+                m = max(m, max(e0 == 255u ? 0u : e0, e1 == 255u ? 0u : e1));
+            }
+        }
+        st.left = (int)__reduce_max_sync(kFull, m) - ((1 << kHistBits) - 1);
+        st.neg_left = ((uint32_t)(-st.left) & 0xFFFFu) * 0x10001u;
+        st.units = 0;
+    }
+    uint32_t g[V], todo = 0;
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+        const uint32_t c = join_codes<kHistBits>(
+            encode_pair<kHistBits>(v[k].x, st.neg_left), encode_pair<kHistBits>(v[k].y, st.neg_left),
+            encode_pair<kHistBits>(v[k].z, st.neg_left), encode_pair<kHistBits>(v[k].w, st.neg_left));
+        g[k] = k < have ? c : 0u;
+        const uint32_t z = k < have ? compress_slots<kHistBits>(zero_slots<kHistBits>(c)) : 0u;
+        todo |= z << (24 - 8 * k);                             // element 0 in the most significant bit
+    }
+    count_codes_overlaid<kHistBits, V>(g, st.cnt);
+    bump_field<kHistBits>(st.cnt, 0, (uint32_t)(8 * have));
+    bump_field<kHistBits>(st.cnt, (1 << kHistBits) - 1, (uint32_t)__popc(todo));
+    if (__any_sync(kFull, todo != 0)) {
+#pragma unroll
+        for (int k = 0; k < V; ++k) scratch[k * 32 + lane] = v[k];
+        const uint16_t *mine = reinterpret_cast<const uint16_t *>(scratch + lane);
+        int *bins = s_hist + (lane & (kHistCopies - 1)) * 256;
+        while (todo) {
+            const int i = __clz((int)todo);
+            todo &= ~(0x80000000u >> i);
+            atomicAdd(&bins[(mine[(i >> 3) * 256 + (i & 7)] >> 7) & 0xFFu], 1);      // (a vector is 8 elements, a row of them 256)
+        }
+    }
+    if (++st.units == kHistFlush) {
+        flush_code_counts<kHistBits>(st.cnt, st.left, s_hist);
+        st.units = 0;
+    }
+}
+
+template <bool SHORT>
+__global__ void __launch_bounds__(kThreads, kHistCtas) k_hist(const __grid_constant__ HistRuns a) {
+    constexpr int V = SHORT ? 1 : kHistVec;
+    __shared__ uint4 s_scratch[kWarps][V * 32];
+    __shared__ int s_hist[kHistCopies * 256];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < kHistCopies * 256; i += kThreads) s_hist[i] = 0;
+    __syncthreads();
+    uint4 *scratch = s_scratch[warp];
+    HistState st;
+#pragma unroll
+    for (int i = 0; i < HistRegs<kHistBits>::v; ++i) st.cnt[i] = 0;
+    st.neg_left = 0, st.left = 0, st.units = -1;
+    if constexpr (SHORT) {
+        const int64_t n_vec = a.runs * a.run_vec;
+        for (int64_t base = ((int64_t)blockIdx.x * kWarps + warp) * 32; base < n_vec; base += (int64_t)gridDim.x * kThreads) {
+            const int64_t i = base + lane;
+            uint4 v[1] = {make_uint4(0, 0, 0, 0)};
+            if (i < n_vec) {
+                const int64_t r = i / a.run_vec, q = r / a.n0, i2 = q / a.n1;
+                const uint16_t *run = a.src + i2 * a.s2 + (q - i2 * a.n1) * a.s1 + (r - q * a.n0) * a.s0;
+                v[0] = reinterpret_cast<const uint4 *>(run)[i - r * a.run_vec];
+            }
+            hist_count(st, v, i < n_vec ? 1 : 0, scratch, s_hist);
+        }
+    } else {
+        const uint32_t run_vec = (uint32_t)a.run_vec, per_run = (run_vec + 32 * kHistVec - 1) / (32 * kHistVec);
+        const uint32_t units = (uint32_t)a.runs * per_run, step = gridDim.x * kWarps;
+        uint4 cur[kHistVec], nxt[kHistVec];
+        // (a lane beyond the end of its run loads nothing and counts nothing: `have` says how many it has)
+        const auto load = [&](uint32_t u, uint4 (&v)[kHistVec]) {
+            int have = 0;
+            if (u < units) {
+                const uint32_t r = u / per_run, at = (u - r * per_run) * (32 * kHistVec) + lane;
+                const uint4 *p = hist_run(a, r) + at;
+#pragma unroll
+                for (int k = 0; k < kHistVec; ++k)
+                    if (at + 32 * k < run_vec) v[k] = __ldg(p + 32 * k), ++have;
+            }
+            return have;
+        };
+#pragma unroll
+        for (int k = 0; k < kHistVec; ++k) cur[k] = nxt[k] = make_uint4(0, 0, 0, 0);
+        uint32_t u = blockIdx.x * kWarps + warp;
+        int have = load(u, cur);
+        while (u < units) {
+            // (units + step stays below 2**32: both are below 2**31)
+            u += step;
+            const int have_next = load(u, nxt);
+            hist_count(st, cur, have, scratch, s_hist);
+#pragma unroll
+            for (int k = 0; k < kHistVec; ++k) cur[k] = nxt[k];
+            have = have_next;
+        }
+    }
+    if (st.units > 0) flush_code_counts<kHistBits>(st.cnt, st.left, s_hist);
+    __syncthreads();
+    int total = 0;
+#pragma unroll
+    for (int i = 0; i < kHistCopies; ++i) total += s_hist[i * 256 + tid];
+    if (total != 0) atomicAdd(a.hist + tid, total);
+}
+
 
 void stable_order_desc(const int64_t *hist, int *order) {
     for (int i = 0; i < 256; ++i) order[i] = i;
@@ -1354,19 +1389,12 @@ int adacode_hist_bf16(const void *src_bf16, int64_t stride_b, int64_t stride_h, 
     a.src = (const uint16_t *)src_bf16, a.hist = hist256;
     // Runs shorter than half a warp's unit leave most of its lanes idle, and 32-bit indices must do.
     const bool by_vector = a.run_vec < 16 * kHistVec || a.runs * a.run_vec >= (1ll << 31);
-    const size_t smem = (size_t)kWarps * 64 * 32 * 4;
     const int64_t units = by_vector ? (a.runs * a.run_vec + 31) / 32
                                     : a.runs * ((a.run_vec + 32 * kHistVec - 1) / (32 * kHistVec));
-    const int64_t want = (units + kWarps - 1) / kWarps, cap = (int64_t)sm_count() * 3;
+    const int64_t want = (units + kWarps - 1) / kWarps, cap = (int64_t)sm_count() * kHistCtas;
     const int blocks = (int)(want < cap ? want : cap);
-    int rc;
-    if (by_vector) {
-        if ((rc = ensure_dynamic_smem(k_hist<true>, smem)) != ADACODE_OK) return rc;
-        k_hist<true><<<blocks, kThreads, smem, (cudaStream_t)stream>>>(a);
-    } else {
-        if ((rc = ensure_dynamic_smem(k_hist<false>, smem)) != ADACODE_OK) return rc;
-        k_hist<false><<<blocks, kThreads, smem, (cudaStream_t)stream>>>(a);
-    }
+    if (by_vector) k_hist<true><<<blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
+    else k_hist<false><<<blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
     ADACODE_CUDA_TRY(cudaGetLastError());
     return ADACODE_OK;
 }

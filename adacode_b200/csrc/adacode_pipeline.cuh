@@ -1026,7 +1026,7 @@ __device__ __forceinline__ void pack_unit(PackSmemT<G> &s, const PackStageT<G> &
 
 template <int N, bool HIST, class G>
 __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const __grid_constant__ PackPipeArgs pa) {
-    static_assert(G::kConsumers >= 256, "the 256-entry tables are filled by one consumer thread per entry");
+    static_assert(G::kConsumers >= 256, "one consumer thread per histogram bin");
     extern __shared__ __align__(128) uint8_t smem_raw[];
     PackSmemT<G> &s = *reinterpret_cast<PackSmemT<G> *>(smem_raw);
     const int tid = threadIdx.x;

@@ -322,8 +322,11 @@ class _PendingPack:
         self.__dict__.update(kw)
 
 
-def _default_escape_capacity(n: int) -> int:
-    return min(max(4096, n // 8), max(n, 1))
+def _default_escape_capacity(n: int, nbits: int) -> int:
+    """Room for an eighth of the elements, more for the windows of one and of three exponents, of which a third to a
+    half of the elements fall outside: a buffer that is too small costs a second pack of the whole span."""
+    share = n // 8 if nbits > 2 else n // 2 if nbits == 2 else n
+    return min(max(4096, share), max(n, 1))
 
 
 def pack_blocks_launch(x: torch.Tensor, right: int, nbits: int, seq_tile: int = 128, need_hist: bool = False,
@@ -357,7 +360,8 @@ def pack_blocks_launch(x: torch.Tensor, right: int, nbits: int, seq_tile: int = 
     p.hist = None
     if need_hist:
         p.hist = hist_out if hist_out is not None else torch.zeros(256, dtype=torch.int32, device=dev)
-    p.cap = min(int(escape_capacity), max(n, 1)) if escape_capacity is not None else _default_escape_capacity(n)
+    p.guessed = escape_capacity is None
+    p.cap = min(int(escape_capacity), max(n, 1)) if escape_capacity is not None else _default_escape_capacity(n, int(nbits))
     if launch:
         p.escapes = _pack_launch(p, p.cap, p.hist)
     return p
@@ -423,7 +427,8 @@ def pack_blocks_finish(p: _PendingPack, host_meta):
             raise _lib.AdacodeError('adacode_pack_tiles: escape overflow after re-run with exact capacity')
     elif status_other:
         raise _lib.AdacodeError(f'adacode_pack_tiles: device status {status:#x} ({describe_status(status)})')
-    if escapes.numel() > 2 * total + 65536:
+    # (a large first guess is not kept: it is cut to size once an eighth of it is unused)
+    if escapes.numel() > (total + total // 8 if p.guessed and p.nbits <= 2 else 2 * total) + 65536:
         escapes = escapes[:total].clone()
     else:
         escapes = escapes[:total]

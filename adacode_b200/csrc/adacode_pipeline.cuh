@@ -393,7 +393,7 @@ __device__ __noinline__ uint2 gather_escapes(uint32_t z, int r, const uint8_t *e
 }
 
 // One unit: staged planes -> registers -> global memory.  The codes are expanded, the escapes placed
-// and the bf16 words put together in registers (about 6 instructions per element, see spread8), and
+// and the bf16 words put together in registers (see spread8), and
 // whole sectors are stored straight from there.  The only CTA-wide barrier is the one between the
 // escape counts of the warps and their sum.
 // Keys and values of [16, 8, 8192, 128] in one launch (537 M elements), with the lookups, the escape loop and the

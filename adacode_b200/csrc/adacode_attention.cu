@@ -292,32 +292,59 @@ __global__ void __launch_bounds__(kAttnThreads) k_decode_attn(const AttnArgs a) 
     }
 }
 
-// out[b][hq][d] = sum_s w_s o_s / sum_s w_s l_s, w_s = exp(m_s - max m)
-__global__ void k_decode_attn_combine(const float *__restrict__ part_o, const float *__restrict__ part_ml, int Hq,
-                                      int Hkv, int G, int D, int n_splits, uint16_t *__restrict__ out) {
+// out[b][hq][d] = sum_s w_s o_s / sum_s w_s l_s, w_s = exp(m_s - max m).  One CTA per query head, bound by the
+// latency of its reads: the weights of all splits are found at once, and the D columns are summed by
+// GROUPS groups of threads that share the splits.  [1, 8, 20480, 128] with 37 splits, attention and combine:
+// 47.3 us with one thread per column that walked all splits twice, 43.4 us with four groups.  Up to
+// kFewSplits splits the extra threads only cost ([16, 4, 4096, 64] with 16 heads per group, nine splits: 53.9 us
+// with one group, 57.0 us with eight).
+constexpr int kCombineThreads = 512;
+constexpr int kFewSplits = 16;
+constexpr int kMaxSplits = 128;
+
+template <int D, int GROUPS>
+__global__ void __launch_bounds__(GROUPS * D) k_decode_attn_combine(const float *__restrict__ part_o,
+                                                                         const float *__restrict__ part_ml, int Hq, int Hkv,
+                                                                         int G, int n_splits, uint16_t *__restrict__ out) {
+    __shared__ float s_w[kMaxSplits], s_den[kMaxSplits], s_num[GROUPS][D];
+    const int tid = threadIdx.x, lane = tid & 31;
     const int bhq = blockIdx.x;
     const int b = bhq / Hq, hq = bhq - b * Hq;
     const int hkv = hq / G, g = hq - hkv * G;
-    const int d = threadIdx.x;
-    if (d >= D) return;
+    const long long base = ((long long)b * Hkv + hkv) * n_splits;
     // launched as a programmatic dependent of the attention kernel: wait for its partial results
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const long long base = ((long long)b * Hkv + hkv) * n_splits;
     float mx = -INFINITY;
-    for (int sidx = 0; sidx < n_splits; ++sidx) mx = fmaxf(mx, part_ml[((base + sidx) * G + g) * 2]);
-    float num = 0.f, den = 0.f;
-    for (int sidx = 0; sidx < n_splits; ++sidx) {
-        const float ms = part_ml[((base + sidx) * G + g) * 2];
-        if (ms == -INFINITY) continue;
-        const float w = __expf(ms - mx);
-        num = fmaf(w, part_o[((base + sidx) * G + g) * D + d], num);
-        den = fmaf(w, part_ml[((base + sidx) * G + g) * 2 + 1], den);
+    for (int s = lane; s < n_splits; s += 32) mx = fmaxf(mx, part_ml[((base + s) * G + g) * 2]);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, d));
+    for (int s = tid; s < n_splits; s += GROUPS * D) {
+        const float m = part_ml[((base + s) * G + g) * 2], l = part_ml[((base + s) * G + g) * 2 + 1];
+        const float w = __expf(m - mx);
+        s_w[s] = m == -INFINITY ? -1.f : w;                // (negative: a split without tokens, not read)
+        s_den[s] = m == -INFINITY ? 0.f : w * l;
     }
-    const float r = den > 0.f ? num / den : 0.f;
-    // round to nearest even bf16
-    uint32_t u = __float_as_uint(r);
-    u += 0x7FFFu + ((u >> 16) & 1u);
-    out[(long long)bhq * D + d] = (uint16_t)(u >> 16);
+    __syncthreads();
+    const int d = tid % D, grp = tid / D;
+    float num = 0.f;
+#pragma unroll 4
+    for (int s = grp; s < n_splits; s += GROUPS) {
+        const float w = s_w[s];
+        if (!(w < 0.f)) num = fmaf(w, part_o[((base + s) * G + g) * D + d], num);
+    }
+    s_num[grp][d] = num;
+    __syncthreads();
+    if (tid < D) {
+        float n = 0.f, den = 0.f;
+#pragma unroll
+        for (int i = 0; i < GROUPS; ++i) n += s_num[i][tid];
+        for (int s = 0; s < n_splits; ++s) den += s_den[s];
+        const float r = den > 0.f ? n / den : 0.f;
+        // round to nearest even bf16
+        uint32_t u = __float_as_uint(r);
+        u += 0x7FFFu + ((u >> 16) & 1u);
+        out[(long long)bhq * D + tid] = (uint16_t)(u >> 16);
+    }
 }
 
 // =======================================================================================
@@ -812,6 +839,8 @@ __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_
             dense_slab(st, a.k_tail + toff + t0 * a.t_ss, a.v_tail + toff + t0 * a.t_ss, a.t_ss, valid, wide, sc2);
     }
 
+    // the combine kernel may be set up from here on (it waits for this launch to complete before it reads)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // ---------------- merge the warps ----------------
 #pragma unroll
     for (int h = 0; h < HG; ++h) {
@@ -874,8 +903,6 @@ __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_
 }
 
 static_assert(sizeof(AttnPipeSmem<128>) <= 113 * 1024, "two CTAs of the pipelined kernel must fit one SM");
-
-constexpr int kMaxSplits = 128;
 
 // Splits per (batch, KV head): the grid should fill a whole number of waves of resident CTAs
 // (two per SM).  One, two and three waves are
@@ -1006,8 +1033,11 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
         k_decode_attn<<<dim3(B * Hkv, n_splits, head_groups), kAttnThreads, sizeof(AttnSmem), st>>>(a);
     }
     if (cudaGetLastError() != cudaSuccess) return ADACODE_ERR_CUDA;
-    if (launch_as_dependent(k_decode_attn_combine, dim3(B * Hq), D, 0, st, (const float *)a.part_o,
-                            (const float *)a.part_ml, Hq, Hkv, G, D, n_splits, (uint16_t *)out_bf16) != cudaSuccess)
+    const bool few = n_splits <= kFewSplits;
+    auto combine = D == 128 ? (few ? k_decode_attn_combine<128, 1> : k_decode_attn_combine<128, kCombineThreads / 128>)
+                            : (few ? k_decode_attn_combine<64, 1> : k_decode_attn_combine<64, kCombineThreads / 64>);
+    if (launch_as_dependent(combine, dim3(B * Hq), few ? D : kCombineThreads, 0, st, (const float *)a.part_o,
+                            (const float *)a.part_ml, Hq, Hkv, G, n_splits, (uint16_t *)out_bf16) != cudaSuccess)
         return ADACODE_ERR_CUDA;
     return ADACODE_OK;
 }

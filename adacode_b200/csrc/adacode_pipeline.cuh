@@ -39,9 +39,7 @@ using WideGeom = PipeGeom<16, 2>;
 using NarrowGeom = PipeGeom<8, 4>;
 
 // the wide geometry under the names that the helpers default to
-constexpr int kPWarps = WideGeom::kWarps;
 constexpr int kConsumerThreads = WideGeom::kConsumers;
-constexpr int kPipeThreads = WideGeom::kThreads;
 constexpr int kUnitElems = WideGeom::kUnit;
 constexpr int kStages = 2;
 constexpr uint32_t kMaxPolls = 1u << 22;

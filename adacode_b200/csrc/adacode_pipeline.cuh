@@ -397,8 +397,8 @@ __device__ __noinline__ uint2 gather_escapes(uint32_t z, int r, const uint8_t *e
 // Keys and values of [16, 8, 8192, 128] in one launch (537 M elements), with the lookups, the escape loop and the
 // bulk store that were here before and now: n = 3, 5 % escapes 188.6 -> 177.7 us (5.2 TB/s, 81 % of what a plain
 // copy reaches), n = 2, 34 % escapes 340 -> 177 us, n = 4, 0.1 % escapes 169.7 -> 170.8 us; [1, 8, 20480, 128]
-// 38.8 -> 35.0 us.  The integer pipe is 64 % busy, issue slots 60 %; the rest is waiting at the barrier and for
-// loads.  Tried and slower: no producer warp (one warp in turn refills; the others wait for it at the next
+// 38.8 -> 35.0 us; 4 % less each since computed permutes go without the intrinsic's mask.  The integer pipe is
+// 67 % busy; the rest is waiting at the barrier and for loads.  Tried and slower: no producer warp (one warp in turn refills; the others wait for it at the next
 // barrier) 201 us; one tile per warp without shared memory or barriers 217-219 us; the finished unit through
 // shared memory and a bulk store, which leaves room for three CTAs per SM, 229 us; five CTAs per SM (spills) 223 us.
 template <int N, class G>

@@ -11,6 +11,7 @@
 // The reference has no such kernel (its attention path materialises dense K/V first; the module
 // its validation script imports, ops/kv_attention.py, is absent from its tree), so numerics are
 // checked against an fp32 PyTorch attention over the dense cache.
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -322,7 +323,7 @@ __global__ void __launch_bounds__(GROUPS * D) k_decode_attn_combine(const float 
         const float m = part_ml[((base + s) * G + g) * 2], l = part_ml[((base + s) * G + g) * 2 + 1];
         const float w = __expf(m - mx);
         s_w[s] = m == -INFINITY ? -1.f : w;                // (negative: a split without tokens, not read)
-        s_den[s] = m == -INFINITY ? 0.f : w * l;
+        s_den[s] = m == -INFINITY ? l : w * l;             // (without a maximum l is 0, or NaN if all scores are)
     }
     __syncthreads();
     const int d = tid % D, grp = tid / D;
@@ -339,11 +340,9 @@ __global__ void __launch_bounds__(GROUPS * D) k_decode_attn_combine(const float 
 #pragma unroll
         for (int i = 0; i < GROUPS; ++i) n += s_num[i][tid];
         for (int s = 0; s < n_splits; ++s) den += s_den[s];
-        const float r = den > 0.f ? n / den : 0.f;
-        // round to nearest even bf16
-        uint32_t u = __float_as_uint(r);
-        u += 0x7FFFu + ((u >> 16) & 1u);
-        out[(long long)bhq * D + tid] = (uint16_t)(u >> 16);
+        // (no weight at all, every score minus infinity: 0; a NaN score makes den NaN)
+        const float r = den == 0.f ? 0.f : n / den;
+        out[(long long)bhq * D + tid] = __bfloat16_as_ushort(__float2bfloat16_rn(r));
     }
 }
 
@@ -892,7 +891,7 @@ __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_
         for (int w = 1; w < kAWarps; ++w) mx = fmaxf(mx, s.m[w][tid]);
         float l = 0.f;
 #pragma unroll
-        for (int w = 0; w < kAWarps; ++w) l += s.m[w][tid] == -INFINITY ? 0.f : s.l[w][tid] * exp2f(s.m[w][tid] - mx);
+        for (int w = 0; w < kAWarps; ++w) l += s.m[w][tid] == -INFINITY ? s.l[w][tid] : s.l[w][tid] * exp2f(s.m[w][tid] - mx);
         a.part_ml[(slot * Gt + gz + tid) * 2 + 0] = mx == -INFINITY ? -INFINITY : mx / kLog2e;   // natural-log domain
         a.part_ml[(slot * Gt + gz + tid) * 2 + 1] = l;
     }

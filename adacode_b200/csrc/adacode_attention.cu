@@ -293,6 +293,66 @@ __global__ void __launch_bounds__(kAttnThreads) k_decode_attn(const AttnArgs a) 
     }
 }
 
+// The terms of a probability after the first may be 0 or negative (and weights may underflow), so a value that is
+// not finite leaves a sum that is not finite but not always the right one (0 x inf, inf - inf).  What is right follows from
+// the values alone: NaN for a NaN or for infinities of both signs, the infinity otherwise.  A warp of the combine
+// kernel that ends with such sums (`odd`, a column each) looks its columns up here; sums that overflowed stay.
+// A block whose window ends below 255 and whose escapes hold no 255 is done with its escape bytes.
+template <int D>
+__device__ __noinline__ void settle_columns(const AttnArgs &a, int bh, bool odd, unsigned *flags, uint16_t *out) {
+    const int lane = threadIdx.x & 31, d0 = threadIdx.x & ~31;
+    flags += d0;                                           // this warp's columns: bit 0 inf, bit 1 -inf, bit 2 NaN
+    flags[lane] = 0;
+    __syncwarp();
+    const auto note = [flags, d0](int d, bool negative, bool nan) {
+        if ((d & ~31) == d0) atomicOr(flags + (d - d0), nan ? 4u : negative ? 2u : 1u);
+    };
+    for (int t = 0; t < a.n_seg; ++t) {
+        const adacode_segment &sg = a.vseg[t];
+        const int nbits = sg.nbits;
+        int64_t rank = bh > 0 ? sg.tile_base[bh - 1] : 0;
+        int64_t end = sg.tile_base[bh];
+        if (end > sg.escapes_len) end = sg.escapes_len;
+        bool has = sg.left + (1 << nbits) - 1 >= 255;
+#pragma unroll 8
+        for (int64_t i = rank + lane; i < end; i += 32) has |= sg.escapes[i] == 255;
+        if (!__any_sync(kFull, has)) continue;
+        const uint8_t *sm = sg.sign_mant + (int64_t)bh * (kTileTokens * D);
+        const uint8_t *codes = sg.codes + (int64_t)bh * (kTileTokens * D / 8 * nbits);
+        for (int g = lane; g < kTileTokens * D / 8; g += 32) {           // groups of eight elements
+            uint32_t x = 0;
+            for (int i = 0; i < nbits; ++i) x = (x << 8) | codes[g * nbits + i];
+            int escapes = 0;
+            for (int k = 0; k < 8; ++k) escapes += ((x >> (k * nbits)) & ((1u << nbits) - 1)) == 0;
+            int incl = escapes;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int u = __shfl_up_sync(kFull, incl, d);
+                if (lane >= d) incl += u;
+            }
+            int64_t r = rank + incl - escapes;
+            for (int k = 0; k < 8; ++k) {
+                const uint32_t code = (x >> ((7 - k) * nbits)) & ((1u << nbits) - 1);
+                uint32_t e = (code + (uint32_t)sg.left) & 0xFFu;
+                if (code == 0) e = r < end ? sg.escapes[r] : 0u, ++r;
+                const uint8_t b = sm[g * 8 + k];
+                if (e == 255) note((g * 8 + k) % D, (b & 0x80) != 0, (b & 0x7F) != 0);
+            }
+            rank += __shfl_sync(kFull, incl, 31);
+        }
+    }
+    const int b = bh / a.Hkv, hkv = bh - b * a.Hkv;
+    const uint16_t *col = a.v_tail + b * a.t_sb + hkv * a.t_sh + d0 + lane;
+#pragma unroll 8
+    for (int t = 0; t < a.tail_len; ++t) {
+        const uint32_t v = col[t * a.t_ss];
+        if ((v & 0x7F80u) == 0x7F80u) note(d0 + lane, (v & 0x8000u) != 0, (v & 0x7Fu) != 0);
+    }
+    __syncwarp();
+    const unsigned f = flags[lane];
+    if (odd && f != 0) out[lane] = f == 1 ? 0x7F80 : f == 2 ? 0xFF80 : 0x7FFF;
+}
+
 // out[b][hq][d] = sum_s w_s o_s / sum_s w_s l_s, w_s = exp(m_s - max m).  One CTA per query head, bound by the
 // latency of its reads: the weights of all splits are found at once, and the D columns are summed by
 // GROUPS groups of threads that share the splits.  [1, 8, 20480, 128] with 37 splits, attention and combine:
@@ -304,15 +364,17 @@ constexpr int kFewSplits = 16;
 constexpr int kMaxSplits = 128;
 
 template <int D, int GROUPS>
-__global__ void __launch_bounds__(GROUPS * D) k_decode_attn_combine(const float *__restrict__ part_o,
-                                                                         const float *__restrict__ part_ml, int Hq, int Hkv,
-                                                                         int G, int n_splits, uint16_t *__restrict__ out) {
+__global__ void __launch_bounds__(GROUPS * D) k_decode_attn_combine(const __grid_constant__ AttnArgs a, uint16_t *__restrict__ out) {
     __shared__ float s_w[kMaxSplits], s_den[kMaxSplits], s_num[GROUPS][D];
+    __shared__ unsigned s_flags[D];
+    const float *__restrict__ part_o = a.part_o;
+    const float *__restrict__ part_ml = a.part_ml;
+    const int G = a.G, n_splits = a.n_splits;
     const int tid = threadIdx.x, lane = tid & 31;
     const int bhq = blockIdx.x;
-    const int b = bhq / Hq, hq = bhq - b * Hq;
-    const int hkv = hq / G, g = hq - hkv * G;
-    const long long base = ((long long)b * Hkv + hkv) * n_splits;
+    const int b = bhq / a.Hq, hq = bhq - b * a.Hq;
+    const int hkv = hq / G, g = hq - hkv * G, bh = b * a.Hkv + hkv;
+    const long long base = (long long)bh * n_splits;
     // launched as a programmatic dependent of the attention kernel: wait for its partial results
     asm volatile("griddepcontrol.wait;" ::: "memory");
     float mx = -INFINITY;
@@ -335,6 +397,7 @@ __global__ void __launch_bounds__(GROUPS * D) k_decode_attn_combine(const float 
     }
     s_num[grp][d] = num;
     __syncthreads();
+    float n = 0.f, den = 0.f;
     if (tid < D) {
         float n = 0.f, den = 0.f;
 #pragma unroll
@@ -343,6 +406,8 @@ __global__ void __launch_bounds__(GROUPS * D) k_decode_attn_combine(const float 
         // (no weight at all, every score minus infinity: 0; a NaN score makes den NaN)
         const float r = den == 0.f ? 0.f : n / den;
         out[(long long)bhq * D + tid] = __bfloat16_as_ushort(__float2bfloat16_rn(r));
+        const bool odd = !isfinite(n) && isfinite(den);
+        if (__any_sync(kFull, odd)) settle_columns<D>(a, bh, odd, s_flags, out + (long long)bhq * D + (tid & ~31));
     }
 }
 
@@ -1035,8 +1100,7 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
     const bool few = n_splits <= kFewSplits;
     auto combine = D == 128 ? (few ? k_decode_attn_combine<128, 1> : k_decode_attn_combine<128, kCombineThreads / 128>)
                             : (few ? k_decode_attn_combine<64, 1> : k_decode_attn_combine<64, kCombineThreads / 64>);
-    if (launch_as_dependent(combine, dim3(B * Hq), few ? D : kCombineThreads, 0, st, (const float *)a.part_o,
-                            (const float *)a.part_ml, Hq, Hkv, G, n_splits, (uint16_t *)out_bf16) != cudaSuccess)
+    if (launch_as_dependent(combine, dim3(B * Hq), few ? D : kCombineThreads, 0, st, a, (uint16_t *)out_bf16) != cudaSuccess)
         return ADACODE_ERR_CUDA;
     return ADACODE_OK;
 }

@@ -397,7 +397,6 @@ __global__ void __launch_bounds__(GROUPS * D) k_decode_attn_combine(const __grid
     }
     s_num[grp][d] = num;
     __syncthreads();
-    float n = 0.f, den = 0.f;
     if (tid < D) {
         float n = 0.f, den = 0.f;
 #pragma unroll

@@ -34,7 +34,6 @@ from transformers import Cache
 from transformers.cache_utils import DynamicLayer
 
 from . import codec
-from .rows import copy_rows
 from .codec import SegmentRef, TiledCompressedTensor
 
 _SUPPORTED_LAYOUTS = ('segmented_tiled', 'legacy', 'tiled')
@@ -118,14 +117,9 @@ class _Residual:
         q = int(states.shape[-2])
         if q == 0:
             return
-        copy_rows([(states, self.room(states, block))])
-        self.length += q
-
-    def room(self, states: torch.Tensor, block: int) -> torch.Tensor:
-        """Where ``states`` goes, behind the tail; they belong to it once they are copied and counted."""
-        q = int(states.shape[-2])
         self._reserve(states, self.length + q, block)
-        return self.buf[:, :, self.length: self.length + q]
+        self.buf[:, :, self.length: self.length + q].copy_(states)
+        self.length += q
 
     def drop_front(self, count: int) -> None:
         """Forget the first ``count`` tokens, moving what follows to the front."""
@@ -348,11 +342,8 @@ class float11Layer(DynamicLayer):
         return self._res_k.tensor(), self._res_v.tensor()
 
     def _append_residual(self, key_states: torch.Tensor, value_states: torch.Tensor) -> None:
-        new = [(states, res) for states, res in ((key_states, self._res_k), (value_states, self._res_v))
-               if int(states.shape[-2]) > 0]
-        copy_rows([(states, res.room(states, self.block_size)) for states, res in new])
-        for states, res in new:
-            res.length += int(states.shape[-2])
+        self._res_k.append(key_states, self.block_size)
+        self._res_v.append(value_states, self.block_size)
 
     @staticmethod
     def _extract_exponent_histogram(states: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -627,7 +618,7 @@ class float11Layer(DynamicLayer):
         res_len = self._res_k.length if self._res_k.buf is not None else 0
         prefix = self._compressed_prefix_seq_len
         total = prefix + res_len
-        outs, tails = [], []
+        outs = []
         pairs = (('k', self._key_segments, self._res_k), ('v', self._value_segments, self._res_v))
         if self.dense_workspace == 'shared':
             # keys, values and the tails behind them are written by one launch when keys and values have one shape
@@ -659,9 +650,8 @@ class float11Layer(DynamicLayer):
             dense = mirror[:, :, :total]
             self._mirror_valid[which] = total
             if res_len:
-                tails.append((res.tensor(), dense[:, :, prefix:total]))
+                dense[:, :, prefix:total].copy_(res.tensor())
             outs.append(dense)
-        copy_rows(tails)
         return outs[0], outs[1]
 
     def _layer_mirror(self, which: str, bhd: tuple, total: int) -> torch.Tensor:

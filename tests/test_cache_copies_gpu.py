@@ -1,0 +1,37 @@
+"""What the copies of dense tokens inside a cache have to keep beside the bytes: tangents, recorded versions, refusals."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwAD
+
+from tests import synth
+from tests.scenarios import StubConfig
+
+pytestmark = pytest.mark.gpu
+
+
+def _cache(workspace):
+    from adacode_b200 import Float11Cache
+    return Float11Cache(StubConfig(1), 130, 3, block_size=128, layout='segmented_tiled', dense_workspace=workspace)
+
+
+def _dual(shape, dev, seed):
+    g = torch.Generator('cpu').manual_seed(seed)
+    x, t = (torch.randn(shape, generator=g).to(torch.bfloat16).to(dev) for _ in range(2))
+    return fwAD.make_dual(x, t), t
+
+
+def _check_tangents(dev, workspace, prompt):
+    cache = _cache(workspace)
+    k, v = (synth.kv_tensor((1, 2, prompt, 64), seed=s).to(dev) for s in (1, 2))
+    cache.update(k, v, 0)
+    with fwAD.dual_level():
+        (kd, kt), (vd, vt) = _dual((1, 2, 3, 64), dev, 3), _dual((1, 2, 3, 64), dev, 4)
+        for out, new, tangent in zip(cache.update(kd, vd, 0), (kd, vd), (kt, vt)):
+            primal, got = fwAD.unpack_dual(out)
+            assert torch.equal(primal[:, :, prompt:], fwAD.unpack_dual(new).primal)
+            assert got is not None and torch.equal(got[:, :, prompt:], tangent) and not got[:, :, :prompt].any()
+
+
+@pytest.mark.parametrize('workspace,prompt', [('shared', 60), ('layer', 60), ('layer', 300)])
+def test_appended_tokens_keep_their_tangents(cuda_device, workspace, prompt):
+    _check_tangents(cuda_device, workspace, prompt)

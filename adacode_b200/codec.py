@@ -17,7 +17,7 @@ from typing import Any, Optional, Sequence
 import torch
 
 from . import _lib
-from .rows import on_device, stream_ptr
+from .rows import on_device, row_record, stream_ptr
 
 _SUPPORTED_TILE_NBITS = (1, 2, 3, 4)
 _DEFAULT_TILE_NBITS = 3
@@ -689,18 +689,13 @@ def _unpack_with_rows(jobs: Sequence[tuple], shape: tuple) -> None:
 def unpack_with_tails(parts: Sequence[tuple], prefix: int, rows: int) -> None:
     """Dense keys and values of one layer: for every ``(segments, table, dense, tail)`` the segments are unpacked into
     the front of the contiguous ``dense`` [B, H, prefix + rows, D] and the first ``rows`` tokens of ``tail``
-    [B, H, capacity, D] copied behind them, in one launch for parts of one shape."""
-    jobs = []
+    [B, H, capacity, D] copied behind them, in one launch for parts of one shape.  A tail that is more than plain
+    rows (see ``row_record``) is left to ``Tensor.copy_``."""
+    jobs, left = [], []
     for segs, table, dense, tail in parts:
-        row = None
-        if rows:
-            B, H, _, D = dense.shape
-            if tail.shape[0] != B or tail.shape[1] != H or tail.shape[3] != D or tail.shape[2] < rows:
-                raise ValueError(f'tail {tuple(tail.shape)} does not fit {tuple(dense.shape)}')
-            if tail.device != dense.device or tail.dtype != torch.bfloat16 or tail.stride(3) != 1:
-                raise ValueError('tail must be a bf16 tensor with unit stride along head_dim on the device of the dense one')
-            db, dh, ds, _ = dense.stride()
-            row = (tail.data_ptr(), dense.data_ptr() + 2 * prefix * ds, *tail.stride()[:3], db, dh, ds, B, H, rows, D)
+        row = row_record(tail, dense, rows, prefix) if rows else None
+        if rows and row is None:
+            left.append((dense, tail))
         jobs.append((segs, dense, table, row))
     shapes = [tuple(p[0][0].original_shape) for p in parts]
     if all(s == shapes[0] for s in shapes):
@@ -708,6 +703,8 @@ def unpack_with_tails(parts: Sequence[tuple], prefix: int, rows: int) -> None:
     else:
         for job, shape in zip(jobs, shapes):
             _unpack_with_rows([job], shape)
+    for dense, tail in left:
+        dense[:, :, prefix: prefix + rows].copy_(tail[:, :, :rows])
 
 
 def exponent_hist(x: torch.Tensor, hist_out: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -628,14 +628,7 @@ class float11Layer(DynamicLayer):
                 dense = self._workspace.view(self.cache_device, which, (B, H, total, D))
                 parts.append((segs, self._segment_table(which, segs), dense, res.buf))
                 outs.append(dense)
-            if all(dense.is_cuda and (not res_len or (tail.device == dense.device and not tail.requires_grad))
-                   for _, _, dense, tail in parts):
-                codec.unpack_with_tails(parts, prefix, res_len)
-            else:
-                codec.unpack_segments_multi([(segs, dense, table) for segs, table, dense, _ in parts])
-                if res_len:
-                    for _, _, dense, tail in parts:
-                        dense[:, :, prefix:total].copy_(tail[:, :, :res_len])
+            codec.unpack_with_tails(parts, prefix, res_len)
             return outs[0], outs[1]
         for which, segs, res in pairs:
             B, H, _, D = segs[0].original_shape

@@ -7,9 +7,11 @@ import ctypes
 from typing import Optional, Sequence
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib
 
+_is_wrapped = torch._C._functorch.is_functorch_wrapped_tensor
 _HERE = contextlib.nullcontext()
 
 
@@ -25,23 +27,33 @@ def on_device(device: torch.device):
     return _HERE if index is None or index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
-def row_record(src: torch.Tensor, dst: torch.Tensor) -> Optional[tuple]:
-    """``dst.copy_(src)`` as a record of the row-copy kernel, or None if it is not one: it takes plain bf16 CUDA tensors
-    of one [B, H, T, D] shape on one device, rows on 16-byte boundaries, and no gradient to record."""
+def row_record(src: torch.Tensor, dst: torch.Tensor, rows: Optional[int] = None, at: int = 0) -> Optional[tuple]:
+    """``dst[:, :, at: at + rows].copy_(src[:, :, :rows])`` (all of both without ``rows``) as a record of the row-copy
+    kernel, or None if it is not one: it takes plain bf16 CUDA tensors [B, H, T, D] on one device, rows on 16-byte
+    boundaries, and nothing that ``copy_`` would do beyond moving bytes: no gradient or tangent to carry on, no
+    ``torch.func`` wrapper, nothing to refuse."""
     if type(src) is not torch.Tensor or type(dst) is not torch.Tensor:
         return None
     if src.dtype != torch.bfloat16 or dst.dtype != torch.bfloat16 or not src.is_cuda or src.device != dst.device:
         return None
-    shape = src.shape
-    if len(shape) != 4 or shape != dst.shape or ((src.requires_grad or dst.requires_grad) and torch.is_grad_enabled()):
+    if forward_ad._current_level >= 0 or _is_wrapped(src) or _is_wrapped(dst):
+        return None
+    if (src.requires_grad or dst.requires_grad) and torch.is_grad_enabled():
+        return None
+    if src.dim() != 4 or dst.dim() != 4:
+        return None
+    B, H, T, D = src.shape
+    B2, H2, T2, D2 = dst.shape
+    if rows is None:
+        rows = T if T == T2 else -1
+    if B != B2 or H != H2 or D != D2 or not 0 <= rows <= T or at + rows > T2:
         return None
     a, b, c, u = src.stride()
     d, e, f, v = dst.stride()
-    from_ptr, to_ptr = src.data_ptr(), dst.data_ptr()
-    B, H, T, D = shape
-    if u != 1 or v != 1 or (a | b | c | d | e | f | D) & 7 or (from_ptr | to_ptr) & 15 or B * H * T * D >= 2 ** 31:
+    from_ptr, to_ptr = src.data_ptr(), dst.data_ptr() + 2 * at * f
+    if u != 1 or v != 1 or (a | b | c | d | e | f | D) & 7 or (from_ptr | to_ptr) & 15 or B * H * rows * D >= 2 ** 31:
         return None
-    return (from_ptr, to_ptr, a, b, c, d, e, f, B, H, T, D)
+    return (from_ptr, to_ptr, a, b, c, d, e, f, B, H, rows, D)
 
 
 def copy_rows(pairs: Sequence[tuple]) -> None:

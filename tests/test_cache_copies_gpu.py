@@ -35,3 +35,23 @@ def _check_tangents(dev, workspace, prompt):
 @pytest.mark.parametrize('workspace,prompt', [('shared', 60), ('layer', 60), ('layer', 300)])
 def test_appended_tokens_keep_their_tangents(cuda_device, workspace, prompt):
     _check_tangents(cuda_device, workspace, prompt)
+
+
+def test_dense_view_keeps_tangents(cuda_device):
+    """Packed blocks have none; the tail behind them keeps its own."""
+    _check_tangents(cuda_device, 'shared', 300)
+
+
+def test_rows_under_transforms(cuda_device):
+    """``torch.func`` wrappers are no plain rows: what ``copy_`` makes of them holds."""
+    from adacode_b200.rows import copy_rows
+    x, t = (torch.randn(2, 2, 3, 16, device=cuda_device).to(torch.bfloat16) for _ in range(2))
+
+    def copied(a):
+        out = torch.empty_like(a)
+        copy_rows([(a, out)])
+        return out
+
+    out, tangent = torch.func.jvp(copied, (x,), (t,))
+    assert torch.equal(out, x) and torch.equal(tangent, t)
+    assert torch.equal(torch.func.vmap(copied)(x[None].expand(3, 2, 2, 3, 16)), x[None].expand(3, 2, 2, 3, 16))

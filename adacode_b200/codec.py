@@ -17,7 +17,7 @@ from typing import Any, Optional, Sequence
 import torch
 
 from . import _lib
-from .rows import on_device, row_record, stream_ptr
+from .rows import increment_version, on_device, row_record, stream_ptr
 
 _SUPPORTED_TILE_NBITS = (1, 2, 3, 4)
 _DEFAULT_TILE_NBITS = 3
@@ -703,6 +703,8 @@ def unpack_with_tails(parts: Sequence[tuple], prefix: int, rows: int) -> None:
     else:
         for job, shape in zip(jobs, shapes):
             _unpack_with_rows([job], shape)
+    # (autograd has to know that memory that it may have saved was overwritten)
+    increment_version([dense for _, dense, _, row in jobs if row is not None])
     for dense, tail in left:
         dense[:, :, prefix: prefix + rows].copy_(tail[:, :, :rows])
 

@@ -8,6 +8,7 @@ from typing import Optional, Sequence
 
 import torch
 from torch.autograd import forward_ad
+from torch.autograd.graph import increment_version
 
 from . import _lib
 
@@ -74,3 +75,4 @@ def copy_rows(pairs: Sequence[tuple]) -> None:
     with on_device(dev):
         rc = _lib.lib().adacode_copy_rows(ctypes.addressof(arr), len(records), stream_ptr(dev))
     _lib.check(rc, 'adacode_copy_rows')
+    increment_version([d for _, d in pairs])

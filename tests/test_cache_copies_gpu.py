@@ -55,3 +55,16 @@ def test_rows_under_transforms(cuda_device):
     out, tangent = torch.func.jvp(copied, (x,), (t,))
     assert torch.equal(out, x) and torch.equal(tangent, t)
     assert torch.equal(torch.func.vmap(copied)(x[None].expand(3, 2, 2, 3, 16)), x[None].expand(3, 2, 2, 3, 16))
+
+
+def test_overwritten_workspace_is_noticed(cuda_device):
+    """Dense keys saved for a backward pass and overwritten by the next call: autograd refuses."""
+    cache = _cache('shared')
+    k, v = (synth.kv_tensor((1, 2, 303, 64), seed=s).to(cuda_device) for s in (1, 2))
+    cache.update(k[:, :, :300], v[:, :, :300], 0)
+    dense, _ = cache.update(k[:, :, 300:301], v[:, :, 300:301], 0)
+    q = torch.ones(1, 2, 1, 64, dtype=torch.bfloat16, device=cuda_device, requires_grad=True)
+    scores = q @ dense.transpose(2, 3)
+    cache.update(k[:, :, 301:302], v[:, :, 301:302], 0)
+    with pytest.raises(RuntimeError, match='modified by an inplace operation'):
+        scores.float().sum().backward()

@@ -41,6 +41,8 @@ def row_record(src: torch.Tensor, dst: torch.Tensor, rows: Optional[int] = None,
         return None
     if (src.requires_grad or dst.requires_grad) and torch.is_grad_enabled():
         return None
+    if dst.is_inference() and not torch.is_inference_mode_enabled():
+        return None
     if src.dim() != 4 or dst.dim() != 4:
         return None
     B, H, T, D = src.shape
@@ -67,6 +69,10 @@ def copy_rows(pairs: Sequence[tuple]) -> None:
         return
     dev = pairs[0][1].device
     records = [row_record(s, d) for s, d in pairs]
+    for i, (s, d) in enumerate(pairs):
+        # what copy_ refuses: destinations that overlap themselves or their source
+        if records[i] is not None and (0 in d.stride() or s.untyped_storage().data_ptr() == d.untyped_storage().data_ptr()):
+            records[i] = None
     if len(records) > 8 or None in records or any(d.device != dev for _, d in pairs):
         for s, d in pairs:
             d.copy_(s)

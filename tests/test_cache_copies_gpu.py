@@ -68,3 +68,21 @@ def test_overwritten_workspace_is_noticed(cuda_device):
     cache.update(k[:, :, 301:302], v[:, :, 301:302], 0)
     with pytest.raises(RuntimeError, match='modified by an inplace operation'):
         scores.float().sum().backward()
+
+
+def test_what_copy_refuses_is_refused(cuda_device):
+    from adacode_b200 import codec
+    from adacode_b200.rows import copy_rows
+    x = torch.randn(2, 2, 3, 16, device=cuda_device).to(torch.bfloat16)
+    with torch.inference_mode():
+        frozen = torch.zeros_like(x)
+    with pytest.raises(RuntimeError, match='InferenceMode'):
+        copy_rows([(x, frozen)])
+    with pytest.raises(RuntimeError, match='single memory location'):
+        copy_rows([(x, torch.zeros(2, 1, 3, 16, dtype=torch.bfloat16, device=cuda_device).expand(2, 2, 3, 16))])
+    k = synth.kv_tensor((1, 2, 140, 64), seed=1).to(cuda_device)
+    segs = codec.pack_blocks(k[:, :, :128], 130, 3, 128)[0].segments()
+    with torch.inference_mode():
+        dense = torch.zeros_like(k)
+    with pytest.raises(RuntimeError, match='InferenceMode'):
+        codec.unpack_with_tails([(segs, None, dense, k[:, :, 128:].contiguous())], 128, 12)

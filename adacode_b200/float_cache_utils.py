@@ -628,7 +628,13 @@ class float11Layer(DynamicLayer):
                 dense = self._workspace.view(self.cache_device, which, (B, H, total, D))
                 parts.append((segs, self._segment_table(which, segs), dense, res.buf))
                 outs.append(dense)
-            codec.unpack_with_tails(parts, prefix, res_len)
+            if self._res_v.length == res_len:
+                codec.unpack_with_tails(parts, prefix, res_len)
+            else:
+                # tails of two lengths (keys and values were appended unevenly): copy_ says what it thinks of that
+                codec.unpack_with_tails(parts, prefix, 0)
+                for dense, res in zip(outs, (self._res_k, self._res_v)) if res_len else ():
+                    dense[:, :, prefix:total].copy_(res.tensor())
             return outs[0], outs[1]
         for which, segs, res in pairs:
             B, H, _, D = segs[0].original_shape

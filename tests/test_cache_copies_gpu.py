@@ -86,3 +86,13 @@ def test_what_copy_refuses_is_refused(cuda_device):
         dense = torch.zeros_like(k)
     with pytest.raises(RuntimeError, match='InferenceMode'):
         codec.unpack_with_tails([(segs, None, dense, k[:, :, 128:].contiguous())], 128, 12)
+
+
+@pytest.mark.parametrize('nk,nv', [(1, 2), (3, 2)])
+def test_uneven_tails_are_refused(cuda_device, nk, nv):
+    """Keys and values of different numbers of tokens: no dense view with rows that nobody wrote."""
+    cache = _cache('shared')
+    k, v = (synth.kv_tensor((1, 2, 303, 64), seed=s).to(cuda_device) for s in (1, 2))
+    cache.update(k[:, :, :300], v[:, :, :300], 0)
+    with pytest.raises(RuntimeError):
+        cache.update(k[:, :, 300: 300 + nk], v[:, :, 300: 300 + nv], 0)

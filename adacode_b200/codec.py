@@ -693,6 +693,9 @@ def unpack_with_tails(parts: Sequence[tuple], prefix: int, rows: int) -> None:
     rows (see ``row_record``) is left to ``Tensor.copy_``."""
     jobs, left = [], []
     for segs, table, dense, tail in parts:
+        if len(segs) * segs[0].original_shape[2] > prefix or dense.shape[2] < prefix + rows:
+            raise ValueError(f'{len(segs)} segments of {segs[0].original_shape[2]} tokens and {rows} rows behind {prefix} '
+                             f'do not fit {tuple(dense.shape)}')
         row = row_record(tail, dense, rows, prefix) if rows else None
         if rows and row is None:
             left.append((dense, tail))

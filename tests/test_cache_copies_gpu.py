@@ -96,3 +96,15 @@ def test_uneven_tails_are_refused(cuda_device, nk, nv):
     cache.update(k[:, :, :300], v[:, :, :300], 0)
     with pytest.raises(RuntimeError):
         cache.update(k[:, :, 300: 300 + nk], v[:, :, 300: 300 + nv], 0)
+
+
+def test_dense_too_small_for_its_parts(cuda_device):
+    from adacode_b200 import codec
+    k = synth.kv_tensor((1, 2, 300, 64), seed=1).to(cuda_device)
+    segs = codec.pack_blocks(k[:, :, :256], 130, 3, 128)[0].segments()
+    tail = k[:, :, 256:].contiguous()
+    for prefix, rows, length in ((256, 44, 299), (200, 44, 300), (300, 0, 299)):
+        dense = torch.zeros(1, 2, length, 64, dtype=torch.bfloat16, device=cuda_device)
+        with pytest.raises(ValueError, match='do not fit'):
+            codec.unpack_with_tails([(segs, None, dense, tail)], prefix, rows)
+        assert not dense.any()

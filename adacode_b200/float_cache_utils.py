@@ -628,11 +628,11 @@ class float11Layer(DynamicLayer):
                 dense = self._workspace.view(self.cache_device, which, (B, H, total, D))
                 parts.append((segs, self._segment_table(which, segs), dense, res.buf))
                 outs.append(dense)
-            if self._res_v.length == res_len:
+            if self._res_v.length == res_len and all(dense.is_cuda for dense in outs):
                 codec.unpack_with_tails(parts, prefix, res_len)
             else:
-                # tails of two lengths (keys and values were appended unevenly): copy_ says what it thinks of that
-                codec.unpack_with_tails(parts, prefix, 0)
+                # (tails of two lengths, from keys and values appended unevenly: copy_ says what it thinks of that)
+                codec.unpack_segments_multi([(segs, dense, table) for segs, table, dense, _ in parts])
                 for dense, res in zip(outs, (self._res_k, self._res_v)) if res_len else ():
                     dense[:, :, prefix:total].copy_(res.tensor())
             return outs[0], outs[1]

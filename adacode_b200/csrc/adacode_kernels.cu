@@ -847,11 +847,25 @@ HistRuns flatten_runs(int64_t sb, int64_t sh, int64_t ss, int64_t B, int64_t H, 
     return a;
 }
 
+// Vectors per thread that the rows along with an unpack launch ask for.  One, two and four measure the same, eight is
+// up to 3 us slower at tails of 256 to 2000 tokens.  Keys and values, 256 packed tokens: one head with a tail of 16, 1000 and
+// 8000 tokens 11.2, 27.7 and 156 us with a grid for the tiles alone, 11.2, 11.1 and 12.3 us with this; eight heads
+// 11.2, 29.7 and 157 us, and 11.2, 13.1 and 24.6 us.
+constexpr int kRowVecs = 2;
+
 template <class G>
 int launch_unpack_geom(const UnpackJobsArgs &ja, cudaStream_t st) {
     int rc = ensure_dynamic_smem(k_unpack_pipe<G>, sizeof(UnpackSmemT<G>));
     if (rc != ADACODE_OK) return rc;
-    const int grid = grid_for(ja.tile0[ja.n_jobs], G::kCtasPerSm);
+    // CTAs for the tiles, or for the rows that go along if those take more (a CTA without tiles copies and leaves)
+    int64_t vecs = 0;
+    for (int i = 0; i < ja.rows.n; ++i) {
+        const adacode_row_copy &c = ja.rows.copy[i];
+        vecs += (int64_t)c.B * c.H * c.rows * (c.D / 8);
+    }
+    const int64_t for_rows = (vecs + G::kConsumers * kRowVecs - 1) / (G::kConsumers * kRowVecs);
+    const int64_t tiles = ja.tile0[ja.n_jobs];
+    const int grid = grid_for(tiles > for_rows ? tiles : for_rows, G::kCtasPerSm);
     return launch_dependent(k_unpack_pipe<G>, dim3(grid), G::kThreads, sizeof(UnpackSmemT<G>), st, ja);
 }
 

@@ -108,3 +108,17 @@ def test_dense_too_small_for_its_parts(cuda_device):
         with pytest.raises(ValueError, match='do not fit'):
             codec.unpack_with_tails([(segs, None, dense, tail)], prefix, rows)
         assert not dense.any()
+
+
+@pytest.mark.parametrize('H,D,rows', [(1, 128, 5000), (2, 64, 40001), (1, 2048, 700), (3, 72, 3000)])
+def test_tails_longer_than_the_packed_part(cuda_device, H, D, rows):
+    """One packed block: the rows decide the launch's grid, most CTAs have no tile.  2048: the wide geometry, 72: the
+    direct kernels."""
+    from adacode_b200 import codec
+    g = torch.Generator(device=cuda_device).manual_seed(rows)
+    x = [torch.randn(1, H, 128 + rows, D, generator=g, device=cuda_device).to(torch.bfloat16) for _ in range(2)]
+    parts = [(codec.pack_blocks(t[:, :, :128], 129, 3, 128)[0].segments(), None, torch.zeros_like(t), t[:, :, 128:]) for t in x]
+    codec.unpack_with_tails(parts, 128, rows)
+    for t, (_, _, dense, _) in zip(x, parts):
+        assert torch.equal(dense.view(torch.int16), t.view(torch.int16))
+    codec.check_device_status(cuda_device)

@@ -506,9 +506,11 @@ def unpack_chunk(chunk: PackedChunk, dst: torch.Tensor, seq_offset: int = 0) -> 
 
 
 def _check_dst(dst: torch.Tensor, B: int, H: int, D: int, min_seq: int) -> None:
-    if dst.dtype != torch.bfloat16 or dst.dim() != 4:
+    shape = dst.shape
+    if dst.dtype != torch.bfloat16 or len(shape) != 4:
         raise ValueError(f'dst must be a 4D bf16 tensor, got {dst.dtype} {tuple(dst.shape)}')
-    if dst.shape[0] != B or dst.shape[1] != H or dst.shape[3] != D or dst.shape[2] < min_seq:
+    B2, H2, S2, D2 = shape
+    if B2 != B or H2 != H or D2 != D or S2 < min_seq:
         raise ValueError(f'dst shape {tuple(dst.shape)} cannot hold [{B}, {H}, {min_seq}, {D}]')
     if dst.stride(3) != 1:
         raise ValueError('dst must have unit stride along head_dim')
@@ -691,16 +693,16 @@ def unpack_with_tails(parts: Sequence[tuple], prefix: int, rows: int) -> None:
     the front of the contiguous ``dense`` [B, H, prefix + rows, D] and the first ``rows`` tokens of ``tail``
     [B, H, capacity, D] copied behind them, in one launch for parts of one shape.  A tail that is more than plain
     rows (see ``row_record``) is left to ``Tensor.copy_``."""
-    jobs, left = [], []
+    jobs, shapes, left = [], [], []
     for segs, table, dense, tail in parts:
-        if len(segs) * segs[0].original_shape[2] > prefix or dense.shape[2] < prefix + rows:
-            raise ValueError(f'{len(segs)} segments of {segs[0].original_shape[2]} tokens and {rows} rows behind {prefix} '
+        shapes.append(tuple(segs[0].original_shape))
+        if len(segs) * shapes[-1][2] > prefix or dense.shape[2] < prefix + rows:
+            raise ValueError(f'{len(segs)} segments of {shapes[-1][2]} tokens and {rows} rows behind {prefix} '
                              f'do not fit {tuple(dense.shape)}')
         row = row_record(tail, dense, rows, prefix) if rows else None
         if rows and row is None:
             left.append((dense, tail))
         jobs.append((segs, dense, table, row))
-    shapes = [tuple(p[0][0].original_shape) for p in parts]
     if all(s == shapes[0] for s in shapes):
         _unpack_with_rows(jobs, shapes[0])
     else:

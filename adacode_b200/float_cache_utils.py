@@ -25,6 +25,7 @@ meaning; the places are cited at each method.
 """
 from __future__ import annotations
 
+import math
 import time
 import warnings
 from typing import Any, Optional
@@ -71,10 +72,8 @@ class _DenseWorkspace:
         self._bufs: dict = {}
 
     def view(self, device, slot: str, shape: tuple) -> torch.Tensor:
-        n = 1
-        for d in shape:
-            n *= int(d)
-        key = (torch.device(device), slot)
+        n = math.prod(shape)
+        key = (device if type(device) is torch.device else torch.device(device), slot)
         buf = self._bufs.get(key)
         if buf is None or buf.numel() < n:
             buf = torch.empty(max(int(n * 1.25), 1 << 16), dtype=torch.bfloat16, device=device)
@@ -628,7 +627,7 @@ class float11Layer(DynamicLayer):
                 dense = self._workspace.view(self.cache_device, which, (B, H, total, D))
                 parts.append((segs, self._segment_table(which, segs), dense, res.buf))
                 outs.append(dense)
-            if self._res_v.length == res_len and all(dense.is_cuda for dense in outs):
+            if self._res_v.length == res_len and outs[0].is_cuda:
                 codec.unpack_with_tails(parts, prefix, res_len)
             else:
                 # (tails of two lengths, from keys and values appended unevenly: copy_ says what it thinks of that)

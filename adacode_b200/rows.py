@@ -13,6 +13,7 @@ from torch.autograd.graph import increment_version
 from . import _lib
 
 _is_wrapped = torch._C._functorch.is_functorch_wrapped_tensor
+_BF16 = torch.bfloat16
 _HERE = contextlib.nullcontext()
 
 
@@ -35,7 +36,7 @@ def row_record(src: torch.Tensor, dst: torch.Tensor, rows: Optional[int] = None,
     ``torch.func`` wrapper, nothing to refuse."""
     if type(src) is not torch.Tensor or type(dst) is not torch.Tensor:
         return None
-    if src.dtype != torch.bfloat16 or dst.dtype != torch.bfloat16 or not src.is_cuda or src.device != dst.device:
+    if src.dtype is not _BF16 or dst.dtype is not _BF16 or not src.is_cuda or src.get_device() != dst.get_device():
         return None
     if forward_ad._current_level >= 0 or _is_wrapped(src) or _is_wrapped(dst):
         return None
@@ -43,16 +44,17 @@ def row_record(src: torch.Tensor, dst: torch.Tensor, rows: Optional[int] = None,
         return None
     if dst.is_inference() and not torch.is_inference_mode_enabled():
         return None
-    if src.dim() != 4 or dst.dim() != 4:
+    from_strides, to_strides = src.stride(), dst.stride()
+    if len(from_strides) != 4 or len(to_strides) != 4:
         return None
+    a, b, c, u = from_strides
+    d, e, f, v = to_strides
     B, H, T, D = src.shape
     B2, H2, T2, D2 = dst.shape
     if rows is None:
         rows = T if T == T2 else -1
     if B != B2 or H != H2 or D != D2 or not 0 <= rows <= T or at + rows > T2:
         return None
-    a, b, c, u = src.stride()
-    d, e, f, v = dst.stride()
     from_ptr, to_ptr = src.data_ptr(), dst.data_ptr() + 2 * at * f
     if u != 1 or v != 1 or (a | b | c | d | e | f | D) & 7 or (from_ptr | to_ptr) & 15 or B * H * rows * D >= 2 ** 31:
         return None

@@ -427,8 +427,13 @@ def pack_blocks_finish(p: _PendingPack, host_meta):
             raise _lib.AdacodeError('adacode_pack_tiles: escape overflow after re-run with exact capacity')
     elif status_other:
         raise _lib.AdacodeError(f'adacode_pack_tiles: device status {status:#x} ({describe_status(status)})')
-    # (a large first guess is not kept: it is cut to size once an eighth of it is unused)
-    if escapes.numel() > (total + total // 8 if p.guessed and p.nbits <= 2 else 2 * total) + 65536:
+    # (a large first guess is not kept, which packs of single blocks would for the cache's life: it is cut to size
+    # where an eighth more than the escapes and a 32nd of the elements are unused)
+    if p.guessed and p.nbits <= 2:
+        keep = total + total // 8 + min(65536, p.sign_mant.numel() // 32)
+    else:
+        keep = 2 * total + 65536
+    if escapes.numel() > keep:
         escapes = escapes[:total].clone()
     else:
         escapes = escapes[:total]

@@ -543,155 +543,118 @@ __global__ void k_choose_params(const int32_t *__restrict__ hists, int n_hists, 
 
 #include "adacode_pipeline.cuh"
 
-// Exponent histogram.  Nearly all exponents of a tensor lie in a window of fifteen, so they are counted as the
-// pack kernel counts its codes: four-bit codes against a window that each warp takes from the first values
-// it sees, one population count per subset of the code bits over 32 elements (count_codes_overlaid), and one
-// shared-memory atomic for each of the few elements outside.  The window only decides the speed.
-// [16, 8, 8192, 128] (268 MB): one atomic per element on bins shared by a warp 113 us, byte counters of each lane's own
-// 97 us (an atomic of 32 lanes in 32 banks still takes several cycles), this 81 us (3.3 TB/s, bound by the integer
-// pipe); three CTAs per SM 87 us.  One block of [1, 8, 128, 128]: 6.3 -> 4.3 us.
+// Exponent histogram: one shared-memory atomic per element, on one set of bins per CTA; lanes that meet in a bin
+// cost nothing extra (see the figures).  A warp takes units of kHistVec x 32 16-byte vectors and loads the next one
+// while it counts the current one.
+// [16, 8, 4096, 128] (134 MB): 26.9 us (5.0 TB/s) for normal values, half zeros and outliers alike, 36 us for random
+// bits, with three or four CTAs per SM; two 33 us, six 35 us, eight 40 us (each adds its bins to the result at the end), eight
+// with half the vectors per unit 29 us, eight vectors per unit 34 us.  Bins in two to sixteen copies by lane 29 to 78 us, and
+// bins per warp without the load ahead 61 us.  Codes against a window of fifteen exponents, counted by population counts, 41 us
+// where nearly all exponents lie in it and up to 86 us where they do not.
 //
-// The source is `runs` contiguous pieces of `run_vec` 16-byte vectors (the host merges dimensions, see
-// flatten_runs); a warp takes units of kHistVec x 32 vectors of one run, and loads the next unit
-// while it counts the current one.  SHORT: runs too short for that are walked vector by vector.
+// The source is `runs` contiguous pieces of `run_vec` vectors (the host merges dimensions, see flatten_runs).  Units are
+// parts of one run, or, SHORT, of the vectors of all runs together, each with an address of its own: two heads
+// of twelve, [4, 2, 8192, 128], 10.5 us with the former, 6.5 us with the latter.
 constexpr int kHistVec = 4;
-constexpr int kHistBits = 4;
-constexpr int kHistFlush = 1024;                               // units between flushes of the 16-bit counters
-constexpr int kHistCtas = 4;                                   // per SM
-constexpr int kHistCopies = 4;                                 // of the bins that the atomics go to, by lane
+constexpr int kHistCtas = 3;                                   // per SM
+
+// Quotients of numbers below 2**31 by a divisor that the host knows, by multiplication (Granlund and Montgomery,
+// Division by invariant integers using multiplication, 1994: 2**l >= d, m = 2**31 (2**l - d) / d + 2**31 + 1 rounded
+// down, n / d = n m >> (31 + l)).
+struct Quotient {
+    uint32_t d, m, shift;
+};
+Quotient quotient_by(int64_t d) {
+    int l = 0;
+    while ((1ll << l) < d) ++l;
+    return {(uint32_t)d, (uint32_t)(((1ull << 31) * ((1ull << l) - (uint64_t)d)) / (uint64_t)d + (1ull << 31) + 1), (uint32_t)(31 + l)};
+}
+__device__ __forceinline__ uint32_t operator/(uint32_t n, const Quotient &q) { return (uint32_t)((uint64_t)n * q.m >> q.shift); }
 
 struct HistRuns {
     const uint16_t *src;
     int64_t runs, run_vec;
     int64_t n1, n0;              // run r -> (r / (n1 n0), r / n0 % n1, r % n0)
     int64_t s2, s1, s0;          // element strides of those indices
+    Quotient by_run, by_n0, by_n1;                // (below 2**31 vectors)
     int32_t *hist;
 };
 
 __device__ __forceinline__ const uint4 *hist_run(const HistRuns &a, uint32_t r) {
-    const uint32_t q = r / (uint32_t)a.n0, i0 = r - q * (uint32_t)a.n0;
-    const uint32_t i2 = q / (uint32_t)a.n1, i1 = q - i2 * (uint32_t)a.n1;
+    const uint32_t q = r / a.by_n0, i0 = r - q * a.by_n0.d;
+    const uint32_t i2 = q / a.by_n1, i1 = q - i2 * a.by_n1.d;
     return reinterpret_cast<const uint4 *>(a.src + i2 * a.s2 + i1 * a.s1 + i0 * a.s0);
 }
+__device__ __forceinline__ const uint4 *hist_run(const HistRuns &a, int64_t r) {
+    const int64_t q = r / a.n0, i2 = q / a.n1;
+    return reinterpret_cast<const uint4 *>(a.src + i2 * a.s2 + (q - i2 * a.n1) * a.s1 + (r - q * a.n0) * a.s0);
+}
 
-struct HistState {
-    uint32_t cnt[HistRegs<kHistBits>::v];
-    uint32_t neg_left;
-    int left, units;             // units: since the last flush; -1: no window yet
-};
-
-// Count the first `have` of V vectors of this lane (V * 8 elements at most); `scratch`: V vectors per lane.
-template <int V>
-__device__ __forceinline__ void hist_count(HistState &st, const uint4 (&v)[V], int have, uint4 *scratch, int *s_hist) {
-    const int lane = threadIdx.x & 31;
-    if (st.units < 0) {
-        // the window ends at the largest finite exponent among this unit's first vectors
-        uint32_t m = 0;
-        if (have > 0) {
-            const uint32_t w[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
+// Count the first `have` of this lane's vectors.
+__device__ __forceinline__ void hist_count(const uint4 (&v)[kHistVec], int have, int *bins) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint32_t e0 = (w[i] >> 7) & 0xFFu, e1 = (w[i] >> 23) & 0xFFu;
-                m = max(m, max(e0 == 255u ? 0u : e0, e1 == 255u ? 0u : e1));
-            }
+    for (int k = 0; k < kHistVec; ++k) {
+        if (k >= have) break;
+        const uint32_t w[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            atomicAdd(&bins[(w[i] >> 7) & 0xFFu], 1);
+            atomicAdd(&bins[(w[i] >> 23) & 0xFFu], 1);
         }
-        st.left = (int)__reduce_max_sync(kFull, m) - ((1 << kHistBits) - 1);
-        st.neg_left = ((uint32_t)(-st.left) & 0xFFFFu) * 0x10001u;
-        st.units = 0;
-    }
-    uint32_t g[V], todo = 0;
-#pragma unroll
-    for (int k = 0; k < V; ++k) {
-        const uint32_t c = join_codes<kHistBits>(
-            encode_pair<kHistBits>(v[k].x, st.neg_left), encode_pair<kHistBits>(v[k].y, st.neg_left),
-            encode_pair<kHistBits>(v[k].z, st.neg_left), encode_pair<kHistBits>(v[k].w, st.neg_left));
-        g[k] = k < have ? c : 0u;
-        const uint32_t z = k < have ? compress_slots<kHistBits>(zero_slots<kHistBits>(c)) : 0u;
-        todo |= z << (24 - 8 * k);                             // element 0 in the most significant bit
-    }
-    count_codes_overlaid<kHistBits, V>(g, st.cnt);
-    bump_field<kHistBits>(st.cnt, 0, (uint32_t)(8 * have));
-    bump_field<kHistBits>(st.cnt, (1 << kHistBits) - 1, (uint32_t)__popc(todo));
-    if (__any_sync(kFull, todo != 0)) {
-#pragma unroll
-        for (int k = 0; k < V; ++k) scratch[k * 32 + lane] = v[k];
-        const uint16_t *mine = reinterpret_cast<const uint16_t *>(scratch + lane);
-        int *bins = s_hist + (lane & (kHistCopies - 1)) * 256;
-        while (todo) {
-            const int i = __clz((int)todo);
-            todo &= ~(0x80000000u >> i);
-            atomicAdd(&bins[(mine[(i >> 3) * 256 + (i & 7)] >> 7) & 0xFFu], 1);      // (a vector is 8 elements, a row of them 256)
-        }
-    }
-    if (++st.units == kHistFlush) {
-        flush_code_counts<kHistBits>(st.cnt, st.left, s_hist);
-        st.units = 0;
     }
 }
 
-template <bool SHORT>
+template <typename Index, bool SHORT>
 __global__ void __launch_bounds__(kThreads, kHistCtas) k_hist(const __grid_constant__ HistRuns a) {
-    constexpr int V = SHORT ? 1 : kHistVec;
-    __shared__ uint4 s_scratch[kWarps][V * 32];
-    __shared__ int s_hist[kHistCopies * 256];
+    __shared__ int s_hist[256];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < kHistCopies * 256; i += kThreads) s_hist[i] = 0;
+    s_hist[tid] = 0;
     __syncthreads();
-    uint4 *scratch = s_scratch[warp];
-    HistState st;
+    const Index run_vec = (Index)a.run_vec, n_vec = (Index)(a.runs * a.run_vec);
+    const Index per_run = (run_vec + 32 * kHistVec - 1) / (32 * kHistVec);
+    const Index units = SHORT ? (n_vec + 32 * kHistVec - 1) / (32 * kHistVec) : (Index)a.runs * per_run;
+    const Index step = (Index)gridDim.x * kWarps;
+    uint4 cur[kHistVec], nxt[kHistVec];
+    // (a lane beyond the end of its run, or of the source, loads nothing and counts nothing: `have` says how many it has)
+    const auto load = [&](Index u, uint4 (&v)[kHistVec]) {
+        int have = 0;
+        if (u >= units) return have;
+        if constexpr (SHORT) {
+            Index i = u * (32 * kHistVec) + lane;
 #pragma unroll
-    for (int i = 0; i < HistRegs<kHistBits>::v; ++i) st.cnt[i] = 0;
-    st.neg_left = 0, st.left = 0, st.units = -1;
-    if constexpr (SHORT) {
-        const int64_t n_vec = a.runs * a.run_vec;
-        for (int64_t base = ((int64_t)blockIdx.x * kWarps + warp) * 32; base < n_vec; base += (int64_t)gridDim.x * kThreads) {
-            const int64_t i = base + lane;
-            uint4 v[1] = {make_uint4(0, 0, 0, 0)};
-            if (i < n_vec) {
-                const int64_t r = i / a.run_vec, q = r / a.n0, i2 = q / a.n1;
-                const uint16_t *run = a.src + i2 * a.s2 + (q - i2 * a.n1) * a.s1 + (r - q * a.n0) * a.s0;
-                v[0] = reinterpret_cast<const uint4 *>(run)[i - r * a.run_vec];
+            for (int k = 0; k < kHistVec; ++k, i += 32) {
+                if (i < n_vec) {
+                    Index r;
+                    if constexpr (sizeof(Index) == 4) r = i / a.by_run;
+                    else r = i / run_vec;
+                    v[k] = __ldg(hist_run(a, r) + (i - r * run_vec)), ++have;
+                }
             }
-            hist_count(st, v, i < n_vec ? 1 : 0, scratch, s_hist);
+        } else {
+            const Index r = u / per_run, at = (u - r * per_run) * (32 * kHistVec) + lane;
+            const uint4 *p = hist_run(a, r) + at;
+#pragma unroll
+            for (int k = 0; k < kHistVec; ++k)
+                if (at + 32 * k < run_vec) v[k] = __ldg(p + 32 * k), ++have;
         }
-    } else {
-        const uint32_t run_vec = (uint32_t)a.run_vec, per_run = (run_vec + 32 * kHistVec - 1) / (32 * kHistVec);
-        const uint32_t units = (uint32_t)a.runs * per_run, step = gridDim.x * kWarps;
-        uint4 cur[kHistVec], nxt[kHistVec];
-        // (a lane beyond the end of its run loads nothing and counts nothing: `have` says how many it has)
-        const auto load = [&](uint32_t u, uint4 (&v)[kHistVec]) {
-            int have = 0;
-            if (u < units) {
-                const uint32_t r = u / per_run, at = (u - r * per_run) * (32 * kHistVec) + lane;
-                const uint4 *p = hist_run(a, r) + at;
+        return have;
+    };
 #pragma unroll
-                for (int k = 0; k < kHistVec; ++k)
-                    if (at + 32 * k < run_vec) v[k] = __ldg(p + 32 * k), ++have;
-            }
-            return have;
-        };
+    for (int k = 0; k < kHistVec; ++k) cur[k] = nxt[k] = make_uint4(0, 0, 0, 0);
+    Index u = (Index)blockIdx.x * kWarps + warp;
+    int have = load(u, cur);
+    while (u < units) {
+        // (in 32 bits units + step stays below 2**32: both are below 2**31)
+        u += step;
+        const int have_next = load(u, nxt);
+        hist_count(cur, have, s_hist);
 #pragma unroll
-        for (int k = 0; k < kHistVec; ++k) cur[k] = nxt[k] = make_uint4(0, 0, 0, 0);
-        uint32_t u = blockIdx.x * kWarps + warp;
-        int have = load(u, cur);
-        while (u < units) {
-            // (units + step stays below 2**32: both are below 2**31)
-            u += step;
-            const int have_next = load(u, nxt);
-            hist_count(st, cur, have, scratch, s_hist);
-#pragma unroll
-            for (int k = 0; k < kHistVec; ++k) cur[k] = nxt[k];
-            have = have_next;
-        }
+        for (int k = 0; k < kHistVec; ++k) cur[k] = nxt[k];
+        have = have_next;
     }
-    if (st.units > 0) flush_code_counts<kHistBits>(st.cnt, st.left, s_hist);
     __syncthreads();
-    int total = 0;
-#pragma unroll
-    for (int i = 0; i < kHistCopies; ++i) total += s_hist[i * 256 + tid];
-    if (total != 0) atomicAdd(a.hist + tid, total);
+    if (s_hist[tid] != 0) atomicAdd(a.hist + tid, s_hist[tid]);
 }
-
 
 void stable_order_desc(const int64_t *hist, int *order) {
     for (int i = 0; i < 256; ++i) order[i] = i;
@@ -1401,14 +1364,17 @@ int adacode_hist_bf16(const void *src_bf16, int64_t stride_b, int64_t stride_h, 
         return ADACODE_ERR_INVALID_ARG;
     HistRuns a = flatten_runs(stride_b, stride_h, stride_s, B, H, S, D);
     a.src = (const uint16_t *)src_bf16, a.hist = hist256;
-    // Runs shorter than half a warp's unit leave most of its lanes idle, and 32-bit indices must do.
-    const bool by_vector = a.run_vec < 16 * kHistVec || a.runs * a.run_vec >= (1ll << 31);
-    const int64_t units = by_vector ? (a.runs * a.run_vec + 31) / 32
-                                    : a.runs * ((a.run_vec + 32 * kHistVec - 1) / (32 * kHistVec));
+    // Units of one run leave lanes idle behind its end; where those are more than an eighth, units are cut from
+    // the vectors of all runs together, which costs each vector its own address.
+    const int64_t n_vec = a.runs * a.run_vec, per_run = (a.run_vec + 32 * kHistVec - 1) / (32 * kHistVec);
+    const bool big = n_vec >= (1ll << 31), by_vector = big || per_run * (32 * kHistVec) > a.run_vec + a.run_vec / 8;
+    if (!big) a.by_run = quotient_by(a.run_vec), a.by_n0 = quotient_by(a.n0), a.by_n1 = quotient_by(a.n1);
+    const int64_t units = by_vector ? (n_vec + 32 * kHistVec - 1) / (32 * kHistVec) : a.runs * per_run;
     const int64_t want = (units + kWarps - 1) / kWarps, cap = (int64_t)sm_count() * kHistCtas;
     const int blocks = (int)(want < cap ? want : cap);
-    if (by_vector) k_hist<true><<<blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
-    else k_hist<false><<<blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
+    if (big) k_hist<int64_t, true><<<blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
+    else if (by_vector) k_hist<uint32_t, true><<<blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
+    else k_hist<uint32_t, false><<<blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
     ADACODE_CUDA_TRY(cudaGetLastError());
     return ADACODE_OK;
 }

@@ -1,12 +1,14 @@
 // Fused unpack + single-query ("decode") attention over a float11-packed KV cache.
 //
 // The packed planes are read straight from HBM (1 + n/8 + p bytes per cached element instead of
-// 2 for dense bf16), decoded tile by tile into shared memory, and consumed there: scores against
+// 2 for dense bf16), decoded tile by tile on the chip, and consumed there: scores against
 // the G query heads that share a KV head, online softmax in fp32, weighted sum of the decoded V
-// tile.  The cache is split along the sequence (flash-decoding): grid = (splits, B * Hkv), each
+// tile.  The cache is split along the sequence (flash-decoding): grid = (B * Hkv, splits), each
 // CTA owns a run of 128-token tiles of one (batch, kv head) and leaves (max, sum, numerator)
-// partials that a second kernel combines.  The plain kernel comes first; the pipelined tensor-core
-// one, which every call takes unless ADACODE_ATTN_SIMPLE=1 is set, follows below.
+// partials that a second kernel combines.  Every call takes the pipelined tensor-core kernel, which decodes in
+// registers.  The plain one, which comes first, is a second opinion on it for tests and for failure analysis, with
+// other arithmetic (fp32 on the CUDA cores) and another decode (tables, tiles in shared memory); it runs only with
+// ADACODE_ATTN_SIMPLE=1.
 //
 // The reference has no such kernel (its attention path materialises dense K/V first; the module
 // its validation script imports, ops/kv_attention.py, is absent from its tree), so numerics are

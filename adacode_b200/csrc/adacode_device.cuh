@@ -222,19 +222,11 @@ __device__ __forceinline__ int warp_scan4(const int cnt[kCPT], int incl[kCPT]) {
 }
 
 // ---- table-driven decode -------------------------------------------------------------------
-// The integer pipe (half the rate of the issue slots) is what limits these kernels, so the
-// per-element shifts, masks and adds of the decode are replaced by one shared-memory lookup per
-// pair (or quadruple, or octet) of codes: the table maps a run of packed code bits to the
-// finished exponent fields of the corresponding bf16 pairs, `(e0 << 7) | (e1 << 23)`, with the
-// window's left edge already added (and 0 for code 0).  Index width: 8 bits for N = 1, 2, 4; 6 bits for N = 3.
-template <int N>
-struct DecodeLut {
-    static constexpr int index_bits = (N == 3) ? 6 : 8;
-    static constexpr int elems = index_bits / N;          // elements covered by one lookup
-    static constexpr int words = elems / 2;               // 32-bit pair words per entry
-    static constexpr int entries = 1 << index_bits;
-};
-
+// One shared-memory lookup per pair (or quadruple, or octet) of codes: the table maps a run of packed
+// code bits to the finished exponent fields of the corresponding bf16 pairs, `(e0 << 7) | (e1 << 23)`,
+// with the window's left edge already added (and 0 for code 0).  Index width: 8 bits for N = 1, 2, 4; 6 bits
+// for N = 3.  Only the plain attention kernel decodes this way, which makes it independent of the decode
+// in registers below that it is there to check.
 __device__ __forceinline__ void build_decode_lut(uint32_t *lut, int N, int left, int n_threads) {
     const int index_bits = (N == 3) ? 6 : 8;
     const int words = (index_bits / N) / 2;

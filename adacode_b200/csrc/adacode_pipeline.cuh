@@ -1,7 +1,8 @@
 // Pipelined pack / unpack kernels: tiles are staged through shared memory with asynchronous
 // bulk copies (the untiled form of TMA) so that the loads of the next units are in flight
-// while the current unit is processed, and results leave through shared memory with bulk
-// stores.  Included by adacode_kernels.cu inside its anonymous namespace.
+// while the current unit is processed.  Unpacked rows and the sign/mantissa plane are stored straight from
+// registers, packed codes and escapes leave through shared memory with bulk stores.  Included by
+// adacode_kernels.cu and, without the pack part, by adacode_attention.cu inside their anonymous namespaces.
 //
 // One CTA = W consumer warps + 1 producer warp, persistent over tiles.  A "unit" is a run of
 // whole token rows of one tile, at most W x 1024 elements.  Two geometries are built: the wide one
@@ -14,11 +15,10 @@
 //   producer warp : waits for a free stage, issues the unit's bulk loads (sign/mantissa and
 //                   code planes, or source rows) against the stage's "full" mbarrier, and
 //                   stages the tile's escape bytes with plain loads
-//   consumer warps: wait on "full", work out of shared memory, signal "empty", and hand the
-//                   finished unit to a bulk store
-// A unit leaves through ONE bulk store per plane: the copy engine has a sizeable cost per
-// operation, and a variant in which every consumer warp stored its own 2 KB slice (no CTA-wide
-// barrier inside a unit) ran 40 % slower than this one.
+//   consumer warps: wait on "full", work out of shared memory, signal "empty"
+// The pack kernel's codes and escapes of a unit leave through ONE bulk store each: the copy engine has a
+// sizeable cost per operation, and a variant in which every consumer warp stored its own slice (no
+// CTA-wide barrier inside a unit) ran 40 % slower.
 // Every mbarrier wait is bounded: after kMaxPolls failed polls the waiter records
 // ADACODE_STATUS_TIMEOUT in the status word and carries on (the result is then wrong but the
 // kernel still reaches every barrier and terminates).
@@ -990,8 +990,9 @@ __device__ __forceinline__ void pack_unit(PackSmemT<G> &s, const PackStageT<G> &
         }
     }
     if (zc[0] + zc[1] != 0) {
-        // One loop over the escapes of both chunks (see unpack_unit): chunk 0 elements 0..15, then
-        // chunk 1 elements 0..15, from the most significant bit of the mask.
+        // One loop over the escapes of both chunks: chunk 0 elements 0..15, then chunk 1 elements 0..15, from the
+        // most significant bit of the mask.  A warp iterates as often as its busiest lane has escapes, and counts over
+        // 32 elements vary much less than those over 8, so this takes about half the iterations of four loops.
         uint32_t todo = (compress_slots<N>(zm[0][0]) << 24) | (compress_slots<N>(zm[0][1]) << 16) |
                         (compress_slots<N>(zm[1][0]) << 8) | compress_slots<N>(zm[1][1]);
         uint8_t *out = s.esc + wprefix + incl[0] - zc[0];

@@ -325,7 +325,7 @@ size_t adacode_decode_attn_workspace_bytes(int B, int Hq, int D, int n_splits);
  * records in sequence order; dst_seq_offset is ignored) followed by tail_len dense bf16
  * tokens (the cache's not-yet-packed residual, element strides tail_stride_b/h/s, unit
  * stride along D).  Every cached token is visible to the query (no mask).  The planes are
- * decoded tile by tile in shared memory, so HBM sees the packed bytes only; the work is
+ * decoded tile by tile in registers, so HBM sees the packed bytes only; the work is
  * split along the sequence into n_splits parts (<= 0: chosen by the library; at most 128)
  * whose partial results a second kernel merges.  A CTA serves up to sixteen query heads of a group;
  * larger groups are served by ceil(G / 16) CTAs that each decode the tiles again.
@@ -335,7 +335,8 @@ size_t adacode_decode_attn_workspace_bytes(int B, int Hq, int D, int n_splits);
  *   validation script imports for a fused path (ops/kv_attention.py) is not in its tree.
  * Arithmetic: bf16 x bf16 tensor-core products with fp32 accumulation; probabilities enter the weighted
  * sum as two bf16 terms (head_dim 64: three, all of their 24 bits) and its denominator in fp32; output
- * rounded to bf16 (nearest even).  Requirements: seq_tile == 128, D in {64, 128}, q with unit stride
+ * rounded to bf16 (nearest even).  A NaN score makes its head NaN; an infinite or NaN value gives its column what
+ * it has in exact arithmetic with weights above 0; a head all of whose scores are minus infinity gives 0.  Requirements: seq_tile == 128, D in {64, 128}, q with unit stride
  * along D and element strides q_stride_b/h, out contiguous [B][Hq][D].
  */
 int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride_h,

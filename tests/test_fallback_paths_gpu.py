@@ -1,6 +1,5 @@
 """The kernels behind the environment switches: ``ADACODE_DISABLE_PIPELINE=1`` (direct pack /
-unpack kernels for every shape) and ``ADACODE_ATTN_SIMPLE=1`` (plain decode attention for
-head_dim 128).  The switches are read once per process, so each case runs in a child process
+unpack kernels for every shape) and ``ADACODE_ATTN_SIMPLE=1`` (plain decode attention).  The switches are read once per process, so each case runs in a child process
 that checks itself against the CPU oracle (bytes) or fp32 attention (tolerance of
 tests/test_attention_gpu.py)."""
 import os

@@ -643,12 +643,12 @@ def unpack_segments(segments: Sequence[TiledCompressedTensor], dst: torch.Tensor
 
 def _check_one_shape(segs: Sequence, shape0: tuple) -> None:
     """Refuse segments of another [batch, kv_heads, seq_tile, head_dim]; segments of one chunk have one shape."""
-    chunk = None
-    for seg in segs:
-        if type(seg) is SegmentRef:
-            if seg.chunk is chunk:
-                continue
-            chunk = seg.chunk
+    try:
+        chunk = segs[0].chunk                 # (of most segments: the prefill's)
+        rest = [seg for seg in segs if seg.chunk is not chunk]
+    except AttributeError:                    # others than SegmentRef among them
+        chunk, rest = None, segs
+    for seg in rest if chunk is None else (segs[0], *rest):
         if tuple(seg.original_shape) != shape0:
             raise ValueError('all segments of one call must share [batch, kv_heads, seq_tile, head_dim]')
 

@@ -78,7 +78,8 @@ class _DenseWorkspace:
         if buf is None or buf.numel() < n:
             buf = torch.empty(max(int(n * 1.25), 1 << 16), dtype=torch.bfloat16, device=device)
             self._bufs[key] = buf
-        return buf[:n].view(shape)
+        B, H, T, D = shape
+        return buf.as_strided(shape, (H * T * D, T * D, D, 1))
 
     def release(self):
         self._bufs.clear()

@@ -122,3 +122,19 @@ def test_tails_longer_than_the_packed_part(cuda_device, H, D, rows):
     for t, (_, _, dense, _) in zip(x, parts):
         assert torch.equal(dense.view(torch.int16), t.view(torch.int16))
     codec.check_device_status(cuda_device)
+
+
+@pytest.mark.parametrize('workspace,prompt', [('shared', 60), ('shared', 300), ('layer', 300)])
+def test_gradients_of_appended_tokens(cuda_device, workspace, prompt):
+    cache = _cache(workspace)
+    k, v = (synth.kv_tensor((2, 2, prompt, 64), seed=s).to(cuda_device) for s in (1, 2))
+    cache.update(k, v, 0)
+    kn, vn = (synth.kv_tensor((2, 2, 3, 64), seed=s).to(cuda_device).requires_grad_() for s in (3, 4))
+    dk, dv = cache.update(kn, vn, 0)
+    assert torch.equal(dk[:, :, prompt:], kn) and torch.equal(dv[:, :, :prompt], v)
+    w = torch.randn(2, 2, prompt + 3, 64, device=cuda_device)
+    ((dk.float() + 2 * dv.float()) * w).sum().backward()
+    want = w[:, :, prompt:].to(torch.bfloat16)
+    assert torch.equal(kn.grad, want) and torch.equal(vn.grad, 2 * want)
+    from adacode_b200.float_cache_utils import _GLOBAL_WORKSPACE
+    _GLOBAL_WORKSPACE.release()               # (it took part in this graph)

@@ -13,6 +13,7 @@
 // The reference has no such kernel (its attention path materialises dense K/V first; the module
 // its validation script imports, ops/kv_attention.py, is absent from its tree), so numerics are
 // checked against an fp32 PyTorch attention over the dense cache.
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -9,6 +9,7 @@
 //            warp-level access is a contiguous run and the escape rank of an element is
 //            a warp scan plus an 8-entry cross-warp prefix
 // Both kernels are bandwidth work: no tensor cores, no reshaping into GEMMs.
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -859,11 +860,54 @@ int launch_unpack_pipe(const UnpackPipeArgs &a, cudaStream_t st) {
     return launch_unpack_pipe(ja, st);
 }
 
+// The driver's encoder of tensor maps (the library is not linked against the driver), or null.
+decltype(&cuTensorMapEncodeTiled) tensor_map_encoder() {
+    static const auto encode = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            (void)cudaGetLastError();
+            f = nullptr;
+        }
+        return (decltype(&cuTensorMapEncodeTiled))f;
+    }();
+    return encode;
+}
+
+// A tensor map of a pack source whose rows do not follow each other: boxes of `unit_rows` rows of one (head, batch).
+// The kernel copies sources without one (false) row by row.  A box has at most 256 entries along a dimension, which
+// is why a row is taken as 8-byte words; its first word is always word 0, so that every copy starts on a 16-byte boundary.
+// One copy per unit in place of one per row, whose issue bounded the kernel: a [1, S, 8, D] projection of 21 M elements,
+// 3 bits, the pack kernel alone: D = 128 33.5 -> 20.4 us, 64 34.1 -> 19.3, 16 33.3 -> 14.3, [1, S, 4, D] 256 25.1 -> 22.2,
+// 512 28.3 -> 27.2, 1024 27.4 -> 26.8; a contiguous source takes 19.7, 19.4, 14.2, 21.3, 26.1 and 26.6.  Above 1024 columns
+// rows are long enough for copies of their own (2048: 32.6 against 31.2 us contiguous).
+bool map_rows(CUtensorMap &map, const PackJob &jb, int64_t B, int H, int seq_tile, int D, int unit_rows) {
+    const int64_t S = (int64_t)jb.n_blocks * seq_tile;
+    if (jb.ss == D || D % 16 != 0 || D / 4 > 256 || unit_rows > 256) return false;
+    // (a dimension of one entry may have any stride)
+    const int64_t ss = S > 1 ? jb.ss : D, sh = H > 1 ? jb.sh : D, sb = B > 1 ? jb.sb : D;
+    constexpr int64_t kMost = 1ll << 38;
+    if (ss <= 0 || sh <= 0 || sb <= 0 || ss >= kMost || sh >= kMost || sb >= kMost || S >= (1ll << 31) || B >= (1ll << 31)) return false;
+    const auto encode = tensor_map_encoder();
+    if (!encode) return false;
+    const cuuint64_t dims[4] = {(cuuint64_t)D / 4, (cuuint64_t)S, (cuuint64_t)H, (cuuint64_t)B};
+    const cuuint64_t strides[3] = {(cuuint64_t)ss * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
+    const cuuint32_t box[4] = {(cuuint32_t)D / 4, (cuuint32_t)unit_rows, 1, 1}, step[4] = {1, 1, 1, 1};
+    return encode(&map, CU_TENSOR_MAP_DATA_TYPE_INT64, 4, const_cast<uint16_t *>(jb.src), dims, strides, box, step,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <class G, typename Kernel>
 int launch_pack_kernel(Kernel kernel, const PackPipeArgs &pa, cudaStream_t st) {
     int rc = ensure_dynamic_smem(kernel, sizeof(PackSmemT<G>));
     if (rc != ADACODE_OK) return rc;
-    return launch_dependent(kernel, dim3(grid_for(pa.n_tiles, G::kCtasPerSm)), G::kThreads, sizeof(PackSmemT<G>), st, pa);
+    PackKernelArgs ka = {};
+    ka.pa = pa;
+    for (int j = 0; j < kMaxJobs; ++j)
+        ka.use_map[j] = j < pa.n_jobs && map_rows(ka.map[j], pa.job[j], pa.BH / pa.H, pa.H, pa.seq_tile, pa.D, pa.unit_rows);
+    return launch_dependent(kernel, dim3(grid_for(pa.n_tiles, G::kCtasPerSm)), G::kThreads, sizeof(PackSmemT<G>), st, ka);
 }
 
 template <int N, class G>

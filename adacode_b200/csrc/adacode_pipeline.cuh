@@ -92,6 +92,14 @@ __device__ __forceinline__ void bulk_load(void *sdst, const void *gsrc, uint32_t
                  "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
+// the box of a four-dimensional tensor map that begins at element 0 of row `row` of (head, batch)
+__device__ __forceinline__ void tensor_load(void *sdst, const CUtensorMap *map, int row, int head, int batch, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
+            smem_u32(sdst)),
+        "l"(map), "r"(0), "r"(row), "r"(head), "r"(batch), "r"(smem_u32(bar))
+        : "memory");
+}
 // shared -> global bulk copy, tracked by the issuing thread's bulk group
 __device__ __forceinline__ void bulk_store(void *gdst, const void *ssrc, uint32_t bytes) {
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gdst), "r"(smem_u32(ssrc)),
@@ -764,6 +772,14 @@ struct PackPipeArgs {
     uint32_t poll_limit;      // bound of every on-chip wait (kMaxPolls unless a test lowered it)
 };
 
+// What the pack kernel gets.  map[j] describes job j's source as rows of D elements over (row, head, batch) if
+// use_map[j]: sources whose rows do not follow each other, e.g. a [B, S, H, D] projection seen as [B, H, S, D].
+struct PackKernelArgs {
+    PackPipeArgs pa;
+    int use_map[kMaxJobs];
+    alignas(64) CUtensorMap map[kMaxJobs];
+};
+
 __device__ __forceinline__ int job_of_tile(const PackPipeArgs &pa, int64_t tile) {
     int j = 0;
     while (j + 1 < pa.n_jobs && tile >= pa.job[j + 1].tile0) ++j;
@@ -1024,7 +1040,8 @@ __device__ __forceinline__ void pack_unit(PackSmemT<G> &s, const PackStageT<G> &
 }
 
 template <int N, bool HIST, class G>
-__global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const __grid_constant__ PackPipeArgs pa) {
+__global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const __grid_constant__ PackKernelArgs ka) {
+    const PackPipeArgs &pa = ka.pa;
     static_assert(G::kConsumers >= 256, "one consumer thread per histogram bin");
     extern __shared__ __align__(128) uint8_t smem_raw[];
     PackSmemT<G> &s = *reinterpret_cast<PackSmemT<G> *>(smem_raw);
@@ -1062,7 +1079,7 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const 
             const int bh = (int)(lt - blk * pa.BH);
             const int b = bh / pa.H, h = bh - b * pa.H;
             const uint16_t *tsrc = jb.src + (int64_t)b * jb.sb + (int64_t)h * jb.sh + blk * pa.seq_tile * jb.ss;
-            const bool rows_contig = (jb.ss == pa.D);
+            const bool rows_contig = (jb.ss == pa.D), use_map = ka.use_map[j] != 0;
             for (int u = 0; u < upt; ++u, ++it) {
                 const int stg = it % kStages;
                 PackStageT<G> &st = s.stage[stg];
@@ -1082,12 +1099,15 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const 
                     m.first_unit_of_tile = (u == 0);
                     m.last_unit_of_tile = (u == upt - 1);
                     m.job = j;
-                    mbar_arrive_expect_tx(&s.full[stg], (uint32_t)elems * 2u);
+                    // (a box is a whole unit; what lies behind the last rows of a tile is loaded and not used)
+                    mbar_arrive_expect_tx(&s.full[stg], (uint32_t)(use_map ? unit_rows * pa.D : elems) * 2u);
                 }
                 __syncwarp();
                 const uint16_t *usrc = tsrc + (int64_t)row0 * jb.ss;
                 if (rows_contig) {
                     if (lane == 0) bulk_load(st.in, usrc, (uint32_t)elems * 2u, &s.full[stg]);
+                } else if (use_map) {
+                    if (lane == 0) tensor_load(st.in, &ka.map[j], (int)(blk * pa.seq_tile) + row0, h, b, &s.full[stg]);
                 } else {
                     for (int r = lane; r < rows; r += 32)
                         bulk_load(st.in + r * pa.D, usrc + (int64_t)r * jb.ss, (uint32_t)pa.D * 2u, &s.full[stg]);

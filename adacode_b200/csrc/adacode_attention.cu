@@ -3,8 +3,8 @@
 // The packed planes are read straight from HBM (1 + n/8 + p bytes per cached element instead of
 // 2 for dense bf16), decoded tile by tile on the chip, and consumed there: scores against
 // the G query heads that share a KV head, online softmax in fp32, weighted sum of the decoded V
-// tile.  The cache is split along the sequence (flash-decoding): grid = (B * Hkv, splits), each
-// CTA owns a run of 128-token tiles of one (batch, kv head) and leaves (max, sum, numerator)
+// tile.  The cache is split along the sequence (flash-decoding): each CTA owns a run of 128-token tiles of one
+// (batch, kv head), or of several that follow each other, and leaves (max, sum, numerator)
 // partials that a second kernel combines.  Every call takes the pipelined tensor-core kernel, which decodes in
 // registers.  The plain one, which comes first, is a second opinion on it for tests and for failure analysis, with
 // other arithmetic (fp32 on the CUDA cores) and another decode (tables, tiles in shared memory); it runs only with
@@ -45,11 +45,27 @@ struct AttnArgs {
     long long t_sb, t_sh, t_ss;
     int B, Hq, Hkv, G, D;
     float scale;
-    int n_splits;
+    int n_splits;                 // partial results kept per (batch, KV head): as many as its row is cut into, or more
     float *part_o;                // [B*Hkv][splits][G][D]
     float *part_ml;               // [B*Hkv][splits][G][2]
     int32_t *status;
+    // The work is rows (batch, KV head, group of query heads) of `items` tiles each, one after the other.  A CTA takes a
+    // run of consecutive items: every `cut_items` of them are cut into `cut_ctas` runs, the r-th from cut_items r / cut_ctas
+    // on.  cut_items is either one row (whole splits) or all rows together, in which case a run may end in one row
+    // and go on in the next.  (cut_items x cut_ctas < 2**31)
+    int items, head_groups, heads_per_row;
+    int cut_items, cut_ctas;
 };
+
+// Item at which the run of CTA c begins, and the CTA whose run holds item x.
+__device__ __forceinline__ int run_begin(const AttnArgs &a, int c) {
+    const int cut = c / a.cut_ctas, r = c - cut * a.cut_ctas;
+    return cut * a.cut_items + a.cut_items * r / a.cut_ctas;
+}
+__device__ __forceinline__ int cta_of(const AttnArgs &a, int x) {
+    const int cut = x / a.cut_items, y = x - cut * a.cut_items;
+    return cut * a.cut_ctas + ((y + 1) * a.cut_ctas - 1) / a.cut_items;
+}
 
 struct AttnSmem {
     alignas(16) uint8_t sm[kTileTokens * kMaxD];          // staged sign/mantissa plane of one tile
@@ -181,10 +197,12 @@ __global__ void __launch_bounds__(kAttnThreads) k_decode_attn(const AttnArgs a) 
     extern __shared__ __align__(128) uint8_t smem_raw[];
     AttnSmem &s = *reinterpret_cast<AttnSmem *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int bh = blockIdx.x, split = blockIdx.y;      // (batch, KV head) on x: no 65 535 limit
+    // (it always takes whole splits)
+    const int r = blockIdx.x / a.n_splits, split = blockIdx.x - r * a.n_splits;
+    const int bh = r / a.head_groups;
     const int b = bh / a.Hkv, hkv = bh - b * a.Hkv;
-    // query heads of the group are handled eight at a time: blockIdx.z picks the eight
-    const int Gt = a.G, gz = blockIdx.z * kMaxGroup;
+    // query heads of the group are handled eight at a time
+    const int Gt = a.G, gz = (r - bh * a.head_groups) * kMaxGroup;
     const int G = Gt - gz < kMaxGroup ? Gt - gz : kMaxGroup, D = a.D;
 
     // queries of this KV head's group, as fp32, pre-multiplied by the softmax scale
@@ -197,10 +215,7 @@ __global__ void __launch_bounds__(kAttnThreads) k_decode_attn(const AttnArgs a) 
     if (tid == 0) s.lut_nbits[0] = s.lut_nbits[1] = 0;
     __syncthreads();
 
-    const int tail_tiles = (a.tail_len + kTileTokens - 1) / kTileTokens;
-    const int items = a.n_seg + tail_tiles;
-    const int first = (int)((long long)items * split / a.n_splits);
-    const int last = (int)((long long)items * (split + 1) / a.n_splits);
+    const int first = run_begin(a, blockIdx.x) - r * a.items, last = run_begin(a, blockIdx.x + 1) - r * a.items;
 
     float m[kMaxGroup], l[kMaxGroup], o[kMaxGroup];     // o: column `tid` of the numerator
 #pragma unroll
@@ -372,12 +387,15 @@ __global__ void __launch_bounds__(GROUPS * D) k_decode_attn_combine(const __grid
     __shared__ unsigned s_flags[D];
     const float *__restrict__ part_o = a.part_o;
     const float *__restrict__ part_ml = a.part_ml;
-    const int G = a.G, n_splits = a.n_splits;
+    const int G = a.G;
     const int tid = threadIdx.x, lane = tid & 31;
     const int bhq = blockIdx.x;
     const int b = bhq / a.Hq, hq = bhq - b * a.Hq;
     const int hkv = hq / G, g = hq - hkv * G, bh = b * a.Hkv + hkv;
-    const long long base = (long long)bh * n_splits;
+    const long long base = (long long)bh * a.n_splits;
+    // parts that this head's row was cut into
+    const int x = (bh * a.head_groups + g / a.heads_per_row) * a.items;
+    const int n_splits = cta_of(a, x + a.items - 1) - cta_of(a, x) + 1;
     // launched as a programmatic dependent of the attention kernel: wait for its partial results
     asm volatile("griddepcontrol.wait;" ::: "memory");
     float mx = -INFINITY;
@@ -454,7 +472,7 @@ struct AttnPipeSmem {
     AttnStage<D> stage[kAStages];
     alignas(16) UnitMeta meta[kAStages];
     alignas(16) uint16_t q[16 * (D + 8)];         // queries (sixteen heads per CTA only)
-    alignas(16) TileSrc src[32];                  // where the units of the current run of 32 lie
+    alignas(16) TileSrc src[32];                  // where the current 32 units lie
     float m[kAWarps][16];                         // running max per warp and head (log2 domain)
     float l[kAWarps][16];
     alignas(8) uint64_t full[kAStages];
@@ -783,21 +801,17 @@ __device__ __forceinline__ void dense_slab(AttnState<D, HG> &st, const uint16_t 
     }
 }
 
-struct AttnPipeArgs {
-    AttnArgs a;
-    UnpackPipeArgs k, v;      // table form, used through resolve_tile
-};
+// See the merge of the warps: a permutation of the D / 16 pairs of a column group (of eight) for heads 2 j and 2 j + 1.
+template <int D>
+__device__ __forceinline__ int merge_swizzle(int i, int j) {
+    return D == 128 ? (i >> 1) ^ ((j & 1) * 4) : (i >> 2) ^ ((j & 1) * 2);
+}
 
 template <int D, int HG>
-__global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_constant__ AttnPipeArgs pa) {
+__global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_constant__ AttnArgs a) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     AttnPipeSmem<D> &s = *reinterpret_cast<AttnPipeSmem<D> *>(smem_raw);
-    const AttnArgs &a = pa.a;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int bh = blockIdx.x, split = blockIdx.y;      // (batch, KV head) on x: no 65 535 limit
-    const int b = bh / a.Hkv, hkv = bh - b * a.Hkv;
-    const int Gt = a.G, gz = blockIdx.z * 8 * HG;        // 8 or 16 query heads of the group per CTA
-    const int G = Gt - gz < 8 * HG ? Gt - gz : 8 * HG;
 
     if (tid == 0) {
 #pragma unroll
@@ -813,171 +827,217 @@ __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_
         m.elems = 0, m.left = 0, m.nbits = 1, m.first_unit_of_tile = 1, m.ds = 0;
     }
     __syncthreads();
+    // this CTA's items [begin, end), and the units that are to be decoded for them (two per packed item)
+    const int begin = run_begin(a, blockIdx.x), end = run_begin(a, blockIdx.x + 1);
+    const int row0 = begin / a.items, item0 = begin - row0 * a.items, row1 = end / a.items;
+    const int n_units = 2 * ((row1 - row0) * a.n_seg + min(end - row1 * a.items, a.n_seg) - min(item0, a.n_seg));
     // launched as a programmatic dependent of its predecessor in the stream: no global memory is touched above
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    const int tail_tiles = (a.tail_len + kTileTokens - 1) / kTileTokens;
-    const int items = a.n_seg + tail_tiles;
-    const int first = (int)((long long)items * split / a.n_splits);
-    const int last = (int)((long long)items * (split + 1) / a.n_splits);
-    const int pk_first = first < a.n_seg ? first : a.n_seg;
-    const int pk_last = last < a.n_seg ? last : a.n_seg;
-    const int n_units = 2 * (pk_last - pk_first);          // K tile, V tile, K tile, ...
+    const int i = lane >> 2, j = lane & 3;
+    const float sc2 = a.scale * kLog2e;                      // scores are kept in the log2 domain
 
-    // Start the copies of unit u (a whole warp; units in ascending order).  The sources of 32 units are looked
-    // up at a time, one per lane: two dependent round trips to global memory for all of them.
-    const auto issue = [&](int u) {
-        if (u >= n_units) return;
-        if ((u & 31) == 0) {
-            const int mine = u + lane;
-            if (mine < n_units) {
-                const long long tile = (long long)(pk_first + (mine >> 1)) * pa.k.BH + bh;
-                s.src[lane] = (mine & 1) ? resolve_tile(pa.v, tile) : resolve_tile(pa.k, tile);
+    // Start the copies of unit n (a whole warp; units in ascending order): K tile, V tile, K tile, ... of the packed items
+    // of the run, from one row on to the next.  The sources of 32 units are looked up at a time, one per lane:
+    // two dependent round trips to global memory for all of them.
+    const auto issue = [&](int n) {
+        if (n >= n_units) return;
+        if ((n & 31) == 0) {
+            const int pair = (n + lane) >> 1;
+            if (n + lane < n_units) {
+                int row = row0, item = item0 + pair;
+                if (item >= a.n_seg) {                       // beyond the first row's (n_units > 0: there are packed items)
+                    const int more = pair - max(0, a.n_seg - item0);
+                    row += 1 + more / a.n_seg;
+                    item = more % a.n_seg;
+                }
+                const adacode_segment sg = ((n + lane) & 1 ? a.vseg : a.kseg)[item];
+                s.src[lane] = resolve_segment_tile(sg, row / a.head_groups, kTileTokens * D, nullptr, 0);
             }
             __syncwarp();
         }
-        const TileSrc &t = s.src[u & 31];
+        const TileSrc &t = s.src[n & 31];
         const EscWindow w = esc_window(t, AttnStage<D>::kEscStage);
-        const int stg = u % kAStages;
+        const int stg = n % kAStages;
         AttnStage<D> &st = s.stage[stg];
         issue_unit(st.sm, st.codes, st.esc + kEscFront, s.meta[stg], &s.full[stg], t, w, 0, kTileTokens, D, nullptr, true, a.status);
     };
     if (warp == 0) {
-        for (int u = 0; u < kAStages - 1; ++u) issue(u);
+#pragma unroll 1
+        for (int n = 0; n < kAStages - 1; ++n) issue(n);
     }
+    int u = 0;                                               // units of this CTA so far
+    for (int x = begin; x < end;) {
+        // the part [first, last) of one row's items
+        const int row = x / a.items, first = x - row * a.items;
+        const int last = min(a.items, first + (end - x));
+        x += last - first;
+        const int bh = row / a.head_groups;
+        const int b = bh / a.Hkv, hkv = bh - b * a.Hkv;
+        const int gz = (row - bh * a.head_groups) * (8 * HG);    // 8 or 16 query heads of the group at a time
+        const int G = min(a.G - gz, 8 * HG);
+        const int u1 = u + 2 * (min(last, a.n_seg) - min(first, a.n_seg));
 
-    const int i = lane >> 2, j = lane & 3;
-    const float sc2 = a.scale * kLog2e;                      // scores are kept in the log2 domain
-    AttnState<D, HG> st;
+        AttnState<D, HG> st;
 #pragma unroll
-    for (int h = 0; h < HG; ++h) {
-        st.m[h] = -INFINITY, st.l[h] = 0.f;
+        for (int h = 0; h < HG; ++h) {
+            st.m[h] = -INFINITY, st.l[h] = 0.f;
 #pragma unroll
-        for (int e = 0; e < D / 16; ++e) st.o[h][e][0] = st.o[h][e][1] = st.o[h][e][2] = st.o[h][e][3] = 0.f;
-    }
-    const uint16_t *qb = a.q + (long long)b * a.q_sb + (long long)(hkv * Gt + gz) * a.q_sh;
-    if constexpr (HG == 1) {                                 // (query rows are only known to be 2-byte aligned)
-        const uint16_t *row = qb + (long long)i * a.q_sh + j * (D / 4);
-#pragma unroll
-        for (int u = 0; u < D / 8; ++u) st.q[u] = i < G ? (uint32_t)row[2 * u] | ((uint32_t)row[2 * u + 1] << 16) : 0u;
-    } else {
-        for (int x = tid; x < 16 * D; x += kAThreads) {
-            const int g = x / D, d = x - g * D;
-            s.q[g * kQRow<D> + d] = g < G ? qb[(long long)g * a.q_sh + d] : (uint16_t)0;
+            for (int e = 0; e < D / 16; ++e) st.o[h][e][0] = st.o[h][e][1] = st.o[h][e][2] = st.o[h][e][3] = 0.f;
         }
-        st.q_smem = s.q + i * kQRow<D> + j * (D / 4);
-        __syncthreads();
-    }
-    for (int u = 0; u < n_units; ++u) {
-        const int stg = u % kAStages;
-        mbar_wait(&s.full[stg], (u / kAStages) & 1, a.status);      // (every lane: the ready case is three instructions)
-        __syncwarp();
-        const AttnStage<D> &stage = s.stage[stg];
-        const UnitMeta &meta = s.meta[stg];
-        int *wt = s.warp_tot[u & 1];
-        if ((u & 1) == 0) {
-            switch (meta.nbits) {
-                case 1: score_unit<1, D, HG>(st, stage, meta, wt, sc2, a.status); break;
-                case 2: score_unit<2, D, HG>(st, stage, meta, wt, sc2, a.status); break;
-                case 3: score_unit<3, D, HG>(st, stage, meta, wt, sc2, a.status); break;
-                default: score_unit<4, D, HG>(st, stage, meta, wt, sc2, a.status); break;
+        const uint16_t *qb = a.q + (long long)b * a.q_sb + (long long)(hkv * a.G + gz) * a.q_sh;
+        if constexpr (HG == 1) {
+            const uint16_t *qrow = qb + (long long)i * a.q_sh + j * (D / 4);
+#pragma unroll
+            for (int w = 0; w < D / 8; ++w) st.q[w] = 0u;
+            if (i < G) {
+                if (((uintptr_t)qrow & 15) == 0) load_row(qrow, true, st.q);
+                else                                             // (query rows are only known to be 2-byte aligned)
+#pragma unroll
+                    for (int w = 0; w < D / 8; ++w) st.q[w] = (uint32_t)qrow[2 * w] | ((uint32_t)qrow[2 * w + 1] << 16);
             }
         } else {
-            switch (meta.nbits) {
-                case 1: accumulate_unit<1, D, HG>(st, stage, meta, wt, a.status); break;
-                case 2: accumulate_unit<2, D, HG>(st, stage, meta, wt, a.status); break;
-                case 3: accumulate_unit<3, D, HG>(st, stage, meta, wt, a.status); break;
-                default: accumulate_unit<4, D, HG>(st, stage, meta, wt, a.status); break;
+            for (int n = tid; n < 16 * D; n += kAThreads) {
+                const int g = n / D, d = n - g * D;
+                s.q[g * kQRow<D> + d] = g < G ? qb[(long long)g * a.q_sh + d] : (uint16_t)0;
             }
+            st.q_smem = s.q + i * kQRow<D> + j * (D / 4);
+            __syncthreads();
         }
-        // every warp has passed this unit's barrier, so the stage of the unit before it is free
-        if (warp == (u & (kAWarps - 1))) issue(u + kAStages - 1);
-    }
-    // dense residual tiles that fall into this split, a slab per warp
-    const int tl_first = first > a.n_seg ? first - a.n_seg : 0;
-    const int tl_last = last > a.n_seg ? last - a.n_seg : 0;
-    const long long toff = (long long)b * a.t_sb + (long long)hkv * a.t_sh;
-    const bool wide = ((((uintptr_t)a.k_tail | (uintptr_t)a.v_tail) & 15) | (uintptr_t)((a.t_sb | a.t_sh | a.t_ss) & 7)) == 0;
-    for (int t = tl_first; t < tl_last; ++t) {
-        const int t0 = t * kTileTokens + warp * 16;
-        const int valid = a.tail_len - t0 < 16 ? a.tail_len - t0 : 16;
-        if (valid > 0)
-            dense_slab(st, a.k_tail + toff + t0 * a.t_ss, a.v_tail + toff + t0 * a.t_ss, a.t_ss, valid, wide, sc2);
-    }
+        for (; u < u1; ++u) {
+            const int stg = u % kAStages;
+            mbar_wait(&s.full[stg], (u / kAStages) & 1, a.status);      // (every lane: the ready case is three instructions)
+            __syncwarp();
+            const AttnStage<D> &stage = s.stage[stg];
+            const UnitMeta &meta = s.meta[stg];
+            int *wt = s.warp_tot[u & 1];
+            if ((u & 1) == 0) {
+                switch (meta.nbits) {
+                    case 1: score_unit<1, D, HG>(st, stage, meta, wt, sc2, a.status); break;
+                    case 2: score_unit<2, D, HG>(st, stage, meta, wt, sc2, a.status); break;
+                    case 3: score_unit<3, D, HG>(st, stage, meta, wt, sc2, a.status); break;
+                    default: score_unit<4, D, HG>(st, stage, meta, wt, sc2, a.status); break;
+                }
+            } else {
+                switch (meta.nbits) {
+                    case 1: accumulate_unit<1, D, HG>(st, stage, meta, wt, a.status); break;
+                    case 2: accumulate_unit<2, D, HG>(st, stage, meta, wt, a.status); break;
+                    case 3: accumulate_unit<3, D, HG>(st, stage, meta, wt, a.status); break;
+                    default: accumulate_unit<4, D, HG>(st, stage, meta, wt, a.status); break;
+                }
+            }
+            // every warp has passed this unit's barrier, so the stage of the unit before it is free
+            if (warp == (u & (kAWarps - 1))) issue(u + kAStages - 1);
+        }
+        // dense residual tiles that fall into this part, a slab per warp
+        const int tl_first = first > a.n_seg ? first - a.n_seg : 0;
+        const int tl_last = last > a.n_seg ? last - a.n_seg : 0;
+        const long long toff = (long long)b * a.t_sb + (long long)hkv * a.t_sh;
+        const bool wide = ((((uintptr_t)a.k_tail | (uintptr_t)a.v_tail) & 15) | (uintptr_t)((a.t_sb | a.t_sh | a.t_ss) & 7)) == 0;
+        for (int t = tl_first; t < tl_last; ++t) {
+            const int t0 = t * kTileTokens + warp * 16;
+            const int valid = a.tail_len - t0 < 16 ? a.tail_len - t0 : 16;
+            if (valid > 0)
+                dense_slab(st, a.k_tail + toff + t0 * a.t_ss, a.v_tail + toff + t0 * a.t_ss, a.t_ss, valid, wide, sc2);
+        }
 
-    // the combine kernel may be set up from here on (it waits for this launch to complete before it reads)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // ---------------- merge the warps ----------------
+        // the combine kernel may be set up from here on (it waits for this launch to complete before it reads)
+        if (x >= end) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        // ---------------- merge the warps ----------------
 #pragma unroll
-    for (int h = 0; h < HG; ++h) {
-        st.l[h] += __shfl_xor_sync(kFull, st.l[h], 1);
-        st.l[h] += __shfl_xor_sync(kFull, st.l[h], 2);
-        if (j == 0) {
-            s.m[warp][8 * h + i] = st.m[h];
-            s.l[warp][8 * h + i] = st.l[h];
-        }
-    }
-    __syncthreads();                       // also: every unit has been read, the stages are free
-    // numerators of all warps, one group of eight heads at a time: [warp][head][d], rows padded by four words
-    constexpr int kRow = D + 4;
-    float *acc = reinterpret_cast<float *>(s.stage);
-    static_assert(sizeof(s.stage) >= sizeof(float) * kAWarps * 8 * kRow, "the stages hold the numerators of the merge");
-    const long long slot = (long long)bh * a.n_splits + split;
-#pragma unroll
-    for (int h = 0; h < HG; ++h) {
-        float f[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int g = 8 * h + 2 * j + u;
-            float mx = s.m[0][g];
-#pragma unroll
-            for (int w = 1; w < kAWarps; ++w) mx = fmaxf(mx, s.m[w][g]);
-            f[u] = s.m[warp][g] == -INFINITY ? 0.f : exp2f(s.m[warp][g] - mx);
-        }
-#pragma unroll
-        for (int e = 0; e < D / 16; ++e) {
-            float *r0 = acc + (warp * 8 + 2 * j) * kRow + i * (D / 8) + 2 * e, *r1 = r0 + kRow;
-            *reinterpret_cast<float2 *>(r0) = make_float2(st.o[h][e][0] * f[0], st.o[h][e][2] * f[0]);
-            *reinterpret_cast<float2 *>(r1) = make_float2(st.o[h][e][1] * f[1], st.o[h][e][3] * f[1]);
-        }
-        __syncthreads();
-        for (int x = tid; x < 8 * D; x += kAThreads) {
-            const int g = x / D, d = x - g * D;
-            if (8 * h + g < G) {
-                float v = 0.f;
-#pragma unroll
-                for (int w = 0; w < kAWarps; ++w) v += acc[(w * 8 + g) * kRow + d];
-                a.part_o[(slot * Gt + gz + 8 * h + g) * D + d] = v;
+        for (int h = 0; h < HG; ++h) {
+            st.l[h] += __shfl_xor_sync(kFull, st.l[h], 1);
+            st.l[h] += __shfl_xor_sync(kFull, st.l[h], 2);
+            if (j == 0) {
+                s.m[warp][8 * h + i] = st.m[h];
+                s.l[warp][8 * h + i] = st.l[h];
             }
         }
-        if (h + 1 < HG) __syncthreads();
-    }
-    if (tid < G) {
-        float mx = s.m[0][tid];
+        __syncthreads();                       // also: every unit so far has been read
+        // Numerators of all warps, one group of eight heads at a time: [warp][head][d], in the stage that comes after those
+        // which the next row's first units are on their way to.  The pairs of a column group of sixteen are
+        // permuted so that a warp's writes, eight column groups of four heads, spread over the banks.
+        float *acc = reinterpret_cast<float *>(&s.stage[(u + kAStages - 1) % kAStages]);
+        static_assert(sizeof(AttnStage<D>) >= sizeof(float) * kAWarps * 8 * D, "a stage holds the numerators of the merge");
+        const long long slot = (long long)bh * a.n_splits + ((int)blockIdx.x - cta_of(a, row * a.items));
 #pragma unroll
-        for (int w = 1; w < kAWarps; ++w) mx = fmaxf(mx, s.m[w][tid]);
-        float l = 0.f;
+        for (int h = 0; h < HG; ++h) {
+            float f[2];
 #pragma unroll
-        for (int w = 0; w < kAWarps; ++w) l += s.m[w][tid] == -INFINITY ? s.l[w][tid] : s.l[w][tid] * exp2f(s.m[w][tid] - mx);
-        a.part_ml[(slot * Gt + gz + tid) * 2 + 0] = mx == -INFINITY ? -INFINITY : mx / kLog2e;   // natural-log domain
-        a.part_ml[(slot * Gt + gz + tid) * 2 + 1] = l;
+            for (int w = 0; w < 2; ++w) {
+                const int g = 8 * h + 2 * j + w;
+                float mx = s.m[0][g];
+#pragma unroll
+                for (int k = 1; k < kAWarps; ++k) mx = fmaxf(mx, s.m[k][g]);
+                f[w] = s.m[warp][g] == -INFINITY ? 0.f : exp2f(s.m[warp][g] - mx);
+            }
+#pragma unroll
+            for (int e = 0; e < D / 16; ++e) {
+                float *r0 = acc + (warp * 8 + 2 * j) * D + i * (D / 8) + 2 * (e ^ merge_swizzle<D>(i, j)), *r1 = r0 + D;
+                *reinterpret_cast<float2 *>(r0) = make_float2(st.o[h][e][0] * f[0], st.o[h][e][2] * f[0]);
+                *reinterpret_cast<float2 *>(r1) = make_float2(st.o[h][e][1] * f[1], st.o[h][e][3] * f[1]);
+            }
+            __syncthreads();
+            for (int n = tid; n < 8 * D; n += kAThreads) {
+                const int g = n / D, d = n - g * D;
+                if (8 * h + g < G) {
+                    const int at = d ^ (2 * merge_swizzle<D>(d / (D / 8), g >> 1));
+                    float v = 0.f;
+#pragma unroll
+                    for (int w = 0; w < kAWarps; ++w) v += acc[(w * 8 + g) * D + at];
+                    a.part_o[(slot * a.G + gz + 8 * h + g) * D + d] = v;
+                }
+            }
+            if (h + 1 < HG) __syncthreads();
+        }
+        if (tid < G) {
+            float mx = s.m[0][tid];
+#pragma unroll
+            for (int w = 1; w < kAWarps; ++w) mx = fmaxf(mx, s.m[w][tid]);
+            float l = 0.f;
+#pragma unroll
+            for (int w = 0; w < kAWarps; ++w) l += s.m[w][tid] == -INFINITY ? s.l[w][tid] : s.l[w][tid] * exp2f(s.m[w][tid] - mx);
+            a.part_ml[(slot * a.G + gz + tid) * 2 + 0] = mx == -INFINITY ? -INFINITY : mx / kLog2e;   // natural-log domain
+            a.part_ml[(slot * a.G + gz + tid) * 2 + 1] = l;
+        }
+        if (x < end) {
+            // (the stage is written again, by a copy, behind the next unit's barrier; the warps' sums by the next row)
+            fence_async_smem();
+            __syncthreads();
+        }
     }
     // do not leave while a copy into this CTA's shared memory may still be in flight (see k_unpack_pipe)
     if (warp == 0 && launch_timed_out(a.status))
-        for (int u = n_units > kAStages ? n_units - kAStages : 0; u < n_units; ++u)
-            mbar_wait(&s.full[u % kAStages], (u / kAStages) & 1, a.status);
+        for (int n = u > kAStages ? u - kAStages : 0; n < u; ++n)
+            mbar_wait(&s.full[n % kAStages], (n / kAStages) & 1, a.status);
 }
 
 static_assert(sizeof(AttnPipeSmem<128>) <= 113 * 1024, "two CTAs of the pipelined kernel must fit one SM");
 
-// Splits per (batch, KV head): the grid should fill a whole number of waves of resident CTAs
-// (two per SM).  One, two and three waves are
-// tried and the fullest wins; fewer waves on ties (more tiles per CTA, less per-CTA overhead).
-int pick_splits(int B, int Hkv, int items) {
+// CTAs of the pipelined kernel that are resident at a time: two per SM.
+long long resident_ctas() {
     int sms = 148;
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long slots = (long long)sms * 2;
+    return (long long)sms * 2;
+}
+
+// CTAs that the items of all rows are dealt out to evenly: all that are resident at a time, fewer if there are
+// fewer items or if a row would be cut into more than kMaxSplits parts (at most n / rows + 2, or n / rows where
+// that is a whole number).
+long long even_ctas(long long rows, int items) {
+    long long n = resident_ctas();
+    if (n > rows * items) n = rows * items;
+    if (n >= rows * kMaxSplits) n = rows * kMaxSplits;
+    else if (n > rows * (kMaxSplits - 1)) n = rows * (kMaxSplits - 1);
+    return n;
+}
+
+// Whole splits per (batch, KV head), for workspaces that hold no more: the grid should fill a whole number of waves
+// of resident CTAs.  One, two and three waves are
+// tried and the fullest wins; fewer waves on ties (more tiles per CTA, less per-CTA overhead).
+int pick_splits(int B, int Hkv, int items) {
+    const long long slots = resident_ctas();
     const long long bh = (long long)B * Hkv;
     int best = 1;
     double best_fill = 0.0;
@@ -1011,7 +1071,7 @@ cudaError_t launch_as_dependent(void (*kernel)(KArgs...), dim3 grid, int threads
 }
 
 template <int D, int HG>
-int launch_attn_pipe(const AttnPipeArgs &pa, dim3 grid, cudaStream_t st) {
+int launch_attn_pipe(const AttnArgs &a, dim3 grid, cudaStream_t st) {
     // the kernel's limit of dynamic shared memory is raised once per device
     static std::atomic<bool> done[64];
     int dev = 0;
@@ -1022,7 +1082,7 @@ int launch_attn_pipe(const AttnPipeArgs &pa, dim3 grid, cudaStream_t st) {
             return ADACODE_ERR_CUDA;
         if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
     }
-    return launch_as_dependent(k_decode_attn_pipe<D, HG>, grid, kAThreads, sizeof(AttnPipeSmem<D>), st, pa) == cudaSuccess
+    return launch_as_dependent(k_decode_attn_pipe<D, HG>, grid, kAThreads, sizeof(AttnPipeSmem<D>), st, a) == cudaSuccess
                ? ADACODE_OK
                : ADACODE_ERR_CUDA;
 }
@@ -1063,10 +1123,33 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
         return ADACODE_ERR_INVALID_ARG;
     const int items = n_segments + (tail_len + kTileTokens - 1) / kTileTokens;
     if (items == 0) return ADACODE_ERR_INVALID_ARG;
-    if (n_splits <= 0) n_splits = pick_splits(B, Hkv * head_groups, items);
+    const long long rows = (long long)B * Hkv * head_groups;
+    if (rows * items >= (1ll << 31)) return ADACODE_ERR_INVALID_ARG;
+    const bool given = n_splits > 0;
+    if (!given) n_splits = pick_splits(B, Hkv * head_groups, items);
     if (n_splits > kMaxSplits) n_splits = kMaxSplits;
     if (workspace_bytes < adacode_decode_attn_workspace_bytes(B, Hq, D, n_splits)) return ADACODE_ERR_WORKSPACE;
+    if (n_splits > items) n_splits = items;                // (the others would be empty)
+    if ((long long)items * n_splits >= (1ll << 31)) n_splits = 1;
+    // Whole splits of every row, or one cut through all rows where that makes the longest run of items shorter: it is worth
+    // the time of about one item to end a row and to begin the next.  256 rows of 33 items on 296 CTAs (keys and values
+    // [32, 8, 4146, 128], 4 heads each): 33 items per CTA and 210 us, or 29 and 187 us; 20 rows of 71 items ([5, 4, 9000, 128], 7 heads each): 6 items and
+    // 54.8 us, or 5 and 52.6 us; 128 rows of 3 items ([64, 2, 300, 128]): 2 either way, 18.4 us whole, 21.1 us cut.
+    long long n_ctas = rows * n_splits, cut_items = items, cut_ctas = n_splits;
+    if (!given && !force_simple) {
+        const long long slots = resident_ctas(), even = even_ctas(rows, items);
+        const int parts = (int)(even % rows == 0 ? even / rows : even / rows + 2);
+        const long long whole_run = (n_ctas + slots - 1) / slots * ((items + n_splits - 1) / n_splits);
+        const long long even_run = (rows * items + even - 1) / even + (even % rows != 0);
+        // (a caller's workspace may be for the whole splits only)
+        if (even_run < whole_run && rows * items * even < (1ll << 31) &&
+            workspace_bytes >= adacode_decode_attn_workspace_bytes(B, Hq, D, parts))
+            n_ctas = cut_ctas = even, cut_items = rows * items, n_splits = parts;
+    }
+    if (n_ctas >= (1ll << 31)) return ADACODE_ERR_INVALID_ARG;
     AttnArgs a;
+    a.items = items, a.head_groups = head_groups, a.heads_per_row = heads_per_cta;
+    a.cut_items = (int)cut_items, a.cut_ctas = (int)cut_ctas;
     a.q = (const uint16_t *)q_bf16, a.q_sb = q_stride_b, a.q_sh = q_stride_h;
     a.kseg = k_segments_dev, a.vseg = v_segments_dev, a.n_seg = n_segments;
     a.k_tail = (const uint16_t *)k_tail_bf16, a.v_tail = (const uint16_t *)v_tail_bf16, a.tail_len = tail_len;
@@ -1077,26 +1160,15 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
     a.status = status;
     cudaStream_t st = (cudaStream_t)stream;
     if (!force_simple) {
-        AttnPipeArgs pa;
-        pa.a = a;
-        UnpackPipeArgs u;
-        u.sign_mant = nullptr, u.codes = nullptr, u.escapes = nullptr, u.escapes_len = 0;
-        u.tile_base = nullptr, u.seg_off = nullptr, u.left = 0, u.nbits = 0;
-        u.tb_stride = 1, u.tb_before = 0;
-        u.H = Hkv, u.BH = B * Hkv, u.seq_tile = kTileTokens, u.D = D, u.tile_elems = kTileTokens * D;
-        u.n_tiles = (long long)n_segments * B * Hkv;
-        u.dst = nullptr, u.db = 0, u.dh = 0, u.ds = 0, u.status = status;
-        pa.k = u, pa.v = u;
-        pa.k.seg = k_segments_dev, pa.v.seg = v_segments_dev;
-        const dim3 grid(B * Hkv, n_splits, head_groups);
-        const int rc = D == 128 ? (two_groups ? launch_attn_pipe<128, 2>(pa, grid, st) : launch_attn_pipe<128, 1>(pa, grid, st))
-                                : (two_groups ? launch_attn_pipe<64, 2>(pa, grid, st) : launch_attn_pipe<64, 1>(pa, grid, st));
+        const dim3 grid((unsigned)n_ctas);
+        const int rc = D == 128 ? (two_groups ? launch_attn_pipe<128, 2>(a, grid, st) : launch_attn_pipe<128, 1>(a, grid, st))
+                                : (two_groups ? launch_attn_pipe<64, 2>(a, grid, st) : launch_attn_pipe<64, 1>(a, grid, st));
         if (rc != ADACODE_OK) return rc;
     } else {
         if (cudaFuncSetAttribute(k_decode_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AttnSmem)) !=
             cudaSuccess)
             return ADACODE_ERR_CUDA;
-        k_decode_attn<<<dim3(B * Hkv, n_splits, head_groups), kAttnThreads, sizeof(AttnSmem), st>>>(a);
+        k_decode_attn<<<dim3((unsigned)n_ctas), kAttnThreads, sizeof(AttnSmem), st>>>(a);
     }
     if (cudaGetLastError() != cudaSuccess) return ADACODE_ERR_CUDA;
     const bool few = n_splits <= kFewSplits;

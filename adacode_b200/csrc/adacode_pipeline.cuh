@@ -236,6 +236,21 @@ struct TileSrc {
     long long ds;
 };
 
+// Tile bh of a segment (its destination, for a caller that has one, is `base` and the segment's offset).
+__device__ __forceinline__ TileSrc resolve_segment_tile(const adacode_segment &sg, int bh, int tile_elems, uint16_t *base, long long ds) {
+    TileSrc t;
+    t.nbits = sg.nbits, t.left = sg.left;
+    t.sm = sg.sign_mant + (long long)bh * tile_elems;
+    t.codes = sg.codes + (long long)bh * (tile_elems * sg.nbits / 8);
+    t.esc = sg.escapes, t.esc_len = sg.escapes_len;
+    const int prev = bh > 0 ? sg.tile_base[bh - 1] : 0;
+    t.esc_start = prev;
+    t.esc_cnt = sg.tile_base[bh] - prev;
+    t.dst = base + sg.dst_seq_offset * ds;
+    t.ds = ds;
+    return t;
+}
+
 __device__ __forceinline__ TileSrc resolve_tile(const UnpackPipeArgs &a, long long tile) {
     TileSrc t;
     const long long blk = tile / a.BH;
@@ -245,14 +260,7 @@ __device__ __forceinline__ TileSrc resolve_tile(const UnpackPipeArgs &a, long lo
     t.ds = a.ds;
     if (a.seg) {
         const adacode_segment sg = a.seg[blk];
-        t.nbits = sg.nbits, t.left = sg.left;
-        t.sm = sg.sign_mant + (long long)bh * a.tile_elems;
-        t.codes = sg.codes + (long long)bh * (a.tile_elems * sg.nbits / 8);
-        t.esc = sg.escapes, t.esc_len = sg.escapes_len;
-        const int prev = bh > 0 ? sg.tile_base[bh - 1] : 0;
-        t.esc_start = prev;
-        t.esc_cnt = sg.tile_base[bh] - prev;
-        t.dst = base + sg.dst_seq_offset * a.ds;
+        t = resolve_segment_tile(sg, bh, a.tile_elems, base, a.ds);
     } else {
         t.nbits = a.nbits, t.left = a.left;
         t.sm = a.sign_mant + tile * a.tile_elems;

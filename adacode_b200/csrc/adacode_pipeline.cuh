@@ -413,13 +413,17 @@ __device__ __noinline__ uint2 gather_escapes(uint32_t z, int r, const uint8_t *e
 // Keys and values of [16, 8, 8192, 128] in one launch (537 M elements), with the lookups, the escape loop and the
 // bulk store that were here before and now: n = 3, 5 % escapes 188.6 -> 177.7 us (5.2 TB/s, 81 % of what a plain
 // copy reaches), n = 2, 34 % escapes 340 -> 177 us, n = 4, 0.1 % escapes 169.7 -> 170.8 us; [1, 8, 20480, 128]
-// 38.8 -> 35.0 us; 4 % less each since computed permutes go without the intrinsic's mask.  The integer pipe is
-// 67 % busy; the rest is waiting at the barrier and for loads.  Tried and slower: no producer warp (one warp in turn refills; the others wait for it at the next
+// 38.8 -> 35.0 us; 4 % less each since computed permutes go without the intrinsic's mask, and 4-5 % less since fewer
+// registers live across the barrier (the escape masks are found again behind it from the codes' nibbles, and a chunk's row
+// and column share a register): n = 3 161.9 -> 154.5 us, n = 2 160.0 -> 154.7 us, n = 4 161.5 -> 160.9 us, the flat
+// form of 4096 x 14336 40.2 -> 38.2 us.  What is left over a plain copy (143 us) is waiting at the barrier and for loads, and
+// the last round of a launch.  Tried and slower: no producer warp (one warp in turn refills; the others wait for it at the next
 // barrier) 201 us; one tile per warp without shared memory or barriers 217-219 us; the finished unit through
-// shared memory and a bulk store, which leaves room for three CTAs per SM, 229 us; five CTAs per SM (spills) 223 us.
+// shared memory and a bulk store, which leaves room for three CTAs per SM, 229 us; five CTAs per SM (spills) 223 us;
+// four chunks per thread in eight warps, three CTAs per SM, 168 us, in four warps, six CTAs, 220 us.
 template <int N, class G>
 __device__ __forceinline__ void unpack_unit(const UnpackStageT<G> &st, const UnitMeta &meta, int *warp_tot, int &consumed,
-                                            const ExpTable &tab, const int (&row)[kPCPT], const int (&col)[kPCPT],
+                                            const ExpTable &tab, const uint32_t (&at)[kPCPT],
                                             uint64_t *empty_bar, int32_t *status, bool broken) {
     constexpr int CB = 2 * N;   // code bytes per 16-element chunk
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -427,7 +431,7 @@ __device__ __forceinline__ void unpack_unit(const UnpackStageT<G> &st, const Uni
     const int chunks = meta.elems >> 4;
     const int c0 = warp * (kPCPT * 32) + lane;
 
-    uint32_t nib[kPCPT][2], z[kPCPT][2];
+    uint32_t nib[kPCPT][2];
     int zc[kPCPT];
 #pragma unroll
     for (int k = 0; k < kPCPT; ++k) {
@@ -436,10 +440,9 @@ __device__ __forceinline__ void unpack_unit(const UnpackStageT<G> &st, const Uni
         load_codes16<N>(st.codes + c * CB, x);             // (beyond the unit's end: what lies there, not used)
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            nib[k][q] = spread8<N>(x[q]);
-            z[k][q] = c < chunks ? escape_mask<N>(nib[k][q]) : 0u;
+            nib[k][q] = c < chunks ? spread8<N>(x[q]) : 0x11111111u;      // (beyond the end: no escapes)
         }
-        zc[k] = escapes_of(z[k][0]) + escapes_of(z[k][1]);
+        zc[k] = escapes_of(escape_mask<N>(nib[k][0])) + escapes_of(escape_mask<N>(nib[k][1]));
     }
     int incl[kPCPT];
     const int wtot = warp_scan_counts(zc, incl);
@@ -460,17 +463,20 @@ __device__ __forceinline__ void unpack_unit(const UnpackStageT<G> &st, const Uni
 #pragma unroll
     for (int k = 0; k < kPCPT; ++k) {
         const int r0 = before + incl[k] - zc[k];               // rank inside the tile of the chunk's first escape
-        const int r1 = r0 + escapes_of(z[k][0]);
+        // (the masks from before the barrier would be kept in registers, and others spilled for them)
+        asm volatile("" : "+r"(nib[k][0]), "+r"(nib[k][1]));
+        const uint32_t z0 = escape_mask<N>(nib[k][0]), z1 = escape_mask<N>(nib[k][1]);
+        const int r1 = r0 + escapes_of(z0);
         uint32_t e0[2], e1[2];
         lookup8<N>(nib[k][0], tab, e0);
         lookup8<N>(nib[k][1], tab, e1);
         if (in_window) {
-            place_escapes(z[k][0], shift + r0, word, e0);
-            place_escapes(z[k][1], shift + r1, word, e1);
+            place_escapes(z0, shift + r0, word, e0);
+            place_escapes(z1, shift + r1, word, e1);
         } else {
-            const uint2 g0 = gather_escapes(z[k][0], r0, esc + shift, staged, meta, status);
+            const uint2 g0 = gather_escapes(z0, r0, esc + shift, staged, meta, status);
             e0[0] |= g0.x, e0[1] |= g0.y;
-            const uint2 g1 = gather_escapes(z[k][1], r1, esc + shift, staged, meta, status);
+            const uint2 g1 = gather_escapes(z1, r1, esc + shift, staged, meta, status);
             e1[0] |= g1.x, e1[1] |= g1.y;
         }
         const uint4 sv = *reinterpret_cast<const uint4 *>(st.sm + (c0 + k * 32) * 16);
@@ -479,7 +485,7 @@ __device__ __forceinline__ void unpack_unit(const UnpackStageT<G> &st, const Uni
         assemble4(sv.y, e0[1], w[2], w[3]);
         assemble4(sv.z, e1[0], w[4], w[5]);
         assemble4(sv.w, e1[1], w[6], w[7]);
-        if (c0 + k * 32 < chunks && !broken) store_chunk(dst + (long long)row[k] * ds + col[k], w, wide);
+        if (c0 + k * 32 < chunks && !broken) store_chunk(dst + (long long)(at[k] >> 16) * ds + (at[k] & 0xFFFFu), w, wide);
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(empty_bar);    // this warp no longer reads the stage
@@ -496,12 +502,12 @@ __device__ __forceinline__ bool wait_loaded(UnpackSmemT<G> &s, uint32_t it, int3
 // that does not, already waited for, or n_units.
 template <int N, class G>
 __device__ __forceinline__ uint32_t unpack_run(UnpackSmemT<G> &s, uint32_t it, uint32_t n_units, int left, int &consumed,
-                                               const int (&row)[kPCPT], const int (&col)[kPCPT], bool &broken,
+                                               const uint32_t (&at)[kPCPT], bool &broken,
                                                int32_t *status, uint32_t poll_limit) {
     const ExpTable tab = exp_table<N>(left);
     for (;;) {
         const int stg = it % kStages;
-        unpack_unit<N>(s.stage[stg], s.meta_ring[it % (2 * kStages)], s.warp_tot[it & 1], consumed, tab, row, col,
+        unpack_unit<N>(s.stage[stg], s.meta_ring[it % (2 * kStages)], s.warp_tot[it & 1], consumed, tab, at,
                        &s.empty[stg], status, broken);
         if (++it >= n_units) return it;
         broken |= !wait_loaded(s, it, status, poll_limit);
@@ -617,13 +623,12 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_unpack_pipe(cons
         copy_rows(ja.rows.copy[j], blockIdx.x * (uint32_t)G::kConsumers + tid, gridDim.x * (uint32_t)G::kConsumers);
     int consumed = 0;
     bool broken = false;                  // a wait of this warp ran out: compute on, store nothing
-    // row and column of this thread's chunks inside a unit (a chunk never crosses a row: D % 16 == 0)
-    int row[kPCPT], col[kPCPT];
+    // row (upper half) and column of this thread's chunks inside a unit (a chunk never crosses a row: D % 16 == 0)
+    uint32_t at[kPCPT];
 #pragma unroll
     for (int k = 0; k < kPCPT; ++k) {
         const int e0 = ((tid >> 5) * (kPCPT * 32) + k * 32 + (tid & 31)) * 16;
-        row[k] = e0 / a0.D;
-        col[k] = e0 - row[k] * a0.D;
+        at[k] = ((uint32_t)(e0 / a0.D) << 16) | (uint32_t)(e0 % a0.D);
     }
     // (the consumers only count units: which tile a unit belongs to is in its description)
     const uint32_t my_units =
@@ -639,10 +644,10 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_unpack_pipe(cons
         const UnitMeta &meta = s.meta_ring[it % (2 * kStages)];
         const int lf = meta.left;
         switch (meta.nbits) {
-            case 1: it = unpack_run<1>(s, it, my_units, lf, consumed, row, col, broken, a0.status, ja.poll_limit); break;
-            case 2: it = unpack_run<2>(s, it, my_units, lf, consumed, row, col, broken, a0.status, ja.poll_limit); break;
-            case 3: it = unpack_run<3>(s, it, my_units, lf, consumed, row, col, broken, a0.status, ja.poll_limit); break;
-            default: it = unpack_run<4>(s, it, my_units, lf, consumed, row, col, broken, a0.status, ja.poll_limit); break;
+            case 1: it = unpack_run<1>(s, it, my_units, lf, consumed, at, broken, a0.status, ja.poll_limit); break;
+            case 2: it = unpack_run<2>(s, it, my_units, lf, consumed, at, broken, a0.status, ja.poll_limit); break;
+            case 3: it = unpack_run<3>(s, it, my_units, lf, consumed, at, broken, a0.status, ja.poll_limit); break;
+            default: it = unpack_run<4>(s, it, my_units, lf, consumed, at, broken, a0.status, ja.poll_limit); break;
         }
     }
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

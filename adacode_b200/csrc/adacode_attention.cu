@@ -486,10 +486,11 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ uint32_t f32_to_bf16_bits(float x) {
-    uint32_t u = __float_as_uint(x);
-    u += 0x7FFFu + ((u >> 16) & 1u);
-    return u >> 16;
+// two fp32 rounded to bf16, `lo` in the low half
+__device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
 }
 
 // Elements from one query row to the next in shared memory (padded: the rows start in different banks).
@@ -547,21 +548,14 @@ __device__ __forceinline__ void softmax_slab(AttnState<D, HG> &st, const float (
         const float alpha = exp2f(st.m[h] - ref);
         st.m[h] = mn;
         float sum = 0.f;
-        uint32_t b[4], b2[4], b3[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const float p = exp2f(s[t] - ref);
-            sum += p;
-            b[t] = f32_to_bf16_bits(p);
-            const float r = p - __uint_as_float(b[t] << 16);
-            b2[t] = f32_to_bf16_bits(r);
-            b3[t] = f32_to_bf16_bits(r - __uint_as_float(b2[t] << 16));
-        }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-            st.p[h][u] = b[2 * u] | (b[2 * u + 1] << 16);
-            st.p2[h][u] = b2[2 * u] | (b2[2 * u + 1] << 16);
-            if (kTermsP<D> == 3) st.p3[h][u] = b3[2 * u] | (b3[2 * u + 1] << 16);
+            const float p0 = exp2f(s[2 * u] - ref), p1 = exp2f(s[2 * u + 1] - ref);
+            sum += p0 + p1;
+            st.p[h][u] = bf16_pair(p0, p1);
+            const float r0 = p0 - bf16_lo(st.p[h][u]), r1 = p1 - bf16_hi(st.p[h][u]);
+            st.p2[h][u] = bf16_pair(r0, r1);
+            if (kTermsP<D> == 3) st.p3[h][u] = bf16_pair(r0 - bf16_lo(st.p2[h][u]), r1 - bf16_hi(st.p2[h][u]));
         }
         st.l[h] = st.l[h] * alpha + sum;
         // the accumulators hold heads 2 j and 2 j + 1: fetch those heads' factors

@@ -29,7 +29,7 @@ EXPORTED_SYMBOLS = (
     'adacode_pack_tiles', 'adacode_unpack_tiles', 'adacode_unpack_segments', 'adacode_hist_bf16',
     'adacode_choose_params', 'adacode_choose_params_host', 'adacode_calibrate_host', 'adacode_pack_tiles_static',
     'adacode_decode_attn_workspace_bytes', 'adacode_decode_attn', 'adacode_copy_to_host',
-    'adacode_pack_jobs', 'adacode_unpack_jobs', 'adacode_unpack_jobs_with_rows', 'adacode_copy_rows', 'adacode_max_jobs', 'adacode_debug_set_wait_limit',
+    'adacode_pack_jobs', 'adacode_pack_jobs_report', 'adacode_wait_report', 'adacode_unpack_jobs', 'adacode_unpack_jobs_with_rows', 'adacode_copy_rows', 'adacode_max_jobs', 'adacode_debug_set_wait_limit',
     'adacode_flat_block_elems', 'adacode_unpack_flat',
 )
 
@@ -132,6 +132,10 @@ def lib() -> ctypes.CDLL:
     L.adacode_debug_set_wait_limit.argtypes = [ctypes.c_uint, i32]
     L.adacode_pack_jobs.restype = i32
     L.adacode_pack_jobs.argtypes = [vp, i32, i32, i32, i32, i32, i32, vp, sz, vp, vp]
+    L.adacode_pack_jobs_report.restype = i32
+    L.adacode_pack_jobs_report.argtypes = [vp, i32, i32, i32, i32, i32, i32, vp, sz, vp, vp, vp, sz, ctypes.c_uint32, vp]
+    L.adacode_wait_report.restype = i32
+    L.adacode_wait_report.argtypes = [vp, sz, ctypes.c_uint32, vp]
     L.adacode_unpack_jobs.restype = i32
     L.adacode_unpack_jobs.argtypes = [vp, i32, i32, i32, i32, i32, vp, vp]
     L.adacode_unpack_jobs_with_rows.restype = i32

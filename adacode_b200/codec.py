@@ -11,6 +11,7 @@ path: on a CPU tensor, or without the built library, these functions raise.
 from __future__ import annotations
 
 import ctypes
+import threading
 from dataclasses import dataclass, field
 from typing import Any, Optional, Sequence
 
@@ -87,6 +88,26 @@ def read_back(t: torch.Tensor):
     import numpy as np
     out = sc.mailbox[:nbytes].numpy().copy()
     return out.view(np.dtype(str(t.dtype).replace('torch.', ''))).reshape(tuple(t.shape))
+
+
+class _ReportBox(threading.local):
+    """A thread's page-locked bytes that a pack's kernels report into, and the token that marks the next report."""
+
+    def __init__(self):
+        self.buf: Optional[torch.Tensor] = None
+        self.token = 0
+
+    def open(self, nbytes: int) -> tuple:
+        """(address, token) for a report of ``nbytes`` bytes."""
+        if self.buf is None or self.buf.numel() < nbytes + 4:
+            self.buf = torch.zeros(max(1 << 14, 2 * nbytes), dtype=torch.uint8).pin_memory()
+        self.token = self.token % 0xFFFFFFFF + 1
+        # (whatever an earlier report of another length left where this one's token goes)
+        ctypes.c_uint32.from_address(self.buf.data_ptr() + nbytes).value = 0
+        return self.buf.data_ptr(), self.token
+
+
+_report_box = _ReportBox()
 
 
 def check_device_status(device) -> None:
@@ -383,9 +404,10 @@ def _pack_launch(p: _PendingPack, capacity: int, hist_t) -> torch.Tensor:
     return esc
 
 
-def _pack_launch_jobs(ps: Sequence[_PendingPack]) -> None:
-    """One ``adacode_pack_jobs`` launch for pending packs of one shape and code length (the keys and
-    the values of a span); every pack gets its own escape buffer, the status word is the first one's."""
+def _pack_launch_jobs(ps: Sequence[_PendingPack], mail: torch.Tensor):
+    """One ``adacode_pack_jobs_report`` launch for pending packs of one shape and code length (as the keys and
+    the values of a span are); every pack gets its own escape buffer, the status word is the first one's.  ``mail``, which
+    their ``meta`` (and histograms that start from zero) are views of, is cleared by the call; returns its contents on the host."""
     first = ps[0]
     dev = first.dev
     sc = _scratch_for(dev)
@@ -401,11 +423,18 @@ def _pack_launch_jobs(ps: Sequence[_PendingPack]) -> None:
         jb.escapes_capacity = p.cap
         jb.tile_base, jb.seg_escape_offsets = p.tile_base.data_ptr(), p.meta.data_ptr()
         jb.hist256 = 0 if p.hist is None else p.hist.data_ptr()
+    nbytes = 8 * mail.numel()
+    host, token = _report_box.open(nbytes)
+    L, stream = _lib.lib(), stream_ptr(dev)
     with on_device(dev):
-        rc = _lib.lib().adacode_pack_jobs(
+        rc = L.adacode_pack_jobs_report(
             ctypes.addressof(jobs), len(ps), first.B, first.H, first.seq_tile, first.D, first.nbits,
-            ws.data_ptr(), ws.numel(), first.meta.data_ptr() + 8 * (first.n_blocks + 1), stream_ptr(dev))
-    _lib.check(rc, 'adacode_pack_jobs')
+            ws.data_ptr(), ws.numel(), first.meta.data_ptr() + 8 * (first.n_blocks + 1), mail.data_ptr(), host, nbytes,
+            token, stream)
+        _lib.check(rc, 'adacode_pack_jobs_report')
+        _lib.check(L.adacode_wait_report(host, nbytes, token, stream), 'adacode_wait_report')
+    import numpy as np
+    return _report_box.buf[:nbytes].numpy().copy().view(np.int64)
 
 
 def pack_blocks_finish(p: _PendingPack, host_meta):
@@ -451,8 +480,13 @@ def pack_blocks(x: torch.Tensor, right: int, nbits: int, seq_tile: int = 128, ne
     ``need_hist`` (``hist_out`` is added to instead when given).  One small device-to-host read
     (segment escape totals and the status word) ends the call.
     """
-    p = pack_blocks_launch(x, right, nbits, seq_tile, need_hist, hist_out, escape_capacity)
-    return pack_blocks_finish(p, read_back(p.meta))
+    words = x.shape[-2] // seq_tile + 2 if x.dim() == 4 and seq_tile > 0 else 0
+    if not 0 < words < 1 << 17:
+        p = pack_blocks_launch(x, right, nbits, seq_tile, need_hist, hist_out, escape_capacity)
+        return pack_blocks_finish(p, read_back(p.meta))
+    mail = torch.empty(words, dtype=torch.int64, device=x.device)
+    p = pack_blocks_launch(x, right, nbits, seq_tile, need_hist, hist_out, escape_capacity, mail, launch=False)
+    return pack_blocks_finish(p, _pack_launch_jobs([p], mail))
 
 
 def pack_pair(k: torch.Tensor, v: torch.Tensor, k_params, v_params, seq_tile: int = 128, need_hist: bool = False,
@@ -466,24 +500,24 @@ def pack_pair(k: torch.Tensor, v: torch.Tensor, k_params, v_params, seq_tile: in
     nk = k.shape[-2] // seq_tile + 2
     nv = v.shape[-2] // seq_tile + 2
     words = nk + nv + (256 if need_hist else 0)          # int64 words; two int32[256] histograms = 256 words
-    mail = torch.zeros(words, dtype=torch.int64, device=dev)
+    # keys and values of one shape and code length go through ONE launch (their windows may differ)
+    together = (tuple(k.shape) == tuple(v.shape) and int(k_params[1]) == int(v_params[1]) and k.numel() > 0
+                and k.shape[-1] % 8 == 0 and 2 * k.numel() < 2 ** 31 and words < 1 << 17)
+    mail = (torch.empty if together else torch.zeros)(words, dtype=torch.int64, device=dev)
     k_hist = v_hist = None
     if need_hist:
         h = mail[nk + nv:].view(torch.int32)
         k_hist, v_hist = h[:256], h[256:]
-    # keys and values of one shape and code length go through ONE launch (their windows may differ)
-    together = (tuple(k.shape) == tuple(v.shape) and int(k_params[1]) == int(v_params[1]) and k.numel() > 0
-                and k.shape[-1] % 8 == 0 and 2 * k.numel() < 2 ** 31)
     pk = pack_blocks_launch(k, k_params[0], k_params[1], seq_tile, need_hist, k_hist, capacities[0], mail[:nk],
                             launch=not together)
     pv = pack_blocks_launch(v, v_params[0], v_params[1], seq_tile, need_hist, v_hist, capacities[1],
                             mail[nk:nk + nv], launch=not together)
     if together:
-        _pack_launch_jobs([pk, pv])
-    host = read_back(mail)
-    if together:
+        host = _pack_launch_jobs([pk, pv], mail)
         # one status word (the keys') serves both packs
         host[nk + nv - 1] = int(host[nk + nv - 1]) | int(host[nk - 1])
+    else:
+        host = read_back(mail)
     k_chunk, _ = pack_blocks_finish(pk, host[:nk])
     v_chunk, _ = pack_blocks_finish(pv, host[nk:nk + nv])
     kh = vh = None

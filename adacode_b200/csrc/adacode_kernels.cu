@@ -704,7 +704,7 @@ size_t unit_counts_bytes(int64_t n_tiles, int64_t tile_elems) {
     return align_up((size_t)n_tiles * (size_t)(tile_elems / 128 + 1) * 4, 256);
 }
 
-// Layout of the pack scratch: [completion counter, 256 B][tile_counts int32][unit_counts int32]
+// Layout of the pack scratch: [completion counters, 256 B][tile_counts int32][unit_counts int32]
 // [block offsets int64, one more than blocks][escape slots, tile_elems bytes per tile].
 struct PackScratch {
     unsigned int *done;
@@ -1014,6 +1014,18 @@ __global__ void k_copy_to_host(const uint32_t *__restrict__ src, uint32_t *dst, 
     __threadfence_system();
 }
 
+// A report on its own, behind kernels that send none.
+__global__ void __launch_bounds__(kThreads) k_send_report(const Report r) { send_report(r); }
+
+// Where the device finds host memory: only page-locked memory that it can address, anything else is refused, not tried.
+int host_view(void *host, uint32_t *&dev) {
+    cudaPointerAttributes attr;
+    ADACODE_CUDA_TRY(cudaPointerGetAttributes(&attr, host));
+    if (attr.type != cudaMemoryTypeHost || attr.devicePointer == nullptr) return ADACODE_ERR_INVALID_ARG;
+    dev = (uint32_t *)attr.devicePointer;
+    return ADACODE_OK;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------------------
@@ -1043,12 +1055,10 @@ int adacode_copy_to_host(const void *src_dev, void *dst_host_pinned, size_t byte
     if (!src_dev || !dst_host_pinned || (bytes & 3) != 0 || (((uintptr_t)src_dev | (uintptr_t)dst_host_pinned) & 3) != 0)
         return ADACODE_ERR_INVALID_ARG;
     if (bytes > (1u << 20)) return ADACODE_ERR_TOO_LARGE;
-    cudaPointerAttributes attr;
-    ADACODE_CUDA_TRY(cudaPointerGetAttributes(&attr, dst_host_pinned));
-    // only page-locked host memory that this device can address; anything else is refused, not tried
-    if (attr.type != cudaMemoryTypeHost || attr.devicePointer == nullptr) return ADACODE_ERR_INVALID_ARG;
-    k_copy_to_host<<<1, 256, 0, (cudaStream_t)stream>>>((const uint32_t *)src_dev, (uint32_t *)attr.devicePointer,
-                                                       bytes / 4);
+    uint32_t *dst;
+    const int rc = host_view(dst_host_pinned, dst);
+    if (rc != ADACODE_OK) return rc;
+    k_copy_to_host<<<1, 256, 0, (cudaStream_t)stream>>>((const uint32_t *)src_dev, dst, bytes / 4);
     ADACODE_CUDA_TRY(cudaGetLastError());
     return ADACODE_OK;
 }
@@ -1113,8 +1123,9 @@ int pack_direct(const adacode_pack_job &jb, int B, int H, int seq_tile, int D, i
     return ADACODE_OK;
 }
 
+// `report` (nullable): its words are cleared before the jobs run and sent to the host after them.
 int pack_jobs_impl(const adacode_pack_job *jobs, int n_jobs, int B, int H, int seq_tile, int D, int nbits,
-                   void *workspace, size_t workspace_bytes, int32_t *status, cudaStream_t st) {
+                   void *workspace, size_t workspace_bytes, int32_t *status, const Report *report, cudaStream_t st) {
     if (n_jobs < 0 || n_jobs > kMaxJobs || (n_jobs > 0 && !jobs)) return ADACODE_ERR_INVALID_ARG;
     if (B < 0 || H < 0 || seq_tile <= 0 || D <= 0) return ADACODE_ERR_INVALID_ARG;
     if (nbits < 1 || nbits > 4 || D % 8 != 0 || !status) return ADACODE_ERR_INVALID_ARG;
@@ -1134,17 +1145,19 @@ int pack_jobs_impl(const adacode_pack_job *jobs, int n_jobs, int B, int H, int s
         n_tiles += jt;
         max_job_tiles = jt > max_job_tiles ? jt : max_job_tiles;
     }
+    if (n_tiles * tile_elems >= (1ll << 31)) return ADACODE_ERR_TOO_LARGE;
+    const bool pipelined = pipeline_enabled() && pipeline_shape_ok(seq_tile, D) && tile_elems <= (1 << 24);
+    if (n_tiles > 0) {
+        // (the pipelined kernel's unit bookkeeping is 32-bit: keep tiles below 2**24 elements)
+        if (!workspace || ((uintptr_t)workspace & 15) != 0) return ADACODE_ERR_INVALID_ARG;
+        if (workspace_bytes < adacode_pack_workspace_bytes(pipelined ? n_tiles : max_job_tiles, tile_elems)) return ADACODE_ERR_WORKSPACE;
+    }
+    if (report) ADACODE_CUDA_TRY(cudaMemsetAsync(const_cast<uint32_t *>(report->src), 0, (size_t)report->words * 4, st));
     for (int j = 0; j < n_jobs; ++j)
         if (BH * jobs[j].n_blocks == 0)
             ADACODE_CUDA_TRY(cudaMemsetAsync(jobs[j].seg_escape_offsets, 0,
                                              sizeof(int64_t) * (size_t)(jobs[j].n_blocks + 1), st));
-    if (n_tiles == 0) return ADACODE_OK;
-    if (n_tiles * tile_elems >= (1ll << 31)) return ADACODE_ERR_TOO_LARGE;
-    if (!workspace || ((uintptr_t)workspace & 15) != 0) return ADACODE_ERR_INVALID_ARG;
-
-    // (the pipelined kernel's unit bookkeeping is 32-bit: keep tiles below 2**24 elements)
-    if (pipeline_enabled() && pipeline_shape_ok(seq_tile, D) && tile_elems <= (1 << 24)) {
-        if (workspace_bytes < adacode_pack_workspace_bytes(n_tiles, tile_elems)) return ADACODE_ERR_WORKSPACE;
+    if (n_tiles > 0 && pipelined) {
         const PackScratch sc = carve_pack_scratch(workspace, n_tiles, tile_elems);
         PackPipeArgs pa;
         memset(&pa, 0, sizeof(pa));
@@ -1171,14 +1184,20 @@ int pack_jobs_impl(const adacode_pack_job *jobs, int n_jobs, int B, int H, int s
         pa.blk_off = sc.blk_off, pa.done = sc.done;
         pa.status = status;
         pa.poll_limit = g_poll_limit;
+        if (report) pa.report = *report;
         return launch_pack_pipe(pa, nbits, st);
     }
-    if (workspace_bytes < adacode_pack_workspace_bytes(max_job_tiles, tile_elems)) return ADACODE_ERR_WORKSPACE;
-    const PackScratch sc = carve_pack_scratch(workspace, max_job_tiles, tile_elems);
-    for (int j = 0; j < n_jobs; ++j) {
-        if (BH * jobs[j].n_blocks == 0) continue;
-        const int rc = pack_direct(jobs[j], B, H, seq_tile, D, nbits, sc, status, st);
-        if (rc != ADACODE_OK) return rc;
+    if (n_tiles > 0) {
+        const PackScratch sc = carve_pack_scratch(workspace, max_job_tiles, tile_elems);
+        for (int j = 0; j < n_jobs; ++j) {
+            if (BH * jobs[j].n_blocks == 0) continue;
+            const int rc = pack_direct(jobs[j], B, H, seq_tile, D, nbits, sc, status, st);
+            if (rc != ADACODE_OK) return rc;
+        }
+    }
+    if (report) {
+        k_send_report<<<1, kThreads, 0, st>>>(*report);
+        ADACODE_CUDA_TRY(cudaGetLastError());
     }
     return ADACODE_OK;
 }
@@ -1189,8 +1208,41 @@ extern "C" {
 
 int adacode_pack_jobs(const adacode_pack_job *jobs, int n_jobs, int B, int H, int seq_tile, int D, int nbits,
                       void *workspace, size_t workspace_bytes, int32_t *status, void *stream) {
-    return pack_jobs_impl(jobs, n_jobs, B, H, seq_tile, D, nbits, workspace, workspace_bytes, status,
+    return pack_jobs_impl(jobs, n_jobs, B, H, seq_tile, D, nbits, workspace, workspace_bytes, status, nullptr,
                           (cudaStream_t)stream);
+}
+
+int adacode_pack_jobs_report(const adacode_pack_job *jobs, int n_jobs, int B, int H, int seq_tile, int D, int nbits,
+                             void *workspace, size_t workspace_bytes, int32_t *status, void *report_dev, void *report_host_pinned,
+                             size_t report_bytes, uint32_t token, void *stream) {
+    if (!report_dev || !report_host_pinned || report_bytes == 0 || (report_bytes & 3) != 0 ||
+        (((uintptr_t)report_dev | (uintptr_t)report_host_pinned) & 3) != 0)
+        return ADACODE_ERR_INVALID_ARG;
+    if (report_bytes > (1u << 20)) return ADACODE_ERR_TOO_LARGE;
+    Report r;
+    const int rc = host_view(report_host_pinned, r.dst);
+    if (rc != ADACODE_OK) return rc;
+    r.src = (const uint32_t *)report_dev;
+    r.words = (uint32_t)(report_bytes / 4), r.token = token;
+    return pack_jobs_impl(jobs, n_jobs, B, H, seq_tile, D, nbits, workspace, workspace_bytes, status, &r, (cudaStream_t)stream);
+}
+
+int adacode_wait_report(const void *report_host_pinned, size_t report_bytes, uint32_t token, void *stream) {
+    if (!report_host_pinned || (report_bytes & 3) != 0) return ADACODE_ERR_INVALID_ARG;
+    const volatile uint32_t *flag = (const volatile uint32_t *)((const uint8_t *)report_host_pinned + report_bytes);
+    for (uint32_t i = 1;; ++i) {
+        if (*flag == token) break;
+        if (i % 512 == 0) {
+            // the stream has run dry, or failed: the token is there by now, or never comes
+            const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
+            if (e == cudaErrorNotReady) continue;
+            if (e != cudaSuccess) return cuda_fail(e);
+            if (*flag == token) break;
+            return ADACODE_ERR_CUDA;
+        }
+    }
+    __atomic_thread_fence(__ATOMIC_ACQUIRE);
+    return ADACODE_OK;
 }
 
 int adacode_max_jobs(void) { return kMaxJobs; }
@@ -1212,7 +1264,7 @@ int adacode_pack_tiles(const void *src_bf16, int64_t stride_b, int64_t stride_h,
     jb.sign_mant = sign_mant, jb.codes = codes, jb.escapes = escapes;
     jb.escapes_capacity = escapes_capacity;
     jb.tile_base = tile_base, jb.seg_escape_offsets = seg_escape_offsets, jb.hist256 = hist256;
-    return pack_jobs_impl(&jb, 1, B, H, seq_tile, D, nbits, workspace, workspace_bytes, status, (cudaStream_t)stream);
+    return pack_jobs_impl(&jb, 1, B, H, seq_tile, D, nbits, workspace, workspace_bytes, status, nullptr, (cudaStream_t)stream);
 }
 
 static int check_unpack_common(int B, int H, int seq_tile, int D, const void *dst, int64_t db, int64_t dh,

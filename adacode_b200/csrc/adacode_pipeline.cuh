@@ -769,6 +769,21 @@ struct PackJob {
     int blk0, n_blocks, left, pad;
 };
 
+// A small device buffer that goes to page-locked host memory, followed there by a 32-bit token that says it has arrived.
+struct Report {
+    const uint32_t *src;
+    uint32_t *dst;
+    uint32_t words, token;
+};
+
+// By a whole CTA: what the host's poll of the token finds in front of it is complete.
+__device__ __forceinline__ void send_report(const Report &r) {
+    for (uint32_t i = threadIdx.x; i < r.words; i += blockDim.x) r.dst[i] = __ldcg(r.src + i);
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) *reinterpret_cast<volatile uint32_t *>(r.dst + r.words) = r.token;
+}
+
 struct PackPipeArgs {
     PackJob job[kMaxJobs];
     int n_jobs;
@@ -778,9 +793,10 @@ struct PackPipeArgs {
     int32_t *tile_counts;     // n_tiles
     int32_t *unit_counts;     // n_tiles * units_per_tile
     int64_t *blk_off;         // over all blocks of the launch: escapes before global block i (n_blocks_total + 1)
-    unsigned int *done;       // zero on entry, zero on exit
+    unsigned int *done;       // two counters (CTAs of the pack, of the compaction), zero on entry, zero on exit
     int unit_rows, units_per_tile;
     int scan_in_pack;         // offsets by the pack kernel's last CTA (else by the compaction's CTAs)
+    Report report;            // what the compaction's last CTA hands to the host (words == 0: nothing)
     int32_t *status;
     uint32_t poll_limit;      // bound of every on-chip wait (kMaxPolls unless a test lowered it)
 };
@@ -1382,6 +1398,21 @@ __global__ void __launch_bounds__(kThreads) k_compact_units(const __grid_constan
         for (int i = 0; i < kWarps; ++i)
             total += s_hist[i][0][tid] + s_hist[i][1][tid] + s_hist[i][2][tid] + s_hist[i][3][tid];
         if (total != 0) atomicAdd(hist + tid, total);
+    }
+    if (pa.report.words != 0) {
+        // The CTA that comes last has everyone's offsets, counts and status bits before it.  (A launch that only copies them
+        // took 4.2 us behind a compaction of 6 us, and its host side as long; keys and values of one block through
+        // pack_pair 103 -> 95 us, of [1, 8, 20480, 128] 169 -> 157 us, with the clearing launch before the pack a memset.)
+        __shared__ bool last;
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) last = atomicAdd(pa.done + 1, 1u) == gridDim.x * gridDim.y - 1;
+        __syncthreads();
+        if (last) {
+            __threadfence();
+            send_report(pa.report);
+            if (tid == 0) pa.done[1] = 0u;
+        }
     }
 }
 

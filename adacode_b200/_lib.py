@@ -146,6 +146,23 @@ def lib() -> ctypes.CDLL:
     return L
 
 
+_native = None
+
+
+def native():
+    """The extension module with the host side of packs and decode steps; raises if it was never built."""
+    global _native
+    if _native is None:
+        lib()
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise AdacodeError(f'the _native module is missing or does not load ({e}): build it with '
+                               '`python -m adacode_b200.build`') from e
+        _native = module
+    return _native
+
+
 def check(rc: int, what: str) -> None:
     """Raise for a non-zero return code of the library."""
     if rc == OK:

@@ -1,18 +1,22 @@
-"""In-tree build of the sm_100a shared library (``libadacode_sm100.so``).
+"""In-tree build of the sm_100a shared library (``libadacode_sm100.so``) and of the extension module that calls it
+(``_native.so``).
 
-``python -m adacode_b200.build`` compiles ``csrc/*.cu`` with nvcc for ``sm_100a`` only.
-nvcc cross-compiles without a GPU, so this also runs on a CPU-only machine.
+``python -m adacode_b200.build`` compiles ``csrc/*.cu`` with nvcc for ``sm_100a`` only, and ``csrc/host_path.cpp`` with the
+host compiler against the installed torch.  nvcc cross-compiles without a GPU, so this also runs on a CPU-only machine.
 """
 from __future__ import annotations
 
 import glob
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 ROOT_DIR = os.path.dirname(PKG_DIR)
 LIB_PATH = os.path.join(PKG_DIR, 'libadacode_sm100.so')
+NATIVE_PATH = os.path.join(PKG_DIR, '_native.so')
 NVCC_FLAGS = [
     '-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17',
     '-Xcompiler', '-fPIC', '-shared',
@@ -23,29 +27,54 @@ def sources() -> list[str]:
     return sorted(glob.glob(os.path.join(PKG_DIR, 'csrc', '*.cu')))
 
 
-def _stale() -> bool:
-    if not os.path.exists(LIB_PATH):
-        return True
-    built = os.path.getmtime(LIB_PATH)
-    deps = sources() + glob.glob(os.path.join(ROOT_DIR, 'include', '*.h')) + glob.glob(os.path.join(PKG_DIR, 'csrc', '*.cuh'))
-    return any(os.path.getmtime(p) > built for p in deps)
+def _stale(path: str, deps: list[str]) -> bool:
+    return not os.path.exists(path) or any(os.path.getmtime(p) > os.path.getmtime(path) for p in deps)
+
+
+def _run(cmd: list[str]) -> str:
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f'{cmd[0]} failed ({proc.returncode}):\n{proc.stdout}\n{proc.stderr}')
+    return proc.stderr
+
+
+def build_native(force: bool = False) -> str:
+    """Compile the extension module if it is missing or older than its sources; return its path."""
+    source = os.path.join(PKG_DIR, 'csrc', 'host_path.cpp')
+    headers = glob.glob(os.path.join(ROOT_DIR, 'include', '*.h'))
+    if not force and not _stale(NATIVE_PATH, [source, *headers]):
+        return NATIVE_PATH
+    torch_dir = os.path.dirname(importlib.util.find_spec('torch').origin)
+    cuda = os.environ.get('CUDA_HOME', '/usr/local/cuda')
+    include = [os.path.join(ROOT_DIR, 'include'), os.path.join(torch_dir, 'include'),
+               os.path.join(torch_dir, 'include', 'torch', 'csrc', 'api', 'include'), sysconfig.get_paths()['include'],
+               os.path.join(cuda, 'include')]
+    _run([os.environ.get('CXX', 'g++'), '-O2', '-std=c++17', '-fPIC', '-shared', '-D_GLIBCXX_USE_CXX11_ABI=1',
+          *(f'-I{p}' for p in include), source, '-o', NATIVE_PATH, f'-L{PKG_DIR}', '-l:' + os.path.basename(LIB_PATH),
+          '-L' + os.path.join(torch_dir, 'lib'), '-ltorch_python', '-ltorch', '-ltorch_cpu', '-ltorch_cuda', '-lc10', '-lc10_cuda',
+          '-L' + os.path.join(cuda, 'lib64'), '-lcudart', '-Wl,-rpath,$ORIGIN'])
+    return NATIVE_PATH
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the library if it is missing or older than its sources; return its path."""
-    if not force and not _stale():
-        return LIB_PATH
+    """Compile the library, then the extension module, where they are missing or older than their sources; return the
+    library's path."""
+    deps = sources() + glob.glob(os.path.join(ROOT_DIR, 'include', '*.h')) + glob.glob(os.path.join(PKG_DIR, 'csrc', '*.cuh'))
+    if force or _stale(LIB_PATH, deps):
+        _build_library(verbose)
+    build_native(force)
+    return LIB_PATH
+
+
+def _build_library(verbose: bool) -> None:
     nvcc = os.environ.get('NVCC', 'nvcc')
     cmd = [nvcc, *NVCC_FLAGS, '-I', os.path.join(ROOT_DIR, 'include'), '-o', LIB_PATH, *sources()]
     if verbose:
         cmd.insert(1, '-Xptxas')
         cmd.insert(2, '-v')
-    proc = subprocess.run(cmd, capture_output=True, text=True)
-    if proc.returncode != 0:
-        raise RuntimeError(f'nvcc failed ({proc.returncode}):\n{proc.stdout}\n{proc.stderr}')
+    log = _run(cmd)
     if verbose:
-        sys.stderr.write(proc.stderr)
-    return LIB_PATH
+        sys.stderr.write(log)
 
 
 if __name__ == '__main__':

@@ -11,7 +11,6 @@ path: on a CPU tensor, or without the built library, these functions raise.
 from __future__ import annotations
 
 import ctypes
-import threading
 from dataclasses import dataclass, field
 from typing import Any, Optional, Sequence
 
@@ -88,26 +87,6 @@ def read_back(t: torch.Tensor):
     import numpy as np
     out = sc.mailbox[:nbytes].numpy().copy()
     return out.view(np.dtype(str(t.dtype).replace('torch.', ''))).reshape(tuple(t.shape))
-
-
-class _ReportBox(threading.local):
-    """A thread's page-locked bytes that a pack's kernels report into, and the token that marks the next report."""
-
-    def __init__(self):
-        self.buf: Optional[torch.Tensor] = None
-        self.token = 0
-
-    def open(self, nbytes: int) -> tuple:
-        """(address, token) for a report of ``nbytes`` bytes."""
-        if self.buf is None or self.buf.numel() < nbytes + 4:
-            self.buf = torch.zeros(max(1 << 14, 2 * nbytes), dtype=torch.uint8).pin_memory()
-        self.token = self.token % 0xFFFFFFFF + 1
-        # (whatever an earlier report of another length left where this one's token goes)
-        ctypes.c_uint32.from_address(self.buf.data_ptr() + nbytes).value = 0
-        return self.buf.data_ptr(), self.token
-
-
-_report_box = _ReportBox()
 
 
 def check_device_status(device) -> None:
@@ -343,6 +322,13 @@ class _PendingPack:
         self.__dict__.update(kw)
 
 
+def _check_blocks(S: int, seq_tile: int) -> None:
+    if seq_tile <= 0:
+        raise ValueError('seq_tile_size must be positive')
+    if S % seq_tile != 0:
+        raise ValueError(f'sequence length {S} is not a multiple of seq_tile_size {seq_tile}')
+
+
 def _default_escape_capacity(n: int, nbits: int) -> int:
     """Room for an eighth of the elements, more for the windows of one and of three exponents, of which a third to a
     half of the elements fall outside: a buffer that is too small costs a second pack of the whole span."""
@@ -361,10 +347,7 @@ def pack_blocks_launch(x: torch.Tensor, right: int, nbits: int, seq_tile: int = 
         raise ValueError(f'Tiled compressed path supports nbits in {_SUPPORTED_TILE_NBITS}, got {nbits}')
     x = _check_src(x)
     B, H, S, D = x.shape
-    if seq_tile <= 0:
-        raise ValueError('seq_tile_size must be positive')
-    if S % seq_tile != 0:
-        raise ValueError(f'sequence length {S} is not a multiple of seq_tile_size {seq_tile}')
+    _check_blocks(S, seq_tile)
     n_blocks = S // seq_tile
     dev = x.device
     tile_elems = seq_tile * D
@@ -404,52 +387,52 @@ def _pack_launch(p: _PendingPack, capacity: int, hist_t) -> torch.Tensor:
     return esc
 
 
-def _pack_launch_jobs(ps: Sequence[_PendingPack], mail: torch.Tensor):
-    """One ``adacode_pack_jobs_report`` launch for pending packs of one shape and code length (as the keys and
-    the values of a span are); every pack gets its own escape buffer, the status word is the first one's.  ``mail``, which
-    their ``meta`` (and histograms that start from zero) are views of, is cleared by the call; returns its contents on the host."""
-    first = ps[0]
-    dev = first.dev
-    sc = _scratch_for(dev)
-    n_tiles = sum(p.B * p.H * p.n_blocks for p in ps)
-    ws = sc.workspace_for(n_tiles, first.seq_tile * first.D)
-    jobs = (_lib.PackJob * len(ps))()
-    for jb, p in zip(jobs, ps):
-        p.escapes = torch.empty(p.cap, dtype=torch.uint8, device=dev)
-        sb, sh, ss, _ = p.x.stride()
-        jb.src_bf16, jb.stride_b, jb.stride_h, jb.stride_s = p.x.data_ptr(), sb, sh, ss
-        jb.n_blocks, jb.right = p.n_blocks, p.right
-        jb.sign_mant, jb.codes, jb.escapes = p.sign_mant.data_ptr(), p.codes.data_ptr(), p.escapes.data_ptr()
-        jb.escapes_capacity = p.cap
-        jb.tile_base, jb.seg_escape_offsets = p.tile_base.data_ptr(), p.meta.data_ptr()
-        jb.hist256 = 0 if p.hist is None else p.hist.data_ptr()
-    nbytes = 8 * mail.numel()
-    host, token = _report_box.open(nbytes)
-    L, stream = _lib.lib(), stream_ptr(dev)
-    with on_device(dev):
-        rc = L.adacode_pack_jobs_report(
-            ctypes.addressof(jobs), len(ps), first.B, first.H, first.seq_tile, first.D, first.nbits,
-            ws.data_ptr(), ws.numel(), first.meta.data_ptr() + 8 * (first.n_blocks + 1), mail.data_ptr(), host, nbytes,
-            token, stream)
-        _lib.check(rc, 'adacode_pack_jobs_report')
-        _lib.check(L.adacode_wait_report(host, nbytes, token, stream), 'adacode_wait_report')
-    import numpy as np
-    return _report_box.buf[:nbytes].numpy().copy().view(np.int64)
+def _pack_now(xs: Sequence[torch.Tensor], rights: Sequence[int], nbits: Sequence[int], seq_tile: int, need_hist, capacities: Sequence):
+    """Pack tensors (in one launch those that share shape and code length, as the keys and the values of a span do),
+    wait for the escape totals and finish.  ``need_hist``: whether, or for a single tensor the int32[256] device histogram
+    to add to.
+    Returns ``[(PackedChunk, device histogram or None), ...]`` and the new histograms on the host (int32 [n, 256]) or None."""
+    pending, caps, tiles, tile_elems = [], [], 0, 0
+    for x, right, bits, cap in zip(xs, rights, nbits, capacities):
+        if bits not in _SUPPORTED_TILE_NBITS:
+            raise ValueError(f'Tiled compressed path supports nbits in {_SUPPORTED_TILE_NBITS}, got {bits}')
+        x = _check_src(x)
+        B, H, S, D = x.shape
+        _check_blocks(S, seq_tile)
+        n, n_blocks = B * H * S * D, S // seq_tile
+        guessed = cap is None
+        cap = _default_escape_capacity(n, bits) if guessed else min(int(cap), max(n, 1))
+        pending.append(_PendingPack(x=x, right=right, nbits=bits, seq_tile=seq_tile, B=B, H=H, D=D, n_blocks=n_blocks, dev=x.device,
+                                    n=n, guessed=guessed, cap=cap))
+        caps.append(cap)
+        tiles, tile_elems = tiles + B * H * n_blocks, max(tile_elems, seq_tile * D)
+    ws = _scratch_for(pending[0].dev).workspace_for(tiles, tile_elems)
+    parts, host_hist = _lib.native().pack(tuple([p.x for p in pending]), tuple(rights), tuple(nbits), seq_tile, tuple(caps), need_hist, ws)
+    out = []
+    for p, part in zip(pending, parts):
+        p.sign_mant, p.codes, p.escapes, p.tile_base, p.meta, p.hist, offsets, status = part
+        out.append(_finish_pack(p, offsets, status))
+    if host_hist is not None:
+        import numpy as np
+        host_hist = np.frombuffer(host_hist, dtype=np.int32).reshape(len(xs), 256).copy()
+    return out, host_hist
 
 
 def pack_blocks_finish(p: _PendingPack, host_meta):
     """Finish a launch given the host copy of its ``meta`` (int64[n_blocks + 2]): re-run with the
     exact capacity if the escape buffer was too small, trim it, build the ``PackedChunk``."""
+    return _finish_pack(p, host_meta[: p.n_blocks + 1].tolist(), int(host_meta[p.n_blocks + 1]) & 0xFFFFFFFF)
+
+
+def _finish_pack(p: _PendingPack, offsets: list, status: int):
     n_blocks = p.n_blocks
-    offsets = host_meta[: n_blocks + 1].tolist()
     total = offsets[-1]
-    status = int(host_meta[n_blocks + 1]) & 0xFFFFFFFF
     escapes = p.escapes
     # the kernels flag an overflow exactly when a stream does not fit its buffer; packs that shared
     # a launch share the status word, so each one decides by its own total
     status_other = status & ~_lib.STATUS_ESCAPE_OVERFLOW
     if total > p.cap:
-        p.meta.zero_()
+        p.meta = torch.zeros(n_blocks + 2, dtype=torch.int64, device=p.dev)
         escapes = _pack_launch(p, total, None)   # histogram already complete from the first pass
         host = read_back(p.meta)
         if int(host[n_blocks + 1]) & 0xFFFFFFFF:
@@ -466,7 +449,8 @@ def pack_blocks_finish(p: _PendingPack, host_meta):
         escapes = escapes[:total].clone()
     else:
         escapes = escapes[:total]
-    chunk = PackedChunk(p.sign_mant, p.codes, escapes, p.tile_base, offsets, p.meta[: n_blocks + 1],
+    meta = p.meta if p.meta.shape[0] == n_blocks + 1 else p.meta[: n_blocks + 1]
+    chunk = PackedChunk(p.sign_mant, p.codes, escapes, p.tile_base, offsets, meta,
                         p.right - 2 ** p.nbits + 1, p.right, p.nbits, p.B, p.H, p.seq_tile, p.D)
     return chunk, p.hist
 
@@ -480,51 +464,22 @@ def pack_blocks(x: torch.Tensor, right: int, nbits: int, seq_tile: int = 128, ne
     ``need_hist`` (``hist_out`` is added to instead when given).  One small device-to-host read
     (segment escape totals and the status word) ends the call.
     """
-    words = x.shape[-2] // seq_tile + 2 if x.dim() == 4 and seq_tile > 0 else 0
-    if not 0 < words < 1 << 17:
-        p = pack_blocks_launch(x, right, nbits, seq_tile, need_hist, hist_out, escape_capacity)
-        return pack_blocks_finish(p, read_back(p.meta))
-    mail = torch.empty(words, dtype=torch.int64, device=x.device)
-    p = pack_blocks_launch(x, right, nbits, seq_tile, need_hist, hist_out, escape_capacity, mail, launch=False)
-    return pack_blocks_finish(p, _pack_launch_jobs([p], mail))
+    [done], _ = _pack_now([x], [int(right)], [int(nbits)], seq_tile, hist_out if need_hist and hist_out is not None else need_hist,
+                          [escape_capacity])
+    return done
 
 
 def pack_pair(k: torch.Tensor, v: torch.Tensor, k_params, v_params, seq_tile: int = 128, need_hist: bool = False,
               capacities=(None, None)):
-    """Pack the keys and the values of one span with one round trip to the host: both launches
-    write their segment offsets, status words and (with ``need_hist``) exponent histograms into
-    one device buffer that a single ``read_back`` fetches.  Returns
+    """Pack the keys and the values of one span, with one launch and one round trip to the host where they have one
+    shape and code length: segment offsets, status and (with ``need_hist``) exponent histograms come back together.  Returns
     ``(k_chunk, v_chunk, k_hist, v_hist, k_hist_host, v_hist_host)``; the ``*_host`` entries are
     numpy int32[256] copies of the histograms (None without ``need_hist``)."""
-    dev = k.device
-    nk = k.shape[-2] // seq_tile + 2
-    nv = v.shape[-2] // seq_tile + 2
-    words = nk + nv + (256 if need_hist else 0)          # int64 words; two int32[256] histograms = 256 words
-    # keys and values of one shape and code length go through ONE launch (their windows may differ)
-    together = (tuple(k.shape) == tuple(v.shape) and int(k_params[1]) == int(v_params[1]) and k.numel() > 0
-                and k.shape[-1] % 8 == 0 and 2 * k.numel() < 2 ** 31 and words < 1 << 17)
-    mail = (torch.empty if together else torch.zeros)(words, dtype=torch.int64, device=dev)
-    k_hist = v_hist = None
-    if need_hist:
-        h = mail[nk + nv:].view(torch.int32)
-        k_hist, v_hist = h[:256], h[256:]
-    pk = pack_blocks_launch(k, k_params[0], k_params[1], seq_tile, need_hist, k_hist, capacities[0], mail[:nk],
-                            launch=not together)
-    pv = pack_blocks_launch(v, v_params[0], v_params[1], seq_tile, need_hist, v_hist, capacities[1],
-                            mail[nk:nk + nv], launch=not together)
-    if together:
-        host = _pack_launch_jobs([pk, pv], mail)
-        # one status word (the keys') serves both packs
-        host[nk + nv - 1] = int(host[nk + nv - 1]) | int(host[nk - 1])
-    else:
-        host = read_back(mail)
-    k_chunk, _ = pack_blocks_finish(pk, host[:nk])
-    v_chunk, _ = pack_blocks_finish(pv, host[nk:nk + nv])
-    kh = vh = None
-    if need_hist:
-        hh = host[nk + nv:].view('int32')
-        kh, vh = hh[:256].copy(), hh[256:].copy()
-    return k_chunk, v_chunk, k_hist, v_hist, kh, vh
+    # (keys and values of one shape and code length go through ONE launch, their windows may differ)
+    (kd, vd), hists = _pack_now([k, v], [int(k_params[0]), int(v_params[0])], [int(k_params[1]), int(v_params[1])], seq_tile,
+                                need_hist, capacities)
+    kh, vh = (None, None) if hists is None else hists
+    return kd[0], vd[0], kd[1], vd[1], kh, vh
 
 
 def unpack_chunk(chunk: PackedChunk, dst: torch.Tensor, seq_offset: int = 0) -> None:
@@ -673,6 +628,17 @@ def unpack_segments(segments: Sequence[TiledCompressedTensor], dst: torch.Tensor
         rc = _lib.lib().adacode_unpack_segments(table.data_ptr(), len(segments), B, H, T, D, dst.data_ptr(),
                                                 db, dh, ds, sc.status.data_ptr(), stream_ptr(dev))
     _lib.check(rc, 'adacode_unpack_segments')
+
+
+def device_status(device: torch.device) -> torch.Tensor:
+    """The status word of a GPU that unpack launches write to."""
+    return _scratch_for(device).status
+
+
+def check_one_shape(segs: Sequence) -> None:
+    """Refuse a list whose segments differ in [batch, kv_heads, seq_tile, head_dim]."""
+    if segs:
+        _check_one_shape(segs, tuple(segs[0].original_shape))
 
 
 def _check_one_shape(segs: Sequence, shape0: tuple) -> None:

@@ -34,8 +34,8 @@ import torch
 from transformers import Cache
 from transformers.cache_utils import DynamicLayer
 
-from . import codec
-from .codec import SegmentRef, TiledCompressedTensor
+from . import _lib, codec
+from .codec import SegmentRef, TiledCompressedTensor, check_one_shape
 
 _SUPPORTED_LAYOUTS = ('segmented_tiled', 'legacy', 'tiled')
 _LEGACY_BLOCK_GAPS = (8, 4, 8, 2)      # escape-base blocks of the flat layout: 128 x gap elements
@@ -71,21 +71,30 @@ class _DenseWorkspace:
     def __init__(self):
         self._bufs: dict = {}
 
-    def view(self, device, slot: str, shape: tuple) -> torch.Tensor:
-        n = math.prod(shape)
+    def flat(self, device, slot: str, n: int) -> torch.Tensor:
+        """The slot's buffer, of at least ``n`` elements."""
         key = (device if type(device) is torch.device else torch.device(device), slot)
         buf = self._bufs.get(key)
         if buf is None or buf.numel() < n:
             buf = torch.empty(max(int(n * 1.25), 1 << 16), dtype=torch.bfloat16, device=device)
             self._bufs[key] = buf
+        return buf
+
+    def view(self, device, slot: str, shape: tuple) -> torch.Tensor:
         B, H, T, D = shape
-        return buf.as_strided(shape, (H * T * D, T * D, D, 1))
+        return self.flat(device, slot, math.prod(shape)).as_strided(shape, (H * T * D, T * D, D, 1))
 
     def release(self):
         self._bufs.clear()
 
 
 _GLOBAL_WORKSPACE = _DenseWorkspace()
+
+
+def _copy_tokens(buf: torch.Tensor, at: int, states: torch.Tensor) -> None:
+    """``buf[:, :, at: at + T].copy_(states)`` for ``states`` of T tokens."""
+    if not (states.is_cuda and _lib.native().append(buf, at, states)):
+        buf[:, :, at: at + states.shape[2]].copy_(states)
 
 
 class _Residual:
@@ -118,7 +127,7 @@ class _Residual:
         if q == 0:
             return
         self._reserve(states, self.length + q, block)
-        self.buf[:, :, self.length: self.length + q].copy_(states)
+        _copy_tokens(self.buf, self.length, states)
         self.length += q
 
     def drop_front(self, count: int) -> None:
@@ -597,6 +606,7 @@ class float11Layer(DynamicLayer):
         cached = self._tables.get(which)
         if cached is not None and cached[0] == len(segments):
             return cached[1]
+        check_one_shape(segments)
         table = codec.build_segment_table(segments, None, self.cache_device)
         self._tables[which] = (len(segments), table)
         return table
@@ -623,6 +633,16 @@ class float11Layer(DynamicLayer):
         if self.dense_workspace == 'shared':
             # keys, values and the tails behind them are written by one launch when keys and values have one shape
             parts = []
+            if self._res_v.length == res_len:
+                for which, segs, res in pairs:
+                    B, H, T, D = segs[0].original_shape
+                    parts.append((self._workspace.flat(self.cache_device, which, B * H * total * D), self._segment_table(which, segs),
+                                  len(segs), B, H, T, D, res.buf))
+                if parts[0][0].is_cuda:
+                    dense = _lib.native().dense_view(tuple(parts), prefix, res_len, codec.device_status(parts[0][0].device))
+                    if dense is not None:
+                        return dense
+                parts = []
             for which, segs, res in pairs:
                 B, H, _, D = segs[0].original_shape
                 dense = self._workspace.view(self.cache_device, which, (B, H, total, D))
@@ -649,7 +669,7 @@ class float11Layer(DynamicLayer):
             dense = mirror[:, :, :total]
             self._mirror_valid[which] = total
             if res_len:
-                dense[:, :, prefix:total].copy_(res.tensor())
+                _copy_tokens(dense, prefix, res.tensor())
             outs.append(dense)
         return outs[0], outs[1]
 

@@ -23,7 +23,7 @@ from typing import Any, Optional
 import torch
 from transformers import Cache
 
-from . import codec
+from . import _lib, codec
 from .float_cache_utils import Float11Cache, _Residual, float11Layer
 
 
@@ -224,10 +224,18 @@ class MLALatentFloat11DenseRopeLayer(float11Layer):
                 self.materialize_cache_hits += 1
             self._materialized_prefix_seq_len = int(self._compressed_prefix_seq_len)
             segs = self._key_segments
-            B, H, _, D = segs[0].original_shape
+            B, H, T, D = segs[0].original_shape
             prefix = self._compressed_prefix_seq_len
             total = prefix + self._res_k.length
+            dense = None
             if self.dense_workspace == 'shared':
+                flat = self._workspace.flat(self.cache_device, 'k', B * H * total * D)
+                if flat.is_cuda:
+                    part = (flat, self._segment_table('k', segs), len(segs), B, H, T, D, self._res_k.buf)
+                    dense = _lib.native().dense_view((part,), prefix, self._res_k.length, codec.device_status(flat.device))
+            if dense is not None:
+                latent, res_latent = dense[0], None              # (the tail is in its place)
+            elif self.dense_workspace == 'shared':
                 latent = self._workspace.view(self.cache_device, 'k', (B, H, total, D))
                 codec.unpack_segments(segs, latent, table=self._segment_table('k', segs))
             else:

@@ -135,7 +135,7 @@ def lib() -> ctypes.CDLL:
     L.adacode_pack_jobs_report.restype = i32
     L.adacode_pack_jobs_report.argtypes = [vp, i32, i32, i32, i32, i32, i32, vp, sz, vp, vp, vp, sz, ctypes.c_uint32, vp]
     L.adacode_wait_report.restype = i32
-    L.adacode_wait_report.argtypes = [vp, sz, ctypes.c_uint32, vp]
+    L.adacode_wait_report.argtypes = [vp, sz, ctypes.c_uint32, vp, vp]
     L.adacode_unpack_jobs.restype = i32
     L.adacode_unpack_jobs.argtypes = [vp, i32, i32, i32, i32, i32, vp, vp]
     L.adacode_unpack_jobs_with_rows.restype = i32

@@ -942,10 +942,10 @@ int launch_pack_pipe(PackPipeArgs &pa, int nbits, cudaStream_t st) {
         hist = hist || pa.job[j].hist != nullptr;
         max_blocks = pa.job[j].n_blocks > max_blocks ? pa.job[j].n_blocks : max_blocks;
     }
-    // one warp per tile; few enough CTAs that the final per-bin atomics of the histogram stay cheap
+    // one warp per tile, as many CTAs as are resident (48 registers)
     const int64_t job_tiles = (int64_t)max_blocks * pa.BH;
     const int64_t want = (job_tiles + kWarps - 1) / kWarps;
-    const int64_t cap = ((int64_t)sm_count() * 4 + pa.n_jobs - 1) / pa.n_jobs;
+    const int64_t cap = ((int64_t)sm_count() * 5 + pa.n_jobs - 1) / pa.n_jobs;
     const dim3 cgrid((unsigned)(want < cap ? want : cap), (unsigned)pa.n_jobs);
     // The compaction's CTAs find their tiles' offsets themselves as long as each can add up all counts
     // before its tiles and has a thread for each of them; beyond that the pack kernel's last CTA scans.
@@ -1216,32 +1216,38 @@ int adacode_pack_jobs_report(const adacode_pack_job *jobs, int n_jobs, int B, in
                              void *workspace, size_t workspace_bytes, int32_t *status, void *report_dev, void *report_host_pinned,
                              size_t report_bytes, uint32_t token, void *stream) {
     if (!report_dev || !report_host_pinned || report_bytes == 0 || (report_bytes & 3) != 0 ||
-        (((uintptr_t)report_dev | (uintptr_t)report_host_pinned) & 3) != 0)
+        ((uintptr_t)report_dev & 3) != 0 || ((uintptr_t)report_host_pinned & 7) != 0)
         return ADACODE_ERR_INVALID_ARG;
     if (report_bytes > (1u << 20)) return ADACODE_ERR_TOO_LARGE;
     Report r;
-    const int rc = host_view(report_host_pinned, r.dst);
+    uint32_t *dst;
+    const int rc = host_view(report_host_pinned, dst);
     if (rc != ADACODE_OK) return rc;
+    r.dst = (uint2 *)dst;
     r.src = (const uint32_t *)report_dev;
     r.words = (uint32_t)(report_bytes / 4), r.token = token;
     return pack_jobs_impl(jobs, n_jobs, B, H, seq_tile, D, nbits, workspace, workspace_bytes, status, &r, (cudaStream_t)stream);
 }
 
-int adacode_wait_report(const void *report_host_pinned, size_t report_bytes, uint32_t token, void *stream) {
-    if (!report_host_pinned || (report_bytes & 3) != 0) return ADACODE_ERR_INVALID_ARG;
-    const volatile uint32_t *flag = (const volatile uint32_t *)((const uint8_t *)report_host_pinned + report_bytes);
-    for (uint32_t i = 1;; ++i) {
-        if (*flag == token) break;
-        if (i % 512 == 0) {
-            // the stream has run dry, or failed: the token is there by now, or never comes
-            const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
-            if (e == cudaErrorNotReady) continue;
-            if (e != cudaSuccess) return cuda_fail(e);
-            if (*flag == token) break;
-            return ADACODE_ERR_CUDA;
+int adacode_wait_report(const void *report_host_pinned, size_t report_bytes, uint32_t token, void *out, void *stream) {
+    if (!report_host_pinned || !out || (report_bytes & 3) != 0 || ((uintptr_t)report_host_pinned & 7) != 0) return ADACODE_ERR_INVALID_ARG;
+    const uint64_t *words = (const uint64_t *)report_host_pinned;
+    uint32_t *to = (uint32_t *)out;
+    bool dry = false;                                      // the stream has: what has not come by now never comes
+    for (size_t i = 0; i < report_bytes / 4; ++i)
+        for (uint32_t poll = 1;; ++poll) {
+            const uint64_t w = __atomic_load_n(words + i, __ATOMIC_RELAXED);
+            if ((uint32_t)(w >> 32) == token) {
+                to[i] = (uint32_t)w;
+                break;
+            }
+            if (dry) return ADACODE_ERR_CUDA;
+            if (poll % 512 == 0) {
+                const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
+                if (e != cudaSuccess && e != cudaErrorNotReady) return cuda_fail(e);
+                dry = e == cudaSuccess;
+            }
         }
-    }
-    __atomic_thread_fence(__ATOMIC_ACQUIRE);
     return ADACODE_OK;
 }
 

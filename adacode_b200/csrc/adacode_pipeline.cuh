@@ -769,19 +769,20 @@ struct PackJob {
     int blk0, n_blocks, left, pad;
 };
 
-// A small device buffer that goes to page-locked host memory, followed there by a 32-bit token that says it has arrived.
+// A small device buffer that goes to page-locked host memory, every word together with a token that says it has arrived:
+// a flag behind the words would have to wait for them to cross the bus.
 struct Report {
     const uint32_t *src;
-    uint32_t *dst;
+    uint2 *dst;
     uint32_t words, token;
 };
 
-// By a whole CTA: what the host's poll of the token finds in front of it is complete.
+// By a whole CTA.
 __device__ __forceinline__ void send_report(const Report &r) {
-    for (uint32_t i = threadIdx.x; i < r.words; i += blockDim.x) r.dst[i] = __ldcg(r.src + i);
-    __threadfence_system();
-    __syncthreads();
-    if (threadIdx.x == 0) *reinterpret_cast<volatile uint32_t *>(r.dst + r.words) = r.token;
+    for (uint32_t i = threadIdx.x; i < r.words; i += blockDim.x) {
+        const uint32_t v = __ldcg(r.src + i);
+        asm volatile("st.relaxed.sys.global.v2.b32 [%0], {%1, %2};" ::"l"(r.dst + i), "r"(v), "r"(r.token) : "memory");
+    }
 }
 
 struct PackPipeArgs {
@@ -1228,58 +1229,63 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const 
     scan_tile_counts<G>(pa, &s.carry, s.scan, s.job_off, reinterpret_cast<long long *>(&s.stage[0]));
 }
 
-// One warp copies the escape bytes of tile t (its units follow each other in the scratch) to `dst`
-// of its job's stream.  The bytes move as aligned 32-bit words: the source words are funnel-shifted
-// into the alignment of the destination; only the first and last word of a run use byte stores.
-// With do_hist the escaped exponents are counted into `my_hist` (256 bins in shared memory).
+// One warp copies the escape bytes of tile t (its units follow each other in the scratch, `count` bytes in all) to `dst`
+// of its job's stream, a kilobyte at a time whose loads are all under way together.  The bytes move as aligned 32-bit words,
+// one per lane: a destination word is put together from a lane's source word and its neighbour's; only the first and
+// last word of a run use byte stores.  With do_hist the escaped exponents are counted into `my_hist` (256 bins in shared
+// memory).
+// Pack and compaction together, in steps of 16 bytes per lane with a load of the word before each, four copies of the bins
+// per warp, four CTAs per SM (64 registers) and now: keys and values [64, 8, 4096, 128] at 3 bits with histograms 440 -> 416 us,
+// [16, 8, 8192, 128] at 2 bits, 34 % escapes, 249 -> 224 us; the compaction is bound by the latency of its reads.
+constexpr int kCompactWords = 8;               // words per lane under way
+
 __device__ __forceinline__ void compact_tile_units(const PackPipeArgs &pa, const PackJob &jb, int64_t t, int64_t dst,
-                                                   int c, int *my_hist, bool do_hist) {
+                                                   int count, int *my_hist, bool do_hist) {
     const int lane = threadIdx.x & 31;
     const int upt = pa.units_per_tile;
     const int unit_elems = pa.unit_rows * pa.D;
-    const bool fits = dst >= 0 && dst + c <= jb.capacity;
+    const bool fits = dst >= 0 && dst + count <= jb.capacity;
     if (!fits && lane == 0) atomicOr(pa.status, ADACODE_STATUS_ESCAPE_OVERFLOW);
     for (int u = 0; u < upt; ++u) {
-        const int cu = __ldcg(pa.unit_counts + t * upt + u);
+        const int cu = upt == 1 ? count : __ldcg(pa.unit_counts + t * upt + u);
         // unit slots start on 16-byte boundaries
-        const uint32_t *src4 =
-            reinterpret_cast<const uint32_t *>(pa.esc_scratch + t * pa.tile_elems + (int64_t)u * unit_elems);
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(pa.esc_scratch + t * pa.tile_elems + (int64_t)u * unit_elems);
         uint8_t *d8 = jb.escapes + dst;
         const int r = (int)((uintptr_t)d8 & 3);
         uint32_t *dst32 = reinterpret_cast<uint32_t *>(d8 - r);
         const int n_words = (r + cu + 3) >> 2;             // destination words touched
-        // four destination words (16 bytes) per lane and step: one 16-byte load of the source
-        // words behind them plus the word before (for the shift)
-        const uint4 *src16 = reinterpret_cast<const uint4 *>(src4);
-        const int n_quads = (n_words + 3) >> 2;
-#pragma unroll 2
-        for (int q = lane; q < n_quads; q += 32) {
-            const uint4 cur = 16 * q < cu ? __ldcg(src16 + q) : make_uint4(0u, 0u, 0u, 0u);
-            const uint32_t prev = (r != 0 && q > 0) ? __ldcg(src4 + 4 * q - 1) : 0u;
-            const uint32_t w[5] = {prev, cur.x, cur.y, cur.z, cur.w};
+        uint32_t carry = 0;                                // lane 0: the source word before its next one
+#pragma unroll 1
+        for (int base = 0; base < n_words; base += 32 * kCompactWords) {
+            uint32_t w[kCompactWords];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int j = 4 * q + k;                       // destination word
-                const int s0 = 4 * j - r;                      // source index of the byte that lands in its byte 0
-                const uint32_t v = r != 0 ? __funnelshift_r(w[k], w[k + 1], 8 * (4 - r)) : w[k + 1];
-                if (fits && j < n_words) {
-                    if (s0 >= 0 && s0 + 4 <= cu) {
-                        dst32[j] = v;
-                    } else {
+            for (int k = 0; k < kCompactWords; ++k) {
+                const int j = base + 32 * k + lane;
+                w[k] = 4 * j < cu ? __ldcg(src + j) : 0u;
+            }
 #pragma unroll
-                        for (int b = 0; b < 4; ++b)
-                            if (s0 + b >= 0 && s0 + b < cu)
-                                reinterpret_cast<uint8_t *>(dst32 + j)[b] = (uint8_t)(v >> (8 * b));
-                    }
+            for (int k = 0; k < kCompactWords; ++k) {
+                if (base + 32 * k >= n_words) break;       // (uniform)
+                const int j = base + 32 * k + lane;
+                const uint32_t turned = __shfl_sync(kFull, w[k], (lane + 31) & 31);
+                const uint32_t prev = lane == 0 ? carry : turned;
+                carry = turned;
+                // bytes 4 j - r .. 4 j - r + 3 of the unit
+                const uint32_t v = __funnelshift_lc(prev, w[k], 8 * r);
+                const int s0 = 4 * j - r;
+                if (fits && s0 >= 0 && s0 + 4 <= cu) {
+                    dst32[j] = v;
+                } else if (fits && j < n_words) {
+#pragma unroll
+                    for (int b = 0; b < 4; ++b)
+                        if (s0 + b >= 0 && s0 + b < cu) reinterpret_cast<uint8_t *>(dst32 + j)[b] = (uint8_t)(v >> (8 * b));
                 }
                 if (do_hist) {
-                    // source word j holds source bytes 4j .. 4j+3: each source byte is counted once
-                    uint32_t x = w[k + 1];
+                    // source word j holds source bytes 4 j .. 4 j + 3: each source byte is counted once
+                    const int left = cu - 4 * j;
 #pragma unroll
-                    for (int b = 0; b < 4; ++b) {
-                        if (4 * j + b < cu) atomicAdd(my_hist + (x & 0xFFu), 1);
-                        x >>= 8;
-                    }
+                    for (int b = 0; b < 4; ++b)
+                        if (b < left) atomicAdd(my_hist + ((w[k] >> (8 * b)) & 0xFFu), 1);
                 }
             }
         }
@@ -1349,23 +1355,21 @@ __device__ __forceinline__ void tile_offsets(const PackPipeArgs &pa, const PackJ
 // count[t] in its job's stream.  blockIdx.y is the job; one warp per tile; all of a tile's metadata
 // is fetched with independent loads (one memory round trip).
 // With HIST the escaped exponents are counted here (whole warps of escape bytes) rather than one
-// by one inside the pack kernel.  Escaped exponents cluster on a few values, so each warp keeps
-// four copies of the 256 bins (picked by lane & 3): one copy would serialise most of a warp's
-// shared-memory atomics.
+// by one inside the pack kernel, into one set of 256 bins per CTA.
 template <bool HIST>
 __global__ void __launch_bounds__(kThreads) k_compact_units(const __grid_constant__ PackPipeArgs pa) {
-    __shared__ int s_hist[HIST ? kWarps : 1][HIST ? 4 : 1][HIST ? 256 : 1];
+    __shared__ int s_hist[HIST ? 256 : 1];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const PackJob &jb = pa.job[blockIdx.y];
     int32_t *hist = jb.hist;
     const bool do_hist = HIST && hist != nullptr;
     if (HIST) {
-        for (int i = tid; i < kWarps * 4 * 256; i += kThreads) (&s_hist[0][0][0])[i] = 0;
+        for (int i = tid; i < 256; i += kThreads) s_hist[i] = 0;
         __syncthreads();
     }
     // launched as a programmatic dependent of the pack kernel: nothing that kernel wrote is read above
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    int *my_hist = &s_hist[HIST ? warp : 0][HIST ? (lane & 3) : 0][0];
+    int *my_hist = s_hist;
     const int64_t job_tiles = (int64_t)jb.n_blocks * pa.BH;
     if (!pa.scan_in_pack) {
         __shared__ int s_off[kThreads], s_cnt[kThreads], s_red[3 * kWarps];
@@ -1393,23 +1397,22 @@ __global__ void __launch_bounds__(kThreads) k_compact_units(const __grid_constan
     }
     if (do_hist) {
         __syncthreads();
-        int total = 0;
-#pragma unroll
-        for (int i = 0; i < kWarps; ++i)
-            total += s_hist[i][0][tid] + s_hist[i][1][tid] + s_hist[i][2][tid] + s_hist[i][3][tid];
+        const int total = s_hist[tid];
         if (total != 0) atomicAdd(hist + tid, total);
     }
     if (pa.report.words != 0) {
         // The CTA that comes last has everyone's offsets, counts and status bits before it.  (A launch that only copies them
-        // took 4.2 us behind a compaction of 6 us, and its host side as long; keys and values of one block through
-        // pack_pair 103 -> 95 us, of [1, 8, 20480, 128] 169 -> 157 us, with the clearing launch before the pack a memset.)
+        // took 4.2 us behind the compaction, and its host side as long; this takes less than one, 7 us with fences
+        // at the system's scope around a single flag.)
         __shared__ bool last;
-        __threadfence();
         __syncthreads();
-        if (tid == 0) last = atomicAdd(pa.done + 1, 1u) == gridDim.x * gridDim.y - 1;
+        if (tid == 0) {
+            unsigned before;
+            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(pa.done + 1) : "memory");
+            last = before == gridDim.x * gridDim.y - 1;
+        }
         __syncthreads();
         if (last) {
-            __threadfence();
             send_report(pa.report);
             if (tid == 0) pa.done[1] = 0u;
         }

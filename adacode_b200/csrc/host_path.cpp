@@ -72,12 +72,16 @@ int64_t integer(PyObject *o) {
     return v;
 }
 
-// This thread's page-locked bytes that packs report into: it grows with the largest report (a MiB at most) and goes
-// with the thread.
+// This thread's page-locked bytes that packs report into: they grow with the largest report (of a MiB at most) and go
+// with the thread.  A token never comes twice while the bytes live: they are cleared before the tokens start over.
 struct ReportBox {
     void *host = nullptr;
     size_t bytes = 0;
     uint32_t token = 0;
+    uint32_t next_token() {
+        if (token == 0xFFFFFFFFu) memset(host, 0, bytes), token = 0;
+        return ++token;
+    }
     ~ReportBox() {
         if (host) (void)cudaFreeHost(host);
     }
@@ -88,6 +92,7 @@ struct ReportBox {
         const size_t n = need < (1 << 14) ? (1 << 14) : 2 * need;
         C10_CUDA_CHECK(cudaHostAlloc(&host, n, cudaHostAllocPortable | cudaHostAllocMapped));
         bytes = n;
+        memset(host, 0, n);
     }
 };
 
@@ -124,7 +129,7 @@ PyObject *pack(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
         int first, n, nbits;
         int64_t B, H, D, elems, offs, words;                      // [segment offsets of its tensors | status | 128 words of histogram each]
         Tensor mail;
-        size_t host_at;                                    // where its report begins
+        size_t at;                                         // where its report begins
         uint32_t token;
     } launch[kMost];
     int n_launches = 0;
@@ -165,16 +170,15 @@ PyObject *pack(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
                               : given_hist.defined() ? (int32_t *)given_hist.mutable_data_ptr()
                                                      : nullptr;
         }
-        l.host_at = host_bytes;
-        host_bytes += (size_t)l.words * 8 + 8;             // (and the token)
+        l.at = host_bytes;
+        host_bytes += (size_t)l.words * 8;
     }
     // a report holds a MiB at most; more offsets than that are fetched by a copy
     const bool reports = host_bytes <= (1 << 20);
     static thread_local ReportBox box;
-    std::vector<uint8_t> fetched;
-    if (reports) box.reserve(host_bytes);
-    else fetched.resize(host_bytes);
-    uint8_t *const host = reports ? (uint8_t *)box.host : fetched.data();
+    if (reports) box.reserve(2 * host_bytes);
+    std::vector<uint8_t> fetched(host_bytes);
+    uint8_t *const host = fetched.data();
     const char *what = "adacode_pack_jobs";
     int rc = ADACODE_OK;
     {
@@ -185,17 +189,15 @@ PyObject *pack(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
             int32_t *const status = (int32_t *)(m + l.n * l.offs);
             const size_t report = (size_t)l.words * 8;
             if (reports) {
-                l.token = box.token = box.token == 0xFFFFFFFFu ? 1 : box.token + 1;
-                // (an earlier report of another length may have left anything there)
-                *(volatile uint32_t *)(host + l.host_at + report) = 0;
+                l.token = box.next_token();
                 what = "adacode_pack_jobs_report";
                 rc = adacode_pack_jobs_report(jobs + l.first, l.n, (int)l.B, (int)l.H, (int)T, (int)l.D, l.nbits, ws.mutable_data_ptr(),
-                                              ws.nbytes(), status, m, host + l.host_at, report, l.token, stream);
+                                              ws.nbytes(), status, m, (uint8_t *)box.host + 2 * l.at, report, l.token, stream);
             } else {
                 C10_CUDA_CHECK(cudaMemsetAsync(m, 0, report, stream));
                 rc = adacode_pack_jobs(jobs + l.first, l.n, (int)l.B, (int)l.H, (int)T, (int)l.D, l.nbits, ws.mutable_data_ptr(), ws.nbytes(),
                                        status, stream);
-                C10_CUDA_CHECK(cudaMemcpyAsync(host + l.host_at, m, report, cudaMemcpyDeviceToHost, stream));
+                C10_CUDA_CHECK(cudaMemcpyAsync(host + l.at, m, report, cudaMemcpyDeviceToHost, stream));
             }
         }
         // (what is under way still reports, or writes, into this thread's bytes)
@@ -203,7 +205,7 @@ PyObject *pack(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
         if (rc == ADACODE_OK && !reports) C10_CUDA_CHECK(cudaStreamSynchronize(stream));
         for (int i = 0; i < n_launches && rc == ADACODE_OK && reports; ++i) {
             what = "adacode_wait_report";
-            rc = adacode_wait_report(host + launch[i].host_at, (size_t)launch[i].words * 8, launch[i].token, stream);
+            rc = adacode_wait_report((uint8_t *)box.host + 2 * launch[i].at, (size_t)launch[i].words * 8, launch[i].token, host + launch[i].at, stream);
         }
     }
     check(rc, what);
@@ -212,7 +214,7 @@ PyObject *pack(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
     if (!parts.p || !hists.p) fail();
     for (int i = 0; i < n_launches; ++i) {
         const Launch &l = launch[i];
-        const int64_t *const got = (const int64_t *)(host + l.host_at);
+        const int64_t *const got = (const int64_t *)(host + l.at);
         const Owned status(PyLong_FromUnsignedLong(*(const uint32_t *)(got + l.n * l.offs)));
         const Tensor counts = need_hist ? l.mail.slice(0, l.n * l.offs + 1).view(at::kInt) : Tensor();
         for (int k = 0; k < l.n; ++k) {

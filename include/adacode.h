@@ -131,16 +131,17 @@ int adacode_pack_jobs(const adacode_pack_job *jobs, int n_jobs, int B, int H, in
 /*
  * adacode_pack_jobs for a caller that needs to know the result: report_bytes bytes of device memory (a multiple of 4, at
  * most 1 MiB) are cleared before the jobs run and written to page-locked host memory after them, by the
- * compaction's last CTA, followed by the 32-bit `token`.  The jobs' seg_escape_offsets, hist256 and `status` are meant
- * to lie in report_dev.  report_host_pinned has room for report_bytes + 4 bytes; pinned memory as for adacode_copy_to_host.
- * adacode_wait_report polls for the token (any value that the 4 bytes do not hold before the call) and returns when the
- * report is complete; ADACODE_ERR_CUDA if the stream fails or runs dry without it.
+ * compaction's last CTA, each 32-bit word followed by the 32-bit `token`.  The jobs' seg_escape_offsets, hist256 and
+ * `status` are meant to lie in report_dev.  report_host_pinned has room for 2 * report_bytes bytes, 8-byte aligned; pinned
+ * memory as for adacode_copy_to_host.
+ * adacode_wait_report polls for the words with this token (one that none of the room's odd words holds before the pack) and
+ * returns when all report_bytes are in `out`; ADACODE_ERR_CUDA if the stream fails or runs dry without them.
  * Replaces: a clearing launch before, and a copying launch and an event behind every pack whose escape totals the host reads.
  */
 int adacode_pack_jobs_report(const adacode_pack_job *jobs, int n_jobs, int B, int H, int seq_tile, int D, int nbits,
                              void *workspace, size_t workspace_bytes, int32_t *status, void *report_dev,
                              void *report_host_pinned, size_t report_bytes, uint32_t token, void *stream);
-int adacode_wait_report(const void *report_host_pinned, size_t report_bytes, uint32_t token, void *stream);
+int adacode_wait_report(const void *report_host_pinned, size_t report_bytes, uint32_t token, void *out, void *stream);
 
 /*
  * Maximum size of the library-owned scratch used by adacode_pack_tiles_static, in bytes.

@@ -58,9 +58,12 @@ def test_refusals(cuda_device):
                                           torch.cuda.current_stream().cuda_stream)
     assert call(dev.data_ptr(), pinned.data_ptr(), 6) == _lib.ERR_INVALID_ARG
     assert call(dev.data_ptr() + 2, pinned.data_ptr(), 8) == _lib.ERR_INVALID_ARG
+    assert call(dev.data_ptr(), pinned.data_ptr() + 4, 8) == _lib.ERR_INVALID_ARG
     assert call(dev.data_ptr(), torch.zeros(128, dtype=torch.uint8).data_ptr(), 8) == _lib.ERR_INVALID_ARG      # not page-locked
     assert call(dev.data_ptr(), pinned.data_ptr(), (1 << 20) + 4) == _lib.ERR_TOO_LARGE
     assert call(dev.data_ptr(), pinned.data_ptr(), 8) == _lib.OK                                            # no jobs: the cleared words
-    assert L.adacode_wait_report(pinned.data_ptr(), 8, 1, torch.cuda.current_stream().cuda_stream) == _lib.OK
+    out = torch.full((2,), -1, dtype=torch.int32)
+    stream = torch.cuda.current_stream().cuda_stream
+    assert L.adacode_wait_report(pinned.data_ptr(), 8, 1, out.data_ptr(), stream) == _lib.OK and not out.any()
     # a token that nothing will send: an error as soon as the stream is idle
-    assert L.adacode_wait_report(pinned.data_ptr(), 8, 77, torch.cuda.current_stream().cuda_stream) == _lib.ERR_CUDA
+    assert L.adacode_wait_report(pinned.data_ptr(), 8, 77, out.data_ptr(), stream) == _lib.ERR_CUDA

@@ -55,16 +55,17 @@ struct AttnArgs {
     // and go on in the next.  (cut_items x cut_ctas < 2**31)
     int items, head_groups, heads_per_row;
     int cut_items, cut_ctas;
+    Quotient by_items, by_head_groups, by_heads, by_cut_items, by_cut_ctas;      // (by_heads: Hkv)
 };
 
 // Item at which the run of CTA c begins, and the CTA whose run holds item x.
 __device__ __forceinline__ int run_begin(const AttnArgs &a, int c) {
-    const int cut = c / a.cut_ctas, r = c - cut * a.cut_ctas;
-    return cut * a.cut_items + a.cut_items * r / a.cut_ctas;
+    const int cut = (uint32_t)c / a.by_cut_ctas, r = c - cut * a.cut_ctas;
+    return cut * a.cut_items + (int)((uint32_t)(a.cut_items * r) / a.by_cut_ctas);
 }
 __device__ __forceinline__ int cta_of(const AttnArgs &a, int x) {
-    const int cut = x / a.cut_items, y = x - cut * a.cut_items;
-    return cut * a.cut_ctas + ((y + 1) * a.cut_ctas - 1) / a.cut_items;
+    const int cut = (uint32_t)x / a.by_cut_items, y = x - cut * a.cut_items;
+    return cut * a.cut_ctas + (int)((uint32_t)((y + 1) * a.cut_ctas - 1) / a.by_cut_items);
 }
 
 struct AttnSmem {
@@ -823,7 +824,7 @@ __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_
     __syncthreads();
     // this CTA's items [begin, end), and the units that are to be decoded for them (two per packed item)
     const int begin = run_begin(a, blockIdx.x), end = run_begin(a, blockIdx.x + 1);
-    const int row0 = begin / a.items, item0 = begin - row0 * a.items, row1 = end / a.items;
+    const int row0 = (uint32_t)begin / a.by_items, item0 = begin - row0 * a.items, row1 = (uint32_t)end / a.by_items;
     const int n_units = 2 * ((row1 - row0) * a.n_seg + min(end - row1 * a.items, a.n_seg) - min(item0, a.n_seg));
     // launched as a programmatic dependent of its predecessor in the stream: no global memory is touched above
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -846,7 +847,7 @@ __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_
                     item = more % a.n_seg;
                 }
                 const adacode_segment sg = ((n + lane) & 1 ? a.vseg : a.kseg)[item];
-                s.src[lane] = resolve_segment_tile(sg, row / a.head_groups, kTileTokens * D, nullptr, 0);
+                s.src[lane] = resolve_segment_tile(sg, (uint32_t)row / a.by_head_groups, kTileTokens * D, nullptr, 0);
             }
             __syncwarp();
         }
@@ -863,11 +864,11 @@ __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_
     int u = 0;                                               // units of this CTA so far
     for (int x = begin; x < end;) {
         // the part [first, last) of one row's items
-        const int row = x / a.items, first = x - row * a.items;
+        const int row = (uint32_t)x / a.by_items, first = x - row * a.items;
         const int last = min(a.items, first + (end - x));
         x += last - first;
-        const int bh = row / a.head_groups;
-        const int b = bh / a.Hkv, hkv = bh - b * a.Hkv;
+        const int bh = (uint32_t)row / a.by_head_groups;
+        const int b = (uint32_t)bh / a.by_heads, hkv = bh - b * a.Hkv;
         const int gz = (row - bh * a.head_groups) * (8 * HG);    // 8 or 16 query heads of the group at a time
         const int G = min(a.G - gz, 8 * HG);
         const int u1 = u + 2 * (min(last, a.n_seg) - min(first, a.n_seg));
@@ -1010,17 +1011,21 @@ static_assert(sizeof(AttnPipeSmem<128>) <= 113 * 1024, "two CTAs of the pipeline
 
 // CTAs of the pipelined kernel that are resident at a time: two per SM.
 long long resident_ctas() {
-    int sms = 148;
+    static std::atomic<int> known[64];
     int dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148 * 2;
+    int sms = known[dev].load(std::memory_order_relaxed);
+    if (sms == 0) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148 * 2;
+        known[dev].store(sms, std::memory_order_relaxed);
+    }
     return (long long)sms * 2;
 }
 
-// CTAs that the items of all rows are dealt out to evenly: all that are resident at a time, fewer if there are
+// CTAs that the items of all rows are dealt out to evenly: the n that are resident at a time, fewer if there are
 // fewer items or if a row would be cut into more than kMaxSplits parts (at most n / rows + 2, or n / rows where
 // that is a whole number).
-long long even_ctas(long long rows, int items) {
-    long long n = resident_ctas();
+long long even_ctas(long long n, long long rows, int items) {
     if (n > rows * items) n = rows * items;
     if (n >= rows * kMaxSplits) n = rows * kMaxSplits;
     else if (n > rows * (kMaxSplits - 1)) n = rows * (kMaxSplits - 1);
@@ -1030,8 +1035,7 @@ long long even_ctas(long long rows, int items) {
 // Whole splits per (batch, KV head), for workspaces that hold no more: the grid should fill a whole number of waves
 // of resident CTAs.  One, two and three waves are
 // tried and the fullest wins; fewer waves on ties (more tiles per CTA, less per-CTA overhead).
-int pick_splits(int B, int Hkv, int items) {
-    const long long slots = resident_ctas();
+int pick_splits(long long slots, int B, int Hkv, int items) {
     const long long bh = (long long)B * Hkv;
     int best = 1;
     double best_fill = 0.0;
@@ -1120,7 +1124,8 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
     const long long rows = (long long)B * Hkv * head_groups;
     if (rows * items >= (1ll << 31)) return ADACODE_ERR_INVALID_ARG;
     const bool given = n_splits > 0;
-    if (!given) n_splits = pick_splits(B, Hkv * head_groups, items);
+    const long long slots = given ? 0 : resident_ctas();
+    if (!given) n_splits = pick_splits(slots, B, Hkv * head_groups, items);
     if (n_splits > kMaxSplits) n_splits = kMaxSplits;
     if (workspace_bytes < adacode_decode_attn_workspace_bytes(B, Hq, D, n_splits)) return ADACODE_ERR_WORKSPACE;
     if (n_splits > items) n_splits = items;                // (the others would be empty)
@@ -1131,7 +1136,7 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
     // 54.8 us, or 5 and 52.6 us; 128 rows of 3 items ([64, 2, 300, 128]): 2 either way, 18.4 us whole, 21.1 us cut.
     long long n_ctas = rows * n_splits, cut_items = items, cut_ctas = n_splits;
     if (!given && !force_simple) {
-        const long long slots = resident_ctas(), even = even_ctas(rows, items);
+        const long long even = even_ctas(slots, rows, items);
         const int parts = (int)(even % rows == 0 ? even / rows : even / rows + 2);
         const long long whole_run = (n_ctas + slots - 1) / slots * ((items + n_splits - 1) / n_splits);
         const long long even_run = (rows * items + even - 1) / even + (even % rows != 0);
@@ -1144,6 +1149,8 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
     AttnArgs a;
     a.items = items, a.head_groups = head_groups, a.heads_per_row = heads_per_cta;
     a.cut_items = (int)cut_items, a.cut_ctas = (int)cut_ctas;
+    a.by_items = quotient_by(items), a.by_head_groups = quotient_by(head_groups), a.by_heads = quotient_by(Hkv);
+    a.by_cut_items = quotient_by(cut_items), a.by_cut_ctas = quotient_by(cut_ctas);
     a.q = (const uint16_t *)q_bf16, a.q_sb = q_stride_b, a.q_sh = q_stride_h;
     a.kseg = k_segments_dev, a.vseg = v_segments_dev, a.n_seg = n_segments;
     a.k_tail = (const uint16_t *)k_tail_bf16, a.v_tail = (const uint16_t *)v_tail_bf16, a.tail_len = tail_len;

@@ -10,6 +10,19 @@ constexpr int kCPT = 4;                          // chunks per thread per slab
 constexpr int kSlabChunks = kThreads * kCPT;     // 1024
 constexpr unsigned kFull = 0xFFFFFFFFu;
 
+// Quotients of numbers below 2**31 by a divisor that the host knows, by multiplication (Granlund and Montgomery,
+// Division by invariant integers using multiplication, 1994: 2**l >= d, m = 2**31 (2**l - d) / d + 2**31 + 1 rounded
+// down, n / d = n m >> (31 + l)).
+struct Quotient {
+    uint32_t d, m, shift;
+};
+Quotient quotient_by(int64_t d) {
+    int l = 0;
+    while ((1ll << l) < d) ++l;
+    return {(uint32_t)d, (uint32_t)(((1ull << 31) * ((1ull << l) - (uint64_t)d)) / (uint64_t)d + (1ull << 31) + 1), (uint32_t)(31 + l)};
+}
+__device__ __forceinline__ uint32_t operator/(uint32_t n, const Quotient &q) { return (uint32_t)((uint64_t)n * q.m >> q.shift); }
+
 // ---------------------------------------------------------------------------------------
 // bit helpers
 // ---------------------------------------------------------------------------------------

@@ -559,19 +559,6 @@ __global__ void k_choose_params(const int32_t *__restrict__ hists, int n_hists, 
 constexpr int kHistVec = 4;
 constexpr int kHistCtas = 3;                                   // per SM
 
-// Quotients of numbers below 2**31 by a divisor that the host knows, by multiplication (Granlund and Montgomery,
-// Division by invariant integers using multiplication, 1994: 2**l >= d, m = 2**31 (2**l - d) / d + 2**31 + 1 rounded
-// down, n / d = n m >> (31 + l)).
-struct Quotient {
-    uint32_t d, m, shift;
-};
-Quotient quotient_by(int64_t d) {
-    int l = 0;
-    while ((1ll << l) < d) ++l;
-    return {(uint32_t)d, (uint32_t)(((1ull << 31) * ((1ull << l) - (uint64_t)d)) / (uint64_t)d + (1ull << 31) + 1), (uint32_t)(31 + l)};
-}
-__device__ __forceinline__ uint32_t operator/(uint32_t n, const Quotient &q) { return (uint32_t)((uint64_t)n * q.m >> q.shift); }
-
 struct HistRuns {
     const uint16_t *src;
     int64_t runs, run_vec;
@@ -844,6 +831,7 @@ bool unpack_prefers_wide() {
 }
 
 int launch_unpack_pipe(UnpackJobsArgs &ja, cudaStream_t st) {
+    for (int j = 0; j < ja.n_jobs; ++j) ja.job[j].by_BH = quotient_by(ja.job[j].BH), ja.job[j].by_H = quotient_by(ja.job[j].H);
     ja.poll_limit = g_poll_limit;
     ja.withhold_unit = g_withhold_unit;
     // a unit holds at least eight token rows: the narrow geometry takes head_dim up to 1024
@@ -1179,6 +1167,7 @@ int pack_jobs_impl(const adacode_pack_job *jobs, int n_jobs, int B, int H, int s
         }
         pa.n_jobs = n;
         pa.H = H, pa.BH = (int)BH, pa.seq_tile = seq_tile, pa.D = D, pa.tile_elems = (int)tile_elems;
+        pa.by_BH = quotient_by(BH), pa.by_H = quotient_by(H);
         pa.n_tiles = n_tiles;
         pa.esc_scratch = sc.esc, pa.tile_counts = sc.tile_counts, pa.unit_counts = sc.unit_counts;
         pa.blk_off = sc.blk_off, pa.done = sc.done;

@@ -221,6 +221,7 @@ struct UnpackPipeArgs {
     const adacode_segment *seg;
     // common
     int H, BH, seq_tile, D, tile_elems;
+    Quotient by_BH, by_H;
     long long n_tiles;
     uint16_t *dst;
     long long db, dh, ds;
@@ -253,9 +254,9 @@ __device__ __forceinline__ TileSrc resolve_segment_tile(const adacode_segment &s
 
 __device__ __forceinline__ TileSrc resolve_tile(const UnpackPipeArgs &a, long long tile) {
     TileSrc t;
-    const long long blk = tile / a.BH;
+    const long long blk = (uint32_t)tile / a.by_BH;       // (fewer than 2**31 tiles: their planes fit a GPU)
     const int bh = (int)(tile - blk * a.BH);
-    const int b = bh / a.H, h = bh - b * a.H;
+    const int b = (uint32_t)bh / a.by_H, h = bh - b * a.H;
     uint16_t *base = a.dst + (long long)b * a.db + (long long)h * a.dh;
     t.ds = a.ds;
     if (a.seg) {
@@ -789,6 +790,7 @@ struct PackPipeArgs {
     PackJob job[kMaxJobs];
     int n_jobs;
     int H, BH, seq_tile, D, tile_elems;
+    Quotient by_BH, by_H;
     int64_t n_tiles;          // over all jobs
     uint8_t *esc_scratch;     // n_tiles * tile_elems bytes, global tile t owns [t * tile_elems, ...)
     int32_t *tile_counts;     // n_tiles
@@ -1105,9 +1107,9 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const 
             const int j = job_of_tile(pa, tile);
             const PackJob &jb = pa.job[j];
             const int64_t lt = tile - jb.tile0;
-            const int64_t blk = lt / pa.BH;
+            const int64_t blk = (uint32_t)lt / pa.by_BH;
             const int bh = (int)(lt - blk * pa.BH);
-            const int b = bh / pa.H, h = bh - b * pa.H;
+            const int b = (uint32_t)bh / pa.by_H, h = bh - b * pa.H;
             const uint16_t *tsrc = jb.src + (int64_t)b * jb.sb + (int64_t)h * jb.sh + blk * pa.seq_tile * jb.ss;
             const bool rows_contig = (jb.ss == pa.D), use_map = ka.use_map[j] != 0;
             for (int u = 0; u < upt; ++u, ++it) {

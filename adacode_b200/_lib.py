@@ -30,7 +30,7 @@ EXPORTED_SYMBOLS = (
     'adacode_choose_params', 'adacode_choose_params_host', 'adacode_calibrate_host', 'adacode_pack_tiles_static',
     'adacode_decode_attn_workspace_bytes', 'adacode_decode_attn', 'adacode_copy_to_host',
     'adacode_pack_jobs', 'adacode_pack_jobs_report', 'adacode_wait_report', 'adacode_unpack_jobs', 'adacode_unpack_jobs_with_rows', 'adacode_copy_rows', 'adacode_max_jobs', 'adacode_debug_set_wait_limit',
-    'adacode_flat_block_elems', 'adacode_unpack_flat',
+    'adacode_flat_block_elems', 'adacode_pack_flat', 'adacode_unpack_flat', 'adacode_unpack_flat_ragged',
 )
 
 
@@ -128,6 +128,10 @@ def lib() -> ctypes.CDLL:
     L.adacode_flat_block_elems.argtypes = [i32]
     L.adacode_unpack_flat.restype = i32
     L.adacode_unpack_flat.argtypes = [vp, vp, vp, i64, vp, i64, i32, i32, vp, vp, vp]
+    L.adacode_pack_flat.restype = i32
+    L.adacode_pack_flat.argtypes = [vp, i64, i32, i32, vp, vp, vp, i64, vp, vp, vp, sz, vp, vp, ctypes.c_uint32, vp]
+    L.adacode_unpack_flat_ragged.restype = i32
+    L.adacode_unpack_flat_ragged.argtypes = L.adacode_unpack_flat.argtypes
     L.adacode_debug_set_wait_limit.restype = i32
     L.adacode_debug_set_wait_limit.argtypes = [ctypes.c_uint, i32]
     L.adacode_pack_jobs.restype = i32

@@ -424,6 +424,13 @@ def pack_blocks_finish(p: _PendingPack, host_meta):
     return _finish_pack(p, host_meta[: p.n_blocks + 1].tolist(), int(host_meta[p.n_blocks + 1]) & 0xFFFFFFFF)
 
 
+def _trim_escapes(escapes: torch.Tensor, total: int, large_guess: bool, n: int) -> torch.Tensor:
+    # (a large first guess is not kept, which packs of single blocks would for the cache's life: it is cut to size
+    # where an eighth more than the escapes and a 32nd of the elements are unused)
+    keep = total + total // 8 + min(65536, n // 32) if large_guess else 2 * total + 65536
+    return escapes[:total].clone() if escapes.numel() > keep else escapes[:total]
+
+
 def _finish_pack(p: _PendingPack, offsets: list, status: int):
     n_blocks = p.n_blocks
     total = offsets[-1]
@@ -439,16 +446,7 @@ def _finish_pack(p: _PendingPack, offsets: list, status: int):
             raise _lib.AdacodeError('adacode_pack_tiles: escape overflow after re-run with exact capacity')
     elif status_other:
         raise _lib.AdacodeError(f'adacode_pack_tiles: device status {status:#x} ({describe_status(status)})')
-    # (a large first guess is not kept, which packs of single blocks would for the cache's life: it is cut to size
-    # where an eighth more than the escapes and a 32nd of the elements are unused)
-    if p.guessed and p.nbits <= 2:
-        keep = total + total // 8 + min(65536, p.sign_mant.numel() // 32)
-    else:
-        keep = 2 * total + 65536
-    if escapes.numel() > keep:
-        escapes = escapes[:total].clone()
-    else:
-        escapes = escapes[:total]
+    escapes = _trim_escapes(escapes, total, p.guessed and p.nbits <= 2, p.n)
     meta = p.meta if p.meta.shape[0] == n_blocks + 1 else p.meta[: n_blocks + 1]
     chunk = PackedChunk(p.sign_mant, p.codes, escapes, p.tile_base, offsets, meta,
                         p.right - 2 ** p.nbits + 1, p.right, p.nbits, p.B, p.H, p.seq_tile, p.D)
@@ -480,6 +478,27 @@ def pack_pair(k: torch.Tensor, v: torch.Tensor, k_params, v_params, seq_tile: in
                                 need_hist, capacities)
     kh, vh = (None, None) if hists is None else hists
     return kd[0], vd[0], kd[1], vd[1], kh, vh
+
+
+def pack_flat(x: torch.Tensor, right: int, nbits: int, block_elems: int, hist: Optional[torch.Tensor] = None) -> tuple:
+    """``(sign_mant, codes, escapes, block_base int32)`` of a contiguous bf16 CUDA tensor in the flat layout, whose
+    element count is a multiple of 8; ``hist`` (int32[256] on the device) is added to."""
+    n = x.numel()
+    if x.data_ptr() % 16 and n % block_elems:
+        x = x.clone()                            # (a ragged tensor may begin anywhere)
+    dev = x.device
+    cap, guessed = _default_escape_capacity(n, nbits), True
+    while True:
+        ws = _scratch_for(dev).workspace_for(n // block_elems, block_elems)
+        sm, cd, escapes, base, total, status = _lib.native().pack_flat(x, right, nbits, block_elems, cap, hist if guessed else None, ws)
+        if total <= cap:
+            break
+        if not guessed:
+            raise _lib.AdacodeError('adacode_pack_flat: escape overflow after re-run with exact capacity')
+        cap, guessed = total, False              # (the histogram is complete from the first pass)
+    if status:
+        raise _lib.AdacodeError(f'adacode_pack_flat: device status {status:#x} ({describe_status(status)})')
+    return sm, cd, _trim_escapes(escapes, total, guessed and nbits <= 2, n), base
 
 
 def unpack_chunk(chunk: PackedChunk, dst: torch.Tensor, seq_offset: int = 0) -> None:

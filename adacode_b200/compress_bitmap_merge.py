@@ -6,7 +6,7 @@ one sign/mantissa byte per element, n-bit exponent codes, one compact list of es
 in flat order and ``block_base``: the inclusive running escape count per ``invalid_block_size``
 (= 128 x {8, 4, 8, 2}[nbits - 1]) elements.  These are exactly the planes ``adacode_pack_tiles``
 writes for tiles of one block each, so ``compress`` is one such launch; ``uncompress`` goes
-through ``adacode_unpack_flat``, which decodes 16384-element tiles and takes every
+through ``adacode_unpack_flat_ragged``, which decodes 16384-element tiles and takes every
 (16384 / block)-th base.  There is no CPU path.
 """
 from __future__ import annotations
@@ -18,13 +18,6 @@ from .rows import on_device, stream_ptr
 
 _BLOCK_GAPS = (8, 4, 8, 2)
 _MAX_ELEMS_PER_CALL = 1 << 30
-
-
-def _ones_code_bytes(nbits: int, n_bytes: int, device) -> torch.Tensor:
-    """Code bytes in which every code is 1 (an in-window code): padding that needs no escape."""
-    pattern = {1: [0xFF], 2: [0x55], 3: [0x24, 0x92, 0x49], 4: [0x11]}[nbits]
-    reps = (n_bytes + len(pattern) - 1) // len(pattern)
-    return torch.tensor(pattern * reps, dtype=torch.uint8, device=device)[:n_bytes]
 
 
 class CompressorBitMap:
@@ -128,44 +121,22 @@ class CompressorBitMap:
         flat = x.reshape(-1)
         if not flat.is_contiguous():
             flat = flat.contiguous()
-        n_blocks = (n + ibs - 1) // ibs
-        n_pad = n_blocks * ibs
-        real_tail_escapes = None
-        if n_pad != n:
-            # whole blocks only: pad with zeros (they escape, after every real element of the last
-            # block) and drop their escape bytes again below
-            tail = flat[(n_blocks - 1) * ibs:]
-            e = (tail.view(torch.int16).to(torch.int32) >> 7) & 0xFF
-            real_tail_escapes = int(((e <= self.left) | (e > self.right)).sum().item())
-            flat = torch.cat([flat, torch.zeros(n_pad - n, dtype=torch.bfloat16, device=x.device)])
         hist = torch.zeros(256, dtype=torch.int32, device=x.device) if need_adjust else None
+        # one call; beyond _MAX_ELEMS_PER_CALL one per run of whole blocks
         per_call = max(ibs, (_MAX_ELEMS_PER_CALL // ibs) * ibs)
         signs, codes, escs, bases = [], [], [], []
         carried = 0
-        for lo in range(0, n_pad, per_call):
-            hi = min(n_pad, lo + per_call)
-            part = flat[lo:hi].view(1, (hi - lo) // ibs, ibs // 32, 32)
-            chunk, _ = codec.pack_blocks(part, self.right, self.nbits, ibs // 32, need_hist=need_adjust, hist_out=hist)
-            signs.append(chunk.sign_mant.reshape(-1))
-            codes.append(chunk.codes.reshape(-1))
-            escs.append(chunk.escapes)
-            bases.append(chunk.tile_base.reshape(-1) + carried if carried else chunk.tile_base.reshape(-1))
-            carried += chunk.n_escapes
+        for lo in range(0, n, per_call):
+            sm, cd, esc, base = codec.pack_flat(flat[lo: lo + per_call], self.right, self.nbits, ibs, hist)
+            signs.append(sm)
+            codes.append(cd)
+            escs.append(esc)
+            bases.append(base + carried if carried else base)
+            carried += esc.numel()
         self.sign_mass_data = signs[0] if len(signs) == 1 else torch.cat(signs)
         self.exp_data = codes[0] if len(codes) == 1 else torch.cat(codes)
         self.invalid_exp = escs[0] if len(escs) == 1 else torch.cat(escs)
         base = (bases[0] if len(bases) == 1 else torch.cat(bases)).to(torch.int32)
-        if n_pad != n:
-            pad = n_pad - n
-            before_last = int(base[-2].item()) if n_blocks > 1 else 0
-            keep = before_last + real_tail_escapes
-            self.invalid_exp = self.invalid_exp[:keep].clone()
-            base = base.clone()
-            base[-1] = keep
-            self.sign_mass_data = self.sign_mass_data[:n].clone()
-            self.exp_data = self.exp_data[: n * self.nbits // 8].clone()
-            if hist is not None:
-                hist[0] -= pad                       # the padding's exponent is 0
         self._base_i32 = base
         self.block_base = base.to(torch.int64)
         self.n_exp_data = n * self.nbits // 8
@@ -183,36 +154,24 @@ class CompressorBitMap:
         out = uncompressed_odb
         if out.numel() != self.n_elements or out.element_size() != 2 or not out.is_contiguous():
             raise ValueError('uncompress_with_weights needs a contiguous 16-bit buffer of n_elements elements')
-        n, ibs = self.n_elements, self.invalid_block_size
-        n_whole = (n // ibs) * ibs
+        n = self.n_elements
+        if n == 0:
+            return
         dev = self.device
         sc = codec._scratch_for(dev)
-        esc = self.invalid_exp
-        stream = stream_ptr(dev)
-        L = _lib.lib()
+        sm, cd, esc, dst = self.sign_mass_data, self.exp_data, self.invalid_exp, out
+        if n < self.invalid_block_size:
+            # (one short block may lie anywhere; the kernels want 16-byte boundaries)
+            sm, cd = (t if t.data_ptr() % 16 == 0 else t.clone() for t in (sm, cd))
+            if out.data_ptr() % 16:
+                dst = torch.empty_like(out)
         with on_device(dev):
-            if n_whole:
-                rc = L.adacode_unpack_flat(self.sign_mass_data.data_ptr(), self.exp_data.data_ptr(),
-                                           esc.data_ptr() if esc.numel() else 0, esc.numel(),
-                                           self._kernel_base().data_ptr(), n_whole, self.left, self.nbits,
-                                           out.data_ptr(), sc.status.data_ptr(), stream)
-                _lib.check(rc, 'adacode_unpack_flat')
-            if n_whole != n:
-                # ragged last block: decode a padded copy of its planes (padding codes are in-window)
-                r = n - n_whole
-                sm = torch.zeros(ibs, dtype=torch.uint8, device=dev)
-                sm[:r] = self.sign_mass_data[n_whole:]
-                cd = _ones_code_bytes(self.nbits, ibs * self.nbits // 8, dev).clone()
-                cd[: r * self.nbits // 8] = self.exp_data[n_whole * self.nbits // 8:]
-                prev = int(self.block_base[-2].item()) if self.block_base.numel() > 1 else 0
-                tail_esc = esc[prev:].contiguous()
-                base = torch.tensor([tail_esc.numel()], dtype=torch.int32, device=dev)
-                tmp = torch.empty(ibs, dtype=torch.int16, device=dev)
-                rc = L.adacode_unpack_flat(sm.data_ptr(), cd.data_ptr(), tail_esc.data_ptr() if tail_esc.numel() else 0,
-                                           tail_esc.numel(), base.data_ptr(), ibs, self.left, self.nbits,
-                                           tmp.data_ptr(), sc.status.data_ptr(), stream)
-                _lib.check(rc, 'adacode_unpack_flat')
-                out.view(torch.int16)[n_whole:] = tmp[:r]
+            rc = _lib.lib().adacode_unpack_flat_ragged(sm.data_ptr(), cd.data_ptr(), esc.data_ptr() if esc.numel() else 0, esc.numel(),
+                                                       self._kernel_base().data_ptr(), n, self.left, self.nbits, dst.data_ptr(),
+                                                       sc.status.data_ptr(), stream_ptr(dev))
+        _lib.check(rc, 'adacode_unpack_flat_ragged')
+        if dst is not out:
+            out.copy_(dst)
 
     def uncompress(self):
         out = torch.empty(self.n_elements, dtype=torch.bfloat16, device=self.device)

@@ -808,15 +808,17 @@ template <class G>
 int launch_unpack_geom(const UnpackJobsArgs &ja, cudaStream_t st) {
     int rc = ensure_dynamic_smem(k_unpack_pipe<G>, sizeof(UnpackSmemT<G>));
     if (rc != ADACODE_OK) return rc;
-    // CTAs for the tiles, or for the rows that go along if those take more (a CTA without tiles copies and leaves)
+    // CTAs for the tiles, or for the rows or blocks that go along if those take more (a CTA without tiles leaves after them)
     int64_t vecs = 0;
     for (int i = 0; i < ja.rows.n; ++i) {
         const adacode_row_copy &c = ja.rows.copy[i];
         vecs += (int64_t)c.B * c.H * c.rows * (c.D / 8);
     }
     const int64_t for_rows = (vecs + G::kConsumers * kRowVecs - 1) / (G::kConsumers * kRowVecs);
-    const int64_t tiles = ja.tile0[ja.n_jobs];
-    const int grid = grid_for(tiles > for_rows ? tiles : for_rows, G::kCtasPerSm);
+    int64_t want = ja.tile0[ja.n_jobs];
+    if (want < for_rows) want = for_rows;
+    if (want < ja.rest.blocks) want = ja.rest.blocks;
+    const int grid = grid_for(want, G::kCtasPerSm);
     return launch_dependent(k_unpack_pipe<G>, dim3(grid), G::kThreads, sizeof(UnpackSmemT<G>), st, ja);
 }
 
@@ -845,6 +847,7 @@ int launch_unpack_pipe(const UnpackPipeArgs &a, cudaStream_t st) {
     ja.tile0[0] = 0, ja.tile0[1] = a.n_tiles;
     ja.n_jobs = 1;
     ja.rows.n = 0;
+    ja.rest.blocks = 0;
     return launch_unpack_pipe(ja, st);
 }
 
@@ -1000,6 +1003,83 @@ int launch_copy_rows(const RowCopies &rc, int64_t most, cudaStream_t st) {
 __global__ void k_copy_to_host(const uint32_t *__restrict__ src, uint32_t *dst, size_t words) {
     for (size_t i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
     __threadfence_system();
+}
+
+// The last, short block of a flat tensor behind the whole ones, which are packed already: fewer than 1024 elements, eight per
+// thread of one CTA, bound by the latency of its loads.  Whatever it needs of the others (where its escapes begin) lies in
+// device memory, so nothing waits for the host in between, and the tensor is not copied to be padded.
+struct FlatTail {
+    const uint16_t *src;                                   // the block's first element
+    uint8_t *sign_mant, *codes;                            // its planes
+    uint8_t *escapes;                                      // the tensor's stream
+    int64_t capacity;
+    int32_t *base;                                         // the block's entry
+    int64_t *total;                                        // in: escapes before it, out: with it
+    int32_t *hist;                                         // nullable
+    int32_t *status;
+    int elems, left, nbits;
+    Report report;
+};
+
+__global__ void __launch_bounds__(128) k_flat_tail(const __grid_constant__ FlatTail a) {
+    __shared__ int s_hist[256], s_tot[4];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, groups = a.elems / 8;
+    s_hist[tid] = s_hist[tid + 128] = 0;
+    __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int64_t before = __ldcg(a.total);
+    uint32_t e[8];
+    uint32_t x = 0, escaped = 0;
+    if (tid < groups) {
+        alignas(16) uint16_t v[8];
+        *reinterpret_cast<uint4 *>(v) = reinterpret_cast<const uint4 *>(a.src)[tid];
+        alignas(8) uint8_t s[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            e[k] = (v[k] >> 7) & 0xFFu;
+            s[k] = (uint8_t)(((v[k] >> 8) & 0x80u) | (v[k] & 0x7Fu));
+            const uint32_t c = e[k] - (uint32_t)a.left, code = c < (1u << a.nbits) ? c : 0u;
+            x = (x << a.nbits) | code;
+            escaped |= (uint32_t)(code == 0u) << k;
+            if (a.hist) atomicAdd(&s_hist[e[k]], 1);
+        }
+        reinterpret_cast<uint2 *>(a.sign_mant)[tid] = *reinterpret_cast<const uint2 *>(s);
+        for (int i = 0; i < a.nbits; ++i) a.codes[tid * a.nbits + i] = (uint8_t)(x >> (8 * (a.nbits - 1 - i)));
+    }
+    const int count = __popc(escaped);
+    int incl = count;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int u = __shfl_up_sync(kFull, incl, d);
+        if (lane >= d) incl += u;
+    }
+    if (lane == 31) s_tot[warp] = incl;
+    __syncthreads();
+    int all = 0;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        if (w < warp) incl += s_tot[w];
+        all += s_tot[w];
+    }
+    int64_t r = before + incl - count;
+    bool fits = true;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if ((escaped >> k) & 1u) {
+            if (r < a.capacity) a.escapes[r] = (uint8_t)e[k];
+            else fits = false;
+            ++r;
+        }
+    if (!fits) atomicOr(a.status, ADACODE_STATUS_ESCAPE_OVERFLOW);
+    if (a.hist)
+        for (int i = tid; i < 256; i += 128)
+            if (s_hist[i] != 0) atomicAdd(a.hist + i, s_hist[i]);
+    if (tid == 0) {
+        *a.base = (int32_t)(before + all);
+        *a.total = before + all;
+    }
+    __syncthreads();
+    if (a.report.words != 0) send_report(a.report);
 }
 
 // A report on its own, behind kernels that send none.
@@ -1218,6 +1298,47 @@ int adacode_pack_jobs_report(const adacode_pack_job *jobs, int n_jobs, int B, in
     return pack_jobs_impl(jobs, n_jobs, B, H, seq_tile, D, nbits, workspace, workspace_bytes, status, &r, (cudaStream_t)stream);
 }
 
+int adacode_pack_flat(const void *src_bf16, int64_t n_elems, int right, int nbits, uint8_t *sign_mant, uint8_t *codes, uint8_t *escapes,
+                      int64_t escapes_capacity, int32_t *block_base, int32_t *hist256, void *workspace, size_t workspace_bytes,
+                      void *report_dev, void *report_host_pinned, uint32_t token, void *stream) {
+    const int be = adacode_flat_block_elems(nbits);
+    if (be == 0 || n_elems <= 0 || n_elems % 8 != 0 || escapes_capacity < 0 || !src_bf16 || !sign_mant || !codes || !block_base ||
+        (!escapes && escapes_capacity > 0) || !report_dev || ((uintptr_t)report_dev & 7) != 0 || !report_host_pinned ||
+        ((uintptr_t)report_host_pinned & 7) != 0 || (((uintptr_t)src_bf16 | (uintptr_t)sign_mant | (uintptr_t)codes) & 15) != 0)
+        return ADACODE_ERR_INVALID_ARG;
+    if (n_elems >= (1ll << 31)) return ADACODE_ERR_TOO_LARGE;
+    uint32_t *host;
+    int rc = host_view(report_host_pinned, host);
+    if (rc != ADACODE_OK) return rc;
+    // report: [offsets of the whole blocks' escapes: 0 and their total, in the end the tensor's | status]
+    int64_t *const offsets = (int64_t *)report_dev;
+    int32_t *const status = (int32_t *)(offsets + 2);
+    const Report report = {(const uint32_t *)report_dev, (uint2 *)host, ADACODE_FLAT_REPORT_BYTES / 4, token};
+    const cudaStream_t st = (cudaStream_t)stream;
+    const int64_t whole = n_elems / be, n_whole = whole * be;
+    const int tail = (int)(n_elems - n_whole);
+    if (whole > 0) {
+        const adacode_pack_job jb = {src_bf16, n_whole, be, 32, 1, right, sign_mant, codes, escapes, escapes_capacity, block_base, offsets, hist256};
+        if (tail > 0) {
+            // (the short block's kernel reports)
+            if (!workspace || workspace_bytes < adacode_pack_workspace_bytes(whole, be)) return ADACODE_ERR_WORKSPACE;
+            ADACODE_CUDA_TRY(cudaMemsetAsync(report_dev, 0, ADACODE_FLAT_REPORT_BYTES, st));
+        }
+        rc = pack_jobs_impl(&jb, 1, 1, (int)whole, be / 32, 32, nbits, workspace, workspace_bytes, status, tail > 0 ? nullptr : &report, st);
+        if (rc != ADACODE_OK || tail == 0) return rc;
+    } else {
+        ADACODE_CUDA_TRY(cudaMemsetAsync(report_dev, 0, ADACODE_FLAT_REPORT_BYTES, st));
+    }
+    FlatTail t;
+    t.src = (const uint16_t *)src_bf16 + n_whole;
+    t.sign_mant = sign_mant + n_whole, t.codes = codes + n_whole * nbits / 8;
+    t.escapes = escapes, t.capacity = escapes_capacity;
+    t.base = block_base + whole, t.total = offsets + 1, t.hist = hist256, t.status = status;
+    t.elems = tail, t.left = right - (1 << nbits) + 1, t.nbits = nbits;
+    t.report = report;
+    return launch_dependent(k_flat_tail, dim3(1), 128, 0, st, t);
+}
+
 int adacode_wait_report(const void *report_host_pinned, size_t report_bytes, uint32_t token, void *out, void *stream) {
     if (!report_host_pinned || !out || (report_bytes & 3) != 0 || ((uintptr_t)report_host_pinned & 7) != 0) return ADACODE_ERR_INVALID_ARG;
     const uint64_t *words = (const uint64_t *)report_host_pinned;
@@ -1350,47 +1471,52 @@ int adacode_flat_block_elems(int nbits) {
     return (nbits < 1 || nbits > 4) ? 0 : 128 * gaps[nbits - 1];
 }
 
-int adacode_unpack_flat(const uint8_t *sign_mant, const uint8_t *codes, const uint8_t *escapes, int64_t escapes_len,
-                        const int32_t *block_base, int64_t n_elems, int left, int nbits, void *dst_bf16,
-                        int32_t *status, void *stream) {
+static int unpack_flat_impl(const uint8_t *sign_mant, const uint8_t *codes, const uint8_t *escapes, int64_t escapes_len,
+                            const int32_t *block_base, int64_t n_elems, int64_t multiple, int left, int nbits, void *dst_bf16,
+                            int32_t *status, void *stream) {
     const int be = adacode_flat_block_elems(nbits);
-    if (be == 0 || n_elems < 0 || n_elems % be != 0 || !status) return ADACODE_ERR_INVALID_ARG;
+    if (be == 0 || n_elems < 0 || n_elems % multiple != 0 || !status) return ADACODE_ERR_INVALID_ARG;
     if (n_elems == 0) return ADACODE_OK;
     if (n_elems >= (1ll << 31)) return ADACODE_ERR_TOO_LARGE;
     if (!sign_mant || !codes || !block_base || !dst_bf16) return ADACODE_ERR_INVALID_ARG;
     if ((((uintptr_t)sign_mant | (uintptr_t)codes | (uintptr_t)dst_bf16) & 15) != 0) return ADACODE_ERR_INVALID_ARG;
     if (!pipeline_enabled()) return ADACODE_ERR_INVALID_ARG;
-    cudaStream_t st = (cudaStream_t)stream;
     // the bulk of the tensor as 128 x 128 tiles whose escape base is every (16384 / be)-th block base,
-    // the rest (fewer than 16384 elements) block by block
+    // the rest (fewer than 16384 elements) block by block in the same launch
     const int64_t big = 128 * 128;
     const int64_t n_big = n_elems / big;
-    const int64_t n_main = n_big * big;
-    UnpackPipeArgs pa;
-    memset(&pa, 0, sizeof(pa));
-    pa.escapes = escapes, pa.escapes_len = escapes_len, pa.seg_off = nullptr, pa.left = left, pa.nbits = nbits;
-    pa.seg = nullptr, pa.status = status;
-    if (n_big > 0) {
-        pa.sign_mant = sign_mant, pa.codes = codes, pa.tile_base = block_base;
-        pa.tb_stride = (int)(big / be), pa.tb_before = 0;
-        pa.H = (int)n_big, pa.BH = (int)n_big, pa.seq_tile = 128, pa.D = 128, pa.tile_elems = (int)big;
-        pa.n_tiles = n_big, pa.dst = (uint16_t *)dst_bf16;
-        pa.db = 0, pa.dh = big, pa.ds = 128;
-        int rc = launch_unpack_pipe(pa, st);
-        if (rc != ADACODE_OK) return rc;
-    }
-    const int64_t n_rest = (n_elems - n_main) / be;
-    if (n_rest > 0) {
-        pa.sign_mant = sign_mant + n_main, pa.codes = codes + n_main * nbits / 8;
-        pa.tile_base = block_base + n_main / be;
-        pa.tb_stride = 1, pa.tb_before = n_main > 0 ? 1 : 0;
-        pa.H = (int)n_rest, pa.BH = (int)n_rest, pa.seq_tile = be / 32, pa.D = 32, pa.tile_elems = be;
-        pa.n_tiles = n_rest, pa.dst = (uint16_t *)dst_bf16 + n_main;
-        pa.db = 0, pa.dh = be, pa.ds = 32;
-        int rc = launch_unpack_pipe(pa, st);
-        if (rc != ADACODE_OK) return rc;
-    }
-    return ADACODE_OK;
+    UnpackJobsArgs ja;
+    memset(&ja, 0, sizeof(ja));
+    UnpackPipeArgs &pa = ja.job[0];
+    pa.escapes = escapes, pa.escapes_len = escapes_len, pa.left = left, pa.nbits = nbits, pa.status = status;
+    pa.sign_mant = sign_mant, pa.codes = codes, pa.tile_base = block_base;
+    pa.tb_stride = (int)(big / be);
+    pa.H = pa.BH = (int)(n_big > 0 ? n_big : 1), pa.seq_tile = 128, pa.D = 128, pa.tile_elems = (int)big;
+    pa.n_tiles = n_big, pa.dst = (uint16_t *)dst_bf16;
+    pa.dh = big, pa.ds = 128;
+    ja.n_jobs = 1;
+    ja.tile0[1] = n_big;
+    FlatRest &f = ja.rest;
+    const int64_t rest = n_elems - n_big * big;
+    f.sign_mant = sign_mant, f.codes = codes, f.escapes = escapes, f.escapes_len = escapes_len, f.block_base = block_base;
+    f.dst = (uint16_t *)dst_bf16, f.left = left, f.nbits = nbits, f.block_elems = be;
+    f.first = (int)(n_big * (big / be)), f.blocks = (int)((rest + be - 1) / be);
+    f.last_elems = (int)(rest - (int64_t)(f.blocks - 1) * be);
+    return launch_unpack_pipe(ja, (cudaStream_t)stream);
+}
+
+int adacode_unpack_flat(const uint8_t *sign_mant, const uint8_t *codes, const uint8_t *escapes, int64_t escapes_len,
+                        const int32_t *block_base, int64_t n_elems, int left, int nbits, void *dst_bf16,
+                        int32_t *status, void *stream) {
+    const int be = adacode_flat_block_elems(nbits);
+    return unpack_flat_impl(sign_mant, codes, escapes, escapes_len, block_base, n_elems, be > 0 ? be : 1, left, nbits, dst_bf16, status,
+                            stream);
+}
+
+int adacode_unpack_flat_ragged(const uint8_t *sign_mant, const uint8_t *codes, const uint8_t *escapes, int64_t escapes_len,
+                               const int32_t *block_base, int64_t n_elems, int left, int nbits, void *dst_bf16,
+                               int32_t *status, void *stream) {
+    return unpack_flat_impl(sign_mant, codes, escapes, escapes_len, block_base, n_elems, 8, left, nbits, dst_bf16, status, stream);
 }
 
 int adacode_copy_rows(const adacode_row_copy *copies, int n_copies, void *stream) {

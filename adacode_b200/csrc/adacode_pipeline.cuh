@@ -538,10 +538,67 @@ struct RowCopies {
     int n;
 };
 
+// The end of a flat tensor that is less than a tile: `blocks` blocks of `block_elems` elements from block `first` on, the last
+// one of last_elems (a multiple of 8).
+struct FlatRest {
+    const uint8_t *sign_mant, *codes, *escapes;            // of the whole tensor
+    long long escapes_len;
+    const int32_t *block_base;
+    uint16_t *dst;
+    int first, blocks, block_elems, last_elems, left, nbits;
+};
+
+// One of those blocks by the consumer threads of a CTA, eight elements per thread (a block has 1024 at most): bound by
+// the latency of its loads, beside the tiles of the same launch.
+template <class G>
+__device__ __noinline__ void unpack_flat_block(const FlatRest &f, int b, int *warp_tot, int32_t *status) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nbits = f.nbits, groups = (b == f.blocks - 1 ? f.last_elems : f.block_elems) / 8;
+    const long long blk = f.first + b, g = blk * (f.block_elems / 8) + tid;        // this thread's group of the tensor
+    const uint32_t mask = (1u << nbits) - 1u;
+    uint32_t x = 0;
+    uint2 sv = make_uint2(0u, 0u);
+    long long start = 0;
+    int count = 0;
+    if (tid < groups) {
+        for (int i = 0; i < nbits; ++i) x = (x << 8) | f.codes[g * nbits + i];
+        sv = *reinterpret_cast<const uint2 *>(f.sign_mant + g * 8);
+        for (int k = 0; k < 8; ++k) count += ((x >> (k * nbits)) & mask) == 0u;
+    }
+    if (blk > 0) start = f.block_base[blk - 1];
+    int incl = count;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int u = __shfl_up_sync(kFull, incl, d);
+        if (lane >= d) incl += u;
+    }
+    if (lane == 31) warp_tot[warp] = incl;
+    consumer_sync<G::kConsumers>();
+    for (int w = 0; w < warp; ++w) incl += warp_tot[w];
+    if (tid < groups) {
+        long long r = start + incl - count;
+        alignas(16) uint16_t out[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t code = (x >> ((7 - k) * nbits)) & mask, s = ((k < 4 ? sv.x : sv.y) >> (8 * (k & 3))) & 0xFFu;
+            uint32_t e = (code + (uint32_t)f.left) & 0xFFu;
+            if (code == 0u) {
+                if (r < f.escapes_len) e = f.escapes[r];
+                else e = 0u, atomicOr(status, ADACODE_STATUS_ESCAPE_UNDERRUN);
+                ++r;
+            }
+            out[k] = (uint16_t)(((s & 0x80u) << 8) | (e << 7) | (s & 0x7Fu));
+        }
+        *reinterpret_cast<uint4 *>(f.dst + g * 8) = *reinterpret_cast<const uint4 *>(out);
+    }
+    consumer_sync<G::kConsumers>();                        // (the counts are read)
+}
+
 // Up to kMaxJobs destinations in one launch; job j owns the tiles [tile0[j], tile0[j + 1]).
 struct UnpackJobsArgs {
     UnpackPipeArgs job[kMaxJobs];
     RowCopies rows;           // dense rows that go along
+    FlatRest rest;            // blocks that go along (rest.blocks == 0: none)
     long long tile0[kMaxJobs + 1];
     int n_jobs;
     uint32_t poll_limit;      // bound of every on-chip wait (kMaxPolls unless a test lowered it)
@@ -622,6 +679,7 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_unpack_pipe(cons
     // the dense rows first, while the first units are on their way
     for (int j = 0; j < ja.rows.n; ++j)
         copy_rows(ja.rows.copy[j], blockIdx.x * (uint32_t)G::kConsumers + tid, gridDim.x * (uint32_t)G::kConsumers);
+    for (int b = blockIdx.x; b < ja.rest.blocks; b += gridDim.x) unpack_flat_block<G>(ja.rest, b, s.warp_tot[0], a0.status);
     int consumed = 0;
     bool broken = false;                  // a wait of this warp ran out: compute on, store nothing
     // row (upper half) and column of this thread's chunks inside a unit (a chunk never crosses a row: D % 16 == 0)

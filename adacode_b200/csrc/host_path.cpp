@@ -96,6 +96,11 @@ struct ReportBox {
     }
 };
 
+ReportBox &report_box() {
+    static thread_local ReportBox box;
+    return box;
+}
+
 // pack(tensors, rights, nbits, seq_tile, capacities, need_hist, workspace)
 //   -> (((sign_mant, codes, escapes, tile_base, seg_offsets, histogram or None, offsets, status), ...), hist bytes or None)
 // Tensors that follow each other and share shape and code length go through one launch; all launches are under way before the
@@ -175,7 +180,7 @@ PyObject *pack(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
     }
     // a report holds a MiB at most; more offsets than that are fetched by a copy
     const bool reports = host_bytes <= (1 << 20);
-    static thread_local ReportBox box;
+    ReportBox &box = report_box();
     if (reports) box.reserve(2 * host_bytes);
     std::vector<uint8_t> fetched(host_bytes);
     uint8_t *const host = fetched.data();
@@ -234,6 +239,50 @@ PyObject *pack(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
         }
     }
     return PyTuple_Pack(2, parts.p, hists.p);
+    END_HANDLE_TH_ERRORS
+}
+
+// pack_flat(x, right, nbits, block, capacity, histogram or None, workspace)
+//   -> (sign_mant, codes, escapes, block_base, total, status)
+// A contiguous bf16 tensor on a GPU, a multiple of 8 and fewer than 2**31 elements on a 16-byte boundary.  As with pack,
+// trimming and packing again are the caller's.
+PyObject *pack_flat(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
+    HANDLE_TH_ERRORS
+    TORCH_CHECK_TYPE(n_args == 7, "pack_flat: arguments");
+    const Tensor &x = tensor(args[0]), &ws = tensor(args[6]);
+    const int right = (int)integer(args[1]), nbits = (int)integer(args[2]);
+    const int64_t block = integer(args[3]), cap = integer(args[4]), n = x.numel();
+    const Tensor hist = args[5] == Py_None ? Tensor() : tensor(args[5]);
+    TORCH_CHECK(x.scalar_type() == at::kBFloat16 && x.is_cuda() && x.is_contiguous() && n > 0 && block > 0 && cap >= 0 && nbits >= 1 && nbits <= 4,
+                "pack_flat: a contiguous bf16 tensor on a GPU");
+    TORCH_CHECK(!hist.defined() || (hist.scalar_type() == at::kInt && hist.numel() == 256 && hist.is_contiguous() && hist.device() == x.device()),
+                "pack_flat: a histogram is 256 contiguous int32 on the GPU");
+    const c10::cuda::CUDAGuard on(x.device());
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+    const auto bytes = at::TensorOptions().device(x.device()).dtype(at::kByte);
+    const Tensor sm = at::empty({n}, bytes), cd = at::empty({n * nbits / 8}, bytes), esc = at::empty({cap}, bytes);
+    const Tensor base = at::empty({(n + block - 1) / block}, bytes.dtype(at::kInt)), mail = at::empty({ADACODE_FLAT_REPORT_BYTES / 8}, bytes.dtype(at::kLong));
+    int64_t got[ADACODE_FLAT_REPORT_BYTES / 8];
+    ReportBox &box = report_box();
+    box.reserve(2 * sizeof(got));
+    const uint32_t token = box.next_token();
+    const char *what = "adacode_pack_flat";
+    int rc;
+    {
+        pybind11::gil_scoped_release waits;
+        rc = adacode_pack_flat(x.const_data_ptr(), n, right, nbits, (uint8_t *)sm.mutable_data_ptr(), (uint8_t *)cd.mutable_data_ptr(),
+                               (uint8_t *)esc.mutable_data_ptr(), cap, (int32_t *)base.mutable_data_ptr(),
+                               hist.defined() ? (int32_t *)hist.mutable_data_ptr() : nullptr, ws.mutable_data_ptr(), ws.nbytes(),
+                               mail.mutable_data_ptr(), box.host, token, stream);
+        if (rc == ADACODE_OK) {
+            what = "adacode_wait_report";
+            rc = adacode_wait_report(box.host, sizeof(got), token, got, stream);
+        }
+    }
+    check(rc, what);
+    const Owned o_sm(THPVariable_Wrap(sm)), o_cd(THPVariable_Wrap(cd)), o_esc(THPVariable_Wrap(esc)), o_base(THPVariable_Wrap(base)),
+        total(PyLong_FromLongLong(got[1])), status(PyLong_FromUnsignedLong((uint32_t)got[2]));
+    return PyTuple_Pack(6, o_sm.p, o_cd.p, o_esc.p, o_base.p, total.p, status.p);
     END_HANDLE_TH_ERRORS
 }
 
@@ -351,6 +400,7 @@ PyObject *dense_view(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
 
 PyMethodDef methods[] = {
     {"pack", (PyCFunction)(void (*)(void))pack, METH_FASTCALL, nullptr},
+    {"pack_flat", (PyCFunction)(void (*)(void))pack_flat, METH_FASTCALL, nullptr},
     {"append", (PyCFunction)(void (*)(void))append, METH_FASTCALL, nullptr},
     {"dense_view", (PyCFunction)(void (*)(void))dense_view, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},

@@ -144,6 +144,18 @@ int adacode_pack_jobs_report(const adacode_pack_job *jobs, int n_jobs, int B, in
 int adacode_wait_report(const void *report_host_pinned, size_t report_bytes, uint32_t token, void *out, void *stream);
 
 /*
+ * Pack a FLAT tensor of n_elems elements (a multiple of 8, see adacode_unpack_flat): sign_mant has n_elems bytes, codes
+ * n_elems * nbits / 8, block_base an entry per block, the last of which may be short.  Reports as
+ * adacode_pack_jobs_report does, ADACODE_FLAT_REPORT_BYTES bytes of its own: int64 0, int64 number of escapes, the status
+ * word, padding.  The scratch must hold adacode_pack_workspace_bytes(n_elems / block, block).
+ * Replaces: CompressorBitMap.compress (compress_bitmap_merge.py:179-420, :768-822), where a ragged end is padded.
+ */
+#define ADACODE_FLAT_REPORT_BYTES 24u
+int adacode_pack_flat(const void *src_bf16, int64_t n_elems, int right, int nbits, uint8_t *sign_mant, uint8_t *codes, uint8_t *escapes,
+                      int64_t escapes_capacity, int32_t *block_base, int32_t *hist256, void *workspace, size_t workspace_bytes,
+                      void *report_dev, void *report_host_pinned, uint32_t token, void *stream);
+
+/*
  * Maximum size of the library-owned scratch used by adacode_pack_tiles_static, in bytes.
  * A call fits when adacode_pack_workspace_bytes(n_tiles, tile_elems) is not larger (roughly
  * 4 Mi bf16 elements per call, e.g. thirty-two 128-token blocks of an [8, 128]-shaped head set).
@@ -265,6 +277,11 @@ int adacode_copy_rows(const adacode_row_copy *copies, int n_copies, void *stream
 /* adacode_unpack_jobs and adacode_copy_rows (the not yet packed tails behind the segments) in ONE launch. */
 int adacode_unpack_jobs_with_rows(const adacode_unpack_job *jobs, int n_jobs, int B, int H, int seq_tile, int D,
                                   const adacode_row_copy *copies, int n_copies, int32_t *status, void *stream);
+
+/* adacode_unpack_flat for any number of elements that is a multiple of 8: the last block may be shorter than the others. */
+int adacode_unpack_flat_ragged(const uint8_t *sign_mant, const uint8_t *codes, const uint8_t *escapes, int64_t escapes_len,
+                               const int32_t *block_base, int64_t n_elems, int left, int nbits, void *dst_bf16,
+                               int32_t *status, void *stream);
 
 /* Elements per escape-base block of the flat layout for a code length: 128 * {8, 4, 8, 2}[nbits - 1]
  * (compress_bitmap_merge.py:653-657, invalid_block_size); 0 for an invalid nbits. */

@@ -903,8 +903,12 @@ int launch_pack_kernel(Kernel kernel, const PackPipeArgs &pa, cudaStream_t st) {
 
 template <int N, class G>
 int launch_pack_pipe_n(const PackPipeArgs &pa, bool hist, cudaStream_t st) {
-    return hist ? launch_pack_kernel<G>(k_pack_pipe<N, true, G>, pa, st)
-                : launch_pack_kernel<G>(k_pack_pipe<N, false, G>, pa, st);
+    if constexpr (G::kUnit == WideGeom::kUnit)
+        if (pa.block_base)
+            return hist ? launch_pack_kernel<G>(k_pack_pipe<N, true, true, G>, pa, st)
+                        : launch_pack_kernel<G>(k_pack_pipe<N, false, true, G>, pa, st);
+    return hist ? launch_pack_kernel<G>(k_pack_pipe<N, true, false, G>, pa, st)
+                : launch_pack_kernel<G>(k_pack_pipe<N, false, false, G>, pa, st);
 }
 
 // The pack kernel takes the narrow geometry where a unit of the wide one would stay half empty
@@ -923,7 +927,7 @@ bool pack_takes_narrow(int seq_tile, int D) {
 
 // Pipelined pack of all jobs of `pa` with one pack launch and one compaction launch.
 int launch_pack_pipe(PackPipeArgs &pa, int nbits, cudaStream_t st) {
-    const bool narrow = pack_takes_narrow(pa.seq_tile, pa.D);
+    const bool narrow = !pa.block_base && pack_takes_narrow(pa.seq_tile, pa.D);
     pa.unit_rows = narrow ? unit_rows_for<NarrowGeom::kUnit>(pa.seq_tile, pa.D)
                           : unit_rows_for<WideGeom::kUnit>(pa.seq_tile, pa.D);
     pa.units_per_tile = (pa.seq_tile + pa.unit_rows - 1) / pa.unit_rows;
@@ -955,8 +959,11 @@ int launch_pack_pipe(PackPipeArgs &pa, int nbits, cudaStream_t st) {
     if (rc != ADACODE_OK) return rc;
     // (a programmatic dependent of the pack kernel: it is set up, and clears its histogram copies, while
     // the pack kernel's last CTAs still run)
-    return hist ? launch_dependent(k_compact_units<true>, cgrid, kThreads, 0, st, pa)
-                : launch_dependent(k_compact_units<false>, cgrid, kThreads, 0, st, pa);
+    if (pa.block_base)
+        return hist ? launch_dependent(k_compact_units<true, true>, cgrid, kThreads, 0, st, pa)
+                    : launch_dependent(k_compact_units<false, true>, cgrid, kThreads, 0, st, pa);
+    return hist ? launch_dependent(k_compact_units<true, false>, cgrid, kThreads, 0, st, pa)
+                : launch_dependent(k_compact_units<false, false>, cgrid, kThreads, 0, st, pa);
 }
 
 template <int N, int CH>
@@ -1005,49 +1012,60 @@ __global__ void k_copy_to_host(const uint32_t *__restrict__ src, uint32_t *dst, 
     __threadfence_system();
 }
 
-// The last, short block of a flat tensor behind the whole ones, which are packed already: fewer than 1024 elements, eight per
-// thread of one CTA, bound by the latency of its loads.  Whatever it needs of the others (where its escapes begin) lies in
-// device memory, so nothing waits for the host in between, and the tensor is not copied to be padded.
+// The end of a flat tensor behind its 16384-element tiles, which are packed already: blocks of block_elems, the last one
+// perhaps short, sixteen elements per thread of one CTA, bound by the latency of its loads.  Whatever it needs of the others
+// (where its escapes begin) lies in device memory, so nothing waits for the host in between, and the tensor is not
+// copied to be padded.
+constexpr int kTailThreads = 1024;
+constexpr int64_t kBigFlat = 4 << 20;         // elements from which adacode_pack_flat takes tiles of 16384
+
 struct FlatTail {
-    const uint16_t *src;                                   // the block's first element
+    const uint16_t *src;                                   // the first element behind the tiles
     uint8_t *sign_mant, *codes;                            // its planes
     uint8_t *escapes;                                      // the tensor's stream
     int64_t capacity;
-    int32_t *base;                                         // the block's entry
-    int64_t *total;                                        // in: escapes before it, out: with it
+    int32_t *base;                                         // its first block's entry
+    int64_t *total;                                        // in: escapes before it, out: of the tensor
     int32_t *hist;                                         // nullable
     int32_t *status;
-    int elems, left, nbits;
+    int elems, block_elems, left, nbits;
     Report report;
 };
 
-__global__ void __launch_bounds__(128) k_flat_tail(const __grid_constant__ FlatTail a) {
-    __shared__ int s_hist[256], s_tot[4];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, groups = a.elems / 8;
-    s_hist[tid] = s_hist[tid + 128] = 0;
+__global__ void __launch_bounds__(kTailThreads) k_flat_tail(const __grid_constant__ FlatTail a) {
+    __shared__ int s_hist[256], s_tot[kTailThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, groups = a.elems / 8, per_block = a.block_elems / 8;
+    if (tid < 256) s_hist[tid] = 0;
     __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int64_t before = __ldcg(a.total);
-    uint32_t e[8];
-    uint32_t x = 0, escaped = 0;
-    if (tid < groups) {
-        alignas(16) uint16_t v[8];
-        *reinterpret_cast<uint4 *>(v) = reinterpret_cast<const uint4 *>(a.src)[tid];
-        alignas(8) uint8_t s[8];
+    // two groups per thread: the longest end, of 16376 elements, in one go
+    uint32_t e[16], escaped = 0;
+    int count[2] = {0, 0};
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            e[k] = (v[k] >> 7) & 0xFFu;
-            s[k] = (uint8_t)(((v[k] >> 8) & 0x80u) | (v[k] & 0x7Fu));
-            const uint32_t c = e[k] - (uint32_t)a.left, code = c < (1u << a.nbits) ? c : 0u;
-            x = (x << a.nbits) | code;
-            escaped |= (uint32_t)(code == 0u) << k;
-            if (a.hist) atomicAdd(&s_hist[e[k]], 1);
+    for (int q = 0; q < 2; ++q) {
+        const int g = 2 * tid + q;
+        if (g < groups) {
+            alignas(16) uint16_t v[8];
+            *reinterpret_cast<uint4 *>(v) = reinterpret_cast<const uint4 *>(a.src)[g];
+            alignas(8) uint8_t s[8];
+            uint32_t x = 0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const uint32_t ex = (v[k] >> 7) & 0xFFu;
+                e[8 * q + k] = ex;
+                s[k] = (uint8_t)(((v[k] >> 8) & 0x80u) | (v[k] & 0x7Fu));
+                const uint32_t c = ex - (uint32_t)a.left, code = c < (1u << a.nbits) ? c : 0u;
+                x = (x << a.nbits) | code;
+                escaped |= (uint32_t)(code == 0u) << (8 * q + k);
+                count[q] += code == 0u;
+                if (a.hist) atomicAdd(&s_hist[ex], 1);
+            }
+            reinterpret_cast<uint2 *>(a.sign_mant)[g] = *reinterpret_cast<const uint2 *>(s);
+            for (int i = 0; i < a.nbits; ++i) a.codes[g * a.nbits + i] = (uint8_t)(x >> (8 * (a.nbits - 1 - i)));
         }
-        reinterpret_cast<uint2 *>(a.sign_mant)[tid] = *reinterpret_cast<const uint2 *>(s);
-        for (int i = 0; i < a.nbits; ++i) a.codes[tid * a.nbits + i] = (uint8_t)(x >> (8 * (a.nbits - 1 - i)));
     }
-    const int count = __popc(escaped);
-    int incl = count;
+    int incl = count[0] + count[1];
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
         const int u = __shfl_up_sync(kFull, incl, d);
@@ -1055,29 +1073,26 @@ __global__ void __launch_bounds__(128) k_flat_tail(const __grid_constant__ FlatT
     }
     if (lane == 31) s_tot[warp] = incl;
     __syncthreads();
-    int all = 0;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-        if (w < warp) incl += s_tot[w];
-        all += s_tot[w];
-    }
-    int64_t r = before + incl - count;
+    const int t = s_tot[lane];
+    incl += (int)__reduce_add_sync(kFull, (unsigned)(lane < warp ? t : 0));
+    const int all = (int)__reduce_add_sync(kFull, (unsigned)t);
     bool fits = true;
+    int64_t r = before + incl - count[0] - count[1];
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
+    for (int k = 0; k < 16; ++k)
         if ((escaped >> k) & 1u) {
             if (r < a.capacity) a.escapes[r] = (uint8_t)e[k];
             else fits = false;
             ++r;
         }
-    if (!fits) atomicOr(a.status, ADACODE_STATUS_ESCAPE_OVERFLOW);
-    if (a.hist)
-        for (int i = tid; i < 256; i += 128)
-            if (s_hist[i] != 0) atomicAdd(a.hist + i, s_hist[i]);
-    if (tid == 0) {
-        *a.base = (int32_t)(before + all);
-        *a.total = before + all;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int g = 2 * tid + q;
+        if (g < groups && (g % per_block == per_block - 1 || g == groups - 1)) a.base[g / per_block] = (int32_t)(before + incl - (q ? 0 : count[1]));
     }
+    if (!fits) atomicOr(a.status, ADACODE_STATUS_ESCAPE_OVERFLOW);
+    if (a.hist && tid < 256 && s_hist[tid] != 0) atomicAdd(a.hist + tid, s_hist[tid]);
+    if (tid == 0) *a.total = before + all;
     __syncthreads();
     if (a.report.words != 0) send_report(a.report);
 }
@@ -1310,33 +1325,53 @@ int adacode_pack_flat(const void *src_bf16, int64_t n_elems, int right, int nbit
     uint32_t *host;
     int rc = host_view(report_host_pinned, host);
     if (rc != ADACODE_OK) return rc;
-    // report: [offsets of the whole blocks' escapes: 0 and their total, in the end the tensor's | status]
+    // report: [offsets of the tiles' escapes: 0 and their total, in the end the tensor's | status]
     int64_t *const offsets = (int64_t *)report_dev;
     int32_t *const status = (int32_t *)(offsets + 2);
     const Report report = {(const uint32_t *)report_dev, (uint2 *)host, ADACODE_FLAT_REPORT_BYTES / 4, token};
     const cudaStream_t st = (cudaStream_t)stream;
-    const int64_t whole = n_elems / be, n_whole = whole * be;
-    const int tail = (int)(n_elems - n_whole);
-    if (whole > 0) {
-        const adacode_pack_job jb = {src_bf16, n_whole, be, 32, 1, right, sign_mant, codes, escapes, escapes_capacity, block_base, offsets, hist256};
-        if (tail > 0) {
-            // (the short block's kernel reports)
-            if (!workspace || workspace_bytes < adacode_pack_workspace_bytes(whole, be)) return ADACODE_ERR_WORKSPACE;
-            ADACODE_CUDA_TRY(cudaMemsetAsync(report_dev, 0, ADACODE_FLAT_REPORT_BYTES, st));
-        }
-        rc = pack_jobs_impl(&jb, 1, 1, (int)whole, be / 32, 32, nbits, workspace, workspace_bytes, status, tail > 0 ? nullptr : &report, st);
-        if (rc != ADACODE_OK || tail == 0) return rc;
-    } else {
-        ADACODE_CUDA_TRY(cudaMemsetAsync(report_dev, 0, ADACODE_FLAT_REPORT_BYTES, st));
+    // Tiles of 16384 elements (a unit of the pack kernel, in which a warp has 1024) and the rest in one CTA, or tiles of one
+    // block, which leave most of a unit's warps without work but need the last CTA for a short block only: 4096 x 14336
+    // weights 343 and 108 us through the Python call, 4001 x 8008 216 and 93 us, 211 x 696 57 and 71 us.
+    const int64_t big = 128 * 128, tile = pipeline_enabled() && n_elems >= kBigFlat ? big : be, n_big = n_elems / tile, done = n_big * tile;
+    const int rest = (int)(n_elems - done);
+    if (n_big > 0 && (!workspace || ((uintptr_t)workspace & 15) != 0)) return ADACODE_ERR_INVALID_ARG;
+    if (n_big > 0 && workspace_bytes < adacode_pack_workspace_bytes(n_big, tile)) return ADACODE_ERR_WORKSPACE;
+    ADACODE_CUDA_TRY(cudaMemsetAsync(report_dev, 0, ADACODE_FLAT_REPORT_BYTES, st));
+    if (n_big > 0 && tile != big) {
+        const adacode_pack_job jb = {src_bf16, done, be, 32, 1, right, sign_mant, codes, escapes, escapes_capacity, block_base, offsets, hist256};
+        rc = pack_jobs_impl(&jb, 1, 1, (int)n_big, be / 32, 32, nbits, workspace, workspace_bytes, status, rest == 0 ? &report : nullptr, st);
+        if (rc != ADACODE_OK || rest == 0) return rc;
+    } else if (n_big > 0) {
+        const PackScratch sc = carve_pack_scratch(workspace, n_big, big);
+        PackPipeArgs pa;
+        memset(&pa, 0, sizeof(pa));
+        PackJob &d = pa.job[0];
+        d.src = (const uint16_t *)src_bf16, d.sb = n_elems, d.sh = big, d.ss = 128;
+        d.sign_mant = sign_mant, d.codes = codes, d.escapes = escapes, d.capacity = escapes_capacity;
+        d.seg_off = offsets, d.hist = hist256, d.n_blocks = 1, d.left = right - (1 << nbits) + 1;
+        pa.n_jobs = 1;
+        pa.H = pa.BH = (int)n_big, pa.seq_tile = 128, pa.D = 128, pa.tile_elems = (int)big, pa.n_tiles = n_big;
+        pa.by_BH = pa.by_H = quotient_by(n_big);
+        pa.esc_scratch = sc.esc, pa.tile_counts = sc.tile_counts, pa.unit_counts = sc.unit_counts;
+        pa.blk_off = sc.blk_off, pa.done = sc.done, pa.status = status, pa.poll_limit = g_poll_limit;
+        // (the scratch has 129 words per tile for unit counts, of which there are two at most: room for the blocks' counts,
+        // 64 at most, and for the tiles' bases, which nobody reads)
+        pa.block_counts = sc.unit_counts + 2 * n_big;
+        pa.block_base = block_base, pa.block_per_1024 = 1024 / be;
+        d.tile_base = sc.unit_counts + 66 * n_big;
+        if (rest == 0) pa.report = report;
+        rc = launch_pack_pipe(pa, nbits, st);
+        if (rc != ADACODE_OK || rest == 0) return rc;
     }
     FlatTail t;
-    t.src = (const uint16_t *)src_bf16 + n_whole;
-    t.sign_mant = sign_mant + n_whole, t.codes = codes + n_whole * nbits / 8;
+    t.src = (const uint16_t *)src_bf16 + done;
+    t.sign_mant = sign_mant + done, t.codes = codes + done * nbits / 8;
     t.escapes = escapes, t.capacity = escapes_capacity;
-    t.base = block_base + whole, t.total = offsets + 1, t.hist = hist256, t.status = status;
-    t.elems = tail, t.left = right - (1 << nbits) + 1, t.nbits = nbits;
+    t.base = block_base + done / be, t.total = offsets + 1, t.hist = hist256, t.status = status;
+    t.elems = rest, t.block_elems = be, t.left = right - (1 << nbits) + 1, t.nbits = nbits;
     t.report = report;
-    return launch_dependent(k_flat_tail, dim3(1), 128, 0, st, t);
+    return launch_dependent(k_flat_tail, dim3(1), kTailThreads, 0, st, t);
 }
 
 int adacode_wait_report(const void *report_host_pinned, size_t report_bytes, uint32_t token, void *out, void *stream) {

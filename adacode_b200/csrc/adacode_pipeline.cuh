@@ -785,6 +785,7 @@ struct PackUnitMeta {
     uint8_t *esc_dst;      // the unit's escape slot in the scratch
     int32_t *unit_count;   // where the unit's escape count goes
     int32_t *tile_count;   // where the tile's escape count goes (written with the last unit)
+    int32_t *block_counts; // flat layout: where the counts of the unit's blocks go
     int elems;
     int first_unit_of_tile;
     int last_unit_of_tile;
@@ -856,6 +857,10 @@ struct PackPipeArgs {
     int64_t *blk_off;         // over all blocks of the launch: escapes before global block i (n_blocks_total + 1)
     unsigned int *done;       // two counters (CTAs of the pack, of the compaction), zero on entry, zero on exit
     int unit_rows, units_per_tile;
+    // Flat layout (one job): a tile holds several escape-base blocks.  The pack kernel leaves block_counts, for every 1024
+    // elements the inclusive counts of their blocks (1024 / block_elems of them), the compaction makes block_base of them.
+    int32_t *block_counts, *block_base;
+    int block_per_1024;
     int scan_in_pack;         // offsets by the pack kernel's last CTA (else by the compaction's CTAs)
     Report report;            // what the compaction's last CTA hands to the host (words == 0: nothing)
     int32_t *status;
@@ -1031,7 +1036,7 @@ __device__ __forceinline__ void flush_code_counts(uint32_t (&cnt2)[HistRegs<N>::
 }
 
 // FULL: the unit has G::kUnit elements (every thread has both of its chunks), so nothing is predicated.
-template <int N, bool HIST, class G, bool FULL>
+template <int N, bool HIST, bool FLAT, class G, bool FULL>
 __device__ __forceinline__ void pack_unit(PackSmemT<G> &s, const PackStageT<G> &st, const PackUnitMeta &m,
                                           uint64_t *empty_bar, int &running, uint32_t (&cnt2)[HistRegs<N>::v],
                                           uint32_t neg_left, bool broken) {
@@ -1080,6 +1085,19 @@ __device__ __forceinline__ void pack_unit(PackSmemT<G> &s, const PackStageT<G> &
     int incl[kPCPT];
     const int wtot = warp_scan_counts(zc, incl);
     if (lane == 0) s.warp_tot[warp] = wtot;
+    if (FLAT && !broken && m.elems > 0) {
+        // this warp's 1024 elements are one block (N = 1, 3), two of 512 (2) or four of 256 (4)
+        if (N == 2) {
+            if (lane == 31) *reinterpret_cast<int2 *>(m.block_counts + 2 * warp) = make_int2(incl[0], incl[1]);
+        } else if (N == 4) {
+            if ((lane & 15) == 15) {
+                m.block_counts[4 * warp + (lane >> 4)] = incl[0];
+                m.block_counts[4 * warp + 2 + (lane >> 4)] = incl[1];
+            }
+        } else if (lane == 0) {
+            m.block_counts[warp] = wtot;
+        }
+    }
     bulk_wait_read();      // the previous unit's stores have finished reading the out buffers
     consumer_sync<G::kConsumers>();
     const int others = s.warp_tot[lane & (G::kWarps - 1)];
@@ -1129,7 +1147,7 @@ __device__ __forceinline__ void pack_unit(PackSmemT<G> &s, const PackStageT<G> &
     }
 }
 
-template <int N, bool HIST, class G>
+template <int N, bool HIST, bool FLAT, class G>
 __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const __grid_constant__ PackKernelArgs ka) {
     const PackPipeArgs &pa = ka.pa;
     static_assert(G::kConsumers >= 256, "one consumer thread per histogram bin");
@@ -1148,7 +1166,7 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const 
     if (tid < 2 * kStages) {
         // an empty unit: what a consumer sees if it gives up waiting before the first description is written
         PackUnitMeta &m = s.meta_ring[tid];
-        m.sm_dst = m.code_dst = m.esc_dst = nullptr, m.unit_count = m.tile_count = nullptr;
+        m.sm_dst = m.code_dst = m.esc_dst = nullptr, m.unit_count = m.tile_count = m.block_counts = nullptr;
         m.elems = 0, m.first_unit_of_tile = 1, m.last_unit_of_tile = 0, m.job = 0;
     }
     __syncthreads();
@@ -1185,6 +1203,8 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const 
                     m.esc_dst = pa.esc_scratch + tile * pa.tile_elems + (int64_t)row0 * pa.D;
                     m.unit_count = pa.unit_counts + tile * upt + u;
                     m.tile_count = pa.tile_counts + tile;
+                    constexpr int kPer1024 = N == 2 ? 2 : N == 4 ? 4 : 1;
+                    if (FLAT) m.block_counts = pa.block_counts + (e0 >> 10) * kPer1024;
                     m.elems = elems;
                     m.first_unit_of_tile = (u == 0);
                     m.last_unit_of_tile = (u == upt - 1);
@@ -1255,8 +1275,8 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtasPerSm) k_pack_pipe(const 
         for (;;) {
             const int stg = it % kStages;
             const PackUnitMeta &meta = s.meta_ring[it % (2 * kStages)];
-            if (meta.elems == G::kUnit) pack_unit<N, HIST, G, true>(s, s.stage[stg], meta, &s.empty[stg], running, cnt2, neg_left, broken);
-            else pack_unit<N, HIST, G, false>(s, s.stage[stg], meta, &s.empty[stg], running, cnt2, neg_left, broken);
+            if (meta.elems == G::kUnit) pack_unit<N, HIST, FLAT, G, true>(s, s.stage[stg], meta, &s.empty[stg], running, cnt2, neg_left, broken);
+            else pack_unit<N, HIST, FLAT, G, false>(s, s.stage[stg], meta, &s.empty[stg], running, cnt2, neg_left, broken);
             // the per-thread counters are 16-bit fields and grow by at most 32 per unit
             if (HIST && (it & 1023u) == 1023u) flush_code_counts<N>(cnt2, cur_left, s.hist);
             if (++it >= my_units) break;
@@ -1353,6 +1373,27 @@ __device__ __forceinline__ void compact_tile_units(const PackPipeArgs &pa, const
     }
 }
 
+// Flat layout: the inclusive escape counts of tile t's blocks, whose first escape is number `start` of the tensor; one warp.
+__device__ __forceinline__ void write_block_bases(const PackPipeArgs &pa, int64_t t, int64_t start) {
+    const int lane = threadIdx.x & 31, per = pa.block_per_1024;
+    const int64_t first = t * (pa.tile_elems >> 10);
+    for (int g0 = 0, groups = pa.tile_elems >> 10; g0 < groups; g0 += 32) {
+        const int32_t *counts = pa.block_counts + (first + g0 + lane) * per;
+        int32_t *base = pa.block_base + (first + g0 + lane) * per;
+        const bool mine = g0 + lane < groups;
+        const int all = mine ? __ldcg(counts + per - 1) : 0;
+        int incl = all;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int u = __shfl_up_sync(kFull, incl, d);
+            if (lane >= d) incl += u;
+        }
+        if (mine)
+            for (int i = 0; i < per; ++i) base[i] = (int32_t)start + incl - all + __ldcg(counts + i);
+        start += __shfl_sync(kFull, incl, 31);
+    }
+}
+
 // Offsets of the escapes of tiles [lt0, lt0 + n) of a job (n <= kThreads), by the whole CTA: their inclusive
 // counts inside the segment and the segments' offsets go to the caller's arrays, s_off[i] is tile lt0 + i's
 // first byte in the job's stream and s_cnt[i] its count.  Every CTA adds up all the counts before its own
@@ -1416,7 +1457,7 @@ __device__ __forceinline__ void tile_offsets(const PackPipeArgs &pa, const PackJ
 // is fetched with independent loads (one memory round trip).
 // With HIST the escaped exponents are counted here (whole warps of escape bytes) rather than one
 // by one inside the pack kernel, into one set of 256 bins per CTA.
-template <bool HIST>
+template <bool HIST, bool FLAT>
 __global__ void __launch_bounds__(kThreads) k_compact_units(const __grid_constant__ PackPipeArgs pa) {
     __shared__ int s_hist[HIST ? 256 : 1];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1438,8 +1479,10 @@ __global__ void __launch_bounds__(kThreads) k_compact_units(const __grid_constan
         const int n = (int)(job_tiles - lt0 < per ? job_tiles - lt0 : per);
         if (n > 0) {                                       // (uniform over the CTA)
             tile_offsets(pa, jb, (int)lt0, n, s_off, s_cnt, s_red);
-            for (int i = warp; i < n; i += kWarps)
+            for (int i = warp; i < n; i += kWarps) {
+                if (FLAT) write_block_bases(pa, lt0 + i, s_off[i]);
                 if (s_cnt[i] != 0) compact_tile_units(pa, jb, jb.tile0 + lt0 + i, s_off[i], s_cnt[i], my_hist, do_hist);
+            }
         }
     } else {
         const int64_t warp_global = (int64_t)blockIdx.x * kWarps + warp;
@@ -1451,6 +1494,7 @@ __global__ void __launch_bounds__(kThreads) k_compact_units(const __grid_constan
             const int c = __ldg(pa.tile_counts + t);
             const int tb = __ldg(jb.tile_base + lt);
             const int64_t so = __ldg(pa.blk_off + t / pa.BH) - job_off;
+            if (FLAT) write_block_bases(pa, t, so + tb - c);
             if (c == 0) continue;
             compact_tile_units(pa, jb, t, so + tb - c, c, my_hist, do_hist);
         }

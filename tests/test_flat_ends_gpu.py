@@ -30,7 +30,8 @@ def _check(dev, x_cpu, right, nbits, out_shift=0):
 
 
 @pytest.mark.parametrize('nbits', [1, 2, 3, 4])
-@pytest.mark.parametrize('n', [8, 248, 256, 264, 504, 1016, 1024, 1032, 16384 - 8, 16384, 16384 + 8, 16384 + 1024 + 504, 5 * 16384 + 15 * 1024 + 1016])
+@pytest.mark.parametrize('n', [8, 248, 256, 264, 504, 1016, 1024, 1032, 16384 - 8, 16384, 16384 + 8, 16384 + 1024 + 504, 5 * 16384 + 15 * 1024 + 1016,
+                               4 * 2 ** 20 - 8, 4 * 2 ** 20, 4 * 2 ** 20 + 8, 4 * 2 ** 20 + 16384 + 15 * 1024 + 1016])
 def test_sizes(cuda_device, n, nbits):
     x = synth.inject_escapes(synth.kv_tensor((1, 1, n // 8, 8), seed=n % 89, s=1.5), seed=4, left=121, right=128, p_window=0.05).reshape(-1)
     _check(cuda_device, x, 129, nbits)

@@ -26,7 +26,7 @@ STATUS_MISALIGNED = 8
 # every symbol include/adacode.h declares
 EXPORTED_SYMBOLS = (
     'adacode_version', 'adacode_strerror', 'adacode_last_cuda_error', 'adacode_pack_workspace_bytes',
-    'adacode_pack_tiles', 'adacode_unpack_tiles', 'adacode_unpack_segments', 'adacode_hist_bf16',
+    'adacode_pack_tiles', 'adacode_unpack_tiles', 'adacode_unpack_segments', 'adacode_hist_bf16', 'adacode_hist_bf16_cleared',
     'adacode_choose_params', 'adacode_choose_params_host', 'adacode_calibrate_host', 'adacode_pack_tiles_static',
     'adacode_decode_attn_workspace_bytes', 'adacode_decode_attn', 'adacode_copy_to_host',
     'adacode_pack_jobs', 'adacode_pack_jobs_report', 'adacode_wait_report', 'adacode_unpack_jobs', 'adacode_unpack_jobs_with_rows', 'adacode_copy_rows', 'adacode_max_jobs', 'adacode_debug_set_wait_limit',
@@ -110,6 +110,8 @@ def lib() -> ctypes.CDLL:
     L.adacode_unpack_segments.argtypes = [vp, i32, i32, i32, i32, i32, vp, i64, i64, i64, vp, vp]
     L.adacode_hist_bf16.restype = i32
     L.adacode_hist_bf16.argtypes = [vp, i64, i64, i64, i32, i32, i32, i32, vp, vp]
+    L.adacode_hist_bf16_cleared.restype = i32
+    L.adacode_hist_bf16_cleared.argtypes = L.adacode_hist_bf16.argtypes
     L.adacode_choose_params.restype = i32
     L.adacode_choose_params.argtypes = [vp, i32, vp, vp]
     L.adacode_choose_params_host.restype = i32

@@ -744,11 +744,13 @@ def exponent_hist(x: torch.Tensor, hist_out: Optional[torch.Tensor] = None) -> t
     x = _check_src(x)
     dev = x.device
     _scratch_for(dev)
-    hist = hist_out if hist_out is not None else torch.zeros(256, dtype=torch.int32, device=dev)
+    hist = hist_out if hist_out is not None else torch.empty(256, dtype=torch.int32, device=dev)
     B, H, S, D = x.shape
     sb, sh, ss, _ = x.stride()
+    L = _lib.lib()
     with on_device(dev):
-        rc = _lib.lib().adacode_hist_bf16(x.data_ptr(), sb, sh, ss, B, H, S, D, hist.data_ptr(), stream_ptr(dev))
+        rc = (L.adacode_hist_bf16 if hist_out is not None else L.adacode_hist_bf16_cleared)(
+            x.data_ptr(), sb, sh, ss, B, H, S, D, hist.data_ptr(), stream_ptr(dev))
     _lib.check(rc, 'adacode_hist_bf16')
     return hist
 

@@ -283,6 +283,10 @@ int adacode_unpack_flat_ragged(const uint8_t *sign_mant, const uint8_t *codes, c
                                const int32_t *block_base, int64_t n_elems, int left, int nbits, void *dst_bf16,
                                int32_t *status, void *stream);
 
+/* adacode_hist_bf16 into a histogram that is cleared first (also where there is nothing to count). */
+int adacode_hist_bf16_cleared(const void *src_bf16, int64_t stride_b, int64_t stride_h, int64_t stride_s, int B, int H, int S,
+                              int D, int32_t *hist256, void *stream);
+
 /* Elements per escape-base block of the flat layout for a code length: 128 * {8, 4, 8, 2}[nbits - 1]
  * (compress_bitmap_merge.py:653-657, invalid_block_size); 0 for an invalid nbits. */
 int adacode_flat_block_elems(int nbits);

@@ -1306,7 +1306,7 @@ int adacode_pack_jobs_report(const adacode_pack_job *jobs, int n_jobs, int B, in
     uint32_t *dst;
     const int rc = host_view(report_host_pinned, dst);
     if (rc != ADACODE_OK) return rc;
-    r.dst = (uint2 *)dst;
+    r.dst = (uint64_t *)dst;
     r.src = (const uint32_t *)report_dev;
     r.words = (uint32_t)(report_bytes / 4), r.token = token;
     return pack_jobs_impl(jobs, n_jobs, B, H, seq_tile, D, nbits, workspace, workspace_bytes, status, &r, (cudaStream_t)stream);
@@ -1327,7 +1327,7 @@ int adacode_pack_flat(const void *src_bf16, int64_t n_elems, int right, int nbit
     // report: [offsets of the tiles' escapes: 0 and their total, in the end the tensor's | status]
     int64_t *const offsets = (int64_t *)report_dev;
     int32_t *const status = (int32_t *)(offsets + 2);
-    const Report report = {(const uint32_t *)report_dev, (uint2 *)host, ADACODE_FLAT_REPORT_BYTES / 4, token};
+    const Report report = {(const uint32_t *)report_dev, (uint64_t *)host, ADACODE_FLAT_REPORT_BYTES / 4, token};
     const cudaStream_t st = (cudaStream_t)stream;
     // Tiles of 16384 elements (a unit of the pack kernel, in which a warp has 1024) and the rest in one CTA, or tiles of one
     // block, which leave most of a unit's warps without work but need the last CTA for a short block only: 4096 x 14336

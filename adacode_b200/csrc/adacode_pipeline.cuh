@@ -829,19 +829,20 @@ struct PackJob {
     int blk0, n_blocks, left, pad;
 };
 
-// A small device buffer that goes to page-locked host memory, every word together with a token that says it has arrived:
-// a flag behind the words would have to wait for them to cross the bus.
+// A small device buffer that goes to page-locked host memory, every word (low half of 64 bits) together with a token that says
+// it has arrived: a flag behind the words would have to wait for them to cross the bus.
 struct Report {
     const uint32_t *src;
-    uint2 *dst;
+    uint64_t *dst;
     uint32_t words, token;
 };
 
-// By a whole CTA.
+// By a whole CTA.  Word and token are ONE scalar store: the parts of a vector store may become visible in any order, and the
+// host would take an old word for the one that its token announces.
 __device__ __forceinline__ void send_report(const Report &r) {
     for (uint32_t i = threadIdx.x; i < r.words; i += blockDim.x) {
-        const uint32_t v = __ldcg(r.src + i);
-        asm volatile("st.relaxed.sys.global.v2.b32 [%0], {%1, %2};" ::"l"(r.dst + i), "r"(v), "r"(r.token) : "memory");
+        const uint64_t v = (uint64_t)r.token << 32 | __ldcg(r.src + i);
+        asm volatile("st.relaxed.sys.global.b64 [%0], %1;" ::"l"(r.dst + i), "l"(v) : "memory");
     }
 }
 

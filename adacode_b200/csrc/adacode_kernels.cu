@@ -1092,6 +1092,7 @@ __global__ void __launch_bounds__(kTailThreads) k_flat_tail(const __grid_constan
     if (!fits) atomicOr(a.status, ADACODE_STATUS_ESCAPE_OVERFLOW);
     if (a.hist && tid < 256 && s_hist[tid] != 0) atomicAdd(a.hist + tid, s_hist[tid]);
     if (tid == 0) *a.total = before + all;
+    __threadfence();                                       // (see send_report)
     __syncthreads();
     if (a.report.words != 0) send_report(a.report);
 }
@@ -1380,7 +1381,7 @@ int adacode_wait_report(const void *report_host_pinned, size_t report_bytes, uin
     bool dry = false;                                      // the stream has: what has not come by now never comes
     for (size_t i = 0; i < report_bytes / 4; ++i)
         for (uint32_t poll = 1;; ++poll) {
-            const uint64_t w = __atomic_load_n(words + i, __ATOMIC_RELAXED);
+            const uint64_t w = __atomic_load_n(words + i, __ATOMIC_ACQUIRE);
             if ((uint32_t)(w >> 32) == token) {
                 to[i] = (uint32_t)w;
                 break;

@@ -838,7 +838,9 @@ struct Report {
 };
 
 // By a whole CTA.  Word and token are ONE scalar store: the parts of a vector store may become visible in any order, and the
-// host would take an old word for the one that its token announces.
+// host would take an old word for the one that its token announces.  The caller has seen to it that everything else that its
+// kernel writes (outputs, the scratch's counters) is written for the whole GPU by now: the host goes on when it has the
+// words, not when the kernel ends.  (A fence at the system's scope here costs 1.7 us of 45 for one block, 4 us of 107 for 20 480 tokens.)
 __device__ __forceinline__ void send_report(const Report &r) {
     for (uint32_t i = threadIdx.x; i < r.words; i += blockDim.x) {
         const uint64_t v = (uint64_t)r.token << 32 | __ldcg(r.src + i);
@@ -1515,15 +1517,15 @@ __global__ void __launch_bounds__(kThreads) k_compact_units(const __grid_constan
         __shared__ bool last;
         __syncthreads();
         if (tid == 0) {
+            // (the last one's increment brings the counter back to zero: the scratch is free before the host hears of it.  By it the
+            // outputs of all CTAs are written for the whole GPU, which send_report asks for)
+            const unsigned ctas = gridDim.x * gridDim.y;
             unsigned before;
-            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(pa.done + 1) : "memory");
-            last = before == gridDim.x * gridDim.y - 1;
+            asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;" : "=r"(before) : "l"(pa.done + 1), "r"(ctas - 1) : "memory");
+            last = before == ctas - 1;
         }
         __syncthreads();
-        if (last) {
-            send_report(pa.report);
-            if (tid == 0) pa.done[1] = 0u;
-        }
+        if (last) send_report(pa.report);
     }
 }
 

@@ -135,7 +135,9 @@ int adacode_pack_jobs(const adacode_pack_job *jobs, int n_jobs, int B, int H, in
  * `status` are meant to lie in report_dev.  report_host_pinned has room for 2 * report_bytes bytes, 8-byte aligned; pinned
  * memory as for adacode_copy_to_host.
  * adacode_wait_report polls for the words with this token (one that none of the room's odd words holds before the pack) and
- * returns when all report_bytes are in `out`; ADACODE_ERR_CUDA if the stream fails or runs dry without them.
+ * returns when all report_bytes are in `out`; ADACODE_ERR_CUDA if the stream fails or runs dry without them.  By then the
+ * pack's outputs are written and its workspace is free again, for launches on other streams of the device too, although its last
+ * kernel may not have ended.
  * Replaces: a clearing launch before, and a copying launch and an event behind every pack whose escape totals the host reads.
  */
 int adacode_pack_jobs_report(const adacode_pack_job *jobs, int n_jobs, int B, int H, int seq_tile, int D, int nbits,

@@ -46,6 +46,25 @@ def test_reports_of_different_lengths_and_streams(cuda_device):
     torch.cuda.current_stream(cuda_device).wait_stream(side)
 
 
+@pytest.mark.parametrize('blocks', [1, 40])
+def test_the_host_may_go_on_from_any_stream(cuda_device, blocks):
+    """A pack that has returned has written its outputs and is done with its scratch: other streams need not wait for it."""
+    from adacode_b200 import codec
+    x = synth.kv_tensor((1, 4, 128 * blocks, 128), seed=74).to(cuda_device)
+    want, _ = codec.pack_blocks(x, 129, 3, 128)
+    torch.cuda.synchronize(cuda_device)
+    streams = [torch.cuda.Stream(cuda_device) for _ in range(3)]
+    for turn in range(40):
+        with torch.cuda.stream(streams[turn % 3]):
+            got, _ = codec.pack_blocks(x, 129, 3, 128)
+        with torch.cuda.stream(streams[(turn + 1) % 3]):
+            out = torch.empty_like(x)
+            codec.unpack_chunk(got, out)
+            assert torch.equal(out.view(torch.int16), x.view(torch.int16))
+            for name in ('sign_mant', 'codes', 'escapes', 'tile_base', 'seg_offsets_dev'):
+                assert torch.equal(getattr(got, name), getattr(want, name)), name
+
+
 def test_refusals(cuda_device):
     from adacode_b200 import _lib
     L = _lib.lib()

@@ -11,6 +11,7 @@ path: on a CPU tensor, or without the built library, these functions raise.
 from __future__ import annotations
 
 import ctypes
+import threading
 from dataclasses import dataclass, field
 from typing import Any, Optional, Sequence
 
@@ -27,22 +28,36 @@ _DEFAULT_TILE_NBITS = 3
 # per-device scratch
 # --------------------------------------------------------------------------------------
 
+# Streams of a GPU that keep a pack scratch; beyond it the oldest one's goes back to the allocator.
+_MAX_SCRATCH_STREAMS = 8
+
+
 class _DeviceScratch:
-    """Pack scratch and the device status word of one GPU (grown on demand, reused)."""
+    """Pack scratch (one per stream: packs on two streams are not ordered) and the device status word of one GPU."""
 
     def __init__(self, device: torch.device):
         self.device = device
-        self.workspace = torch.zeros(1 << 20, dtype=torch.uint8, device=device)
+        self.workspaces: dict[int, torch.Tensor] = {}    # by stream, grown on demand, oldest first
+        self.lock = threading.Lock()
         self.status = torch.zeros(2, dtype=torch.int32, device=device)
         self.mailbox: Optional[torch.Tensor] = None      # pinned host bytes that kernels write results into
         self.mail_event = torch.cuda.Event()
 
     def workspace_for(self, n_tiles: int, tile_elems: int) -> torch.Tensor:
+        """The current stream's scratch.  It is allocated on that stream, so one that was replaced or dropped is used again in
+        the stream's order."""
         need = int(_lib.lib().adacode_pack_workspace_bytes(n_tiles, tile_elems))
-        if self.workspace.numel() < need:
+        stream = stream_ptr(self.device)
+        ws = self.workspaces.get(stream)
+        if ws is None or ws.numel() < need:
             # the library wants a zero-filled scratch and leaves it reusable
-            self.workspace = torch.zeros(int(need * 1.25) + 256, dtype=torch.uint8, device=self.device)
-        return self.workspace
+            ws = torch.zeros(max(1 << 20, int(need * 1.25) + 256), dtype=torch.uint8, device=self.device)
+            with self.lock:
+                self.workspaces.pop(stream, None)
+                self.workspaces[stream] = ws
+                while len(self.workspaces) > _MAX_SCRATCH_STREAMS:
+                    del self.workspaces[next(iter(self.workspaces))]
+        return ws
 
 
 _scratch: dict[torch.device, _DeviceScratch] = {}

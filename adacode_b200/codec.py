@@ -40,8 +40,6 @@ class _DeviceScratch:
         self.workspaces: dict[int, torch.Tensor] = {}    # by stream, grown on demand, oldest first
         self.lock = threading.Lock()
         self.status = torch.zeros(2, dtype=torch.int32, device=device)
-        self.mailbox: Optional[torch.Tensor] = None      # pinned host bytes that kernels write results into
-        self.mail_event = torch.cuda.Event()
 
     def workspace_for(self, n_tiles: int, tile_elems: int) -> torch.Tensor:
         """The current stream's scratch.  It is allocated on that stream, so one that was replaced or dropped is used again in
@@ -75,6 +73,17 @@ def _scratch_for(device: torch.device) -> _DeviceScratch:
     return s
 
 
+class _Mailbox(threading.local):
+    """A thread's page-locked host bytes that ``read_back``'s kernel writes into."""
+
+    def __init__(self):
+        self.bytes: Optional[torch.Tensor] = None
+        self.events: dict[torch.device, torch.cuda.Event] = {}
+
+
+_mailbox = _Mailbox()
+
+
 def read_back(t: torch.Tensor):
     """Host copy (numpy array of ``t``'s shape and dtype) of a small device tensor.
 
@@ -88,19 +97,23 @@ def read_back(t: torch.Tensor):
     if nbytes == 0 or nbytes % 4 != 0 or nbytes > (1 << 20):
         return t.cpu().numpy()
     dev = t.device
-    sc = _scratch_for(dev)
-    if sc.mailbox is None or sc.mailbox.numel() < nbytes:
-        sc.mailbox = torch.empty(max(1 << 16, nbytes), dtype=torch.uint8).pin_memory()
+    _scratch_for(dev)
+    box = _mailbox
+    if box.bytes is None or box.bytes.numel() < nbytes:
+        box.bytes = torch.empty(max(1 << 16, nbytes), dtype=torch.uint8).pin_memory()
+    event = box.events.get(dev)
+    if event is None:
+        event = box.events[dev] = torch.cuda.Event()
     stream = torch.cuda.current_stream(dev)
     with on_device(dev):
-        rc = _lib.lib().adacode_copy_to_host(t.data_ptr(), sc.mailbox.data_ptr(), nbytes, int(stream.cuda_stream))
+        rc = _lib.lib().adacode_copy_to_host(t.data_ptr(), box.bytes.data_ptr(), nbytes, int(stream.cuda_stream))
     if rc == _lib.ERR_INVALID_ARG:
         return t.cpu().numpy()           # pinned memory this device cannot address: plain copy
     _lib.check(rc, 'adacode_copy_to_host')
-    sc.mail_event.record(stream)
-    sc.mail_event.synchronize()
+    event.record(stream)
+    event.synchronize()
     import numpy as np
-    out = sc.mailbox[:nbytes].numpy().copy()
+    out = box.bytes[:nbytes].numpy().copy()
     return out.view(np.dtype(str(t.dtype).replace('torch.', ''))).reshape(tuple(t.shape))
 
 

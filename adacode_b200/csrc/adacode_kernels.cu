@@ -16,6 +16,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <mutex>
+
 #include "adacode.h"
 
 namespace {
@@ -924,6 +926,13 @@ bool pack_takes_narrow(int seq_tile, int D) {
     return unit_rows_for<WideGeom::kUnit>(seq_tile, D) * D <= NarrowGeom::kUnit;
 }
 
+// A pack is several launches that hand data on in its scratch: threads that pack on one stream with one scratch
+// must not come between them.  (Taken for the launches alone, some microseconds; two scratches seldom share one.)
+std::mutex &pack_lock(const void *scratch) {
+    static std::mutex locks[64];
+    return locks[((uintptr_t)scratch >> 9) * 0x9E3779B97F4A7C15ull >> 58];
+}
+
 // Pipelined pack of all jobs of `pa` with one pack launch and one compaction launch.
 int launch_pack_pipe(PackPipeArgs &pa, int nbits, cudaStream_t st) {
     const bool narrow = !pa.block_base && pack_takes_narrow(pa.seq_tile, pa.D);
@@ -944,6 +953,7 @@ int launch_pack_pipe(PackPipeArgs &pa, int nbits, cudaStream_t st) {
     // The compaction's CTAs find their tiles' offsets themselves as long as each can add up all counts
     // before its tiles and has a thread for each of them; beyond that the pack kernel's last CTA scans.
     pa.scan_in_pack = pa.n_tiles > kSumTiles || job_tiles > (int64_t)cgrid.x * kThreads;
+    const std::lock_guard<std::mutex> whole(pack_lock(pa.done));
     int rc;
     switch (nbits + (narrow ? 4 : 0)) {
         case 1: rc = launch_pack_pipe_n<1, WideGeom>(pa, hist, st); break;
@@ -1273,6 +1283,7 @@ int pack_jobs_impl(const adacode_pack_job *jobs, int n_jobs, int B, int H, int s
     }
     if (n_tiles > 0) {
         const PackScratch sc = carve_pack_scratch(workspace, max_job_tiles, tile_elems);
+        const std::lock_guard<std::mutex> whole(pack_lock(sc.done));
         for (int j = 0; j < n_jobs; ++j) {
             if (BH * jobs[j].n_blocks == 0) continue;
             const int rc = pack_direct(jobs[j], B, H, seq_tile, D, nbits, sc, status, st);

@@ -60,7 +60,7 @@ const char *adacode_last_cuda_error(void);
  * n_tiles = B*H*n_blocks tiles of tile_elems = seq_tile*D elements.
  * The scratch must be zero-filled once when it is allocated; the library
  * leaves it ready for the next call.  Calls sharing one scratch buffer must
- * be ordered on one stream.
+ * be ordered on one stream; they may come from several threads.
  */
 size_t adacode_pack_workspace_bytes(int64_t n_tiles, int64_t tile_elems);
 

@@ -13,7 +13,7 @@ _PLANES = ('sign_mant', 'codes', 'escapes', 'tile_base', 'seg_offsets_dev')
 
 # pipelined kernels, offsets scanned in the pack kernel (more than 65 536 tiles), direct kernels
 @pytest.mark.parametrize('shape,seq_tile', [((1, 4, 1280, 64), 128), ((16, 64, 520, 16), 8), ((2, 3, 1280, 72), 128)])
-@pytest.mark.parametrize('own_streams', [True])
+@pytest.mark.parametrize('own_streams', [True, False])
 def test_packs_do_not_share_a_scratch(cuda_device, shape, seq_tile, own_streams):
     from adacode_b200 import codec
     xs = [synth.kv_tensor(shape, seed=95 + i, s=0.5 + i).to(cuda_device) for i in range(4)]

@@ -26,15 +26,6 @@ from .rows import on_device, stream_ptr
 _SEQ_TILE = 128
 _MAX_SPLITS = 128
 
-_workspaces: dict = {}
-
-
-def _workspace(device: torch.device, need: int) -> torch.Tensor:
-    ws = _workspaces.get(device)
-    if ws is None or ws.numel() < need:
-        ws = _workspaces[device] = torch.empty(need, dtype=torch.uint8, device=device)
-    return ws
-
 
 def decode_attention(query: torch.Tensor, key_segments: Sequence, value_segments: Sequence,
                      key_tail: Optional[torch.Tensor] = None, value_tail: Optional[torch.Tensor] = None,
@@ -95,7 +86,8 @@ def decode_attention(query: torch.Tensor, key_segments: Sequence, value_segments
             value_table = build_segment_table(value_segments, None, dev)
     L = _lib.lib()
     need = int(L.adacode_decode_attn_workspace_bytes(B, Hq, D, n_splits if n_splits > 0 else _MAX_SPLITS))
-    ws = _workspace(dev, need)
+    # (the call's own: what threads, streams and captured graphs share would have to be ordered between them)
+    ws = torch.empty(need, dtype=torch.uint8, device=dev)
     if out is None:
         out = torch.empty((B, Hq, D), dtype=torch.bfloat16, device=dev)
     elif out.dtype != torch.bfloat16 or tuple(out.shape) != (B, Hq, D) or not out.is_contiguous():

@@ -802,7 +802,10 @@ __device__ __forceinline__ int merge_swizzle(int i, int j) {
     return D == 128 ? (i >> 1) ^ ((j & 1) * 4) : (i >> 2) ^ ((j & 1) * 2);
 }
 
-template <int D, int HG>
+// ROWS: a run of items may go on in the next rows (see AttnArgs); otherwise a CTA has one split of one row, and nothing
+// of the loop over rows, whose counters cost registers: spill loads 60 -> 44 bytes at <128, 1>, 244 -> 172 at <128, 2>;
+// keys and values [1, 8, 20557, 128], 4 heads each, 41.4 -> 40.4 us, [16, 8, 1500, 128], 8 heads, 46.4 -> 45.1 us.
+template <int D, int HG, bool ROWS>
 __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_constant__ AttnArgs a) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     AttnPipeSmem<D> &s = *reinterpret_cast<AttnPipeSmem<D> *>(smem_raw);
@@ -824,7 +827,8 @@ __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_
     __syncthreads();
     // this CTA's items [begin, end), and the units that are to be decoded for them (two per packed item)
     const int begin = run_begin(a, blockIdx.x), end = run_begin(a, blockIdx.x + 1);
-    const int row0 = (uint32_t)begin / a.by_items, item0 = begin - row0 * a.items, row1 = (uint32_t)end / a.by_items;
+    const int row0 = ROWS ? (uint32_t)begin / a.by_items : blockIdx.x / a.by_cut_ctas, item0 = begin - row0 * a.items;
+    const int row1 = ROWS ? (uint32_t)end / a.by_items : row0;
     const int n_units = 2 * ((row1 - row0) * a.n_seg + min(end - row1 * a.items, a.n_seg) - min(item0, a.n_seg));
     // launched as a programmatic dependent of its predecessor in the stream: no global memory is touched above
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -841,7 +845,7 @@ __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_
             const int pair = (n + lane) >> 1;
             if (n + lane < n_units) {
                 int row = row0, item = item0 + pair;
-                if (item >= a.n_seg) {                       // beyond the first row's (n_units > 0: there are packed items)
+                if (ROWS && item >= a.n_seg) {                       // beyond the first row's (n_units > 0: there are packed items)
                     const int more = pair - max(0, a.n_seg - item0);
                     row += 1 + more / a.n_seg;
                     item = more % a.n_seg;
@@ -862,10 +866,11 @@ __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_
         for (int n = 0; n < kAStages - 1; ++n) issue(n);
     }
     int u = 0;                                               // units of this CTA so far
-    for (int x = begin; x < end;) {
+    int x = begin;
+    do {
         // the part [first, last) of one row's items
-        const int row = (uint32_t)x / a.by_items, first = x - row * a.items;
-        const int last = min(a.items, first + (end - x));
+        const int row = ROWS ? (uint32_t)x / a.by_items : row0, first = x - row * a.items;
+        const int last = ROWS ? min(a.items, first + (end - x)) : end - row * a.items;
         x += last - first;
         const int bh = (uint32_t)row / a.by_head_groups;
         const int b = (uint32_t)bh / a.by_heads, hkv = bh - b * a.Hkv;
@@ -937,7 +942,7 @@ __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_
         }
 
         // the combine kernel may be set up from here on (it waits for this launch to complete before it reads)
-        if (x >= end) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        if (!ROWS || x >= end) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         // ---------------- merge the warps ----------------
 #pragma unroll
         for (int h = 0; h < HG; ++h) {
@@ -954,7 +959,7 @@ __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_
         // permuted so that a warp's writes, eight column groups of four heads, spread over the banks.
         float *acc = reinterpret_cast<float *>(&s.stage[(u + kAStages - 1) % kAStages]);
         static_assert(sizeof(AttnStage<D>) >= sizeof(float) * kAWarps * 8 * D, "a stage holds the numerators of the merge");
-        const long long slot = (long long)bh * a.n_splits + ((int)blockIdx.x - cta_of(a, row * a.items));
+        const long long slot = (long long)bh * a.n_splits + ((int)blockIdx.x - (ROWS ? cta_of(a, row * a.items) : row * a.cut_ctas));
 #pragma unroll
         for (int h = 0; h < HG; ++h) {
             float f[2];
@@ -995,12 +1000,12 @@ __global__ void __launch_bounds__(kAThreads, 2) k_decode_attn_pipe(const __grid_
             a.part_ml[(slot * a.G + gz + tid) * 2 + 0] = mx == -INFINITY ? -INFINITY : mx / kLog2e;   // natural-log domain
             a.part_ml[(slot * a.G + gz + tid) * 2 + 1] = l;
         }
-        if (x < end) {
+        if (ROWS && x < end) {
             // (the stage is written again, by a copy, behind the next unit's barrier; the warps' sums by the next row)
             fence_async_smem();
             __syncthreads();
         }
-    }
+    } while (ROWS && x < end);
     // do not leave while a copy into this CTA's shared memory may still be in flight (see k_unpack_pipe)
     if (warp == 0 && launch_timed_out(a.status))
         for (int n = u > kAStages ? u - kAStages : 0; n < u; ++n)
@@ -1068,21 +1073,27 @@ cudaError_t launch_as_dependent(void (*kernel)(KArgs...), dim3 grid, int threads
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-template <int D, int HG>
+template <int D, int HG, bool ROWS>
 int launch_attn_pipe(const AttnArgs &a, dim3 grid, cudaStream_t st) {
     // the kernel's limit of dynamic shared memory is raised once per device
     static std::atomic<bool> done[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return ADACODE_ERR_CUDA;
     if (dev < 0 || dev >= 64 || !done[dev].load(std::memory_order_acquire)) {
-        if (cudaFuncSetAttribute(k_decode_attn_pipe<D, HG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(k_decode_attn_pipe<D, HG, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sizeof(AttnPipeSmem<D>)) != cudaSuccess)
             return ADACODE_ERR_CUDA;
         if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
     }
-    return launch_as_dependent(k_decode_attn_pipe<D, HG>, grid, kAThreads, sizeof(AttnPipeSmem<D>), st, a) == cudaSuccess
+    return launch_as_dependent(k_decode_attn_pipe<D, HG, ROWS>, grid, kAThreads, sizeof(AttnPipeSmem<D>), st, a) == cudaSuccess
                ? ADACODE_OK
                : ADACODE_ERR_CUDA;
+}
+
+template <bool ROWS>
+int launch_attn_heads(const AttnArgs &a, bool two_groups, dim3 grid, cudaStream_t st) {
+    if (a.D == 128) return two_groups ? launch_attn_pipe<128, 2, ROWS>(a, grid, st) : launch_attn_pipe<128, 1, ROWS>(a, grid, st);
+    return two_groups ? launch_attn_pipe<64, 2, ROWS>(a, grid, st) : launch_attn_pipe<64, 1, ROWS>(a, grid, st);
 }
 }  // namespace
 
@@ -1162,8 +1173,7 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
     cudaStream_t st = (cudaStream_t)stream;
     if (!force_simple) {
         const dim3 grid((unsigned)n_ctas);
-        const int rc = D == 128 ? (two_groups ? launch_attn_pipe<128, 2>(a, grid, st) : launch_attn_pipe<128, 1>(a, grid, st))
-                                : (two_groups ? launch_attn_pipe<64, 2>(a, grid, st) : launch_attn_pipe<64, 1>(a, grid, st));
+        const int rc = cut_items > items ? launch_attn_heads<true>(a, two_groups, grid, st) : launch_attn_heads<false>(a, two_groups, grid, st);
         if (rc != ADACODE_OK) return rc;
     } else {
         if (cudaFuncSetAttribute(k_decode_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AttnSmem)) !=

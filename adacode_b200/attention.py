@@ -14,6 +14,7 @@ cache is only promised by the materialising path (``Float11Cache.update``).
 """
 from __future__ import annotations
 
+import functools
 import math
 from typing import Optional, Sequence
 
@@ -25,6 +26,11 @@ from .rows import on_device, stream_ptr
 
 _SEQ_TILE = 128
 _MAX_SPLITS = 128
+
+
+@functools.lru_cache(maxsize=256)
+def _workspace_bytes(B: int, Hq: int, D: int, n_splits: int) -> int:
+    return int(_lib.lib().adacode_decode_attn_workspace_bytes(B, Hq, D, n_splits))
 
 
 def decode_attention(query: torch.Tensor, key_segments: Sequence, value_segments: Sequence,
@@ -84,21 +90,22 @@ def decode_attention(query: torch.Tensor, key_segments: Sequence, value_segments
             key_table = build_segment_table(key_segments, None, dev)
         if value_table is None:
             value_table = build_segment_table(value_segments, None, dev)
-    L = _lib.lib()
-    need = int(L.adacode_decode_attn_workspace_bytes(B, Hq, D, n_splits if n_splits > 0 else _MAX_SPLITS))
-    # (the call's own: what threads, streams and captured graphs share would have to be ordered between them)
-    ws = torch.empty(need, dtype=torch.uint8, device=dev)
+    need = _workspace_bytes(B, Hq, D, n_splits if n_splits > 0 else _MAX_SPLITS)
     if out is None:
         out = torch.empty((B, Hq, D), dtype=torch.bfloat16, device=dev)
     elif out.dtype != torch.bfloat16 or tuple(out.shape) != (B, Hq, D) or not out.is_contiguous():
         raise ValueError('out must be a contiguous bf16 [B, Hq, D] tensor')
     tb, th, ts = (key_tail.stride()[:3] if tail_len else (0, 0, 0))
     with on_device(dev):
-        rc = L.adacode_decode_attn(
+        stream = stream_ptr(dev)
+        # (a captured graph runs on other streams than the one that it is captured on: it has memory of its own)
+        ws = (torch.empty(need, dtype=torch.uint8, device=dev) if torch.cuda.is_current_stream_capturing()
+              else sc.partials.get(stream, need))
+        rc = _lib.lib().adacode_decode_attn(
             q.data_ptr(), q.stride(0), q.stride(1),
             key_table.data_ptr() if n_seg else None, value_table.data_ptr() if n_seg else None, n_seg,
             key_tail.data_ptr() if tail_len else None, value_tail.data_ptr() if tail_len else None, tail_len,
             tb, th, ts, B, Hq, Hkv, _SEQ_TILE, D, float(scale), out.data_ptr(), ws.data_ptr(), ws.numel(),
-            int(n_splits), sc.status.data_ptr(), stream_ptr(dev))
+            int(n_splits), sc.status.data_ptr(), stream)
     _lib.check(rc, 'adacode_decode_attn')
     return out.unsqueeze(2) if squeeze else out

@@ -28,40 +28,53 @@ _DEFAULT_TILE_NBITS = 3
 # per-device scratch
 # --------------------------------------------------------------------------------------
 
-# Streams of a GPU that keep a pack scratch; beyond it the oldest one's goes back to the allocator.
-_MAX_SCRATCH_STREAMS = 8
+# Streams of a GPU that keep buffers; beyond it the oldest one's go back to the allocator.
+_MAX_STREAMS = 8
+
+
+class _StreamBuffers:
+    """Memory that launches hand data on in: one buffer per stream of a GPU (two streams are not ordered), grown on demand."""
+
+    def __init__(self, device: torch.device, make):
+        self.device, self.make = device, make
+        self.by_stream: dict[int, torch.Tensor] = {}      # oldest first
+        self.lock = threading.Lock()
+
+    def get(self, stream: int, need: int) -> torch.Tensor:
+        """At least ``need`` bytes for ``stream``, the current one: they are allocated on it, so a buffer that was replaced
+        or dropped is used again in the stream's order."""
+        buf = self.by_stream.get(stream)
+        if buf is None or buf.numel() < need:
+            buf = self.make(max(1 << 20, need + need // 4 + 256), dtype=torch.uint8, device=self.device)
+            with self.lock:
+                self.by_stream.pop(stream, None)
+                self.by_stream[stream] = buf
+                while len(self.by_stream) > _MAX_STREAMS:
+                    del self.by_stream[next(iter(self.by_stream))]
+        return buf
 
 
 class _DeviceScratch:
-    """Pack scratch (one per stream: packs on two streams are not ordered) and the device status word of one GPU."""
+    """The pack scratch, the memory for the fused attention's partial results and the status word of one GPU."""
 
     def __init__(self, device: torch.device):
         self.device = device
-        self.workspaces: dict[int, torch.Tensor] = {}    # by stream, grown on demand, oldest first
-        self.lock = threading.Lock()
+        self.packs = _StreamBuffers(device, torch.zeros)  # (the library wants a zero-filled scratch and leaves it reusable)
+        self.partials = _StreamBuffers(device, torch.empty)
         self.status = torch.zeros(2, dtype=torch.int32, device=device)
 
     def workspace_for(self, n_tiles: int, tile_elems: int) -> torch.Tensor:
-        """The current stream's scratch.  It is allocated on that stream, so one that was replaced or dropped is used again in
-        the stream's order."""
-        need = int(_lib.lib().adacode_pack_workspace_bytes(n_tiles, tile_elems))
-        stream = stream_ptr(self.device)
-        ws = self.workspaces.get(stream)
-        if ws is None or ws.numel() < need:
-            # the library wants a zero-filled scratch and leaves it reusable
-            ws = torch.zeros(max(1 << 20, int(need * 1.25) + 256), dtype=torch.uint8, device=self.device)
-            with self.lock:
-                self.workspaces.pop(stream, None)
-                self.workspaces[stream] = ws
-                while len(self.workspaces) > _MAX_SCRATCH_STREAMS:
-                    del self.workspaces[next(iter(self.workspaces))]
-        return ws
+        """The current stream's pack scratch."""
+        return self.packs.get(stream_ptr(self.device), int(_lib.lib().adacode_pack_workspace_bytes(n_tiles, tile_elems)))
 
 
 _scratch: dict[torch.device, _DeviceScratch] = {}
 
 
 def _scratch_for(device: torch.device) -> _DeviceScratch:
+    s = _scratch.get(device)
+    if s is not None:
+        return s
     device = torch.device(device)
     if device.type != 'cuda':
         raise _lib.AdacodeError(f'float11 kernels need a CUDA tensor, got device {device} (there is no CPU path)')

@@ -23,6 +23,7 @@
 #include <stdlib.h>
 
 #include <atomic>
+#include <mutex>
 
 namespace {
 
@@ -1171,6 +1172,10 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
     a.part_ml = a.part_o + (size_t)B * Hq * n_splits * D;
     a.status = status;
     cudaStream_t st = (cudaStream_t)stream;
+    // Two launches that hand partial results on in the workspace: threads that share a stream and a workspace must not come
+    // between them.
+    static std::mutex locks[64];
+    const std::lock_guard<std::mutex> both(locks[((uintptr_t)workspace >> 9) * 0x9E3779B97F4A7C15ull >> 58]);
     if (!force_simple) {
         const dim3 grid((unsigned)n_ctas);
         const int rc = cut_items > items ? launch_attn_heads<true>(a, two_groups, grid, st) : launch_attn_heads<false>(a, two_groups, grid, st);

@@ -23,8 +23,8 @@ def test_every_stream_has_a_scratch_of_its_own(monkeypatch):
     grown = at(11, 400)
     assert grown.numel() > first.numel() and at(11) is grown and at(12) is second
     # what streams keep is bounded, and the newest stay
-    kept = [at(s) for s in range(100, 100 + codec._MAX_SCRATCH_STREAMS)]
-    assert len(scratch.workspaces) == codec._MAX_SCRATCH_STREAMS
+    kept = [at(s) for s in range(100, 100 + codec._MAX_STREAMS)]
+    assert len(scratch.packs.by_stream) == codec._MAX_STREAMS
     assert all(at(100 + i) is ws for i, ws in enumerate(kept))
     assert at(12) is not second
 

@@ -525,8 +525,8 @@ def pack_flat(x: torch.Tensor, right: int, nbits: int, block_elems: int, hist: O
     """``(sign_mant, codes, escapes, block_base int32)`` of a contiguous bf16 CUDA tensor in the flat layout, whose
     element count is a multiple of 8; ``hist`` (int32[256] on the device) is added to."""
     n = x.numel()
-    if x.data_ptr() % 16 and n % block_elems:
-        x = x.clone()                            # (a ragged tensor may begin anywhere)
+    if x.data_ptr() % 16:
+        x = x.clone()                            # (a view may begin anywhere, the kernels want 16-byte boundaries)
     dev = x.device
     cap, guessed = _default_escape_capacity(n, nbits), True
     while True:

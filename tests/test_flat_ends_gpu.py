@@ -48,8 +48,8 @@ def test_short_tensors_anywhere(cuda_device):
     x = synth.kv_tensor((1, 1, 12, 8), seed=5).reshape(-1)
     _check(cuda_device, x, 129, 3, out_shift=3)
     from adacode_b200.compress_bitmap_merge import CompressorBitMap
-    room = torch.zeros(2000, dtype=torch.bfloat16, device=cuda_device)
-    for n in (96, 1040):
+    room = torch.zeros(20000, dtype=torch.bfloat16, device=cuda_device)
+    for n in (96, 1024, 1040, 2048, 16384, 16384 + 1032):
         view = room[5: 5 + n]
         view.copy_(synth.kv_tensor((1, 1, n // 8, 8), seed=6).reshape(-1))
         c = CompressorBitMap(129, 3)

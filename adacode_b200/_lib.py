@@ -160,8 +160,11 @@ def native():
     global _native
     if _native is None:
         lib()
+        from .build import built_for
         try:
             from . import _native as module
+            if getattr(module, 'built_for', None) != built_for():
+                raise ImportError(f'it was not made as an {built_for()}')
         except ImportError as e:
             raise AdacodeError(f'the _native module is missing or does not load ({e}): build it with '
                                '`python -m adacode_b200.build`') from e

@@ -1,5 +1,5 @@
 """In-tree build of the sm_100a shared library (``libadacode_sm100.so``) and of the extension module that calls it
-(``_native.so``).
+(``_native``).
 
 ``python -m adacode_b200.build`` compiles ``csrc/*.cu`` with nvcc for ``sm_100a`` only, and ``csrc/host_path.cpp`` with the
 host compiler against the installed torch.  nvcc cross-compiles without a GPU, so this also runs on a CPU-only machine.
@@ -7,7 +7,6 @@ host compiler against the installed torch.  nvcc cross-compiles without a GPU, s
 from __future__ import annotations
 
 import glob
-import importlib.util
 import os
 import subprocess
 import sys
@@ -16,7 +15,6 @@ import sysconfig
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 ROOT_DIR = os.path.dirname(PKG_DIR)
 LIB_PATH = os.path.join(PKG_DIR, 'libadacode_sm100.so')
-NATIVE_PATH = os.path.join(PKG_DIR, '_native.so')
 NVCC_FLAGS = [
     '-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17',
     '-Xcompiler', '-fPIC', '-shared',
@@ -38,22 +36,40 @@ def _run(cmd: list[str]) -> str:
     return proc.stderr
 
 
+def native_path() -> str:
+    """The extension module's file, which no other Python takes for its own."""
+    return os.path.join(PKG_DIR, '_native' + sysconfig.get_config_var('EXT_SUFFIX'))
+
+
+def built_for() -> str:
+    """What a module has to be compiled against to be loaded here: it reads torch's objects through torch's headers."""
+    import torch
+    return f'adacode host path for torch {torch.__version__}'
+
+
+def _compiled_for_this_torch(path: str) -> bool:
+    with open(path, 'rb') as f:
+        return built_for().encode() + b'\0' in f.read()
+
+
 def build_native(force: bool = False) -> str:
-    """Compile the extension module if it is missing or older than its sources; return its path."""
-    source = os.path.join(PKG_DIR, 'csrc', 'host_path.cpp')
+    """Compile the extension module if it is missing, older than its sources or made for another torch; return its path."""
+    import torch
+    source, path = os.path.join(PKG_DIR, 'csrc', 'host_path.cpp'), native_path()
     headers = glob.glob(os.path.join(ROOT_DIR, 'include', '*.h'))
-    if not force and not _stale(NATIVE_PATH, [source, *headers]):
-        return NATIVE_PATH
-    torch_dir = os.path.dirname(importlib.util.find_spec('torch').origin)
+    if not force and not _stale(path, [source, *headers]) and _compiled_for_this_torch(path):
+        return path
+    torch_dir = os.path.dirname(torch.__file__)
     cuda = os.environ.get('CUDA_HOME', '/usr/local/cuda')
     include = [os.path.join(ROOT_DIR, 'include'), os.path.join(torch_dir, 'include'),
                os.path.join(torch_dir, 'include', 'torch', 'csrc', 'api', 'include'), sysconfig.get_paths()['include'],
                os.path.join(cuda, 'include')]
-    _run([os.environ.get('CXX', 'g++'), '-O2', '-std=c++17', '-fPIC', '-shared', '-D_GLIBCXX_USE_CXX11_ABI=1',
-          *(f'-I{p}' for p in include), source, '-o', NATIVE_PATH, f'-L{PKG_DIR}', '-l:' + os.path.basename(LIB_PATH),
+    _run([os.environ.get('CXX', 'g++'), '-O2', '-std=c++17', '-fPIC', '-shared',
+          f'-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}', f'-DADACODE_BUILT_FOR="{built_for()}"',
+          *(f'-I{p}' for p in include), source, '-o', path, f'-L{PKG_DIR}', '-l:' + os.path.basename(LIB_PATH),
           '-L' + os.path.join(torch_dir, 'lib'), '-ltorch_python', '-ltorch', '-ltorch_cpu', '-ltorch_cuda', '-lc10', '-lc10_cuda',
           '-L' + os.path.join(cuda, 'lib64'), '-lcudart', '-Wl,-rpath,$ORIGIN'])
-    return NATIVE_PATH
+    return path
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

@@ -409,4 +409,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nu
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__native(void) {
+    PyObject *m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "built_for", ADACODE_BUILT_FOR) != 0) Py_CLEAR(m);
+    return m;
+}

@@ -357,7 +357,7 @@ def _check_src(x: torch.Tensor) -> torch.Tensor:
 
 
 class _PendingPack:
-    """A pack launch whose escape totals have not been read yet (``pack_blocks_launch``)."""
+    """One tensor of a pack: what was asked for, and the outputs of its launch."""
 
     def __init__(self, **kw):
         self.__dict__.update(kw)
@@ -377,53 +377,16 @@ def _default_escape_capacity(n: int, nbits: int) -> int:
     return min(max(4096, share), max(n, 1))
 
 
-def pack_blocks_launch(x: torch.Tensor, right: int, nbits: int, seq_tile: int = 128, need_hist: bool = False,
-                       hist_out: Optional[torch.Tensor] = None, escape_capacity: Optional[int] = None,
-                       meta_out: Optional[torch.Tensor] = None, launch: bool = True) -> _PendingPack:
-    """Start packing ``x`` (see ``pack_blocks``) and return without reading anything back.
-    ``meta_out``: zeroed int64[n_blocks + 2] device buffer for the segment offsets and the status
-    word (e.g. a slice of a buffer that several launches share, so that one ``read_back`` serves
-    them all); the caller passes its host copy to ``pack_blocks_finish``."""
-    if nbits not in _SUPPORTED_TILE_NBITS:
-        raise ValueError(f'Tiled compressed path supports nbits in {_SUPPORTED_TILE_NBITS}, got {nbits}')
-    x = _check_src(x)
-    B, H, S, D = x.shape
-    _check_blocks(S, seq_tile)
-    n_blocks = S // seq_tile
-    dev = x.device
-    tile_elems = seq_tile * D
-    n = B * H * n_blocks * tile_elems
-    p = _PendingPack(x=x, right=int(right), nbits=int(nbits), seq_tile=seq_tile, B=B, H=H, D=D, n_blocks=n_blocks,
-                     dev=dev, n=n)
-    p.sign_mant = torch.empty((n_blocks, B * H * tile_elems), dtype=torch.uint8, device=dev)
-    p.codes = torch.empty((n_blocks, B * H * tile_elems * nbits // 8), dtype=torch.uint8, device=dev)
-    p.tile_base = torch.empty((n_blocks, B * H), dtype=torch.int32, device=dev)
-    # [segment offsets (n_blocks+1) | status word] in one int64 buffer -> one read
-    p.meta = meta_out if meta_out is not None else torch.zeros(n_blocks + 2, dtype=torch.int64, device=dev)
-    if p.meta.numel() != n_blocks + 2 or p.meta.dtype != torch.int64 or not p.meta.is_contiguous():
-        raise ValueError('meta_out must be a contiguous int64 tensor of n_blocks + 2 entries')
-    p.hist = None
-    if need_hist:
-        p.hist = hist_out if hist_out is not None else torch.zeros(256, dtype=torch.int32, device=dev)
-    p.guessed = escape_capacity is None
-    p.cap = min(int(escape_capacity), max(n, 1)) if escape_capacity is not None else _default_escape_capacity(n, int(nbits))
-    if launch:
-        p.escapes = _pack_launch(p, p.cap, p.hist)
-    return p
-
-
-def _pack_launch(p: _PendingPack, capacity: int, hist_t) -> torch.Tensor:
-    sc = _scratch_for(p.dev)
-    n_tiles = p.B * p.H * p.n_blocks
-    ws = sc.workspace_for(n_tiles, p.seq_tile * p.D)
+def _pack_again(p: _PendingPack, capacity: int) -> torch.Tensor:
+    """Pack ``p`` into its planes once more, with room for ``capacity`` escapes; its histogram is complete."""
+    ws = _scratch_for(p.dev).workspace_for(p.B * p.H * p.n_blocks, p.seq_tile * p.D)
     esc = torch.empty(capacity, dtype=torch.uint8, device=p.dev)
     sb, sh, ss, _ = p.x.stride()
     with on_device(p.dev):
         rc = _lib.lib().adacode_pack_tiles(
             p.x.data_ptr(), sb, sh, ss, p.B, p.H, p.n_blocks, p.seq_tile, p.D, p.right, p.nbits,
             p.sign_mant.data_ptr(), p.codes.data_ptr(), esc.data_ptr(), capacity, p.tile_base.data_ptr(),
-            p.meta.data_ptr(), 0 if hist_t is None else hist_t.data_ptr(), ws.data_ptr(), ws.numel(),
-            p.meta.data_ptr() + 8 * (p.n_blocks + 1), stream_ptr(p.dev))
+            p.meta.data_ptr(), 0, ws.data_ptr(), ws.numel(), p.meta.data_ptr() + 8 * (p.n_blocks + 1), stream_ptr(p.dev))
     _lib.check(rc, 'adacode_pack_tiles')
     return esc
 
@@ -459,12 +422,6 @@ def _pack_now(xs: Sequence[torch.Tensor], rights: Sequence[int], nbits: Sequence
     return out, host_hist
 
 
-def pack_blocks_finish(p: _PendingPack, host_meta):
-    """Finish a launch given the host copy of its ``meta`` (int64[n_blocks + 2]): re-run with the
-    exact capacity if the escape buffer was too small, trim it, build the ``PackedChunk``."""
-    return _finish_pack(p, host_meta[: p.n_blocks + 1].tolist(), int(host_meta[p.n_blocks + 1]) & 0xFFFFFFFF)
-
-
 def _trim_escapes(escapes: torch.Tensor, total: int, large_guess: bool, n: int) -> torch.Tensor:
     # (a large first guess is not kept, which packs of single blocks would for the cache's life: it is cut to size
     # where an eighth more than the escapes and a 32nd of the elements are unused)
@@ -481,7 +438,7 @@ def _finish_pack(p: _PendingPack, offsets: list, status: int):
     status_other = status & ~_lib.STATUS_ESCAPE_OVERFLOW
     if total > p.cap:
         p.meta = torch.zeros(n_blocks + 2, dtype=torch.int64, device=p.dev)
-        escapes = _pack_launch(p, total, None)   # histogram already complete from the first pass
+        escapes = _pack_again(p, total)
         host = read_back(p.meta)
         if int(host[n_blocks + 1]) & 0xFFFFFFFF:
             raise _lib.AdacodeError('adacode_pack_tiles: escape overflow after re-run with exact capacity')

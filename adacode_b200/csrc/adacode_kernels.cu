@@ -1460,7 +1460,7 @@ int adacode_unpack_tiles(const uint8_t *sign_mant, const uint8_t *codes, const u
         UnpackPipeArgs pa;
         pa.sign_mant = sign_mant, pa.codes = codes, pa.escapes = escapes, pa.escapes_len = escapes_len;
         pa.tile_base = tile_base, pa.seg_off = seg_escape_offsets, pa.left = left, pa.nbits = nbits;
-        pa.tb_stride = 1, pa.tb_before = 0;
+        pa.tb_stride = 1;
         pa.seg = nullptr;
         pa.H = H, pa.BH = B * H, pa.seq_tile = seq_tile, pa.D = D, pa.tile_elems = seq_tile * D;
         pa.n_tiles = n_tiles, pa.dst = (uint16_t *)dst_bf16;
@@ -1498,7 +1498,7 @@ int adacode_unpack_segments(const adacode_segment *segments_dev, int n_segments,
         UnpackPipeArgs pa;
         pa.sign_mant = nullptr, pa.codes = nullptr, pa.escapes = nullptr, pa.escapes_len = 0;
         pa.tile_base = nullptr, pa.seg_off = nullptr, pa.left = 0, pa.nbits = 0;
-        pa.tb_stride = 1, pa.tb_before = 0;
+        pa.tb_stride = 1;
         pa.seg = segments_dev;
         pa.H = H, pa.BH = B * H, pa.seq_tile = seq_tile, pa.D = D, pa.tile_elems = seq_tile * D;
         pa.n_tiles = n_tiles, pa.dst = (uint16_t *)dst_bf16;

@@ -1180,7 +1180,7 @@ def config3_block(args, dev) -> dict:
     import kv_synth
     import numpy as np
     import torch
-    from adacode_b200 import MLAFloat11Cache, codec
+    from adacode_b200 import MLAFloat11Cache, _lib, codec
     from oracle import float11_oracle as O
     LAYERS3, B, S, DL, DR = 27, 8, 16384, 512, 64
     pos = torch.arange(S, dtype=torch.float32).view(S, 1)
@@ -1195,6 +1195,7 @@ def config3_block(args, dev) -> dict:
         cl = kv_synth.kv_tensor(39000 + 2 * l, (1, 1, 1024, DL), sl, ol, 'cpu')
         cr = kv_synth.kv_tensor(39001 + 2 * l, (1, 1, 1024, DR), sr, orr, 'cpu', modulation=modulation)
         wins.append((calibrate_from(O.exponent_hist(cl)), calibrate_from(O.exponent_hist(cr))))
+    L = _lib.lib()
     peak, _ = measured_hbm_peak()
     res = {'workload': 'config3: MLA latent cache, 27 layers, latent [8,1,16384,512] + rope key [8,1,16384,64]'}
 
@@ -1206,10 +1207,20 @@ def config3_block(args, dev) -> dict:
         codes = sum(x.numel() * c.nbits // 8 for x, c in zip(tensors, chunks))
         outb = torch.empty_like(tensors[0])
 
+        # (outputs that every tensor's launch writes in turn)
+        D, n_blocks, cap = tensors[0].shape[-1], S // BLOCK, max(c.n_escapes for c in chunks) + 4096
+        plane = torch.empty(tensors[0].numel(), dtype=torch.uint8, device=dev)
+        code, escape, base = torch.empty_like(plane), torch.empty(cap, dtype=torch.uint8, device=dev), torch.empty_like(chunks[0].tile_base)
+        meta, hist = torch.zeros(n_blocks + 2, dtype=torch.int64, device=dev), torch.zeros(256, dtype=torch.int32, device=dev)
+        ws = torch.zeros(L.adacode_pack_workspace_bytes(B * n_blocks, BLOCK * D), dtype=torch.uint8, device=dev)
+        stream = torch.cuda.current_stream(dev).cuda_stream
+
         def pack_all():
             for l, x in enumerate(tensors):
-                codec.pack_blocks_launch(x, wins[l][widx][0], wins[l][widx][1], BLOCK, need_hist=True,
-                                         escape_capacity=chunks[l].n_escapes + 4096)
+                right, nbits = wins[l][widx]
+                _lib.check(L.adacode_pack_tiles(x.data_ptr(), *x.stride()[:3], B, 1, n_blocks, BLOCK, D, right, nbits, plane.data_ptr(),
+                                                code.data_ptr(), escape.data_ptr(), cap, base.data_ptr(), meta.data_ptr(), hist.data_ptr(),
+                                                ws.data_ptr(), ws.numel(), meta.data_ptr() + 8 * (n_blocks + 1), stream), 'adacode_pack_tiles')
 
         def unpack_all():
             for c in chunks:
@@ -1238,7 +1249,7 @@ def config3_block(args, dev) -> dict:
                     and np.array_equal(c.escapes.cpu().numpy(), ref.invalid_exp)):
                 bad.append(l)
         res[name]['byte_parity_vs_oracle_layers_0_13_26'] = 'ok' if not bad else f'MISMATCH {bad}'
-        del chunks, outb
+        del chunks, outb, plane, code, escape, ws
         torch.cuda.empty_cache()
 
     # through the cache API, both modes

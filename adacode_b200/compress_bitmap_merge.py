@@ -4,10 +4,10 @@
 The flat layout packs ANY bf16 tensor (KV blocks of the 'legacy' cache layout, model weights) as
 one sign/mantissa byte per element, n-bit exponent codes, one compact list of escaped exponents
 in flat order and ``block_base``: the inclusive running escape count per ``invalid_block_size``
-(= 128 x {8, 4, 8, 2}[nbits - 1]) elements.  These are exactly the planes ``adacode_pack_tiles``
-writes for tiles of one block each, so ``compress`` is one such launch; ``uncompress`` goes
-through ``adacode_unpack_flat_ragged``, which decodes 16384-element tiles and takes every
-(16384 / block)-th base.  There is no CPU path.
+(= 128 x {8, 4, 8, 2}[nbits - 1]) elements.  ``compress`` is one ``adacode_pack_flat`` (for every 2**30
+elements): tiles of one block each or, from 4 Mi elements on, of 16384 elements, and the end behind them
+in one more launch; ``uncompress`` is one ``adacode_unpack_flat_ragged``, which decodes 16384-element
+tiles, taking every (16384 / block)-th base, and the blocks behind them.  There is no CPU path.
 """
 from __future__ import annotations
 

@@ -1120,7 +1120,7 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
         const char *v = getenv("ADACODE_ATTN_SIMPLE");
         return v && v[0] == '1';
     }();
-    // CTAs along z: up to eight query heads share a CTA, or up to sixteen: what costs is the decode of the
+    // Rows of work per KV head: up to eight query heads share a CTA, or up to sixteen: what costs is the decode of the
     // cache, which they share.  The plain kernel takes eight.
     const bool two_groups = G > 8 && !force_simple;
     const int heads_per_cta = two_groups ? 16 : kMaxGroup;

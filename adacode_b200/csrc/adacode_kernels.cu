@@ -596,7 +596,8 @@ __global__ void __launch_bounds__(kThreads, kHistCtas) k_hist(const __grid_const
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     s_hist[tid] = 0;
     __syncthreads();
-    // (a programmatic dependent of its predecessor: no global memory is touched above)
+    // (a programmatic dependent of its predecessor: no global memory is touched above.  That gains nothing where the
+    // histogram is cleared first: a memset has no end that a kernel could overlap)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const Index run_vec = (Index)a.run_vec, n_vec = (Index)(a.runs * a.run_vec);
     const Index per_run = (run_vec + 32 * kHistVec - 1) / (32 * kHistVec);

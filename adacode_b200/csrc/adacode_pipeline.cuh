@@ -413,9 +413,9 @@ __device__ __noinline__ uint2 gather_escapes(uint32_t z, int r, const uint8_t *e
 // Keys and values of [16, 8, 8192, 128] in one launch (537 M elements), with the lookups, the escape loop and the
 // bulk store that were here before and now: n = 3, 5 % escapes 188.6 -> 177.7 us (5.2 TB/s, 81 % of what a plain
 // copy reaches), n = 2, 34 % escapes 340 -> 177 us, n = 4, 0.1 % escapes 169.7 -> 170.8 us; [1, 8, 20480, 128]
-// 38.8 -> 35.0 us; 4 % less each since computed permutes go without the intrinsic's mask, and 4-5 % less since fewer
-// registers live across the barrier (the escape masks are found again behind it from the codes' nibbles, and a chunk's row
-// and column share a register): n = 3 161.9 -> 154.5 us, n = 2 160.0 -> 154.7 us, n = 4 161.5 -> 160.9 us, the flat
+// 38.8 -> 35.0 us; 4 % less each since computed permutes go without the intrinsic's mask, and 4-5 % less since the
+// escape masks are found again behind the barrier from the codes' nibbles, and a chunk's row and column share a
+// register (spills 72 / 104 -> 68 / 96 bytes of stores / loads, which is not where the time went; what it is has not been measured): n = 3 161.9 -> 154.5 us, n = 2 160.0 -> 154.7 us, n = 4 161.5 -> 160.9 us, the flat
 // form of 4096 x 14336 40.2 -> 38.2 us.  What is left over a plain copy (143 us) is waiting at the barrier and for loads, and
 // the last round of a launch.  Tried and slower: no producer warp (one warp in turn refills; the others wait for it at the next
 // barrier) 201 us; one tile per warp without shared memory or barriers 217-219 us; the finished unit through
@@ -463,7 +463,7 @@ __device__ __forceinline__ void unpack_unit(const UnpackStageT<G> &st, const Uni
 #pragma unroll
     for (int k = 0; k < kPCPT; ++k) {
         const int r0 = before + incl[k] - zc[k];               // rank inside the tile of the chunk's first escape
-        // (the masks from before the barrier would be kept in registers, and others spilled for them)
+        // (hidden from the compiler, which would keep the masks from before the barrier)
         asm volatile("" : "+r"(nib[k][0]), "+r"(nib[k][1]));
         const uint32_t z0 = escape_mask<N>(nib[k][0]), z1 = escape_mask<N>(nib[k][1]);
         const int r1 = r0 + escapes_of(z0);

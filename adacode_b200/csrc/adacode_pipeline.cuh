@@ -410,7 +410,7 @@ __device__ __noinline__ uint2 gather_escapes(uint32_t z, int r, const uint8_t *e
 // and the bf16 words put together in registers (see spread8), and
 // whole sectors are stored straight from there.  The only CTA-wide barrier is the one between the
 // escape counts of the warps and their sum.
-// Keys and values of [16, 8, 8192, 128] in one launch (537 M elements), with the lookups, the escape loop and the
+// Keys and values of [16, 8, 8192, 128] in one launch (268 M elements), with the lookups, the escape loop and the
 // bulk store that were here before and now: n = 3, 5 % escapes 188.6 -> 177.7 us (5.2 TB/s, 81 % of what a plain
 // copy reaches), n = 2, 34 % escapes 340 -> 177 us, n = 4, 0.1 % escapes 169.7 -> 170.8 us; [1, 8, 20480, 128]
 // 38.8 -> 35.0 us; 4 % less each since computed permutes go without the intrinsic's mask, and 4-5 % less since the

@@ -1144,8 +1144,9 @@ int adacode_decode_attn(const void *q_bf16, int64_t q_stride_b, int64_t q_stride
     if ((long long)items * n_splits >= (1ll << 31)) n_splits = 1;
     // Whole splits of every row, or one cut through all rows where that makes the longest run of items shorter: it is worth
     // the time of about one item to end a row and to begin the next.  256 rows of 33 items on 296 CTAs (keys and values
-    // [32, 8, 4146, 128], 4 heads each): 33 items per CTA and 210 us, or 29 and 187 us; 20 rows of 71 items ([5, 4, 9000, 128], 7 heads each): 6 items and
-    // 54.8 us, or 5 and 52.6 us; 128 rows of 3 items ([64, 2, 300, 128]): 2 either way, 18.4 us whole, 21.1 us cut.
+    // [32, 8, 4146, 128], 4 heads each): 33 items per CTA and 206 us, or 29 and 192 us; 20 rows of 71 items ([5, 4, 9000, 128],
+    // 7 heads each): 6 items and 54.3 us, or 5 and a row's end, which counts as 6 and stays whole (cut 52.6 us);
+    // 128 rows of 3 items ([64, 2, 300, 128]): 2 either way, 18.4 us whole, 21.1 us cut.
     long long n_ctas = rows * n_splits, cut_items = items, cut_ctas = n_splits;
     if (!given && !force_simple) {
         const long long even = even_ctas(slots, rows, items);
